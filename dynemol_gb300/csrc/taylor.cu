@@ -7,20 +7,48 @@
 // (ElHl_Chebyshev.f:174-187, :267) for fixed nuclei and records populations
 // (pop_Slater, data_output.f:242-262) after every step.
 //
-// Execution model: one cooperative launch, one CTA per SM.  Each CTA owns a
-// contiguous block of rows; one "round" = one expansion order for every
+// Execution model: one cooperative launch, at most one CTA per SM.  Each CTA
+// owns a contiguous block of rows; one "round" = one expansion order for every
 // active particle:
-//   phase A  each CTA computes its rows of H'^T.bra and H'.ket (H' read from
-//            L2/HBM), the epilogue forms the scaled term, the partial sum and
-//            per-CTA partials (max |delta|, <bra|ket>, populations);
-//   barrier  bounded grid barrier (gives up after kBarrierNs and reports
-//            ELHL_ERR_TIMEOUT instead of hanging);
-//   phase B  every CTA reduces the per-CTA partials in the same fixed order and
-//            advances an identical copy of the per-particle state machine, so
-//            all CTAs take the same branch with no host round trip.
+//   products   the CTA's rows of H'^T.bra and H'.ket;
+//   epilogue   one warp per eight rows forms the scaled term, the partial sum
+//              and, where the round decides something, the CTA's record
+//              (max |delta|^2 of bra and ket, <bra|ket>);
+//   barrier    bounded grid barrier (gives up after kBarrierNs and reports
+//              ELHL_ERR_TIMEOUT instead of hanging);
+//   advance    one warp per particle sums the records in a fixed order and
+//              advances an identical copy of the particle's state machine in
+//              every CTA, with no host round trip, while the other warps
+//              already form the next round's products on the vector that
+//              follows unless this round ended an expansion (then they are
+//              formed again).
 // Vectors live in kSlots slots per particle; "Psi = new" and the term/partial-
 // sum rotation are slot renames, never copies.
+//
+// What bounds a round is GB300's FP64 unit: a warp instruction takes its SM
+// sub-partition 64 cycles whatever the active lanes, and a dependent one waits
+// as long, so a round costs what its FP64 warp instructions and their longest
+// chain cost.  Hence
+//   - kResident (N up to about 1250): H' rows and columns of the CTA stay in
+//     shared memory for the whole launch, and a lane owns one of the four sums
+//     (re, im of ket and bra) of every row over every 64th column, so that a
+//     row's sums meet over eight lanes (one add per row) instead of 32 lanes
+//     and 31 adds per four rows;
+//   - no hypot in the round (|delta|^2 against tol^2, as integers for the
+//     maximum), |<bra|ket>| only where the decision needs it, the expansion's
+//     coefficient ratios kept with the coefficients (computed by the lanes of
+//     one warp in parallel), and no record exchange in rounds that decide
+//     nothing;
+//   - at least kMinRows rows per CTA: with fewer rows the barrier's arrivals
+//     cost more than the products saved;
+//   - grid_arrive / grid_poll (grid_sync.cuh) instead of grid_barrier.
+// Measured, one particle at N = 465 (the 150-atom drop-in call, 3254 rounds): 23 us
+// per round before (one thread per column, 32 accumulators each), 6.4 us now:
+// products 5,900 cycles (5,400 is the FP64 unit's time for the 72 warp instructions
+// of each sub-partition), barrier 2,750, epilogue 1,950, vectors 850.  N = 62: 4 us.
 #include <cooperative_groups.h>
+
+#include <algorithm>
 
 #include "elhl_internal.cuh"
 #include "grid_sync.cuh"
@@ -30,9 +58,13 @@ namespace {
 
 constexpr int RC = 4;            // rows per register chunk
 constexpr int PMAX = 2;          // particles per launch
-constexpr int PW = 16;           // partial record width (doubles)
+constexpr int PW = 16;           // record width (doubles)
+constexpr int kWarps = kTaylorBlock / 32;
+constexpr int kMinRows = 2;      // rows per CTA below which CTAs are left out of the launch
+constexpr size_t kResidentSmem = 220 * 1024;
 
 enum Phase { PH_NORM = 0, PH_CONV = 1, PH_MAIN = 2, PH_DONE = 3 };
+enum { NEED_COEF = 1, NEED_KMAX = 2 };  // what a state change asks of the particle's warp
 
 struct Ctrl {
     int phase, first, k, kmax;
@@ -40,23 +72,8 @@ struct Ctrl {
     int conv_calls, conv_step, substeps, status;
     long long orders;
     double tau, t, norm_ref, save_tau;
-    double cre[kOrder], cim[kOrder];
+    double g[kOrder];  // |c_k / c_{k-1}|, 0-based k: c_k / c_{k-1} = -i g[k]
 };
-
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
-// coefficient(tau): c_1 = 1, c_k = -i c_{k-1} tau/(k-1) (Taylor.f:224-239), 0-based storage
-__device__ void set_coefficients(Ctrl &c) {
-    c.cre[0] = 1.0;
-    c.cim[0] = 0.0;
-    for (int k = 1; k < kOrder; ++k) {
-        const double f = c.tau / k;
-        c.cre[k] = c.cim[k - 1] * f;
-        c.cim[k] = -c.cre[k - 1] * f;
-    }
-}
 
 __device__ void pick_out_slots(Ctrl &c) {
     int found = 0;
@@ -67,26 +84,43 @@ __device__ void pick_out_slots(Ctrl &c) {
     }
 }
 
-__device__ void start_conv(Ctrl &c, int max_calls) {
+// coefficient(tau): c_1 = 1, c_k = -i c_{k-1} tau/(k-1) (Taylor.f:224-239): |c_k| by
+// that recursion and the ratios g, lane k holding order k (0-based); with kmax,
+// the first k >= 2 (1-based) with |c_k| < 1e-16, at most kOrder (Taylor.f:165-171).
+__device__ void set_coefficients(Ctrl &c, int need, int lane) {
+    const double tau = c.tau;
+    const double f = lane >= 1 && lane < kOrder ? tau / (double)lane : 0.0;
+    double m = 1.0, mine = 1.0, before = 1.0;
+    for (int k = 1; k < kOrder; ++k) {
+        const double prev = m;
+        m = m * __shfl_sync(0xffffffffu, f, k);
+        if (k == lane) {
+            mine = m;
+            before = prev;
+        }
+    }
+    if (lane >= 1 && lane < kOrder) c.g[lane] = (mine * before) / (before * before);
+    if (need & NEED_KMAX) {
+        const unsigned small = __ballot_sync(0xffffffffu, lane >= 1 && lane < kOrder && fabs(mine) < 1.0e-16);
+        if (lane == 0) c.kmax = small ? __ffs(small) : kOrder;
+    }
+    __syncwarp();
+}
+
+__device__ int start_conv(Ctrl &c, int max_calls) {
     if (c.conv_step >= max_calls) {
         c.status = ELHL_ERR_NO_CONVERGENCE;
         c.phase = PH_DONE;
-        return;
+        return 0;
     }
     c.conv_calls++;
     c.conv_step++;
-    set_coefficients(c);
-    c.kmax = kOrder;  // 1-based: first k >= 2 with |c_k| < 1e-16 (Taylor.f:165-171)
-    for (int k = 2; k <= kOrder; ++k)
-        if (hypot(c.cre[k - 1], c.cim[k - 1]) < 1.0e-16) {
-            c.kmax = k;
-            break;
-        }
     c.src = c.psi;
     c.old = c.psi;
     c.k = 2;
     c.phase = PH_CONV;
     pick_out_slots(c);
+    return NEED_COEF | NEED_KMAX;
 }
 
 __device__ void start_main(Ctrl &c) {
@@ -98,7 +132,8 @@ __device__ void start_main(Ctrl &c) {
 }
 
 // After an accepted convergence sub-step (Taylor.f:71-78 first time, :116-121 later).
-__device__ void after_accept(Ctrl &c, double t_init, double t_max) {
+__device__ int after_accept(Ctrl &c, double t_init, double t_max) {
+    int need = 0;
     c.substeps++;
     if (c.first) {
         c.save_tau = c.tau;
@@ -109,25 +144,111 @@ __device__ void after_accept(Ctrl &c, double t_init, double t_max) {
     }
     if (t_max - c.t < c.tau * kHbar) {
         c.tau = (t_max - c.t) / kHbar;
-        set_coefficients(c);
+        need = NEED_COEF;
     }
     if (c.t < t_max) start_main(c); else c.phase = PH_DONE;
+    return need;
 }
 
+// the next order of the running expansion
+__device__ void next_order(Ctrl &c) {
+    c.old = c.out_acc;
+    c.src = c.out_term;
+    c.k++;
+    pick_out_slots(c);
+}
+
+// does this round end in a decision (the records are read)?
+__device__ __forceinline__ bool decides(const Ctrl &c) {
+    return c.phase == PH_NORM || c.phase == PH_CONV || (c.phase == PH_MAIN && c.k >= c.kmax);
+}
+
+// State change after a round, lane 0 of the particle's warp; tot = max |delta|^2 of
+// bra and ket, <bra|ket>.  Returns NEED_* flags for the warp.
+__device__ int advance(Ctrl &c, const double *tot, double tol2, double norm_tol, int max_calls, double t_init,
+                       double t_max) {
+    if (c.phase == PH_NORM) {
+        c.norm_ref = hypot(tot[2], tot[3]);  // Taylor.f:62
+        c.first = 1;
+        c.conv_step = 0;
+        return start_conv(c, max_calls);
+    }
+    if (c.phase == PH_CONV) {
+        c.orders++;
+        if (!(tot[0] > tol2) && !(tot[1] > tol2) && fabs(hypot(tot[2], tot[3]) - c.norm_ref) < norm_tol) {
+            c.psi = c.out_acc;
+            return after_accept(c, t_init, t_max);
+        }
+        if (c.k + 1 > c.kmax) {
+            c.tau = c.tau * (c.first ? 0.9 : 0.975);  // Taylor.f:69, :110
+            return start_conv(c, max_calls);
+        }
+        next_order(c);
+        return 0;
+    }
+    if (c.phase == PH_MAIN) {
+        c.orders++;
+        if (c.k < c.kmax) {
+            next_order(c);
+            return 0;
+        }
+        if (fabs(hypot(tot[2], tot[3]) - c.norm_ref) < norm_tol) {  // Taylor.f:103-106
+            int need = 0;
+            c.psi = c.out_acc;
+            c.substeps++;
+            c.t = c.t + (c.tau * kHbar);
+            if (t_max - c.t < c.tau * kHbar) {
+                c.tau = (t_max - c.t) / kHbar;
+                need = NEED_COEF;
+            }
+            if (c.t < t_max) start_main(c); else c.phase = PH_DONE;
+            return need;
+        }
+        c.tau = c.tau * 0.975;  // Taylor.f:107-114
+        return start_conv(c, max_calls);
+    }
+    return 0;
+}
+
+// maximum of two non-negative doubles (NaN counts as the largest), on their bits
+__device__ __forceinline__ double max_bits(double a, double b) {
+    const unsigned long long x = (unsigned long long)__double_as_longlong(a),
+                             y = (unsigned long long)__double_as_longlong(b);
+    return x > y ? a : b;
+}
+
+// columns padded to whole eight-column lane groups
+__host__ __device__ constexpr int pad8(int n) { return (n + 7) & ~7; }
+
+// dynamic shared memory: resident [P][pad8 N][4] vectors, [rows][pad8 N][2] matrix
+// elements (row i, column i) and the warps' sums [kWarps][P][rows][4]; otherwise
+// the row sums [P][rows][4]
+size_t taylor_smem(int N, int rows, int P, bool resident) {
+    const size_t y = (size_t)P * rows * 4 * sizeof(double);
+    if (!resident) return y;
+    return (size_t)pad8(N) * (4 * P + 2 * rows) * sizeof(double) + kWarps * y;
+}
+
+template <int P, bool kResident>
 __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L) {
-    __shared__ Ctrl ctrl[PMAX];
-    __shared__ double red[kTaylorBlock / 32][PMAX * RC * 4];
-    __shared__ double part[PMAX][RC][4];   // per (particle, chunk row) running partials
-    __shared__ double cta_rec[PMAX][PW];
-    __shared__ int s_step, s_it;
+    extern __shared__ __align__(16) double dyn[];
+    __shared__ Ctrl ctrl[P];
+    __shared__ double red[kWarps][16 * P];       // non-resident: a chunk's warp sums
+    __shared__ double unit_rec[kWarps][4];       // records of the epilogue's units
+    __shared__ int s_step, s_it, s_ok;
     __shared__ double s_tinit, s_tmax;
 
     const int G = gridDim.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int N = L.N, ld = L.ld, ldv = L.ldv, P = L.nparticles;
-    const int rows = (N + G - 1) / G;
-    const int r0 = min(N, blockIdx.x * rows), r1 = min(N, r0 + rows);
+    const int N = L.N, ld = L.ld, ldv = L.ldv;
+    const int rows = (N + G - 1) / G;            // rows of a CTA (the last ones may have fewer)
+    const int r0 = min(N, blockIdx.x * rows), r1 = min(N, r0 + rows), nrow = r1 - r0;
+    const int np = pad8(N);
     const int nf = L.nfrag < kMaxFrag ? L.nfrag : kMaxFrag;
+    const double tol2 = L.tol * L.tol;
+    double *sv = dyn;                                    // resident: [P][np][4] ket re, im, bra re, im
+    double *sh = dyn + (size_t)P * np * 4;               // resident: [rows][np][2] H'(i, j), H'(j, i)
+    double *sy = kResident ? sh + (size_t)rows * np * 2 : dyn;  // [kWarps][P][rows][4] or [P][rows][4]
 
     auto vec = [&](int p, int slot, int which) -> double2 * {
         return L.slots + ((size_t)(p * kSlots + slot) * 2 + which) * ldv;
@@ -143,74 +264,99 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
             c.phase = PH_NORM;
             c.first = 1;
             c.psi = 0; c.src = 0; c.old = 0; c.out_term = 1; c.out_acc = 2;
+            c.k = 2; c.kmax = kOrder;
             c.conv_calls = 0; c.conv_step = 0; c.substeps = 0; c.status = ELHL_OK; c.orders = 0;
             c.tau = L.part[p].tau_in;
             c.t = L.t_init;
             c.save_tau = 0.0;
         }
     }
+    if constexpr (kResident) {
+        for (int q = tid; q < rows * np; q += kTaylorBlock) {
+            const int r = q / np, j = q % np;
+            const bool in = r < nrow && j < N;
+            sh[(size_t)q * 2 + 1] = in ? L.H[(size_t)(r0 + r) * ld + j] : 0.0;
+        }
+        for (int q = tid; q < rows * np; q += kTaylorBlock) {  // lanes along the rows of one column
+            const int r = q % rows, j = q / rows;
+            const bool in = r < nrow && j < N;
+            sh[((size_t)r * np + j) * 2] = in ? L.H[(size_t)j * ld + r0 + r] : 0.0;
+        }
+        for (int q = tid; q < P * np * 4; q += kTaylorBlock) sv[q] = 0.0;  // padding columns stay zero
+    }
     __syncthreads();
 
-    int parity = 0;
-    for (;;) {
-        // ------------------------------------------------ phase A
-        bool any_gemv = false;
-        for (int p = 0; p < P; ++p) any_gemv |= (ctrl[p].phase == PH_CONV || ctrl[p].phase == PH_MAIN);
-
-        // norm / population partials on own rows (particles in PH_NORM)
-        if (tid < PMAX * PW) (&cta_rec[0][0])[tid] = 0.0;
-        __syncthreads();
-        if (tid < P && ctrl[tid].phase == PH_NORM) {
-            const int p = tid;
-            const double2 *b = vec(p, ctrl[p].psi, 0), *k = vec(p, ctrl[p].psi, 1);
-            double dre = 0.0, dim = 0.0, pops[kMaxFrag + 1];
-            for (int f = 0; f <= kMaxFrag; ++f) pops[f] = 0.0;
-            for (int i = r0; i < r1; ++i) {
-                const double2 bi = __ldcg(b + i), ki = __ldcg(k + i);
-                dre += bi.x * ki.x + bi.y * ki.y;  // conj(bra) ket
-                dim += bi.x * ki.y - bi.y * ki.x;
-                const double v = ki.x * bi.x + ki.y * bi.y;  // Re conj(ket) bra
-                if (L.ao_frag) {
-                    const int f = L.ao_frag[i];
-                    if (f >= 0 && f < nf) pops[f] += v;
-                }
-                pops[kMaxFrag] += v;
-            }
-            cta_rec[p][2] = dre;
-            cta_rec[p][3] = dim;
-            for (int f = 0; f <= kMaxFrag; ++f) cta_rec[p][4 + f] = pops[f];
+    // resident: the vectors of slot `slot` of particle p into shared memory.  Written by
+    // other CTAs: L2 loads (L1 is not coherent across SMs).
+    auto stage = [&](int p, int slot) {
+        const double2 *k = vec(p, slot, 1), *b = vec(p, slot, 0);
+        double2 *dst = reinterpret_cast<double2 *>(sv + (size_t)p * np * 4);
+#pragma unroll 8
+        for (int q = tid; q < 2 * N; q += kTaylorBlock) {
+            const int j = q >> 1;
+            dst[q] = __ldcg(((q & 1) ? b : k) + j);
         }
-
-        if (any_gemv) {
-            if (tid < PMAX * RC * 4) (&part[0][0][0])[tid] = 0.0;
-            __syncthreads();
-            double2 rr[PMAX];
-            bool act[PMAX];
-            for (int p = 0; p < PMAX; ++p) {
-                act[p] = p < P && (ctrl[p].phase == PH_CONV || ctrl[p].phase == PH_MAIN);
-                if (act[p]) {
-                    const Ctrl &c = ctrl[p];
-                    // r = c_k / c_{k-1} (Taylor.f:93); both pure real or pure imaginary multiples
-                    const double ar = c.cre[c.k - 1], ai = c.cim[c.k - 1];
-                    const double br = c.cre[c.k - 2], bi = c.cim[c.k - 2];
-                    const double d = br * br + bi * bi;
-                    rr[p] = make_double2((ar * br + ai * bi) / d, (ai * br - ar * bi) / d);
+    };
+    // resident: the warp's t-th group of eight columns.  The warps that advance the
+    // particles' states (0 .. P - 1) take half the others' share: their other FP64
+    // instructions fall into the products' time.
+    auto group_of = [&](int t) {
+        constexpr int kOther = kWarps - P, kCycle = 2 * kOther + P;
+        return warp < P ? t * kCycle + 2 * kOther + warp : (t >> 1) * kCycle + (t & 1) * kOther + warp - P;
+    };
+    // the row sums of the active particles' source vectors
+    auto products = [&](const int (&src)[P], const bool (&act)[P]) {
+        if constexpr (kResident) {
+            const int comp = lane & 3, slice = lane >> 2;
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                if (!act[p]) continue;
+                const double *x = sv + (size_t)p * np * 4 + lane;
+                for (int c0 = 0; c0 < nrow; c0 += RC) {
+                    const int nr = min(RC, nrow - c0);
+                    const double *h = sh + ((size_t)c0 * np + slice) * 2 + (comp >> 1);
+                    double v[RC];
+#pragma unroll
+                    for (int r = 0; r < RC; ++r) v[r] = 0.0;
+                    if (nr == RC) {
+#pragma unroll 2
+                        for (int t = 0, jb; (jb = group_of(t)) < np / 8; ++t) {
+                            const double xv = x[jb * 32];
+#pragma unroll
+                            for (int r = 0; r < RC; ++r)
+                                v[r] = fma(h[((size_t)r * np + jb * 8) * 2], xv, v[r]);
+                        }
+                    } else {
+#pragma unroll 2
+                        for (int t = 0, jb; (jb = group_of(t)) < np / 8; ++t) {
+                            const double xv = x[jb * 32];
+#pragma unroll
+                            for (int r = 0; r < RC; ++r)
+                                if (r < nr) v[r] = fma(h[((size_t)r * np + jb * 8) * 2], xv, v[r]);
+                        }
+                    }
+                    // over the eight lanes of a component: rows split over lane bits 4 and 3, then bit 2
+#pragma unroll
+                    for (int o = 16, half = RC / 2; half > 0; o >>= 1, half >>= 1) {
+                        const bool upper = (lane & o) != 0;
+#pragma unroll
+                        for (int i = 0; i < half; ++i) {
+                            const double send = upper ? v[i] : v[i + half];
+                            const double keep = upper ? v[i + half] : v[i];
+                            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                        }
+                    }
+                    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 4);
+                    const int row = c0 + ((lane & 16) ? 2 : 0) + ((lane & 8) ? 1 : 0);
+                    if (!(lane & 4) && row < nrow) sy[((size_t)(warp * P + p) * rows + row) * 4 + comp] = v[0];
                 }
             }
+        } else {
             for (int c0 = r0; c0 < r1; c0 += RC) {
                 const int nr = min(RC, r1 - c0);
-                double acc[PMAX][RC][4];
+                double v[16 * P];
 #pragma unroll
-                for (int p = 0; p < PMAX; ++p)
-#pragma unroll
-                    for (int r = 0; r < RC; ++r)
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) acc[p][r][q] = 0.0;
-                const double2 *xb[PMAX], *xk[PMAX];
-                for (int p = 0; p < PMAX; ++p) {
-                    xb[p] = act[p] ? vec(p, ctrl[p].src, 0) : nullptr;
-                    xk[p] = act[p] ? vec(p, ctrl[p].src, 1) : nullptr;
-                }
+                for (int q = 0; q < 16 * P; ++q) v[q] = 0.0;
                 for (int j = tid; j < N; j += kTaylorBlock) {
                     double hk[RC], hb[RC];
 #pragma unroll
@@ -220,32 +366,27 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
                         hb[r] = L.H[(size_t)i * ld + j];   // H'(j, i): column block (bra, H'^T)
                     }
 #pragma unroll
-                    for (int p = 0; p < PMAX; ++p) {
+                    for (int p = 0; p < P; ++p) {
                         if (!act[p]) continue;
-                        // vectors written by other CTAs: L2 loads (L1 is not coherent across SMs)
-                        const double2 vk = __ldcg(xk[p] + j), vb = __ldcg(xb[p] + j);
+                        const double2 vk = __ldcg(vec(p, src[p], 1) + j), vb = __ldcg(vec(p, src[p], 0) + j);
 #pragma unroll
                         for (int r = 0; r < RC; ++r) {
-                            acc[p][r][0] = fma(hk[r], vk.x, acc[p][r][0]);
-                            acc[p][r][1] = fma(hk[r], vk.y, acc[p][r][1]);
-                            acc[p][r][2] = fma(hb[r], vb.x, acc[p][r][2]);
-                            acc[p][r][3] = fma(hb[r], vb.y, acc[p][r][3]);
+                            double *a = v + (p * RC + r) * 4;
+                            a[0] = fma(hk[r], vk.x, a[0]);
+                            a[1] = fma(hk[r], vk.y, a[1]);
+                            a[2] = fma(hb[r], vb.x, a[2]);
+                            a[3] = fma(hb[r], vb.y, a[3]);
                         }
                     }
                 }
-                // block reduction of the 32 accumulators: transposed butterfly, after
-                // which lane l holds the warp sum of accumulator l (31 shuffles + adds
-                // per lane instead of 5 per accumulator), then a fixed-order sum over warps
-                static_assert(PMAX * RC * 4 == 32, "one accumulator per lane");
-                double v[32];
+                // warp sums: P = 1 first folds the lane halves, then a transposed butterfly,
+                // after which lane l holds the sum of accumulator l % (16 P)
+                if constexpr (P == 1) {
 #pragma unroll
-                for (int p = 0; p < PMAX; ++p)
+                    for (int i = 0; i < 16; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 16);
+                }
 #pragma unroll
-                    for (int r = 0; r < RC; ++r)
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) v[(p * RC + r) * 4 + q] = acc[p][r][q];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
+                for (int o = 8 * P; o > 0; o >>= 1) {
                     const bool upper = (lane & o) != 0;
 #pragma unroll
                     for (int i = 0; i < o; ++i) {
@@ -254,217 +395,278 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
                         v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
                     }
                 }
-                red[warp][lane] = v[0];
+                if (lane < 16 * P) red[warp][lane] = v[0];
                 __syncthreads();
-                if (tid < PMAX * RC * 4) {
-                    double v = 0.0;
-                    for (int w = 0; w < kTaylorBlock / 32; ++w) v += red[w][tid];
-                    red[0][tid] = v;  // safe: each tid reads column tid of all warps before writing row 0
-                }
-                __syncthreads();
-                // epilogue: one thread per (particle, row)
-                if (tid < PMAX * RC) {
-                    const int p = tid / RC, r = tid % RC;
-                    if (act[p] && r < nr) {
-                        const Ctrl &c = ctrl[p];
-                        const int i = c0 + r;
-                        const double2 yk = make_double2(red[0][(p * RC + r) * 4 + 0], red[0][(p * RC + r) * 4 + 1]);
-                        const double2 yb = make_double2(red[0][(p * RC + r) * 4 + 2], red[0][(p * RC + r) * 4 + 3]);
-                        const double2 tk = cmul(rr[p], yk), tb = cmul(rr[p], yb);
-                        const double2 ok = __ldcg(vec(p, c.old, 1) + i), ob = __ldcg(vec(p, c.old, 0) + i);
-                        const double2 nk = make_double2(ok.x + tk.x, ok.y + tk.y);
-                        const double2 nb = make_double2(ob.x + tb.x, ob.y + tb.y);
-                        vec(p, c.out_term, 1)[i] = tk;
-                        vec(p, c.out_term, 0)[i] = tb;
-                        vec(p, c.out_acc, 1)[i] = nk;
-                        vec(p, c.out_acc, 0)[i] = nb;
-                        const double db = hypot(nb.x - ob.x, nb.y - ob.y);
-                        const double dk = hypot(nk.x - ok.x, nk.y - ok.y);
-                        part[p][r][0] = fmax(part[p][r][0], db);
-                        part[p][r][1] = fmax(part[p][r][1], dk);
-                        part[p][r][2] += nb.x * nk.x + nb.y * nk.y;
-                        part[p][r][3] += nb.x * nk.y - nb.y * nk.x;
-                    }
+                if (tid < 16 * P) {
+                    const int p = tid / 16, r = (tid / 4) % 4;
+                    double s = 0.0;
+                    for (int w = 0; w < kWarps; ++w) s += red[w][tid];
+                    if (act[p] && r < nr) sy[((size_t)p * rows + c0 - r0 + r) * 4 + (tid & 3)] = s;
                 }
                 __syncthreads();
             }
-            if (tid < P && act[tid]) {
-                const int p = tid;
-                double mb = 0.0, mk = 0.0, dre = 0.0, dim = 0.0;
-                for (int r = 0; r < RC; ++r) {
-                    mb = fmax(mb, part[p][r][0]);
-                    mk = fmax(mk, part[p][r][1]);
-                    dre += part[p][r][2];
-                    dim += part[p][r][3];
-                }
-                cta_rec[p][0] = mb;
-                cta_rec[p][1] = mk;
-                cta_rec[p][2] = dre;
-                cta_rec[p][3] = dim;
-            }
         }
-        __syncthreads();
-        // publish this CTA's partial record
-        if (tid < P * PW) {
-            const int p = tid / PW, q = tid % PW;
-            L.partials[(((size_t)parity * PMAX + p) * G + blockIdx.x) * PW + q] = cta_rec[p][q];
-        }
+    };
 
-        if (!grid_barrier(L.bar_count, G, L.error)) break;
-
-        // ------------------------------------------------ phase B: reduce + advance
-        // warp p reduces particle p's records in a fixed order (identical in every CTA)
-        __shared__ double tot[PMAX][PW];
-        if (warp < P) {
-            // only the max |delta| and <bra|ket> fields matter after a GEMV round;
-            // the population fields are read after a norm round only
-            const int p = warp;
-            const int nq = (ctrl[p].phase == PH_NORM) ? PW : 4;
-            double v[PW];
+    int parity = 0;
+    unsigned long long arrivals = 0;  // of the whole grid, at the next barrier's end
+    double keep[P];                   // this lane's element of the last partial sum (first unit) ...
+    int keep_slot[P];                 // ... and the slot it went to
 #pragma unroll
-            for (int q = 0; q < PW; ++q) v[q] = 0.0;
-            for (int g = lane; g < G; g += 32) {
-                const double *rec = L.partials + (((size_t)parity * PMAX + p) * G + g) * PW;
-                v[0] = fmax(v[0], __ldcg(rec + 0));
-                v[1] = fmax(v[1], __ldcg(rec + 1));
-                v[2] += __ldcg(rec + 2);
-                v[3] += __ldcg(rec + 3);
-                for (int q = 4; q < nq; ++q) v[q] += __ldcg(rec + q);
+    for (int p = 0; p < P; ++p) {
+        keep[p] = 0.0;
+        keep_slot[p] = -1;
+    }
+    // this CTA's record field q of particle p
+    auto record = [&](int p, int q) -> double * {
+        return L.partials + (((size_t)parity * PMAX + p) * G + blockIdx.x) * PW + q;
+    };
+    // wait for the round's arrivals; false: the launch ends with an error
+    auto wait_round = [&]() -> bool {
+        arrivals += G;
+        if (tid == 0) s_ok = grid_poll(L.bar_count, arrivals, L.error);
+        __syncthreads();
+        return s_ok;
+    };
+    bool ready = false;  // the next round's products are formed
+    for (;;) {
+        int src[P];
+        bool act[P];
+        bool norm = false;
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            src[p] = ctrl[p].src;
+            act[p] = ctrl[p].phase == PH_CONV || ctrl[p].phase == PH_MAIN;
+            norm |= ctrl[p].phase == PH_NORM;
+        }
+        if (!ready) {
+            if constexpr (kResident) {
+#pragma unroll
+                for (int p = 0; p < P; ++p)
+                    if (act[p]) stage(p, src[p]);
+                __syncthreads();
+            }
+            products(src, act);
+        }
+        if (norm && warp < P && ctrl[warp].phase == PH_NORM) {  // <bra|ket> of the own rows
+            const double2 *b = vec(warp, ctrl[warp].psi, 0), *k = vec(warp, ctrl[warp].psi, 1);
+            double dre = 0.0, dim = 0.0;
+            for (int i = r0 + lane; i < r1; i += 32) {
+                const double2 bi = __ldcg(b + i), ki = __ldcg(k + i);
+                dre += bi.x * ki.x + bi.y * ki.y;  // conj(bra) ket
+                dim += bi.x * ki.y - bi.y * ki.x;
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
-                v[0] = fmax(v[0], __shfl_xor_sync(0xffffffffu, v[0], o));
-                v[1] = fmax(v[1], __shfl_xor_sync(0xffffffffu, v[1], o));
-                v[2] += __shfl_xor_sync(0xffffffffu, v[2], o);
-                v[3] += __shfl_xor_sync(0xffffffffu, v[3], o);
+                dre += __shfl_xor_sync(0xffffffffu, dre, o);
+                dim += __shfl_xor_sync(0xffffffffu, dim, o);
             }
-            if (nq > 4)
-                for (int o = 16; o > 0; o >>= 1)
-                    for (int q = 4; q < PW; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-            if (lane == 0)
-                for (int q = 0; q < PW; ++q) tot[p][q] = v[q];
+            if (lane == 0) {
+                *record(warp, 0) = *record(warp, 1) = 0.0;
+                *record(warp, 2) = dre;
+                *record(warp, 3) = dim;
+            }
         }
         __syncthreads();
-        parity ^= 1;
 
-        if (tid == 0) {
-            bool all_done = true;
-            for (int p = 0; p < P; ++p) {
-                Ctrl &c = ctrl[p];
-                const double dotabs = hypot(tot[p][2], tot[p][3]);
-                if (c.phase == PH_NORM) {
-                    c.norm_ref = dotabs;  // Taylor.f:62
-                    c.first = 1;
-                    c.conv_step = 0;
-                    start_conv(c, L.max_conv_calls);
-                } else if (c.phase == PH_CONV) {
-                    c.orders++;
-                    const bool conv = !(tot[p][0] > L.tol) && !(tot[p][1] > L.tol) &&
-                                      fabs(dotabs - c.norm_ref) < L.norm_tol;
-                    if (conv) {
-                        c.psi = c.out_acc;
-                        after_accept(c, s_tinit, s_tmax);
+        // ------------------------------------------------ epilogue
+        // unit u = (particle, eight rows), one warp each: lane = (row, component)
+        const int groups = (nrow + 7) / 8;
+        for (int p = 0; p < P; ++p) {
+            if (!act[p]) continue;
+            const Ctrl &c = ctrl[p];
+            const bool rec = decides(c);
+            const double gk = c.g[c.k - 1];
+            double best = 0.0, dot = 0.0;  // lanes of component 0 / 1: Re / Im of <bra|ket>
+            // units dealt so that both particles' first units go to different warps
+            for (int u = (warp + kWarps - p) % kWarps; u < groups; u += kWarps) {
+                const int row = u * 8 + (lane >> 2), comp = lane & 3, i = r0 + row;
+                const bool in = row < nrow;
+                double y = 0.0;
+                if (in) {
+                    if constexpr (kResident) {
+                        double w[kWarps];
+#pragma unroll
+                        for (int q = 0; q < kWarps; ++q) w[q] = sy[((size_t)(q * P + p) * rows + row) * 4 + comp];
+#pragma unroll
+                        for (int o = kWarps / 2; o > 0; o >>= 1)
+#pragma unroll
+                            for (int q = 0; q < o; ++q) w[q] += w[q + o];
+                        y = w[0];
                     } else {
-                        c.old = c.out_acc;
-                        c.src = c.out_term;
-                        c.k++;
-                        if (c.k > c.kmax) {
-                            c.tau = c.tau * (c.first ? 0.9 : 0.975);  // Taylor.f:69, :110
-                            start_conv(c, L.max_conv_calls);
-                        } else {
-                            pick_out_slots(c);
-                        }
-                    }
-                } else if (c.phase == PH_MAIN) {
-                    c.orders++;
-                    if (c.k < c.kmax) {
-                        c.old = c.out_acc;
-                        c.src = c.out_term;
-                        c.k++;
-                        pick_out_slots(c);
-                    } else if (fabs(dotabs - c.norm_ref) < L.norm_tol) {  // Taylor.f:103-106
-                        c.psi = c.out_acc;
-                        c.substeps++;
-                        c.t = c.t + (c.tau * kHbar);
-                        if (s_tmax - c.t < c.tau * kHbar) {
-                            c.tau = (s_tmax - c.t) / kHbar;
-                            set_coefficients(c);
-                        }
-                        if (c.t < s_tmax) start_main(c); else c.phase = PH_DONE;
-                    } else {  // Taylor.f:107-114
-                        c.tau = c.tau * 0.975;
-                        start_conv(c, L.max_conv_calls);
+                        y = sy[((size_t)p * rows + row) * 4 + comp];
                     }
                 }
-                if (c.phase != PH_DONE) all_done = false;
+                const double yo = __shfl_xor_sync(0xffffffffu, y, 1);  // the other part (re <-> im)
+                double o = keep[p];
+                const size_t e = (size_t)i * 2 + (comp & 1);
+                if (in && (u > 0 || c.old != keep_slot[p])) o = __ldcg(reinterpret_cast<const double *>(vec(p, c.old, comp < 2)) + e);
+                const double t = (comp & 1) ? -gk * yo : gk * yo;  // -i g y
+                const double n = o + t;
+                if (in) {
+                    reinterpret_cast<double *>(vec(p, c.out_term, comp < 2))[e] = t;
+                    reinterpret_cast<double *>(vec(p, c.out_acc, comp < 2))[e] = n;
+                }
+                if (u == 0) keep[p] = n;
+                if (rec) {
+                    const double d = n - o, d2 = d * d;
+                    const double s = d2 + __shfl_xor_sync(0xffffffffu, d2, 1);  // |delta|^2: lanes 0, 1 ket, 2, 3 bra
+                    best = max_bits(best, in ? s : 0.0);
+                    // conj(bra) ket: re = br kr + bi ki, im = br ki - bi kr
+                    const double nb = __shfl_xor_sync(0xffffffffu, n, 2), nbx = __shfl_xor_sync(0xffffffffu, nb, 1);
+                    const double a = comp == 0 ? n * nb : comp == 1 ? n * nbx : 0.0;  // kr br | ki br
+                    const double n1 = __shfl_xor_sync(0xffffffffu, n, 1);
+                    const double b = comp == 0 ? n1 * nbx : comp == 1 ? -n1 * nb : 0.0;  // ki bi | -kr bi
+                    if (in) dot += a + b;
+                }
             }
-            if (all_done) {
-                // populations of the finished step come from a PH_NORM round on the
-                // next step (or the final round below)
-                s_step++;
+            if (rec) {
+                // over the unit's rows (lane bits 2-4), then over the warps' units
+#pragma unroll
+                for (int o = 16; o >= 4; o >>= 1) {
+                    best = max_bits(best, __shfl_xor_sync(0xffffffffu, best, o));
+                    dot += __shfl_xor_sync(0xffffffffu, dot, o);
+                }
+                if (groups <= 1) {
+                    if (warp == p) {
+                        if (lane == 0) {
+                            *record(p, 1) = best;
+                            *record(p, 2) = dot;
+                        } else if (lane == 1) {
+                            *record(p, 3) = dot;
+                        } else if (lane == 2) {
+                            *record(p, 0) = best;
+                        }
+                    }
+                } else {
+                    if (lane == 0) {
+                        unit_rec[warp][1] = best;
+                        unit_rec[warp][2] = dot;
+                    } else if (lane == 1) {
+                        unit_rec[warp][3] = dot;
+                    } else if (lane == 2) {
+                        unit_rec[warp][0] = best;
+                    }
+                    __syncthreads();  // every warp passes here for this particle
+                    if (tid < 4) {
+                        double s = unit_rec[0][tid];
+                        for (int w = 1; w < kWarps; ++w)
+                            s = tid < 2 ? max_bits(s, unit_rec[w][tid]) : s + unit_rec[w][tid];
+                        *record(p, tid) = s;
+                    }
+                    __syncthreads();
+                }
             }
+            keep_slot[p] = c.out_acc;
         }
+        if (P == 1 && groups <= 1) {  // warp 0 alone wrote global memory in this round
+            __syncwarp();
+        } else {
+            __syncthreads();
+        }
+        if (tid == 0) grid_arrive(L.bar_count);
+        if (!wait_round()) break;
+
+        // ------------------------------------------------ advance
+        // The next round's source unless the advance decides otherwise: this round's
+        // term, or the partial sum where a main expansion ends (it is accepted as a rule).
+        int guess[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const Ctrl &c = ctrl[p];
+            guess[p] = !act[p] ? -1 : c.phase == PH_MAIN && c.k >= c.kmax ? c.out_acc : c.out_term;
+        }
+        if constexpr (kResident) {
+#pragma unroll
+            for (int p = 0; p < P; ++p)
+                if (act[p]) stage(p, guess[p]);
+        }
+        __syncthreads();  // ctrl has been read by every thread; the staged vectors are complete
+        if (warp < P) {
+            // warp p: particle p's records summed in a fixed order (identical in every CTA)
+            Ctrl &c = ctrl[warp];
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
+            if (decides(c)) {
+                // lanes 0-15 sum fields 0 and 2 (bra maximum, Re <bra|ket>), lanes 16-31 fields 1 and 3
+                const double *rec = L.partials + ((size_t)parity * PMAX + warp) * G * PW + (lane >> 4);
+                double m = 0.0, d = 0.0;
+#pragma unroll 5
+                for (int g = lane & 15; g < G; g += 16) {
+                    m = max_bits(m, __ldcg(rec + (size_t)g * PW));
+                    d += __ldcg(rec + (size_t)g * PW + 2);
+                }
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) {
+                    m = max_bits(m, __shfl_xor_sync(0xffffffffu, m, o));
+                    d += __shfl_xor_sync(0xffffffffu, d, o);
+                }
+                v[0] = m;
+                v[2] = d;
+                v[1] = __shfl_sync(0xffffffffu, m, 16);
+                v[3] = __shfl_sync(0xffffffffu, d, 16);
+            }
+            int need = 0;
+            if (lane == 0) need = advance(c, v, tol2, L.norm_tol, L.max_conv_calls, s_tinit, s_tmax);
+            need = __shfl_sync(0xffffffffu, need, 0);
+            if (need) set_coefficients(c, need, lane);
+        }
+        products(guess, act);
         __syncthreads();
+        parity ^= 1;
 
         bool all_done = true;
-        for (int p = 0; p < P; ++p) all_done &= (ctrl[p].phase == PH_DONE);
+        ready = true;
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const Ctrl &c = ctrl[p];
+            all_done &= c.phase == PH_DONE;
+            if (c.phase == PH_CONV || c.phase == PH_MAIN) ready &= c.src == guess[p];
+        }
         if (!all_done) continue;
+        ready = false;
 
         // ---- step finished for every particle: population round + step driver
-        // population partials of the final Psi, one more barrier round
-        if (tid < PMAX * PW) (&cta_rec[0][0])[tid] = 0.0;
-        __syncthreads();
-        if (tid < P) {
-            const int p = tid;
-            const double2 *b = vec(p, ctrl[p].psi, 0), *k = vec(p, ctrl[p].psi, 1);
-            double pops[kMaxFrag + 1];
-            for (int f = 0; f <= kMaxFrag; ++f) pops[f] = 0.0;
-            for (int i = r0; i < r1; ++i) {
-                const double2 bi = __ldcg(b + i), ki = __ldcg(k + i);
-                const double v = ki.x * bi.x + ki.y * bi.y;
-                if (L.ao_frag) {
-                    const int f = L.ao_frag[i];
-                    if (f >= 0 && f < nf) pops[f] += v;
-                }
-                pops[kMaxFrag] += v;
-            }
-            for (int f = 0; f <= kMaxFrag; ++f) cta_rec[p][4 + f] = pops[f];
-        }
-        __syncthreads();
-        if (tid < P * PW) {
-            const int p = tid / PW, q = tid % PW;
-            L.partials[(((size_t)parity * PMAX + p) * G + blockIdx.x) * PW + q] = cta_rec[p][q];
-        }
-        if (!grid_barrier(L.bar_count, G, L.error)) break;
-        if (warp < P) {
+        if (L.pops && warp < P) {
             const int p = warp;
-            double v[kMaxFrag + 1];
-            for (int f = 0; f <= kMaxFrag; ++f) v[f] = 0.0;
-            for (int g = lane; g < G; g += 32) {
-                const double *rec = L.partials + (((size_t)parity * PMAX + p) * G + g) * PW;
-                for (int f = 0; f <= kMaxFrag; ++f) v[f] += __ldcg(rec + 4 + f);
-            }
-            for (int o = 16; o > 0; o >>= 1)
-                for (int f = 0; f <= kMaxFrag; ++f) v[f] += __shfl_xor_sync(0xffffffffu, v[f], o);
-            if (lane == 0) {
-                for (int f = 0; f <= kMaxFrag; ++f) tot[p][4 + f] = v[f];
+            const double2 *b = vec(p, ctrl[p].psi, 0), *k = vec(p, ctrl[p].psi, 1);
+            for (int f = 0; f <= nf; ++f) {  // fragments, then the total
+                double s = 0.0;
+                for (int i = r0 + lane; i < r1; i += 32) {
+                    if (f < nf && !(L.ao_frag && L.ao_frag[i] == f)) continue;
+                    const double2 bi = __ldcg(b + i), ki = __ldcg(k + i);
+                    s += ki.x * bi.x + ki.y * bi.y;  // Re conj(ket) bra
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) *record(p, 4 + f) = s;
             }
         }
-        __syncthreads();
+        if (L.pops) {
+            __syncthreads();
+            if (tid == 0) grid_arrive(L.bar_count);
+            if (!wait_round()) break;
+        }
+        if (blockIdx.x == 0 && warp < P && L.pops && s_step < L.nsteps) {
+            const int p = warp;
+            double *dst = L.pops + ((size_t)s_step * P + p) * (L.nfrag + 1);
+            for (int f = 0; f <= nf; ++f) {
+                double s = 0.0;
+                for (int g = lane; g < G; g += 32)
+                    s += __ldcg(L.partials + (((size_t)parity * PMAX + p) * G + g) * PW + 4 + f);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) dst[f == nf ? L.nfrag : f] = s;
+            }
+        }
         parity ^= 1;
-        const int step_done = s_step - 1;
-        if (blockIdx.x == 0 && tid < P && L.pops && step_done < L.nsteps) {
-            const int p = tid;
-            double *dst = L.pops + ((size_t)step_done * P + p) * (L.nfrag + 1);
-            for (int f = 0; f < nf; ++f) dst[f] = tot[p][4 + f];
-            dst[L.nfrag] = tot[p][4 + kMaxFrag];
-        }
         bool failed = false;
         for (int p = 0; p < P; ++p) failed |= (ctrl[p].status != ELHL_OK);
-        if (s_step >= L.nsteps || failed) break;
+        const bool last = s_step + 1 >= L.nsteps;
         __syncthreads();
+        if (last || failed) break;
         if (tid == 0) {
             // next nuclear step (ElHl_Chebyshev.f:174-187, :267): t_init = t, t_max = dt*fs*(it-1)
+            s_step++;
             s_it++;
             s_tinit = s_tinit + L.dt_frame;
             s_tmax = L.dt_frame * (double)(s_it - 1);
@@ -510,24 +712,46 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
     }
 }
 
+template <int P, bool kResident>
+cudaError_t launch_taylor_t(const TaylorLaunch &L, int grid, int block, size_t smem, cudaStream_t st) {
+    auto kern = taylor_kernel<P, kResident>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    TaylorLaunch copy = L;
+    void *args[] = {&copy};
+    e = cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(block), args, smem, st);
+    count_launch();
+    return e;
+}
+
 }  // namespace
 
 int taylor_grid_size(int block, int *grid_out) {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, taylor_kernel, block, 0) != cudaSuccess) return -1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, taylor_kernel<PMAX, false>, block, 0) != cudaSuccess)
+        return -1;
     if (per_sm < 1) return -1;
     *grid_out = sms;  // one CTA per SM
     return 0;
 }
 
+// grid: the CTAs that may run (and that the partials' buffer has room for); the
+// launch takes as many as the rows need at kMinRows or more per CTA.
 cudaError_t launch_taylor(const TaylorLaunch &L, int grid, int block, cudaStream_t st) {
-    TaylorLaunch copy = L;
-    void *args[] = {&copy};
-    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)taylor_kernel, dim3(grid), dim3(block), args, 0, st);
-    count_launch();
-    return e;
+    if (L.N < 1 || grid < 1 || block != kTaylorBlock || L.nparticles < 1 || L.nparticles > PMAX)
+        return cudaErrorInvalidValue;
+    const int rows = std::max((L.N + grid - 1) / grid, kMinRows);
+    const int ctas = (L.N + rows - 1) / rows;
+    const int own = (L.N + ctas - 1) / ctas;  // as the kernel computes it
+    const bool resident = taylor_smem(L.N, own, L.nparticles, true) <= kResidentSmem;
+    const size_t smem = taylor_smem(L.N, own, L.nparticles, resident);
+    if (L.nparticles == 1)
+        return resident ? launch_taylor_t<1, true>(L, ctas, block, smem, st)
+                        : launch_taylor_t<1, false>(L, ctas, block, smem, st);
+    return resident ? launch_taylor_t<2, true>(L, ctas, block, smem, st)
+                    : launch_taylor_t<2, false>(L, ctas, block, smem, st);
 }
 
 }  // namespace elhl
