@@ -399,6 +399,8 @@ __global__ void __launch_bounds__(kBlock, 1) cheb_kernel(ChebLaunch L) {
     const int s0 = L.seg_begin[blockIdx.x], s1 = L.seg_begin[blockIdx.x + 1];
     const unsigned long long bar_ns = L.barrier_ns ? L.barrier_ns : kBarrierNs;
     if ((int)blockIdx.x + 1 == L.exit_cta1) return;  // test hook: the other CTAs' barrier waits run out
+    __shared__ int s_ok;
+    unsigned long long arrivals = 0;
     for (int k = 0; k <= L.kmax; ++k) {
         const int nph = k == 0 ? 1 : L.nphase;
         for (int ph = 0; ph < nph; ++ph) {
@@ -426,7 +428,7 @@ __global__ void __launch_bounds__(kBlock, 1) cheb_kernel(ChebLaunch L) {
                     }
                 }
             }
-            if (!grid_barrier(L.bar_count, G, L.error, bar_ns)) return;
+            if (!grid_round(L.bar_count, arrivals, G, L.error, &s_ok, bar_ns)) return;
         }
     }
 }
@@ -548,8 +550,8 @@ __global__ void reduce_pops_kernel(ChebLaunch L, int nprob) {
 // numbers (48-bit significands, about 4e-15 relative) and evaluates the
 // products on the FP32 pipes: Dekker's exact product error by FMA and Knuth's
 // TwoSum for the running sums (df64.cuh).  Sums leave the row loop in FP64; the recurrence and
-// the accumulation of c_k v_k are FP64 as in the other precisions.  Implicit
-// operator only (G, h/b and G^T stored as float2 = (hi, lo)).
+// the accumulation of c_k v_k are FP64 as in the other precisions.  The operator
+// (G, h/b and G^T, or an explicit Hs) is stored as float2 = (hi, lo).
 
 __device__ __forceinline__ float4 df_split2(double re, double im) {
     const float2 a = df_split(re), b = df_split(im);
@@ -686,8 +688,8 @@ struct StoreEpiDF {
     __device__ void operator()(int i, int c, double yr, double yi) { dst[(size_t)i * MG + c] = df_split2(yr, yi); }
 };
 
-// recurrence in FP64: y -= shift v_{k-1}; v_k = 2 y - v_{k-2} (v_1 = y), stored as
-// DF64; acc += c_k v_k
+// recurrence in FP64: y -= shift v_{k-1} (implicit operator; vprev1 == nullptr:
+// explicit Hs); v_k = 2 y - v_{k-2} (v_1 = y), stored as DF64; acc += c_k v_k
 template <int MG>
 struct OrderEpiDF {
     const float4 *vprev2;
@@ -698,9 +700,11 @@ struct OrderEpiDF {
     const float4 *vprev1;
     double shift;
     __device__ void operator()(int i, int c, double yr, double yi) {
-        const float4 p = __ldcg(vprev1 + (size_t)i * MG + c);
-        yr -= shift * ((double)p.x + (double)p.y);
-        yi -= shift * ((double)p.z + (double)p.w);
+        if (vprev1) {
+            const float4 p = __ldcg(vprev1 + (size_t)i * MG + c);
+            yr -= shift * ((double)p.x + (double)p.y);
+            yi -= shift * ((double)p.z + (double)p.w);
+        }
         double vr = yr, vi = yi;
         if (k > 1) {
             const float4 w = __ldcg(vprev2 + (size_t)i * MG + c);
@@ -776,7 +780,28 @@ __device__ void implicit_phase_df(const ChebLaunch &L, const ChebProblem &pb, in
     }
 }
 
-// one launch per step, implicit operator (one problem, three phases per order)
+// order k >= 1 of an explicit Hs, column group g, over the CTA's segments [s0, s1)
+template <int MG>
+__device__ void explicit_order_df(const ChebLaunch &L, const ChebProblem &pb, int s0, int s1, int k, int g,
+                                  float4 *s_v, float2 *s_part, double cre, double cim) {
+    if (s0 >= s1) return;
+    const int ld = pb.ld, m = pb.m;
+    float4 *vbuf = reinterpret_cast<float4 *>(pb.vbuf);
+    const size_t gstride = (size_t)pb.ldv * MG;
+    const size_t bstride = gstride * (m / MG);
+    const float4 *vprev = vbuf + (size_t)((k + 2) % 3) * bstride + g * gstride;
+    __syncthreads();
+    for (int q = threadIdx.x; q < ld * MG; q += kBlock) s_v[q] = __ldcg(vprev + q);  // padding rows are zero
+    __syncthreads();
+    OrderEpiDF<MG> epi{vbuf + (size_t)((k + 1) % 3) * bstride + g * gstride,
+                       vbuf + (size_t)(k % 3) * bstride + g * gstride,
+                       pb.col[L.parity ^ 1], k, m, g, cre, cim, nullptr, 0.0};
+    for (int s = s0; s < s1; ++s)
+        rows_gemv_df<MG, 0>(reinterpret_cast<const float2 *>(pb.H), ld, s_v, L.segs[s].row0, L.segs[s].row1, s_part,
+                            epi);
+}
+
+// one launch per step, one problem: implicit operator (three phases per order) or explicit Hs (one)
 template <int MG>
 __global__ void __launch_bounds__(kBlock, 1) cheb_df_kernel(ChebLaunch L) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -787,24 +812,29 @@ __global__ void __launch_bounds__(kBlock, 1) cheb_df_kernel(ChebLaunch L) {
     const ChebProblem &pb = L.probs[0];
     const unsigned long long bar_ns = L.barrier_ns ? L.barrier_ns : kBarrierNs;
     if ((int)blockIdx.x + 1 == L.exit_cta1) return;  // test hook: the other CTAs' barrier waits run out
+    __shared__ int s_ok;
+    unsigned long long arrivals = 0;
     for (int k = 0; k <= L.kmax; ++k) {
-        const int nph = k == 0 ? 1 : 3;
+        const int nph = k == 0 ? 1 : L.nphase;
         for (int ph = 0; ph < nph; ++ph) {
             if (k == 0) {
                 for (int s = s0; s < s1; ++s) order_zero_df<MG>(pb, L.segs[s], L.parity);
             } else if (k <= pb.K) {
                 const double cre = pb.coef[k].x, cim = pb.coef[k].y;
-                for (int g = 0; g < pb.m / MG; ++g)
-                    implicit_phase_df<MG>(L, pb, s0, s1, k, ph, g, s_v, s_part, cre, cim);
+                for (int g = 0; g < pb.m / MG; ++g) {
+                    if (L.nphase == 3)
+                        implicit_phase_df<MG>(L, pb, s0, s1, k, ph, g, s_v, s_part, cre, cim);
+                    else
+                        explicit_order_df<MG>(L, pb, s0, s1, k, g, s_v, s_part, cre, cim);
+                }
             }
-            if (!grid_barrier(L.bar_count, G, L.error, bar_ns)) return;
+            if (!grid_round(L.bar_count, arrivals, G, L.error, &s_ok, bar_ns)) return;
         }
     }
 }
 
 template <int MG>
 cudaError_t launch_df(const ChebLaunch &L, cudaStream_t st) {
-    if (L.nphase != 3) return cudaErrorInvalidValue;  // implicit operator only
     auto kern = cheb_df_kernel<MG>;
     const size_t smem = kCheb_part_bytes + (size_t)L.max_ld * MG * sizeof(float4);
     if (smem > kCheb_smem_limit) return cudaErrorInvalidValue;

@@ -307,8 +307,8 @@ int chol_inv64(double *A, double *G, int n, int ld, int row0, double *W, int *in
 // ---- H' = S^-1 h = G^T (G h) ---------------------------------------------------
 struct Factor {
     int N = 0, ld = 0;
-    double *L = nullptr;     // Cholesky factor (lower, zero above the diagonal), N x N, ld
-    double *G = nullptr;     // G = L^-1 (lower, zero above the diagonal), unless factor() put it elsewhere
+    double *L = nullptr;     // Cholesky factor (lower triangle), N x N, ld
+    double *G = nullptr;     // G = L^-1 (lower triangle), unless factor() put it elsewhere
     double *W = nullptr;     // ld x N workspace: the factorisation's off-diagonal blocks, then G h
     int *info = nullptr;     // [2]: first non-positive pivot (1-based global column), 0 = positive definite
     double *cols = nullptr;  // 2 x (N x 2) scratch (S^-1 applied to a complex vector)
@@ -330,8 +330,9 @@ struct Factor {
         dev_free(L); dev_free(G); dev_free(W); dev_free(info); dev_free(cols);
         N = 0;
     }
-    // L <- chol(S) and Gdst (this->G when null) <- L^-1, both with zero upper
-    // triangles and padding rows.  Every block of the recursion is checked
+    // L <- chol(S) and Gdst (this->G when null) <- L^-1, lower triangles (what is
+    // above the diagonal and in the padding rows is undefined: every reader masks
+    // it or stays below the diagonal).  Every block of the recursion is checked
     // against the workspace before the first launch.  Asynchronous.
     int factor(const double *S, int n, double *Gdst = nullptr) {
         cudaStream_t st = g_ctx.stream;
@@ -340,14 +341,7 @@ struct Factor {
         CU_TRY(cudaMemsetAsync(info, 0, 2 * sizeof(int), st));
         CU_TRY(cudaMemcpy2DAsync(L, ld * sizeof(double), S, ld * sizeof(double), n * sizeof(double), n,
                                  cudaMemcpyDeviceToDevice, st));
-        if (int rc = chol_inv64(L, g, n, ld, 0, W, info, tc)) return rc;
-        const dim3 grid((ld + 127) / 128, n);
-        lower_only_kernel<<<grid, 128, 0, st>>>(L, n, ld);
-        count_launch();
-        lower_only_kernel<<<grid, 128, 0, st>>>(g, n, ld);
-        count_launch();
-        CU_TRY(cudaGetLastError());
-        return ELHL_OK;
+        return chol_inv64(L, g, n, ld, 0, W, info, tc);
     }
     // L, G from S; Hp <- G^T (G h) = S^-1 h, 2 N^3 flops with triangular G.  Asynchronous.
     int form_hprime(const double *S, const double *h, double *Hp, int n) {
@@ -795,11 +789,13 @@ struct ChebState {
     bool implicit = false;
     void *Gt = nullptr;
     void *wb = nullptr;      // [2][ld][m] launch precision (phase intermediates)
-    // FP64 L^T and G^T for the column transforms of the implicit operator: B and
-    // Gt on the FP64 path, own copies in the other precisions
+    // FP64 L^T and G^T of a moving-nuclei rebuild for the column transforms: own
+    // copies, except that the implicit operator in FP64 has them as B and Gt
     double *Lt64 = nullptr, *Gt64 = nullptr;
-    const double *lt64() const { return precision == ELHL_PREC_FP64 ? static_cast<const double *>(B) : Lt64; }
-    const double *gt64() const { return precision == ELHL_PREC_FP64 ? static_cast<const double *>(Gt) : Gt64; }
+    bool moving = false;     // the current factor came from a moving-nuclei rebuild: Lt64, Gt64 are its transposes
+    bool t_shared() const { return implicit && precision == ELHL_PREC_FP64; }
+    const double *lt64() const { return !moving ? nullptr : t_shared() ? static_cast<const double *>(B) : Lt64; }
+    const double *gt64() const { return !moving ? nullptr : t_shared() ? static_cast<const double *>(Gt) : Gt64; }
     double *cscratch = nullptr;  // [2m][ld] column-transform output
     int alloc(int N_, int m_, int prec) {
         N = N_;
@@ -1086,10 +1082,12 @@ int cheb_prepare_implicit(ChebState &cs, const double *Lfac, const double *h, do
         convert_kernel<double><<<grid, 128, 0, st>>>(Lfac, cs.Lt64, n, ld, true);
         count_launch();
     }
-    convert_kernel<double><<<grid, 128, 0, st>>>(cs.Ht, const_cast<double *>(cs.gt64()), n, ld, true);
+    convert_kernel<double><<<grid, 128, 0, st>>>(
+        cs.Ht, cs.precision != ELHL_PREC_FP64 ? cs.Gt64 : static_cast<double *>(cs.Gt), n, ld, true);
     count_launch();
     CU_TRY(cudaGetLastError());
-    if (int rc = lanczos_bounds(cs, kLanczosMoving, h, cs.gt64())) return rc;
+    const double *Gt = cs.precision != ELHL_PREC_FP64 ? cs.Gt64 : static_cast<const double *>(cs.Gt);
+    if (int rc = lanczos_bounds(cs, kLanczosMoving, h, Gt)) return rc;
     if (int rc = cheb_prepare(cs, dt, tol, h)) return rc;
     if (cs.precision == ELHL_PREC_DF64) {  // G and G^T as (hi, lo) pairs; no device read-out matrices
         split_df_kernel<<<grid, 128, 0, st>>>(cs.Ht, (float2 *)cs.A, n, ld, 0.0, 1.0, false);
@@ -1097,7 +1095,7 @@ int cheb_prepare_implicit(ChebState &cs, const double *Lfac, const double *h, do
         split_df_kernel<<<grid, 128, 0, st>>>(cs.Ht, (float2 *)cs.Gt, n, ld, 0.0, 1.0, true);
         count_launch();
         CU_TRY(cudaGetLastError());
-        cs.implicit = true;
+        cs.implicit = cs.moving = true;
         cs.readout_ready = false;  // read-out through the FP64 dense transforms
         return ELHL_OK;
     }
@@ -1115,7 +1113,7 @@ int cheb_prepare_implicit(ChebState &cs, const double *Lfac, const double *h, do
         count_launch();
     }
     CU_TRY(cudaGetLastError());
-    cs.implicit = true;
+    cs.implicit = cs.moving = true;
     cs.readout_ready = true;
     return ELHL_OK;
 }
@@ -1396,6 +1394,9 @@ struct ChebPlan {
 
 int tune_plan(ChebPlan &pl, int mgcd);
 
+// may the propagation stage its vector in windows? (explicit Hs, not in DF64)
+bool windowed_plan(int precision, bool implicit) { return !implicit && precision != ELHL_PREC_DF64; }
+
 int cheb_plan(ChebPlan &pl, const std::vector<ChebState *> &states) {
     pl.release();
     pl.probs.clear();
@@ -1418,7 +1419,7 @@ int cheb_plan(ChebPlan &pl, const std::vector<ChebState *> &states) {
         mgcd = a;
     }
     const bool implicit_plan = states[0]->implicit;
-    pl.mg = cheb_group_size(pl.precision, mgcd, pl.max_ld, !implicit_plan);
+    pl.mg = cheb_group_size(pl.precision, mgcd, pl.max_ld, windowed_plan(pl.precision, implicit_plan));
     if (!pl.mg) return ELHL_ERR_UNSUPPORTED;
     int pgcd = 0;  // read-out groups must divide every problem's ket columns
     for (auto *cs : states) {
@@ -1583,8 +1584,9 @@ std::map<std::tuple<int, int, int, int, int>, int> g_tile_cache;
 
 int tune_plan(ChebPlan &pl, int mgcd) {
     std::vector<int> cand;
+    const bool windowed = windowed_plan(pl.precision, pl.nphase == 3);
     for (int mg : {4, 2, 1})
-        if (mgcd % mg == 0 && cheb_group_size(pl.precision, mg, pl.max_ld, pl.nphase == 1) == mg) cand.push_back(mg);
+        if (mgcd % mg == 0 && cheb_group_size(pl.precision, mg, pl.max_ld, windowed) == mg) cand.push_back(mg);
     if (cand.size() < 2 || pl.kmax < 1) return ELHL_OK;
     double elems = 0.0;
     for (const auto &p : pl.probs) elems += (double)p.N * p.ld;
@@ -2041,21 +2043,36 @@ int rebuild(elhl_traj *tr, const double *d_coords) {
     return rc;
 }
 
+// Moving nuclei: form H~ = G h G^T every step (1.5 N^3 flops), or apply its three
+// factors in every order (twice the elements, three grid phases per order instead
+// of one, and the same in the Lanczos recursion)?  H~ wins until its N^3 overtakes
+// the N^2 saved per order (143 orders of a 0.5 fs step): measured whole steps,
+// factors / H~ in ms, FP32 5.8 / 3.4 at N = 744, 24.1 / 20.0 at 3720, 45.5 / 41.8 at
+// 5580; DF64 16.0 / 9.7 at 1860, 85.2 / 63.0 at 5580; FP64, whose H~ is formed on
+// the FP64 pipe, 15.5 / 9.2 at 1032, 31.6 / 28.4 at 1860.  Beyond the measured sizes
+// the lines lie where the two costs extrapolated as N^2 and N^3 meet.  The OZ64
+// kernel propagates an explicit operator only.
+bool moving_explicit(const elhl_traj *tr) {
+    switch (tr->cfg.precision) {
+        case ELHL_PREC_OZ64: return true;
+        case ELHL_PREC_FP64: return tr->N <= 2000;
+        case ELHL_PREC_DF64: return tr->N <= 12000;
+        default: return tr->N <= 6000;
+    }
+}
+
 // Cholesky factor, then the operator for the current S, h: explicit H~ (formed
-// once for fixed nuclei, 2 N^3 flops) or implicit G h G^T (a geometry that
-// changes every step, N^3/3 flops); bounds and coefficients.
-int cheb_rebuild_operator(elhl_traj *tr, bool implicit = false) {
+// once for fixed nuclei; for moving nuclei as moving_explicit says, unless the
+// caller asks for the factors) or implicit G h G^T; bounds and coefficients.
+int cheb_rebuild_operator(elhl_traj *tr, bool implicit = false, bool factors = false) {
     cudaStream_t st = g_ctx.stream;
     ChebState &cs = tr->cs;
     // S = L L^T and G = L^-1 in one recursion, in FP64 for every precision: on the
     // FP64 pipe for FP64 propagation (the plain FP64 path), with the products of
     // 320 or more rows exact on the tensor cores for the others (Factor::tc).
     // The implicit operator keeps G in cs.Ht, the explicit one in the factor's G.
-    if (implicit && cs.oz) {
-        // ELHL_PREC_OZ64: with every product on the tensor cores, forming H~ = G h G^T
-        // (1.5 N^3 flops) costs less than the implicit operator's extra phases (2 N^2
-        // elements and three grid phases per order instead of N^2 and one), so moving
-        // nuclei use the explicit operator too.  FP64 L^T and G^T serve the column transforms.
+    cs.moving = false;
+    if (implicit && !factors && moving_explicit(tr)) {
         if (int rc = tr->fac.factor(tr->S, tr->N)) return rc;
         CU_TRY(cudaEventRecord(g_ctx.ev[5], st));
         if (int rc = tr->fac.check_info(false)) return rc;
@@ -2064,12 +2081,20 @@ int cheb_rebuild_operator(elhl_traj *tr, bool implicit = false) {
         CU_TRY(cudaEventRecord(g_ctx.ev[6], st));
         if (int rc = lanczos_bounds(cs, kLanczosMoving)) return rc;
         if (int rc = cheb_prepare(cs, tr->cfg.dt * tr->cfg.frame_step, tr->cfg.cheb_tol)) return rc;
-        if (int rc = cheb_prepare_readout(cs, tr->fac.L, tr->fac.G)) return rc;  // A = G, B = L^T in FP64
-        if (!cs.Gt) CU_TRY(cudaMalloc(&cs.Gt, (size_t)cs.ld * cs.N * sizeof(double)));
-        convert_kernel<double><<<dim3((cs.ld + 127) / 128, cs.N), 128, 0, st>>>(tr->fac.G, (double *)cs.Gt, cs.N,
-                                                                                cs.ld, true);
+        // FP64 L^T and G^T for the column transforms; the read-out matrices of fixed
+        // nuclei follow when a step without coordinates asks for them
+        if (!cs.Lt64)
+            if (int rc = dev_alloc(&cs.Lt64, (size_t)cs.ld * cs.N)) return rc;
+        if (!cs.Gt64)
+            if (int rc = dev_alloc(&cs.Gt64, (size_t)cs.ld * cs.N)) return rc;
+        const dim3 grid((cs.ld + 127) / 128, cs.N);
+        convert_kernel<double><<<grid, 128, 0, st>>>(tr->fac.L, cs.Lt64, cs.N, cs.ld, true);
+        count_launch();
+        convert_kernel<double><<<grid, 128, 0, st>>>(tr->fac.G, cs.Gt64, cs.N, cs.ld, true);
         count_launch();
         CU_TRY(cudaGetLastError());
+        cs.moving = true;
+        cs.readout_ready = false;
         return ELHL_OK;
     }
     if (int rc = tr->fac.factor(tr->S, tr->N, implicit ? cs.Ht : nullptr)) return rc;
@@ -2107,7 +2132,7 @@ int cheb_load_columns(elhl_traj *tr) {
         return ELHL_OK;
     }
     const double *G = traj_inverse(tr);
-    const double *Lt = cs.oz ? cs.lt64() : nullptr, *Gt = cs.oz ? cs.gt64() : nullptr;  // FP64 transposes
+    const double *Lt = cs.lt64(), *Gt = cs.gt64();  // FP64 transposes (moving nuclei) or null
     if (int rc = cols_apply_dense(tr->fac.L, G, tr->ld, n, in, cs.m, 0, P, false, false, cs.cscratch, Lt, Gt))
         return rc;  // L^T psi
     if (cs.m == 2 * P)
@@ -2135,7 +2160,7 @@ int cheb_readout(elhl_traj *tr, const double2 *cols, double *d_pops) {
             return rc;  // L chi
     } else {
         const double *G = traj_inverse(tr);
-        const double *Lt = cs.oz ? cs.lt64() : nullptr, *Gt = cs.oz ? cs.gt64() : nullptr;  // FP64 transposes
+        const double *Lt = cs.lt64(), *Gt = cs.gt64();  // FP64 transposes (moving nuclei) or null
         if (int rc = cols_apply_dense(tr->fac.L, G, tr->ld, n, tr->psi_ao, P, 0, P, false, true, cs.cscratch, Lt, Gt))
             return rc;  // L^-T phi
         if (int rc = cols_apply_dense(tr->fac.L, G, tr->ld, n, tr->bra_ao, P, 0, P, true, false, cs.cscratch, Lt, Gt))
@@ -2840,7 +2865,7 @@ int elhl_traj_create(const elhl_basis_desc *basis, const double *coords, const e
         if (!rc && cudaMemset(tr->psi_ao, 0, (size_t)tr->ld * tr->P * sizeof(double2)) != cudaSuccess) rc = ELHL_ERR_CUDA;
         if (!rc && cudaMemset(tr->bra_ao, 0, (size_t)tr->ld * tr->P * sizeof(double2)) != cudaSuccess) rc = ELHL_ERR_CUDA;
         const bool df = tr->cfg.precision == ELHL_PREC_DF64;  // DF64: implicit operator from the start
-        if (!rc) rc = cheb_rebuild_operator(tr, df);
+        if (!rc) rc = cheb_rebuild_operator(tr, df, df);
         ChebState &cs = tr->cs;
         cs.P = tr->P; cs.nfrag = tr->nfrag; cs.psi_out = tr->psi_ao; cs.bra_out = tr->bra_ao;
         cs.ao_frag = tr->basis.ao_frag; cs.target = tr->target;

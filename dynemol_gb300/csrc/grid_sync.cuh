@@ -84,5 +84,18 @@ __device__ __forceinline__ bool grid_poll(const unsigned *count, unsigned long l
     __threadfence();  // acquire: the other CTAs' writes before their arrivals
     return ok;
 }
+// One barrier of a block's threads with the grid: `arrivals` counts the grid's
+// arrivals so far in every thread, *s_ok (shared memory) carries the answer.
+__device__ __forceinline__ bool grid_round(unsigned *count, unsigned long long &arrivals, unsigned nblocks, int *err,
+                                           int *s_ok, unsigned long long limit_ns = kBarrierNs) {
+    __syncthreads();
+    arrivals += nblocks;
+    if (threadIdx.x == 0) {
+        grid_arrive(count);
+        *s_ok = grid_poll(count, arrivals, err, limit_ns);
+    }
+    __syncthreads();
+    return *s_ok;
+}
 
 }  // namespace elhl
