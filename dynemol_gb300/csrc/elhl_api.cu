@@ -2477,10 +2477,37 @@ int traj_step_impl(elhl_traj *tr, const double *coords, bool coords_on_device, i
     return ELHL_OK;
 }
 
-// Initial state of particle p from fragment MO `state` (1-based).
-int fmo_particle(elhl_traj *tr, int nat, const int *atoms, int state, double2 *ket, double2 *bra, int stride) {
-    if (nat <= 0 || !atoms || state < 1 || !tr->S) return ELHL_ERR_BAD_ARG;
-    std::vector<int> ao0, nao, n, l, m, nz, aos;
+// The molecular orbitals of one fragment at the current coordinates: H_f C = S_f C E
+// solved once (cuSOLVER dsygvd), any number of its states embedded afterwards.  An
+// ensemble or a served request takes its columns from one fragment: a request of 8
+// states used to build and solve the same problem 8 times (3 ms each at 60 AOs).
+struct FragmentOrbitals {
+    int nf = 0, ldf = 0;
+    double *C = nullptr;  // eigenvectors, ascending energy
+    int *aos = nullptr;   // [nf] their AOs in the full basis
+    ~FragmentOrbitals() {
+        dev_free(C);
+        dev_free(aos);
+    }
+    int solve(elhl_traj *tr, int nat, const int *atoms);
+    // fragment MO `state` (1-based) into ket (zeros outside the fragment), bra = S ket
+    int embed(elhl_traj *tr, int state, double2 *ket, double2 *bra, int stride) const {
+        if (state < 1 || state > nf) return ELHL_ERR_BAD_ARG;
+        cudaStream_t st = g_ctx.stream;
+        zero_strided<<<(tr->N + 255) / 256, 256, 0, st>>>(ket, tr->N, stride);
+        count_launch();
+        embed_fmo<<<1, 256, 0, st>>>(C, ldf, nf, state - 1, aos, ket, stride);
+        count_launch();
+        s_times_sparse<<<(tr->N + 127) / 128, 128, 0, st>>>(tr->S, tr->ld, tr->N, aos, nf, ket, bra, stride);
+        count_launch();
+        CU_TRY(cudaGetLastError());
+        return ELHL_OK;
+    }
+};
+
+int FragmentOrbitals::solve(elhl_traj *tr, int nat, const int *atoms) {
+    if (nat <= 0 || !atoms || !tr->S) return ELHL_ERR_BAD_ARG;
+    std::vector<int> ao0, nao, n, l, m, nz, haos;
     std::vector<double> zeta, coef, ip, kwh, vs;
     for (int a = 0; a < nat; ++a) {
         const int at = atoms[a];
@@ -2489,15 +2516,15 @@ int fmo_particle(elhl_traj *tr, int nat, const int *atoms, int state, double2 *k
         nao.push_back(tr->h_nao[at]);
         for (int j = 0; j < tr->h_nao[at]; ++j) {
             const int i = tr->h_ao0[at] + j;
-            aos.push_back(i);
+            haos.push_back(i);
             n.push_back(tr->h_n[i]); l.push_back(tr->h_l[i]); m.push_back(tr->h_m[i]); nz.push_back(tr->h_nz[i]);
             zeta.push_back(tr->h_zeta[2 * i]); zeta.push_back(tr->h_zeta[2 * i + 1]);
             coef.push_back(tr->h_coef[2 * i]); coef.push_back(tr->h_coef[2 * i + 1]);
             ip.push_back(tr->h_ip[i]); kwh.push_back(tr->h_kwh[i]); vs.push_back(tr->h_vs[i]);
         }
     }
-    const int nf = (int)aos.size();
-    if (state > nf) return ELHL_ERR_BAD_ARG;
+    nf = (int)haos.size();
+    ldf = round_up(nf, 32);
     // fragment coordinates gathered from the current device coordinates
     std::vector<double> all((size_t)tr->natoms * 3), sub((size_t)nat * 3);
     CU_TRY(copy_d2h(all.data(), tr->last_coords, all.size() * sizeof(double)));
@@ -2509,42 +2536,32 @@ int fmo_particle(elhl_traj *tr, int nat, const int *atoms, int state, double2 *k
     d.ao_ip = ip.data(); d.ao_kwh = kwh.data(); d.ao_vshift = vs.data(); d.ao_frag = nullptr; d.nfrag = 0;
     DevBasis fb;
     int rc = upload_basis(fb, &d);
-    const int ldf = round_up(nf, 32);
-    double *Sf = nullptr, *hf = nullptr, *w = nullptr, *dc = nullptr, *work = nullptr;
-    int *info = nullptr, *daos = nullptr, lwork = 0;
+    double *Sf = nullptr, *w = nullptr, *dc = nullptr, *work = nullptr;
+    int *info = nullptr, lwork = 0;
     cudaStream_t st = g_ctx.stream;
     if (!rc) rc = dev_alloc(&Sf, (size_t)ldf * nf);
-    if (!rc) rc = dev_alloc(&hf, (size_t)ldf * nf);
+    if (!rc) rc = dev_alloc(&C, (size_t)ldf * nf);  // h_f, then the eigenvectors
     if (!rc) rc = dev_alloc(&w, (size_t)nf);
     if (!rc) rc = dev_alloc(&dc, sub.size());
     if (!rc) rc = dev_alloc(&info, 1);
-    if (!rc) rc = dev_alloc(&daos, (size_t)nf);
+    if (!rc) rc = dev_alloc(&aos, (size_t)nf);
     if (!rc && copy_h2d(dc, sub.data(), sub.size() * sizeof(double)) != cudaSuccess) rc = ELHL_ERR_CUDA;
-    if (!rc && copy_h2d(daos, aos.data(), nf * sizeof(int)) != cudaSuccess) rc = ELHL_ERR_CUDA;
-    if (!rc && launch_build_sh(fb, dc, tr->cfg.cutoff, Sf, hf, ldf, st) != cudaSuccess) rc = ELHL_ERR_CUDA;
+    if (!rc && copy_h2d(aos, haos.data(), nf * sizeof(int)) != cudaSuccess) rc = ELHL_ERR_CUDA;
+    if (!rc && launch_build_sh(fb, dc, tr->cfg.cutoff, Sf, C, ldf, st) != cudaSuccess) rc = ELHL_ERR_CUDA;
     if (!rc && cusolverDnDsygvd_bufferSize(g_ctx.solver, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_VECTOR,
-                                           CUBLAS_FILL_MODE_LOWER, nf, hf, ldf, Sf, ldf, w, &lwork) !=
+                                           CUBLAS_FILL_MODE_LOWER, nf, C, ldf, Sf, ldf, w, &lwork) !=
                    CUSOLVER_STATUS_SUCCESS)
         rc = ELHL_ERR_CUDA;
     if (!rc) rc = dev_alloc(&work, (size_t)lwork + 1);
     if (!rc && cusolverDnDsygvd(g_ctx.solver, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER,
-                                nf, hf, ldf, Sf, ldf, w, work, lwork, info) != CUSOLVER_STATUS_SUCCESS)
+                                nf, C, ldf, Sf, ldf, w, work, lwork, info) != CUSOLVER_STATUS_SUCCESS)
         rc = ELHL_ERR_CUDA;
-    if (!rc) {
-        zero_strided<<<(tr->N + 255) / 256, 256, 0, st>>>(ket, tr->N, stride);
-        count_launch();
-        embed_fmo<<<1, 256, 0, st>>>(hf, ldf, nf, state - 1, daos, ket, stride);
-        count_launch();
-        s_times_sparse<<<(tr->N + 127) / 128, 128, 0, st>>>(tr->S, tr->ld, tr->N, daos, nf, ket, bra, stride);
-        count_launch();
-        if (cudaGetLastError() != cudaSuccess) rc = ELHL_ERR_CUDA;
-    }
     int hinfo = 0;
     if (!rc && cudaMemcpyAsync(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = ELHL_ERR_CUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess && !rc) rc = ELHL_ERR_CUDA;
     if (!rc && hinfo != 0) rc = hinfo > nf ? ELHL_ERR_NOT_POSITIVE_DEFINITE : ELHL_ERR_CUDA;
     free_basis(fb);
-    dev_free(Sf); dev_free(hf); dev_free(w); dev_free(dc); dev_free(work); dev_free(info); dev_free(daos);
+    dev_free(Sf); dev_free(w); dev_free(dc); dev_free(work); dev_free(info);
     return rc;
 }
 
@@ -2931,22 +2948,32 @@ int elhl_traj_init_fmo(elhl_traj *tr, int n_el_atoms, const int *el_atoms, int e
                        const int *hl_atoms, int hole_state) {
     if (!tr) return ELHL_ERR_BAD_ARG;
     std::lock_guard<std::mutex> lk(g_ctx.mu);
-    if (tr->cheb()) {
-        if (tr->P < 2) return ELHL_ERR_BAD_ARG;
-        if (int rc = fmo_particle(tr, n_el_atoms, el_atoms, electron_state, tr->psi_ao, tr->bra_ao, tr->P)) return rc;
-        if (int rc = fmo_particle(tr, n_hl_atoms, hl_atoms, hole_state, tr->psi_ao + 1, tr->bra_ao + 1, tr->P))
-            return rc;
-        return cheb_set_target(tr);
-    }
-    if (int rc = fmo_particle(tr, n_el_atoms, el_atoms, electron_state, tr->tb.ket(0), tr->tb.bra(0), 1)) return rc;
-    return fmo_particle(tr, n_hl_atoms, hl_atoms, hole_state, tr->tb.ket(1), tr->tb.bra(1), 1);
+    const bool cheb = tr->cheb();
+    if (cheb && tr->P < 2) return ELHL_ERR_BAD_ARG;
+    FragmentOrbitals el, hl;
+    if (int rc = el.solve(tr, n_el_atoms, el_atoms)) return rc;
+    if (int rc = el.embed(tr, electron_state, cheb ? tr->psi_ao : tr->tb.ket(0), cheb ? tr->bra_ao : tr->tb.bra(0),
+                          cheb ? tr->P : 1))
+        return rc;
+    const bool same = n_hl_atoms == n_el_atoms && hl_atoms &&  // one fragment carries both (el.solve checked el_atoms)
+                      std::equal(el_atoms, el_atoms + n_el_atoms, hl_atoms);
+    if (!same)
+        if (int rc = hl.solve(tr, n_hl_atoms, hl_atoms)) return rc;
+    if (int rc = (same ? el : hl).embed(tr, hole_state, cheb ? tr->psi_ao + 1 : tr->tb.ket(1),
+                                        cheb ? tr->bra_ao + 1 : tr->tb.bra(1), cheb ? tr->P : 1))
+        return rc;
+    if (cheb) return cheb_set_target(tr);
+    CU_TRY(cudaStreamSynchronize(g_ctx.stream));
+    return ELHL_OK;
 }
 
 int elhl_traj_init_fmo_states(elhl_traj *tr, int n_atoms, const int *atoms, int nstates, const int *states) {
     if (!tr || !tr->cheb() || nstates < 1 || nstates > tr->P || !states) return ELHL_ERR_BAD_ARG;
     std::lock_guard<std::mutex> lk(g_ctx.mu);
+    FragmentOrbitals fo;
+    if (int rc = fo.solve(tr, n_atoms, atoms)) return rc;
     for (int c = 0; c < nstates; ++c)
-        if (int rc = fmo_particle(tr, n_atoms, atoms, states[c], tr->psi_ao + c, tr->bra_ao + c, tr->P)) return rc;
+        if (int rc = fo.embed(tr, states[c], tr->psi_ao + c, tr->bra_ao + c, tr->P)) return rc;
     return cheb_set_target(tr);
 }
 
