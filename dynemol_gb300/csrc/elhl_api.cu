@@ -797,6 +797,11 @@ struct ChebState {
     const double *lt64() const { return !moving ? nullptr : t_shared() ? static_cast<const double *>(B) : Lt64; }
     const double *gt64() const { return !moving ? nullptr : t_shared() ? static_cast<const double *>(Gt) : Gt64; }
     double *cscratch = nullptr;  // [2m][ld] column-transform output
+    // explicit operator on the shared-memory row kernel (cheb_rows.cuh): rows per CTA (0:
+    // another kernel), its exchange buffers and the launches made on them
+    int rows = 0;
+    ulonglong2 *xbuf = nullptr;
+    unsigned long long row_launches = 0;
     int alloc(int N_, int m_, int prec) {
         N = N_;
         ld = round_up(N, 32);
@@ -847,6 +852,7 @@ struct ChebState {
         dev_free(Lt64);
         dev_free(Gt64);
         dev_free(cscratch);
+        dev_free(xbuf);
         implicit = false;
         dev_free(gpops);
         dev_free(Ht); dev_free(phi); dev_free(acc); dev_free(coef); dev_free(lz); dev_free(scale);
@@ -969,7 +975,7 @@ int cheb_prepare(ChebState &cs, double dt, double tol, const double *h = nullptr
     CU_TRY(cudaMemcpyAsync(cs.coef, c.data(), (K + 1) * sizeof(double2), cudaMemcpyHostToDevice, st));
     CU_TRY(cudaStreamSynchronize(st));  // c is a host temporary
     cs.K = K;
-    if (cs.oz)  // the tensor-core propagation reads Hs as BF16 slices
+    if (cs.oz && !cs.rows)  // the tensor-core propagation reads Hs as BF16 slices
         if (int rc = cs.oz->slice(static_cast<const double *>(cs.Hs), st)) return rc;
     if (cs.umma && !h) {  // the tensor-core GEMM reads Hs as three BF16 terms
         if (int rc = split3_bf16(reinterpret_cast<const float *>(cs.Hs), cs.N, cs.N, cs.ld, cs.hsplit, cs.ld, false, st))
@@ -1385,6 +1391,7 @@ struct ChebPlan {
     int mgcd = 0;              // gcd of the problems' column counts
     bool tuned = false;        // tile measured (on the plan's first run)
     OzRes *oz = nullptr;       // one ELHL_PREC_OZ64 trajectory: the tensor-core propagation
+    ChebState *solo = nullptr; // the state of a plan of one problem
     size_t pops_per_step = 0;  // populations of all problems in one step
     void release() {
         dev_free(d_probs); dev_free(d_segs); dev_free(d_seg_begin); dev_free(d_prob_seg0); dev_free(d_seg_pops);
@@ -1536,6 +1543,7 @@ int cheb_plan(ChebPlan &pl, const std::vector<ChebState *> &states) {
     pl.mgcd = mgcd;
     pl.tuned = false;  // measured on the first run (plans of batch members never run)
     pl.oz = states.size() == 1 ? states[0]->oz : nullptr;
+    pl.solo = states.size() == 1 ? states[0] : nullptr;
     return ELHL_OK;
 }
 
@@ -1670,8 +1678,42 @@ int oz_run(ChebPlan &pl) {
     return ELHL_OK;
 }
 
+// The propagation launch of a plan of one explicit problem on the shared-memory row kernel.
+int rows_run(ChebPlan &pl) {
+    cudaStream_t st = g_ctx.stream;
+    ChebState &cs = *pl.solo;
+    const ChebProblem &p = pl.probs[0];
+    const size_t words = cheb_rows_words(pl.precision, p.N, p.m);
+    if (!cs.xbuf) {
+        if (int rc = dev_alloc(&cs.xbuf, 2 * words)) return rc;
+        CU_TRY(cudaMemsetAsync(cs.xbuf, 0, 2 * words * sizeof(ulonglong2), st));
+    }
+    RowsLaunch L{};
+    L.N = p.N; L.ld = p.ld; L.K = p.K; L.m = p.m; L.P = p.P;
+    L.H = p.H;
+    L.coef = p.coef;
+    L.phi = p.col[pl.parity];
+    L.acc = p.col[pl.parity ^ 1];
+    L.scale = p.scale;
+    L.dcorr = p.dcorr;
+    L.xbuf[0] = cs.xbuf;
+    L.xbuf[1] = cs.xbuf + words;
+    L.tag0 = ++cs.row_launches << 32;
+    L.error = g_ctx.err;
+    L.barrier_ns = g_dbg_barrier_ns;
+    L.exit_cta1 = g_dbg_exit_cta1;
+    g_dbg_exit_cta1 = 0;  // one launch only
+    CU_TRY(cudaMemsetAsync(g_ctx.err, 0, sizeof(int), st));
+    CU_TRY(cudaEventRecord(g_ctx.ev[0], st));
+    CU_TRY(launch_cheb_rows(L, pl.precision, cs.rows, st));
+    CU_TRY(cudaEventRecord(g_ctx.ev[1], st));
+    pl.mg = p.m;  // all columns in one pass
+    return ELHL_OK;
+}
+
 int cheb_run(ChebPlan &pl) {
     cudaStream_t st = g_ctx.stream;
+    if (pl.solo && pl.solo->rows && pl.nphase == 1) return rows_run(pl);
     if (pl.oz) return oz_run(pl);
     if (!pl.tuned) {
         if (int rc = tune_plan(pl, pl.mgcd)) return rc;
@@ -2042,6 +2084,13 @@ int rebuild(elhl_traj *tr, const double *d_coords) {
     CU_TRY(cudaEventRecord(g_ctx.ev[3], g_ctx.stream));
     return rc;
 }
+
+// ELHL_PREC_OZ64 up to this size propagates on the FP64 pipe (cheb_rows.cuh) instead of
+// the tensor cores: an order of oz_cheb_kernel costs at least 7 us of hand-overs
+// (TMA, MMA, flush, partials, barrier) whatever its size.  Moving step, tensor cores /
+// FP64 pipe in ms of propagation: 0.98 / 0.23 at N = 62, 1.22 / 0.61 at 341, 1.89 /
+// 1.49 at 620, 1.92 / 2.04 at 775.
+constexpr int kOzRowsMax = 700;
 
 // Moving nuclei: form H~ = G h G^T every step (1.5 N^3 flops), or apply its three
 // factors in every order (twice the elements, three grid phases per order instead
@@ -2874,6 +2923,11 @@ int elhl_traj_create(const elhl_basis_desc *basis, const double *coords, const e
             int grid = 0;
             tr->cs.oz = new OzRes();
             rc = cheb_grid_size(&grid) ? ELHL_ERR_CUDA : tr->cs.oz->init(tr->N, tr->ld, grid);
+        }
+        if (!rc) {
+            int sms = 0;
+            rc = cheb_grid_size(&sms) ? ELHL_ERR_CUDA : ELHL_OK;
+            if (!oz || tr->N <= kOzRowsMax) tr->cs.rows = cheb_rows_fit(tr->cs.precision, tr->N, tr->cs.m, sms);
         }
         tr->cs.guard = tr->cfg.lanczos_guard;
         if (!rc) rc = dev_alloc(&tr->psi_ao, (size_t)tr->ld * tr->P);

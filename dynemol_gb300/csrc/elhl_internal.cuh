@@ -155,6 +155,32 @@ int cheb_group_size(int precision, int m, int max_ld, bool windowed = false);
 cudaError_t launch_cheb(const ChebLaunch &L, int precision, int mg, cudaStream_t st);
 cudaError_t launch_readout(const ChebLaunch &L, int nprob, int precision, int mg, cudaStream_t st);
 
+// One trajectory of 2 or 4 complex columns on an explicit Hs whose rows fit in the
+// SMs' shared memory (cheb_rows.cuh).  xbuf: two buffers of cheb_rows_words 16-byte
+// words (zero before the first launch); tag0: a value no earlier launch on these
+// buffers used, its low 32 bits zero.
+struct RowsLaunch {
+    int N, ld, K, m, P;
+    const void *H;             // Hs in the launch precision, N columns of ld rows (symmetric)
+    const double2 *coef;       // [K+1]
+    const double2 *phi;        // [ld][m] input columns
+    double2 *acc;              // [ld][m] output columns
+    const double *scale;       // [P] renormalisation factor of the input, or nullptr
+    const float *dcorr;        // FP32: [N] rounding residual of Hs's diagonal, or nullptr
+    ulonglong2 *xbuf[2];
+    unsigned long long tag0;
+    int *error;
+    unsigned long long barrier_ns;  // limit of the waits (0: default)
+    int exit_cta1;                  // test hook: 1 + the CTA that leaves at once (0: none)
+};
+// rows per CTA, or 0 where the kernel does not serve this size
+int cheb_rows_fit(int precision, int N, int m, int sms);
+size_t cheb_rows_words(int precision, int N, int m);
+cudaError_t launch_cheb_rows(const RowsLaunch &L, int precision, int rows, cudaStream_t st);
+cudaError_t launch_cheb_rows_fp64(const RowsLaunch &L, int rows, cudaStream_t st);
+cudaError_t launch_cheb_rows_fp32(const RowsLaunch &L, int rows, cudaStream_t st);
+cudaError_t launch_cheb_rows_df64(const RowsLaunch &L, int rows, cudaStream_t st);
+
 // Split-precision tensor-core GEMM (umma_gemm.cu): sum over s < splits of Y_s
 // (rows x n2, row-major FP32, Y_s = Y + s rows n2) = sum over the BF16 terms
 // (i + j <= 2) of A_i (rows x K, K contiguous, ld lda) times B_j^T (B_j: n2 x K,
