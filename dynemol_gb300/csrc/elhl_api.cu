@@ -875,14 +875,15 @@ __global__ void mirror_lower_kernel(double *A, int n, int ld) {
     if (i < n && j < n && i > j) A[(size_t)i * ld + j] = A[(size_t)j * ld + i];
 }
 
-// H~ = G h G^T with G = L^-1 (lower, zero upper triangle): W = G h, then the
-// lower triangle of W G^T (symmetric result, N^3 + N^3/2 flops), mirrored.
-// tc: products of 320 or more rows on the tensor cores from exact slices.
+// H~ = G h G^T with G = L^-1 (lower triangle): the lower triangle of W = G h, then that
+// of W G^T, mirrored.  H~(i, j), j <= i, sums W(i, l) G(j, l) over l <= j <= i, so W's
+// upper triangle is never needed: 2/3 N^3 + 1/3 N^3 flops.  tc: products of 320 or
+// more rows on the tensor cores from exact slices.
 int form_htilde(ChebState &cs, const double *G, const double *h, int ld, double *W, bool tc) {
     cudaStream_t st = g_ctx.stream;
     const int n = cs.N;
-    CU_TRY(fgemm(tc, n, n, n, 1.0, G, ld, false, h, ld, false, 0.0, W, ld, st, kTriA));
-    CU_TRY(fgemm(tc, n, n, n, 1.0, W, ld, false, G, ld, true, 0.0, cs.Ht, cs.ld, st, kTriBt | kTriLowerC));
+    CU_TRY(fgemm(tc, n, n, n, 1.0, G, ld, false, h, ld, false, 0.0, W, ld, st, kTriA | kTriLowerC));
+    CU_TRY(fgemm(tc, n, n, n, 1.0, W, ld, false, G, ld, true, 0.0, cs.Ht, cs.ld, st, kTriA | kTriBt | kTriLowerC));
     mirror_lower_kernel<<<dim3((n + 127) / 128, n), 128, 0, st>>>(cs.Ht, n, cs.ld);
     count_launch();
     CU_TRY(cudaGetLastError());
