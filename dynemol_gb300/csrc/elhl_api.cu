@@ -2025,6 +2025,11 @@ int upload_basis(DevBasis &d, const elhl_basis_desc *b) {
     rc |= up_i(&d.ao_nzeta, b->ao_nzeta, b->nao);
     rc |= up_d(&d.ao_zeta, b->ao_zeta, 2 * (size_t)b->nao);
     rc |= up_d(&d.ao_coef, b->ao_coef, 2 * (size_t)b->nao);
+    std::vector<double> norm(2 * (size_t)b->nao, 0.0);
+    for (int i = 0; i < b->nao; ++i)
+        for (int z = 0; z < b->ao_nzeta[i]; ++z)
+            norm[2 * i + z] = b->ao_coef[2 * i + z] * sto_norm(b->ao_zeta[2 * i + z], b->ao_n[i], b->ao_l[i]);
+    rc |= up_d(&d.ao_norm, norm.data(), norm.size());
     rc |= up_d(&d.ao_ip, b->ao_ip, b->nao);
     rc |= up_d(&d.ao_kwh, b->ao_kwh, b->nao);
     rc |= up_d(&d.ao_vshift, b->ao_vshift, b->nao);
@@ -2052,7 +2057,7 @@ int upload_basis(DevBasis &d, const elhl_basis_desc *b) {
 
 void free_basis(DevBasis &d) {
     dev_free(d.atom_ao0); dev_free(d.atom_nao); dev_free(d.ao_n); dev_free(d.ao_l); dev_free(d.ao_m);
-    dev_free(d.ao_nzeta); dev_free(d.ao_zeta); dev_free(d.ao_coef); dev_free(d.ao_ip); dev_free(d.ao_kwh);
+    dev_free(d.ao_nzeta); dev_free(d.ao_zeta); dev_free(d.ao_coef); dev_free(d.ao_norm); dev_free(d.ao_ip); dev_free(d.ao_kwh);
     dev_free(d.ao_vshift); dev_free(d.ao_frag); dev_free(d.atom_order);
 }
 

@@ -26,12 +26,15 @@ struct DevBasis {
     int natoms = 0, nao = 0, nfrag = 0;
     int *atom_ao0 = nullptr, *atom_nao = nullptr;
     int *ao_n = nullptr, *ao_l = nullptr, *ao_m = nullptr, *ao_nzeta = nullptr, *ao_frag = nullptr;
+    double *ao_norm = nullptr;  // [nao][2] coefficient times normalisation of each exponent (sto_norm)
     double *ao_zeta = nullptr, *ao_coef = nullptr, *ao_ip = nullptr, *ao_kwh = nullptr, *ao_vshift = nullptr;
     int *atom_order = nullptr;  // atoms grouped by kind (same AO signature): the S/h build's pair order
 };
 
 // One-time per-device fill of the overlap kernel's constant tables.
 cudaError_t init_build_tables();
+// normalisation of an AO's exponent (host)
+double sto_norm(double zeta, int n, int l);
 
 // S and h (both N x N, column-major, leading dimension ld) from coordinates.
 // Hueckel Hamiltonian with environment fields (h zeroed by the caller)
