@@ -26,7 +26,7 @@
 
 #include "df64.cuh"
 #include "elhl_internal.cuh"
-#include "grid_sync.cuh"
+#include "exchange.cuh"
 
 namespace elhl {
 namespace rows {
@@ -34,21 +34,6 @@ namespace rows {
 constexpr int kThreads = 256, kWarps = kThreads / 32;
 constexpr int kBatch = 8;                      // words in flight per lane
 constexpr size_t kSmemLimit = 220 * 1024;
-
-// a published element: its 8 bytes and its tag, one 128-bit word
-__device__ __forceinline__ void publish(ulonglong2 *p, unsigned long long value, unsigned long long tag) {
-    asm volatile(
-        "{\n.reg .b128 w;\nmov.b128 w, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], w;\n}" ::"l"(p), "l"(value), "l"(tag)
-        : "memory");
-}
-__device__ __forceinline__ ulonglong2 fetch(const ulonglong2 *p) {
-    ulonglong2 v;
-    asm volatile("{\n.reg .b128 w;\nld.relaxed.gpu.global.b128 w, [%2];\nmov.b128 {%0, %1}, w;\n}"
-                 : "=l"(v.x), "=l"(v.y)
-                 : "l"(p)
-                 : "memory");
-    return v;
-}
 
 // ---- arithmetics -------------------------------------------------------------
 // Word: what a word carries; C words per column j (components, or complex columns
@@ -259,29 +244,8 @@ __global__ void __launch_bounds__(kThreads, 1) cheb_rows_kernel(const RowsLaunch
                 if (e < N * C) w[u] = fetch(src + e);
             }
         };
-        // The warp polls as one (votes, no lane leaves the loop alone): the block barrier
-        // below counts whole warps.
         auto use = [&](int g, ulonglong2 (&w)[kBatch]) {
-            unsigned long long t0 = 0;
-            for (unsigned polls = 1;; ++polls) {
-                bool miss = false;
-#pragma unroll
-                for (int u = 0; u < kBatch; ++u) miss |= w[u].y != want;
-                if (!__any_sync(0xffffffffu, miss)) break;
-                if ((polls & 63u) == 0) {
-                    const unsigned long long t = globaltimer_ns();
-                    if (!t0) t0 = t;
-                    const bool late = t - t0 > limit;
-                    if (late) atomicExch(L.error, ELHL_ERR_TIMEOUT);
-                    if (__any_sync(0xffffffffu, late || *(volatile int *)L.error)) {
-                        s_abort = 1;
-                        break;
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kBatch; ++u)
-                    if (w[u].y != want) w[u] = fetch(src + (g + u * kWarps) * 32 + lane);
-            }
+            if (!await_words(w, want, src + g * 32 + lane, kWarps * 32, L.error, limit)) s_abort = 1;
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
                 const int gu = g + u * kWarps;

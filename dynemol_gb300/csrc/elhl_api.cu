@@ -818,6 +818,7 @@ struct ChebState {
         CU_TRY(cudaMemset(acc, 0, (size_t)ld * m * sizeof(double2)));
         // 6 Lanczos vectors, per-CTA partial sums, the tridiagonal record
         if (int rc = dev_alloc(&lz, (size_t)6 * ld + kLzPart + 128)) return rc;
+        CU_TRY(cudaMemset(lz, 0, (size_t)4 * ld * sizeof(double)));  // exchanged words: no tag
         if (int rc = dev_alloc(&cscratch, (size_t)2 * m * ld)) return rc;
         if (int rc = dev_alloc(&scale, (size_t)kMaxCols)) return rc;
         if (int rc = dev_alloc(&drift, 1)) return rc;

@@ -1,10 +1,12 @@
 // Spectral bounds of the Chebyshev operator by Lanczos, in FP64 on the FP64
 // pipe, all k steps in one cooperative launch (no host round trip, no library
 // GEMV).  The operator is
-//   explicit: H~ (symmetric, both triangles stored), w = H~ q;
+//   explicit: H~ (symmetric, both triangles stored), w = H~ q:
+//             lanczos_rows_kernel (below), while its rows fit in shared memory;
 //   implicit: H~ = G h G^T with G = L^-1 lower triangular and its transpose
-//             Gt stored, w = G (h (G^T q)) in three column-dot phases.
-// Every product is a set of column dot products M(:, i) . x (columns are
+//             Gt stored, w = G (h (G^T q)) in three column-dot phases:
+//             lanczos64_kernel, which also takes the explicit operator of larger bases.
+// In lanczos64_kernel every product is a set of column dot products M(:, i) . x (columns are
 // contiguous in the column-major storage, so the reads coalesce): CTA c takes
 // the columns i = c, c + grid, ..., one warp per column, so that every SM
 // reads the same share of the matrix; x sits in shared memory when it fits.
@@ -17,6 +19,7 @@
 #include <algorithm>
 
 #include "elhl_internal.cuh"
+#include "exchange.cuh"
 #include "grid_sync.cuh"
 
 namespace elhl {
@@ -199,6 +202,172 @@ __global__ void __launch_bounds__(kLzThreads) lanczos64_kernel(const LzArgs a) {
     }
 }
 
+// ---- explicit operator, every CTA with the whole vectors -----------------------
+// One hand-over per step instead of two grid barriers: each CTA forms w = H~ q for
+// its rows and publishes them (exchange.cuh); every CTA then reads all of w and
+// carries q_j and q_{j-1} and the scalars itself, by the same operations in the same
+// order, so that all agree to the bit.  p = w - beta_{j-1} q_{j-1}, alpha = p . q and
+// beta^2 = |p|^2 - alpha^2 from one pass over p (a second pass sums |p - alpha q|^2
+// where that difference would cancel).  Bound: the FP64 unit for the products above
+// about N = 700, latency below.  Twenty steps: N = 62 217 -> 75 us, N = 744 272 -> 174,
+// N = 932 275 -> 193, N = 1860 379 -> 300.
+constexpr int kLrThreads = 256, kLrWarps = kLrThreads / 32, kLrBatch = 4;
+constexpr size_t kLrSmem = 220 * 1024;
+
+struct LrArgs {
+    int n, ld, k;
+    const double *H;
+    ulonglong2 *x;            // [2][n] exchanged words
+    unsigned long long tag0;  // a value no earlier launch used, its low 32 bits zero
+    double *rec;              // alpha [k], beta [k], steps used [1]
+    int *err;
+};
+
+__global__ void __launch_bounds__(kLrThreads, 1) lanczos_rows_kernel(const LrArgs a) {
+    extern __shared__ double dyn[];
+    __shared__ double s_red[2][kLrWarps], s_sc[4];
+    __shared__ int s_abort;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int n = a.n, rows = (n + gridDim.x - 1) / gridDim.x;
+    const int r0 = min(n, (int)blockIdx.x * rows), nrow = min(n, r0 + rows) - r0;
+    double *q = dyn, *p = dyn + n;        // q_j; q_{j-1}, overwritten by p and then by q_{j+1}
+    double *sh = dyn + 2 * (size_t)n;
+    if (tid == 0) s_abort = 0;
+    for (int r = 0; r < nrow; ++r)
+        for (int j = tid; j < n; j += kLrThreads) sh[(size_t)r * n + j] = a.H[(size_t)(r0 + r) * a.ld + j];
+    // the start vector (every component present), published like a product
+    for (int r = tid; r < nrow; r += kLrThreads)
+        publish(a.x + r0 + r, (unsigned long long)__double_as_longlong(1.0 + 0.5 * sin(1.37 * (r0 + r) + 0.2)), a.tag0);
+    for (int i = tid; i < 2 * n; i += kLrThreads) dyn[i] = 0.0;
+    __syncthreads();
+    double beta = 0.0;
+    for (int j = -1; j < a.k; ++j) {
+        const unsigned long long tag = a.tag0 + (unsigned long long)(j + 1);
+        ulonglong2 *x = a.x + (size_t)((j + 1) & 1) * n;
+        if (j >= 0) {
+            for (int r = warp; r < nrow; r += kLrWarps) {
+                const double *h = sh + (size_t)r * n;
+                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+                int l = lane;
+                for (; l + 96 < n; l += 128) {
+                    s0 = fma(h[l], q[l], s0);
+                    s1 = fma(h[l + 32], q[l + 32], s1);
+                    s2 = fma(h[l + 64], q[l + 64], s2);
+                    s3 = fma(h[l + 96], q[l + 96], s3);
+                }
+                for (; l < n; l += 32) s0 = fma(h[l], q[l], s0);
+                double s = (s0 + s1) + (s2 + s3);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) publish(x + r0 + r, (unsigned long long)__double_as_longlong(s), tag);
+            }
+        }
+        // all of w: p = w - beta q_{j-1}; sums p . q (j >= 0) and |p|^2
+        double pq = 0.0, pp = 0.0;
+        for (int i0 = warp * 32; i0 < n; i0 += kLrBatch * kLrThreads) {
+            ulonglong2 w[kLrBatch];
+#pragma unroll
+            for (int u = 0; u < kLrBatch; ++u) {
+                const int i = i0 + u * kLrThreads + lane;
+                w[u] = make_ulonglong2(0ull, tag);
+                if (i < n) w[u] = fetch(x + i);
+            }
+            if (!await_words(w, tag, x + i0 + lane, kLrThreads, a.err, kBarrierNs)) s_abort = 1;
+#pragma unroll
+            for (int u = 0; u < kLrBatch; ++u) {
+                const int i = i0 + u * kLrThreads + lane;
+                if (i0 + u * kLrThreads >= n) break;  // the same for the warp
+                if (i < n) {
+                    const double v = fma(-beta, p[i], __longlong_as_double((long long)w[u].x));
+                    p[i] = v;
+                    pq = fma(v, q[i], pq);
+                    pp = fma(v, v, pp);
+                }
+            }
+        }
+        // lanes 0-15 sum p . q, lanes 16-31 |p|^2; then the eight warps' sums in warp order
+        auto block_sums = [&](double x0, double x1) {
+            const bool upper = lane & 16;
+            double v = upper ? x1 : x0;
+            v += __shfl_xor_sync(0xffffffffu, upper ? x0 : x1, 16);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if ((lane & 15) == 0) s_red[lane >> 4][warp] = v;
+            __syncthreads();
+        };
+        block_sums(pq, pp);
+        if (s_abort) return;
+        if (warp == 0) {
+            double v = s_red[lane >> 4][lane & 7];
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            const double alpha = __shfl_sync(0xffffffffu, v, 0), p2 = __shfl_sync(0xffffffffu, v, 16);
+            if (lane == 0) {
+                const double b2 = p2 - alpha * alpha, ib = rsqrt(b2);
+                s_sc[0] = alpha;
+                s_sc[1] = b2 > 1.0e-6 * p2 ? 1.0 : 0.0;  // else |p - alpha q|^2 is summed
+                s_sc[2] = b2 * ib;
+                s_sc[3] = ib;
+            }
+        }
+        __syncthreads();
+        const double alpha = s_sc[0];
+        if (s_sc[1] == 0.0) {
+            double rr = 0.0;
+            for (int i = tid; i < n; i += kLrThreads) {
+                const double v = p[i] - alpha * q[i];
+                rr = fma(v, v, rr);
+            }
+            block_sums(rr, 0.0);
+            if (warp == 0) {
+                double v = s_red[0][lane & 7];
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 0) {
+                    s_sc[2] = sqrt(v);
+                    s_sc[3] = 1.0 / s_sc[2];
+                }
+            }
+            __syncthreads();
+        }
+        const double ib = s_sc[3];
+        beta = s_sc[2];
+        if (j >= 0) {
+            const bool stop = !(beta > 1e-10 * (fabs(alpha) + 1.0));  // invariant subspace found
+            if (blockIdx.x == 0 && tid == 0) {
+                a.rec[j] = alpha;
+                a.rec[a.k + j] = beta;
+                if (stop) a.rec[2 * a.k] = j + 1;
+            }
+            if (stop) return;
+        }
+        // q_{j+1} = (p - alpha q_j) / beta (the start vector: j = -1, q = 0); roles swap
+        for (int i = tid; i < n; i += kLrThreads) p[i] = (p[i] - alpha * q[i]) * ib;
+        double *t = q;
+        q = p;
+        p = t;
+        if (j < 0) beta = 0.0;
+        __syncthreads();
+    }
+}
+
+// shared memory of a CTA: its rows of H~ and the two vectors
+size_t rows_smem(int n, int sms) { return (size_t)(2 + (n + sms - 1) / sms) * n * sizeof(double); }
+
+cudaError_t launch_rows(int n, int ld, int k, const double *H, double *x, double *rec, int *err, int sms,
+                        cudaStream_t st) {
+    static unsigned long long launches = 0;  // under the library's lock
+    const int rows = (n + sms - 1) / sms, grid = (n + rows - 1) / rows;
+    const size_t smem = rows_smem(n, sms);
+    cudaError_t e = cudaFuncSetAttribute(lanczos_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    LrArgs a{n, ld, k, H, reinterpret_cast<ulonglong2 *>(x), ++launches << 32, rec, err};
+    void *args[] = {&a};
+    e = cudaLaunchCooperativeKernel((const void *)lanczos_rows_kernel, dim3(grid), dim3(kLrThreads), args, smem, st);
+    count_launch();
+    return e;
+}
+
 }  // namespace
 
 cudaError_t launch_lanczos64(int n, int ld, int k, const double *H, const double *G, const double *Gt, double *r,
@@ -217,6 +386,11 @@ cudaError_t launch_lanczos64(int n, int ld, int k, const double *H, const double
         if (per < 1) return cudaErrorInvalidConfiguration;
         grid = sms;
     }
+    // explicit operator while its rows fit (N up to about 1,900; read from L2 by eight warps
+    // a step at N = 3720 takes 57 us against lanczos64_kernel's 43): the words' [2][n] x 16
+    // bytes lie in r's 4 x ld doubles
+    if (!G && n >= 1 && k >= 1 && rows_smem(n, grid) <= kLrSmem)
+        return launch_rows(n, ld, k, H, r, rec, err, grid, st);
     const size_t smem = (size_t)(std::min(n, kXsCap) + kRedSlots) * sizeof(double);
     if (grid > part_cap || k < 1 || n < 1 || (G && !Gt)) return cudaErrorInvalidValue;
     LzArgs a{n, ld, k, H, G, Gt, r, t, part, rec, bar, err};
