@@ -176,15 +176,6 @@ __device__ void rows_gemv(const T *M, int ld, const typename Vec2<T>::type *s_v,
     }
 }
 
-// (a + b) + c rounded once for |c| far below ulp(a + b): TwoSum gives a + b = t + e
-// exactly, then t + (e + c)
-__device__ __forceinline__ float two_sum_plus(float a, float b, float c) {
-    const float t = __fadd_rn(a, b);
-    const float z = __fsub_rn(t, a);
-    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(b, z));
-    return __fadd_rn(t, __fadd_rn(e, c));
-}
-
 // epilogue of one order: recurrence + FP64 accumulation of c_k v_k
 template <typename T, int MG>
 struct OrderEpi {

@@ -84,15 +84,6 @@ __device__ __forceinline__ unsigned long long pack2(float x, float y) {
     return (unsigned long long)__float_as_uint(x) | ((unsigned long long)__float_as_uint(y) << 32);
 }
 
-// (a + b) + c rounded once for |c| far below ulp(a + b): TwoSum gives a + b = t + e
-// exactly, then t + (e + c)
-__device__ __forceinline__ float two_sum_plus(float a, float b, float c) {
-    const float t = __fadd_rn(a, b);
-    const float z = __fsub_rn(t, a);
-    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(b, z));
-    return __fadd_rn(t, __fadd_rn(e, c));
-}
-
 // One output word (row, component or complex column) of a CTA: the recurrence
 // state, held by the four lanes that sum its partials.
 template <typename A> struct Out;

@@ -37,4 +37,13 @@ __device__ __forceinline__ void df_add(float &ah, float &al, float bh, float bl)
     ah = t;
 }
 
+// (a + b) + c rounded once for |c| far below ulp(a + b): TwoSum gives a + b = t + e
+// exactly, then t + (e + c)
+__device__ __forceinline__ float two_sum_plus(float a, float b, float c) {
+    const float t = __fadd_rn(a, b);
+    const float z = __fsub_rn(t, a);
+    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(b, z));
+    return __fadd_rn(t, __fadd_rn(e, c));
+}
+
 }  // namespace elhl

@@ -20,6 +20,7 @@
 #include <tuple>
 #include <vector>
 
+#include "df64.cuh"
 #include "elhl_internal.cuh"
 
 using namespace elhl;
@@ -1227,29 +1228,35 @@ __global__ void gemm_order0_kernel(const double2 *__restrict__ phi, const double
     acc[q] = make_double2(c0.x * p.x - c0.y * p.y, c0.x * p.y + c0.y * p.x);
 }
 
-// y = sum of the nsplit partial products (FP64, fixed order), v_k = 2 y - v_{k-2}
-// (v_1 = y) rounded to FP32, acc += c_k v_k in FP64
-__global__ void gemm_epilogue_kernel(const float2 *__restrict__ Y, int nsplit, size_t split_stride,
-                                     const float2 *__restrict__ vprev2, float2 *__restrict__ vout,
-                                     double2 *__restrict__ acc, const double2 *coef, int k, int nm) {
+// y = sum of the nsplit partial products (fixed order, as an FP32 pair: TwoSum, so
+// exact to 2^-48), v_k = 2 y - v_{k-2} (v_1 = y) rounded once to FP32, acc += c_k v_k
+// in FP64.  The sums in FP64 bound this kernel by the FP64 unit (32 of its 40 FP64
+// instructions per element at 16 splits): 30 us per order at N = 4092, 64 columns,
+// 8 us on the FP32 pipes.
+__global__ void __launch_bounds__(256) gemm_epilogue_kernel(const float2 *__restrict__ Y, int nsplit,
+                                                            size_t split_stride, const float2 *__restrict__ vprev2,
+                                                            float2 *__restrict__ vout, double2 *__restrict__ acc,
+                                                            const double2 *coef, int k, int nm) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nm) return;
-    double yx = 0.0, yy = 0.0;
-    for (int s = 0; s < nsplit; ++s) {
+    double2 a = acc[q];
+    const float2 w = k == 1 ? make_float2(0.f, 0.f) : vprev2[q];
+    float2 h = Y[q], l = make_float2(0.f, 0.f);
+#pragma unroll 8
+    for (int s = 1; s < nsplit; ++s) {
         const float2 t = Y[s * split_stride + q];
-        yx += (double)t.x;
-        yy += (double)t.y;
+        df_add(h.x, l.x, t.x, 0.f);
+        df_add(h.y, l.y, t.y, 0.f);
     }
     float2 v;
     if (k == 1) {
-        v = make_float2((float)yx, (float)yy);
+        v = make_float2(__fadd_rn(h.x, l.x), __fadd_rn(h.y, l.y));
     } else {
-        const float2 w = vprev2[q];
-        v = make_float2((float)(2.0 * yx - (double)w.x), (float)(2.0 * yy - (double)w.y));
+        v.x = two_sum_plus(__fmul_rn(2.f, h.x), -w.x, __fmul_rn(2.f, l.x));
+        v.y = two_sum_plus(__fmul_rn(2.f, h.y), -w.y, __fmul_rn(2.f, l.y));
     }
     vout[q] = v;
     const double2 c = coef[k];
-    double2 a = acc[q];
     a.x += c.x * (double)v.x - c.y * (double)v.y;
     a.y += c.x * (double)v.y + c.y * (double)v.x;
     acc[q] = a;
@@ -2057,7 +2064,8 @@ struct elhl_traj {
     // Chebyshev method: AO-basis Psi_ket / Psi_bra as [ld][2] (row i, particle p)
     ChebState cs;
     ChebPlan plan;
-    double2 *psi_ao = nullptr, *bra_ao = nullptr, *ro_ket = nullptr, *ro_bra = nullptr;
+    double2 *psi_ao = nullptr, *bra_ao = nullptr;
+    double2 *psi_cols = nullptr;  // [2][P][N] their columns, for reading back (allocated on first use)
     double *target = nullptr;  // per-particle total population to hold (reduced precision)
     bool cheb() const { return cfg.method == ELHL_METHOD_CHEBYSHEV; }
 };
@@ -2684,6 +2692,47 @@ int FragmentOrbitals::solve(elhl_traj *tr, int nat, const int *atoms) {
 
 int cheb_set_target(elhl_traj *tr);
 
+// [N][P] rows -> column-major N x P, 32 x 32 tiles (P on x) through shared memory
+__global__ void __launch_bounds__(256) columns_kernel(const double2 *__restrict__ src, double2 *__restrict__ dst, int n,
+                                                      int P) {
+    __shared__ double2 t[32][33];
+    const int p0 = blockIdx.y * 32, i0 = blockIdx.x * 32;
+    for (int q = threadIdx.x; q < 1024; q += 256) {
+        const int i = i0 + q / 32, p = p0 + q % 32;
+        if (i < n && p < P) t[q / 32][q % 32] = src[(size_t)i * P + p];
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < 1024; q += 256) {
+        const int p = p0 + q / 32, i = i0 + q % 32;
+        if (i < n && p < P) dst[(size_t)p * n + i] = t[q % 32][q / 32];
+    }
+}
+
+// Psi as host columns.  The AO arrays hold the particles side by side ([ld][P]); they
+// are transposed on the device and copied whole: a strided copy of 16-byte elements
+// per particle and state took 18 us each (64 columns: 2.3 ms).
+int cheb_psi_columns(elhl_traj *tr, elhl_zcomplex *bra, elhl_zcomplex *ket) {
+    cudaStream_t st = g_ctx.stream;
+    const int P = tr->P, n = tr->N;
+    const size_t len = (size_t)n * P;
+    if (!tr->psi_cols)
+        if (int rc = dev_alloc(&tr->psi_cols, 2 * len)) return rc;
+    const dim3 grid((n + 31) / 32, (P + 31) / 32);
+    if (ket) {
+        columns_kernel<<<grid, 256, 0, st>>>(tr->psi_ao, tr->psi_cols, n, P);
+        count_launch();
+        CU_TRY(cudaMemcpyAsync(ket, tr->psi_cols, len * sizeof(double2), cudaMemcpyDeviceToHost, st));
+    }
+    if (bra) {
+        columns_kernel<<<grid, 256, 0, st>>>(tr->bra_ao, tr->psi_cols + len, n, P);
+        count_launch();
+        CU_TRY(cudaMemcpyAsync(bra, tr->psi_cols + len, len * sizeof(double2), cudaMemcpyDeviceToHost, st));
+    }
+    CU_TRY(cudaGetLastError());
+    CU_TRY(cudaStreamSynchronize(st));
+    return ELHL_OK;
+}
+
 // Psi (host, column-major N x P) into the [ld][P] AO arrays; bra = S ket when
 // bra is NULL.  The norm target of each particle is its initial total population.
 int cheb_set_psi(elhl_traj *tr, const elhl_zcomplex *bra, const elhl_zcomplex *ket) {
@@ -3061,7 +3110,7 @@ int elhl_traj_destroy(elhl_traj *tr) {
     tr->tb.release();
     tr->cs.release();
     tr->plan.release();
-    dev_free(tr->psi_ao); dev_free(tr->bra_ao); dev_free(tr->target);
+    dev_free(tr->psi_ao); dev_free(tr->bra_ao); dev_free(tr->psi_cols); dev_free(tr->target);
     delete tr;
     return ELHL_OK;
 }
@@ -3162,15 +3211,8 @@ int elhl_traj_set_psi(elhl_traj *tr, const elhl_zcomplex *bra, const elhl_zcompl
 int elhl_traj_get_psi(elhl_traj *tr, elhl_zcomplex *bra, elhl_zcomplex *ket) {
     if (!tr) return ELHL_ERR_BAD_ARG;
     std::lock_guard<std::mutex> lk(g_ctx.mu);
+    if (tr->cheb()) return cheb_psi_columns(tr, bra, ket);
     CU_TRY(cudaStreamSynchronize(g_ctx.stream));
-    if (tr->cheb()) {
-        const size_t e = sizeof(double2);
-        for (int p = 0; p < tr->P; ++p) {
-            if (ket) CU_TRY(cudaMemcpy2D(ket + (size_t)p * tr->N, e, tr->psi_ao + p, tr->P * e, e, tr->N, cudaMemcpyDeviceToHost));
-            if (bra) CU_TRY(cudaMemcpy2D(bra + (size_t)p * tr->N, e, tr->bra_ao + p, tr->P * e, e, tr->N, cudaMemcpyDeviceToHost));
-        }
-        return ELHL_OK;
-    }
     for (int p = 0; p < tr->P; ++p) {
         if (bra) CU_TRY(copy_d2h(bra + (size_t)p * tr->N, tr->tb.bra(p), tr->N * sizeof(double2)));
         if (ket) CU_TRY(copy_d2h(ket + (size_t)p * tr->N, tr->tb.ket(p), tr->N * sizeof(double2)));
@@ -3274,15 +3316,14 @@ int traj_psi_host(elhl_traj *tr, std::vector<double2> &bra, std::vector<double2>
     bra.resize((size_t)N * P);
     ket.resize((size_t)N * P);
     const size_t e = sizeof(double2);
+    static_assert(sizeof(elhl_zcomplex) == sizeof(double2), "complex layout");
+    if (tr->cheb())
+        return cheb_psi_columns(tr, reinterpret_cast<elhl_zcomplex *>(bra.data()),
+                                reinterpret_cast<elhl_zcomplex *>(ket.data()));
     CU_TRY(cudaStreamSynchronize(g_ctx.stream));
     for (int p = 0; p < P; ++p) {
-        if (tr->cheb()) {
-            CU_TRY(cudaMemcpy2D(ket.data() + (size_t)p * N, e, tr->psi_ao + p, P * e, e, N, cudaMemcpyDeviceToHost));
-            CU_TRY(cudaMemcpy2D(bra.data() + (size_t)p * N, e, tr->bra_ao + p, P * e, e, N, cudaMemcpyDeviceToHost));
-        } else {
-            CU_TRY(cudaMemcpy(bra.data() + (size_t)p * N, tr->tb.bra(p), N * e, cudaMemcpyDeviceToHost));
-            CU_TRY(cudaMemcpy(ket.data() + (size_t)p * N, tr->tb.ket(p), N * e, cudaMemcpyDeviceToHost));
-        }
+        CU_TRY(cudaMemcpy(bra.data() + (size_t)p * N, tr->tb.bra(p), N * e, cudaMemcpyDeviceToHost));
+        CU_TRY(cudaMemcpy(ket.data() + (size_t)p * N, tr->tb.ket(p), N * e, cudaMemcpyDeviceToHost));
     }
     return ELHL_OK;
 }
@@ -3889,10 +3930,8 @@ int elhl_server_step(elhl_server *sv, int *n_active, int *n_pending) {
                 const double *src = r->group < 0 ? r->tr->cs.gpops : sv->groups[r->group].pops + r->pops_off;
                 CU_TRY(copy_d2h(r->pops.data(), src, np * sizeof(double)));
                 r->psi.resize((size_t)r->nao * r->P);
-                const size_t e = sizeof(double2);
-                for (int p = 0; p < r->P; ++p)
-                    CU_TRY(cudaMemcpy2D(r->psi.data() + (size_t)p * r->nao, e, r->tr->psi_ao + p, r->P * e, e, r->nao,
-                                        cudaMemcpyDeviceToHost));
+                if (int rc = cheb_psi_columns(r->tr, nullptr, reinterpret_cast<elhl_zcomplex *>(r->psi.data())))
+                    return rc;
                 r->t_done = now_s();
                 sv->used -= r->bytes;
                 if (r->group >= 0) {
