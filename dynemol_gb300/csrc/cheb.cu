@@ -535,6 +535,146 @@ __global__ void reduce_pops_kernel(ChebLaunch L, int nprob) {
     }
 }
 
+// Read-out of one trajectory of P particles with FP64 read-out matrices, with the
+// norm control and the populations in the same launch (readout_kernel, the norm
+// kernels and reduce_pops_kernel in one).  One warp per row i: psi_i = sum_{j >= i}
+// A(j, i) phi_j and bra_i = sum_{j <= i} B(j, i) chi_j read N + 1 elements together, so
+// every row costs the same.  Each block leaves its rows' terms of the K sums (squared
+// norms of the input and output columns, totals, populations); the last block sums
+// the blocks' terms in block order.  At N = 450 the separate launches took 27 + 22 +
+// 5.5 us per step (FP64 butterflies of all accumulators over all lanes; 152 segment
+// sums in one thread); this one takes 9.
+constexpr int kRoRows = 8;  // rows (warps) per block
+
+template <int P>
+__global__ void __launch_bounds__(32 * kRoRows) readout_rows_kernel(const ChebProblem *__restrict__ probs, int parity,
+                                                                    double *__restrict__ part,
+                                                                    unsigned *__restrict__ count,
+                                                                    double *__restrict__ pops) {
+    constexpr int V = 4 * P;  // re and im of psi, then of bra
+    constexpr int kMaxVals = 2 * 4 + P + P * (kMaxFrag + 1);
+    __shared__ double s_v[kRoRows][V];
+    __shared__ double s_tot[kMaxVals];
+    __shared__ unsigned s_last;
+    const ChebProblem &pb = probs[0];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int N = pb.N, ld = pb.ld, m = pb.m, nf = min(pb.nfrag, kMaxFrag);
+    const int r0 = blockIdx.x * kRoRows, i = r0 + warp, bcol = m == 2 * P ? P : 0;
+    const double2 *in = pb.col[parity], *out = pb.col[parity ^ 1];
+    double v[V];
+#pragma unroll
+    for (int q = 0; q < V; ++q) v[q] = 0.0;
+    if (i < N) {
+        const double *a = static_cast<const double *>(pb.A) + (size_t)i * ld, *b = static_cast<const double *>(pb.B) + (size_t)i * ld;
+#pragma unroll 4
+        for (int j = i + lane; j < N; j += 32) {
+            const double h = a[j];
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                const double2 x = out[(size_t)j * m + p];
+                v[2 * p] = fma(h, x.x, v[2 * p]);
+                v[2 * p + 1] = fma(h, x.y, v[2 * p + 1]);
+            }
+        }
+#pragma unroll 4
+        for (int j = lane; j <= i; j += 32) {
+            const double h = b[j];
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                const double2 x = out[(size_t)j * m + bcol + p];
+                v[2 * (P + p)] = fma(h, x.x, v[2 * (P + p)]);
+                v[2 * (P + p) + 1] = fma(h, x.y, v[2 * (P + p) + 1]);
+            }
+        }
+    }
+    // lane sums: each lane bit from the top halves the values a lane holds, then plain sums
+    int idx = 0;
+#pragma unroll
+    for (int o = 16, n = V; o > 0; o >>= 1) {
+        if (n > 1) {
+            n /= 2;
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int q = 0; q < V / 2; ++q)
+                if (q < n) {
+                    const double send = upper ? v[q] : v[q + n], keep = upper ? v[q + n] : v[q];
+                    v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            if (upper) idx += n;
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    if ((lane & (32 / V - 1)) == 0) {
+        s_v[warp][idx] = v[0];
+        if (i < N)
+            reinterpret_cast<double *>(idx < 2 * P ? pb.psi : pb.bra)[(size_t)i * 2 * P + (idx < 2 * P ? idx : idx - 2 * P)] =
+                v[0];
+    }
+    __syncthreads();
+    // the block's terms, eight lanes (rows) per value: in and out norms of the m columns,
+    // P totals, P x (nf + 1) populations
+    const int vals = 2 * m + P + P * (nf + 1);
+    for (int t0 = 0; t0 < vals * kRoRows; t0 += 32 * kRoRows) {
+        const int t = t0 + tid, val = t / kRoRows, row = t % kRoRows, r = r0 + row;
+        double x = 0.0;
+        if (val < vals && r < N) {
+            if (val < 2 * m) {
+                const double2 c = (val < m ? in : out)[(size_t)r * m + val % m];
+                x = c.x * c.x + c.y * c.y;
+            } else if (val < 2 * m + P) {
+                const int p = val - 2 * m;
+                const double2 c = out[(size_t)r * m + p], d = m == 2 * P ? out[(size_t)r * m + P + p] : c;
+                x = c.x * d.x + c.y * d.y;
+            } else {
+                const int p = (val - 2 * m - P) / (nf + 1), f = (val - 2 * m - P) % (nf + 1);
+                if (f == nf || (pb.ao_frag && pb.ao_frag[r] == f))
+                    x = s_v[row][2 * p] * s_v[row][2 * (P + p)] + s_v[row][2 * p + 1] * s_v[row][2 * (P + p) + 1];
+            }
+        }
+#pragma unroll
+        for (int o = kRoRows / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (val < vals && row == 0) part[(size_t)blockIdx.x * vals + val] = x;
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(count, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int val = warp; val < vals; val += kRoRows) {
+        double x = 0.0;
+        for (int b = lane; b < (int)gridDim.x; b += 32) x += __ldcg(part + (size_t)b * vals + val);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) s_tot[val] = x;
+    }
+    if (tid == 0) *count = 0u;  // for the next launch
+    __syncthreads();
+    if (tid < m && pb.drift) {  // norm control, as norm_drift_kernel
+        const double s = pb.scale ? pb.scale[tid % P] : 1.0;
+        const double nin = s_tot[tid] * (s * s), nout = s_tot[m + tid];
+        double d = nin > 0.0 ? fabs(nout / nin - 1.0) : (nout > 0.0 ? 1.0e300 : 0.0);
+        if (!(d <= 1.0e300)) d = 1.0e300;
+        atomicMax(reinterpret_cast<unsigned long long *>(pb.drift), (unsigned long long)__double_as_longlong(d));
+    }
+    __shared__ double s_f[P];  // population factor of the renormalised state, as reduce_pops_kernel
+    __syncthreads();           // pb.scale has been read
+    if (tid < P) {
+        const double tot = pb.ntot ? s_tot[2 * m + tid] : s_tot[2 * m + P + tid * (nf + 1) + nf];
+        const double tgt = pb.target ? pb.target[tid] : 0.0;
+        const bool rn = pb.scale_out && tot > 0.0 && tgt > 0.0;
+        if (pb.ntot) pb.ntot[tid] = tot;
+        if (pb.scale_out) pb.scale_out[tid] = rn ? sqrt(tgt / tot) : 1.0;
+        s_f[tid] = rn ? tgt / tot : 1.0;
+    }
+    __syncthreads();
+    for (int t = tid; pops && t < P * (nf + 1); t += 32 * kRoRows) {
+        const int p = t / (nf + 1), f = t % (nf + 1);
+        pops[pb.pops_off + p * (pb.nfrag + 1) + (f == nf ? pb.nfrag : f)] = s_tot[2 * m + P + t] * s_f[p];
+    }
+}
+
 // ============================ double-float (DF64) ================================
 // GB300's FP64 pipe runs at 1/58 of its FP32 rate.  ELHL_PREC_DF64 keeps the
 // operator and the series vectors as unevaluated sums hi + lo of two FP32
@@ -892,6 +1032,18 @@ cudaError_t launch_readout(const ChebLaunch &L, int nprob, int precision, int mg
         }
     }
     return cudaErrorInvalidValue;
+}
+
+// scratch: at least 6 N doubles; count: zero before the first launch
+cudaError_t launch_readout_rows(const ChebProblem *probs, int N, int P, int parity, double *scratch, unsigned *count,
+                                double *pops, cudaStream_t st) {
+    const int grid = (N + kRoRows - 1) / kRoRows;
+    if (P == 1) readout_rows_kernel<1><<<grid, 32 * kRoRows, 0, st>>>(probs, parity, scratch, count, pops);
+    else if (P == 2) readout_rows_kernel<2><<<grid, 32 * kRoRows, 0, st>>>(probs, parity, scratch, count, pops);
+    else if (P == 4) readout_rows_kernel<4><<<grid, 32 * kRoRows, 0, st>>>(probs, parity, scratch, count, pops);
+    else return cudaErrorInvalidValue;
+    count_launch();
+    return cudaGetLastError();
 }
 
 int cheb_block() { return kBlock; }

@@ -1394,6 +1394,7 @@ struct ChebPlan {
     int *d_seg_begin = nullptr, *d_prob_seg0 = nullptr, *d_seg_full_begin = nullptr;
     double *d_seg_pops = nullptr;
     double *d_drift = nullptr;  // [problem] norm drift of the steps since the last reset
+    unsigned *d_ro_count = nullptr;  // blocks done of the one-problem read-out
     int grid = 0, max_ld = 0, kmax = 0, mg = 0, mg_read = 0, precision = 0, parity = 0;
     int ro_precision = 0;      // element type of the read-out matrices (FP64 or the launch precision)
     int nphase = 1;            // 3: one implicit problem
@@ -1404,7 +1405,7 @@ struct ChebPlan {
     size_t pops_per_step = 0;  // populations of all problems in one step
     void release() {
         dev_free(d_probs); dev_free(d_segs); dev_free(d_seg_begin); dev_free(d_prob_seg0); dev_free(d_seg_pops);
-        dev_free(d_drift); dev_free(d_segs_full); dev_free(d_seg_full_begin);
+        dev_free(d_drift); dev_free(d_segs_full); dev_free(d_seg_full_begin); dev_free(d_ro_count);
     }
 };
 
@@ -1785,6 +1786,20 @@ double cheb_norm_tolerance(const elhl_traj_config &c) {
 // columns swap roles.  No host sync.
 int cheb_dev_step(ChebPlan &pl, const std::vector<ChebState *> &states, double *d_pops_step) {
     if (int rc = cheb_run(pl)) return rc;
+    const ChebProblem &p0 = pl.probs[0];
+    if (pl.solo && pl.solo->rows && pl.nphase == 1 && pl.ro_precision == ELHL_PREC_FP64 &&
+        (p0.P == 1 || p0.P == 2 || p0.P == 4)) {
+        if (!pl.d_ro_count) {
+            if (int rc = dev_alloc(&pl.d_ro_count, 1)) return rc;
+            CU_TRY(cudaMemsetAsync(pl.d_ro_count, 0, sizeof(unsigned), g_ctx.stream));
+        }
+        // scratch: the segments' population partials, kMaxCols (kMaxFrag + 1) doubles for each of min(N, SMs) or more
+        CU_TRY(launch_readout_rows(pl.d_probs, p0.N, p0.P, pl.parity, pl.d_seg_pops, pl.d_ro_count, d_pops_step,
+                                   g_ctx.stream));
+        pl.parity ^= 1;
+        states[0]->parity = pl.parity;
+        return ELHL_OK;
+    }
     if (int rc = launch_norm_drift(pl)) return rc;
     ChebLaunch L{};
     L.probs = pl.d_probs;
@@ -1868,13 +1883,23 @@ __global__ void cols_mt_kernel(const double *__restrict__ M, int ld, int n, cons
         for (int r = 0; r < kMaxTransformRows; ++r)
             if (r < R) acc[r] = fma(mk, x[r], acc[r]);
     }
+    // lane sums of the eight accumulators: three lane bits halve what a lane holds, two sum
+    // (9 FP64 adds instead of 40; lane 4 r ends with row r)
+    static_assert(kMaxTransformRows == 8, "lane sums");
 #pragma unroll
-    for (int r = 0; r < kMaxTransformRows; ++r)
+    for (int o = 16, n = 4; n > 0; o >>= 1, n >>= 1) {
+        const bool upper = (lane & o) != 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
-#pragma unroll
-    for (int r = 0; r < kMaxTransformRows; ++r)
-        if (r < R && lane == r) Y[(size_t)j * R + r] = acc[r];
+        for (int r = 0; r < 4; ++r)
+            if (r < n) {
+                const double send = upper ? acc[r] : acc[r + n], keep = upper ? acc[r + n] : acc[r];
+                acc[r] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+    }
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+    const int r = lane >> 2;
+    if ((lane & 3) == 0 && r < R) Y[(size_t)j * R + r] = acc[0];
 }
 
 // The same four transforms with dense FP64 factors (zeros above the diagonal):

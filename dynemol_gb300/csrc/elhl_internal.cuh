@@ -157,6 +157,10 @@ int cheb_grid_size(int *grid_out);
 int cheb_group_size(int precision, int m, int max_ld, bool windowed = false);
 cudaError_t launch_cheb(const ChebLaunch &L, int precision, int mg, cudaStream_t st);
 cudaError_t launch_readout(const ChebLaunch &L, int nprob, int precision, int mg, cudaStream_t st);
+// the same for probs[0] alone (FP64 read-out matrices; m <= 4; P = 1, 2 or 4), with its
+// norm control and populations
+cudaError_t launch_readout_rows(const ChebProblem *probs, int N, int P, int parity, double *scratch, unsigned *count,
+                                double *pops, cudaStream_t st);
 
 // One trajectory of 2 or 4 complex columns on an explicit Hs whose rows fit in the
 // SMs' shared memory (cheb_rows.cuh).  xbuf: two buffers of cheb_rows_words 16-byte
