@@ -311,7 +311,8 @@ struct Factor {
     double *L = nullptr;     // Cholesky factor (lower triangle), N x N, ld
     double *G = nullptr;     // G = L^-1 (lower triangle), unless factor() put it elsewhere
     double *W = nullptr;     // ld x N workspace: the factorisation's off-diagonal blocks, then G h
-    int *info = nullptr;     // [2]: first non-positive pivot (1-based global column), 0 = positive definite
+    int *info = nullptr;     // [2]: first non-positive pivot (1-based global column), 0 = positive definite; a
+                             // leaf's error (ELHL_ERR_TIMEOUT)
     double *cols = nullptr;  // 2 x (N x 2) scratch (S^-1 applied to a complex vector)
     bool tc = false;         // large products on the tensor cores from exact slices (ELHL_PREC_OZ64)
     int reserve(int N_, int ld_) {
@@ -373,6 +374,7 @@ struct Factor {
         CU_TRY(cudaStreamSynchronize(g_ctx.stream));
         if (tc)
             if (int rc = ozgemm_status()) return rc;
+        if (h[1]) return h[1];  // a leaf's wait gave up
         if (h[0] > 0) return ELHL_ERR_NOT_POSITIVE_DEFINITE;
         if (h[0] < 0) return ELHL_ERR_BAD_ARG;
         return ELHL_OK;

@@ -1,270 +1,330 @@
-// Dense Cholesky-with-inverse of one diagonal block of at most L = 64 rows in
-// FP64, one CTA of 256 threads, entirely in shared memory: the leaves of the
-// rebuild's recursive factorisation (S = L L^T with G = L^-1) for every
-// precision, and of the drop-in's H' = S^-1 h.  Library triangular kernels at
-// these sizes (cuSOLVER trtri on 256 rows, cuBLAS DTRMM/DTRSM panels) ran on a
+// Dense Cholesky-with-inverse of one diagonal block of at most 64 rows in FP64:
+// the leaves of the rebuild's recursive factorisation (S = L L^T with G = L^-1) for
+// every precision, and of the drop-in's H' = S^-1 h.  Library triangular kernels
+// at these sizes (cuSOLVER trtri on 256 rows, cuBLAS DTRMM/DTRSM panels) ran on a
 // handful of CTAs for 65-106 us per call.
 //
-// The cost model is GB300's FP64 pipe: one FP64 warp instruction occupies its
-// SM sub-partition (SMSP) for 76 cycles whether 1 or 32 lanes are active, and
-// a dependent FP64 operation waits 64 cycles (rsqrt: about 370).  So the
-// kernel counts warp instructions, not flops:
-//   - every element loop runs over a dense list of the elements that change
-//     (triangles enumerated column by column from the last column, so that
-//     "columns >= c" is a prefix of the list), never over a square with
-//     predicated-off lanes;
-//   - the products of the inverse give the lanes of a warp equal trip counts;
-//   - the serial chain (pivots of the 8 x 8 diagonal blocks) runs in warp 0
-//     alone while the warps of the other three SMSPs do the trailing update
-//     of the previous block (one block of lookahead), so that the chain and
-//     the bulk work overlap instead of adding up.
+// The cost model is GB300's FP64 unit: one FP64 warp instruction occupies its SM
+// sub-partition (SMSP) for 64-76 cycles whether 1 or 32 lanes are active, a
+// dependent one waits as long.  One SM's unit alone needs 27 us for the 2 x 64^3/6
+// FMAs of the factor and its inverse, and the chain of 64 pivots 22 us, so the work
+// is one cluster of four CTAs:
+//   CTA 0    the factor, by 8-column blocks b: F factors and inverts the 8 x 8
+//            diagonal block (warp 0), P forms the panel below it, U updates what the
+//            next block needs.  U runs beside the next F: warps 1-3 first update the
+//            next diagonal block, on which F waits; warps 1-3 and 5-7 (not on warp
+//            0's SMSP) then update the rest of the next block's columns and bring the
+//            columns after that up to date with every panel so far (left-looking, so
+//            that each step carries about the same work);
+//            warp 4 sends the finished panel and the diagonal block's inverse to the
+//            other CTAs (distributed shared memory) and writes L out.
+//   CTAs 1-3 G = L^-1 by column blocks, right-looking: W_ij += L_ib G_bj as panel b
+//            arrives, G_bj = -G_bb W_bj as the inverse of diagonal block b arrives, so
+//            that only one such product remains when the factor ends.
+// The pivots of F: reciprocal instead of reciprocal root in the chain (the roots of
+// all eight pivots together afterwards), the eliminated column of A replaced in place
+// by the inverse's, one FMA per lane and pivot for both.
+// 66 us per leaf before (one CTA, inverse included), see leaf_chol_inv64 for now.
 #include "elhl_internal.cuh"
+#include "grid_sync.cuh"
 
 namespace elhl {
 namespace {
 
-constexpr int kLeafRows = 64, kThreads = 256;
-constexpr int kDiag = 8, kPPitch = kDiag + 1;
-constexpr int kOthers = 192;  // threads of warps 1-3 and 5-7 (not on warp 0's SMSP)
+constexpr int kLeafRows = 64, kThreads = 256, kCluster = 4;
+constexpr int kB = 8, kBlocks = kLeafRows / kB;
+constexpr int kPitch = kLeafRows + 2;      // row pitch of the factor (16-byte rows)
+constexpr int kOwn = 3;                    // column blocks of G per CTA, at most
+constexpr int kGPitch = kOwn * kB + 2;
+constexpr int kUpdaters = 6;               // warps 1-3 and 5-7
+constexpr unsigned long long kWaitNs = 2000000000ull;
+// column blocks of G by CTA (balanced by their products in the last steps)
+__constant__ int c_own[kCluster][kOwn] = {{-1, -1, -1}, {0, 5, -1}, {1, 4, 6}, {2, 3, 7}};
 
-// element e of the lower triangle of an n x n block, columns from the last:
-// column n - 1 - q holds e in [q (q + 1) / 2, (q + 1) (q + 2) / 2), rows from
-// the diagonal down; "columns >= c" are the first (n - c)(n - c + 1) / 2
-__device__ __forceinline__ void tri_elem(int e, int n, int &i, int &j) {
-    int q = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
-    while ((q + 1) * (q + 2) / 2 <= e) ++q;
-    while (q * (q + 1) / 2 > e) --q;
-    j = n - 1 - q;
-    i = j + (e - q * (q + 1) / 2);
+// element e of an 8 x 8 lower triangle, row by row
+__device__ __forceinline__ void tri_elem(int e, int &i, int &j) {
+    i = 0;
+    while ((i + 1) * (i + 2) / 2 <= e) ++i;
+    j = e - i * (i + 1) / 2;
 }
 
-template <int L>
-__host__ __device__ constexpr int tri_count() { return L * (L + 1) / 2; }
-
-// products of the doubling inverse: [L * L / 4] for one level at a time, or for
-// L = 64 the 8-, 16- and 32-row levels side by side (4 x 64 + 2 x 256 + 1024)
-template <int L>
-__host__ __device__ constexpr int leaf_wm() { return 7 * L * L / 16; }
-
-template <int L>
-constexpr size_t leaf_smem() {
-    return (size_t)(2 * L * (L + 1) + L * kPPitch + leaf_wm<L>() + 2 * kDiag) * sizeof(double) +
-           (size_t)tri_count<L>() * sizeof(int);
+// 1 / d for a normal d > 0: third-order Householder iteration y (1 + e + e^2), e = 1 - d y,
+// on the hardware's approximation (20 bits: error e^3 below 2^-57 before rounding)
+__device__ __forceinline__ double reciprocal(double d) {
+    const int ex = (__double2hiint(d) >> 20) & 0x7ff;
+    if (ex < 24 || ex > 2020) return 1.0 / d;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d, y, 1.0);
+    return fma(y, fma(e, e, e), y);
 }
 
-// The doubling inverse of one s x s pair of diagonal blocks at o = 2 s blk
-// (pitch p): W = L21 G11 (G11 lower: t >= j) and G21 = -G22 W (G22 lower: t <= i).
-// W's rows of L21 come from `l21` (row i at l21 + i * lp: As, or the panel while
-// its copy into As is in flight).  Columns j0 .. j1 of W only; lanes along i for
-// W (equal trips s - j), along j for G21 (equal trips i + 1).
-__device__ void inv_w(const double *l21, int lp, const double *Gs, int p, double *W, int s, int o, int j0, int j1,
-                      int tid, int nthr) {
-    const int count = (j1 - j0) * s;
-    for (int e = tid; e < count; e += nthr) {
-        const int j = j0 + e / s, i = e % s;
-        double a = 0.0;
-        for (int t = j; t < s; ++t) a = fma(l21[i * lp + t], Gs[(o + t) * p + o + j], a);
-        W[i * s + j] = a;
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address of this CTA's shared variable in CTA `rank` of the cluster
+__device__ __forceinline__ unsigned remote(const void *p, unsigned rank) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void store_remote(unsigned a, double x, double y) {
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(x), "d"(y) : "memory");
+}
+// whole warp: what its lanes stored in the CTAs 1 .. 3 is visible there before *flag = 1
+__device__ __forceinline__ void raise_flag(int *flag) {
+    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+    __syncwarp();
+    const unsigned lane = threadIdx.x & 31;
+    if (lane >= 1 && lane < kCluster)
+        asm volatile("st.release.cluster.shared::cluster.u32 [%0], %1;" ::"r"(remote(flag, lane)), "r"(1) : "memory");
+}
+// one thread: bounded wait for a flag of this CTA
+__device__ __forceinline__ bool wait_flag(const int *flag) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(flag);
+    unsigned long long t0 = 0;
+    for (unsigned n = 1;; ++n) {
+        int v;
+        asm volatile("ld.acquire.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+        if (v) return true;
+        if ((n & 63u) == 0) {
+            const unsigned long long t = globaltimer_ns();
+            if (!t0) t0 = t;
+            if (t - t0 > kWaitNs) return false;
+        }
     }
 }
-__device__ void inv_g(double *Gs, int p, const double *W, int s, int o, int tid, int nthr) {
-    for (int e = tid; e < s * s; e += nthr) {
-        const int i = e / s, j = e % s;
-        double a = 0.0;
-        for (int t = 0; t <= i; ++t) a = fma(Gs[(o + s + i) * p + o + s + t], W[t * s + j], a);
-        Gs[(o + s + i) * p + o + j] = -a;
-    }
-}
 
-// Warp 0: factor and invert the 8 x 8 diagonal block at Ab / Gb (pitch p):
-// a_ij -= a_ik a_jk / a_kk for the pivots k (the elements of columns > k: a
-// prefix of at most 28 of the block's list, one lane each), then the unit
-// lower inverse x and the scalings G = x_ij / L(i, i), L = a_ij / L(j, j).
-// A non-positive pivot of a real row (< nb) sets *info (first one found) and
-// is carried on with a zero scale, so the launch always ends.
-__device__ void diag_block(double *Ab, double *Gb, int p, double *rb, double *sb, int b0, int nb, int r, int *info) {
-    const int lane = threadIdx.x % 32;
-    int di, dj;
-    tri_elem(lane, kDiag, di, dj);  // this lane's element of the 8 x 8 list (36 elements: 32 here)
-    for (int kk = 0; kk < kDiag; ++kk) {
+struct Smem {
+    double A[kLeafRows * kPitch];          // CTA 0: A, then L; others: the panels of L
+    double Gd[kBlocks][kB * kB];           // inverses of the diagonal blocks (zero above the diagonal)
+    double G[kLeafRows * kGPitch];         // others: W, then G, of the CTA's column blocks
+    double M[kB * (kB + 1)], Lr[kB * (kB + 1)], d[kB], rr[kB];  // F
+    int flag_g[kBlocks], flag_p[kBlocks];  // others: Gd[b], panel b have arrived
+    int ok;
+};
+
+// F, warp 0: the 8 x 8 block at (b0, b0) of s.A, all of its updates done: its Cholesky
+// factor in place and the factor's inverse in s.Gd[b].  At pivot k, with m_i = a_ik / a_kk:
+// a_ij -= m_i a_jk for i >= j > k and, for the unit lower inverse x kept where the
+// columns <= k of A were, x_ij -= m_i x_kj for j < k and x_ik = -m_i.  act[k]: this
+// lane's element (i << 4 | j) of that update, or -1 (28 - k (k + 1) / 2 elements).  A
+// non-positive pivot of a real row (< nb) sets *info (first one found) and is carried
+// on with a zero scale, so the launch always ends.
+__device__ void factor_block(Smem &s, int b, int nb, int row0, const int (&act)[kB - 1], int *info) {
+    const int lane = threadIdx.x & 31, b0 = b * kB;
+    constexpr int p = kB + 1;
+    for (int e = lane; e < kB * (kB + 1) / 2; e += 32) {
+        int i, j;
+        tri_elem(e, i, j);
+        s.M[i * p + j] = s.A[(b0 + i) * kPitch + b0 + j];
+    }
+#pragma unroll
+    for (int k = 0; k < kB; ++k) {
         __syncwarp();
-        const double d = Ab[kk * p + kk];
-        const bool ok = d > 0.0;
-        const double rr = ok ? rsqrt(d) : 0.0, sq = rr * rr;
+        const double d = s.M[k * p + k];
+        const long long bits = __double_as_longlong(d);
+        const bool ok = bits > 0 && bits <= 0x7ff0000000000000ll;  // d > 0
+        const double inv = ok ? reciprocal(d) : 0.0;
         if (lane == 0) {
-            rb[kk] = rr;
-            sb[kk] = sq;
-            if (!ok && b0 + kk < nb) atomicCAS(info, 0, r + b0 + kk + 1);
+            s.d[k] = ok ? d : 0.0;
+            if (!ok && b0 + k < nb) atomicCAS(info, 0, row0 + b0 + k + 1);
         }
-        const int m = kDiag - 1 - kk;  // columns kk + 1 .. 7
-        if (lane < m * (m + 1) / 2)
-            Ab[di * p + dj] = fma(-Ab[di * p + kk] * sq, Ab[dj * p + kk], Ab[di * p + dj]);
+        if (k + 1 < kB) {
+            const int ij = act[k < kB - 1 ? k : 0], i = ij >> 4, j = ij & 15, ic = k + 1 + lane;
+            double v = 0.0, a = 0.0, x = 0.0;
+            if (ij >= 0) {
+                const double t = s.M[i * p + k] * (j > k ? s.M[j * p + k] : s.M[k * p + j]);
+                v = fma(-t, inv, s.M[i * p + j]);
+            }
+            if (ic < kB) {
+                a = s.M[ic * p + k];
+                x = -(a * inv);
+            }
+            __syncwarp();
+            if (ij >= 0) s.M[i * p + j] = v;
+            if (ic < kB) {
+                s.Lr[ic * p + k] = a;
+                s.M[ic * p + k] = x;
+            }
+        }
     }
     __syncwarp();
-    for (int e = lane; e < kDiag * kDiag; e += 32) Gb[(e / kDiag) * p + e % kDiag] = (e / kDiag == e % kDiag) ? 1.0 : 0.0;
-    for (int kk = 0; kk < kDiag - 1; ++kk) {  // x(i, j) -= (a_ik / a_kk) x(k, j), i > k >= j
-        __syncwarp();
-        if (lane < (kDiag - 1 - kk) * (kk + 1)) {
-            const int i = kk + 1 + lane / (kk + 1), j = lane % (kk + 1);
-            Gb[i * p + j] = fma(-Ab[i * p + kk] * sb[kk], Gb[kk * p + j], Gb[i * p + j]);
-        }
-    }
+    if (lane < kB) s.rr[lane] = s.d[lane] > 0.0 ? rsqrt(s.d[lane]) : 0.0;
     __syncwarp();
-    for (int e = lane; e < kDiag * (kDiag + 1) / 2; e += 32) {
-        int i, j;
-        tri_elem(e, kDiag, i, j);
-        Gb[i * p + j] *= rb[i];
-        Ab[i * p + j] *= rb[j];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int e = lane + 32 * u, i = e / kB, j = e % kB;
+        double g = 0.0;
+        if (i >= j) {
+            s.A[(b0 + i) * kPitch + b0 + j] = (i > j ? s.Lr[i * p + j] : s.d[j]) * s.rr[j];
+            g = i > j ? s.M[i * p + j] * s.rr[i] : s.rr[i];
+        }
+        s.Gd[b][e] = g;
     }
     __syncwarp();
 }
 
-// L = chol(A) in place and G = L^-1 for the nb x nb diagonal block at offset r
-// (rows past nb padded with the identity), by 8-column blocks b:
-//   panel   L_rb = A_rb G_bb^T for the rows r >= b0 + 8 below block b;
-//   then, concurrently: warp 0 updates the next diagonal block with the panel
-//   and factors it (diag_block); warps 1-3 and 5-7 update the rest of the
-//   trailing matrix, A_rr -= L_rb L_rb^T (the columns past the next block, and
-//   the next block's own rows below its diagonal block);
-// and the inverse by doubling, s = 8, 16, 32: G21 = -G22 (L21 G11) for all
-// pairs of s x s blocks.
-template <int L>
-__global__ void __launch_bounds__(kThreads) leaf_chol_inv64_kernel(double *A, double *G, int nb, int ld, int r,
-                                                                   int *info) {
-    constexpr int kP = L + 1;
-    extern __shared__ double smem[];
-    double *As = smem;                 // [L][kP], row-major: A, then L
-    double *Gs = As + L * kP;          // [L][kP]: G
-    double *Pn = Gs + L * kP;          // [L][kPPitch]: panel of the current block
-    double *Wm = Pn + L * kPPitch;     // [leaf_wm<L>()]: L21 G11 of the doubling levels
-    double *rb = Wm + leaf_wm<L>(), *sb = rb + kDiag;  // 1/L(k, k) and its square, warp 0's block
-    int *tab = reinterpret_cast<int *>(sb + kDiag);  // [tri_count<L>()]: (i << 8) | j, columns from the last
-    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const bool other = (warp & 3) != 0;
-    const int ot = other ? (warp - 1 - (warp > 4)) * 32 + lane : -1;  // 0 .. kOthers - 1
-    for (int e = tid; e < L * L; e += kThreads) {
-        const int i = e % L, j = e / L;
-        double v = 0.0;
-        if (i < nb && j < nb) {
-            if (i >= j) v = A[(size_t)j * ld + i];
-        } else if (i == j) {
-            v = 1.0;
-        }
-        As[i * kP + j] = v;
-        Gs[i * kP + j] = 0.0;
+// CTA 0: the factor
+__device__ void factor_cta(Smem &s, double *A, int nb, int ld, int row0, int *info) {
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
+    const int blocks = (nb + kB - 1) / kB, end = blocks * kB;  // rows in use (padded to whole blocks)
+    int act[kB - 1];
+#pragma unroll
+    for (int k = 0; k < kB - 1; ++k) {
+        int i = k + 1, e = lane;
+        while (i < kB && e >= i) e -= i++;
+        act[k] = i < kB ? (i << 4) | (e < k ? e : e + 1) : -1;
     }
-    for (int e = tid; e < tri_count<L>(); e += kThreads) {
-        int i, j;
-        tri_elem(e, L, i, j);
-        tab[e] = (i << 8) | j;
-    }
-    __syncthreads();
-    if (warp == 0) diag_block(As, Gs, kP, rb, sb, 0, nb, r, info);
-    __syncthreads();
-    for (int b0 = 0; b0 + kDiag < L; b0 += kDiag) {
-        const int r0 = b0 + kDiag, nr = L - r0;
-        const double *Gb = Gs + b0 * kP + b0;
-        // panel: L(i, b0 + t) = sum_{s <= t} A(i, b0 + s) G_bb(t, s), lanes along i
-        for (int e = tid; e < kDiag * nr; e += kThreads) {
-            const int t = e / nr, i = r0 + e % nr;
-            double a = 0.0;
-            for (int s = 0; s <= t; ++s) a = fma(As[i * kP + b0 + s], Gb[t * kP + s], a);
-            Pn[i * kPPitch + t] = a;
+    if (warp == 0) factor_block(s, 0, nb, row0, act, info);
+    for (int b = 0; b < blocks; ++b) {
+        const int b0 = b * kB, r0 = b0 + kB;
+        const bool last = b + 1 == blocks;
+        __syncthreads();  // F(b) and U(b - 1) done
+        if (!last) {
+            // P: L(i, b0 + t) = sum_{s <= t} A(i, b0 + s) Gd(t, s); a warp takes the columns t and
+            // 7 - t (nine FMAs) of 32 rows, results held until every row has been read
+            const int t0 = warp & 3, t1 = kB - 1 - t0, i = r0 + (warp >> 2) * 32 + lane;
+            double o0 = 0.0, o1 = 0.0;
+            if (i < end) {
+                const double *a = s.A + i * kPitch + b0, *g0 = s.Gd[b] + t0 * kB, *g1 = s.Gd[b] + t1 * kB;
+#pragma unroll
+                for (int q = 0; q < kB; ++q) {
+                    if (q <= t0) o0 = fma(a[q], g0[q], o0);
+                    if (q <= t1) o1 = fma(a[q], g1[q], o1);
+                }
+            }
+            __syncthreads();
+            if (i < end) {
+                s.A[i * kPitch + b0 + t0] = o0;
+                s.A[i * kPitch + b0 + t1] = o1;
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        for (int e = tid; e < kDiag * nr; e += kThreads) {
-            const int t = e / nr, i = r0 + e % nr;
-            As[i * kP + b0 + t] = Pn[i * kPPitch + t];
+        if (warp == 4) {
+            // the inverse of the diagonal block, then the panel, to the CTAs 1 .. 3
+            for (int c = 1; c < kCluster; ++c)
+                store_remote(remote(&s.Gd[b][2 * lane], c), s.Gd[b][2 * lane], s.Gd[b][2 * lane + 1]);
+            raise_flag(&s.flag_g[b]);
+            for (int q = lane; q < (end - r0) * (kB / 2); q += 32) {
+                const double *v = s.A + (r0 + q / (kB / 2)) * kPitch + b0 + 2 * (q % (kB / 2));
+                for (int c = 1; c < kCluster; ++c) store_remote(remote(v, c), v[0], v[1]);
+            }
+            raise_flag(&s.flag_p[b]);
+            for (int j = b0; j < min(r0, nb); ++j)  // column block b of L, zero above the diagonal
+                for (int i = lane; i < nb; i += 32) A[(size_t)j * ld + i] = i >= j ? s.A[i * kPitch + j] : 0.0;
         }
+        if (last) break;
         if (warp == 0) {
-            // the next diagonal block (rows and columns r0 .. r0 + 7), then its factor
-            for (int e = lane; e < kDiag * (kDiag + 1) / 2; e += 32) {
-                int i, j;
-                tri_elem(e, kDiag, i, j);
-                i += r0;
-                j += r0;
-                double a = As[i * kP + j];
+            asm volatile("bar.sync 1, 128;" ::: "memory");  // the next diagonal block is up to date
+            factor_block(s, b + 1, nb, row0, act, info);
+            continue;
+        }
+        if (warp == 4) continue;
+        if (warp < 4) {
+            // the next diagonal block: 12 of its 36 elements per warp, two lanes of four FMAs each
+            const int half = lane >= 12;
+            int i, j;
+            tri_elem((warp - 1) * 12 + lane % 12, i, j);
+            const double *x = s.A + (r0 + i) * kPitch + b0 + 4 * half, *y = s.A + (r0 + j) * kPitch + b0 + 4 * half;
+            double v = 0.0;
 #pragma unroll
-                for (int t = 0; t < kDiag; ++t) a = fma(-Pn[i * kPPitch + t], Pn[j * kPPitch + t], a);
-                As[i * kP + j] = a;
-            }
-            diag_block(As + r0 * kP + r0, Gs + r0 * kP + r0, kP, rb, sb, r0, nb, r, info);
-        } else if (other) {
-            // the trailing triangle of the columns past the next block
-            const int m = L - r0 - kDiag, cnt = m * (m + 1) / 2;
-            for (int e = ot; e < cnt; e += kOthers) {
-                const int i = tab[e] >> 8, j = tab[e] & 255;
-                double a = As[i * kP + j];
+            for (int q = 0; q < 4; ++q) v = fma(x[q], y[q], v);
+            v += __shfl_down_sync(0xffffffffu, v, 12);
+            if (lane < 12) s.A[(r0 + i) * kPitch + r0 + j] -= v;
+            asm volatile("bar.arrive 1, 128;" ::: "memory");
+        }
+        // the rows below it: the next block's columns with this panel (set 0), the columns after
+        // those with every panel so far (set 1), in chunks of 32 elements along the rows
+        const int c0 = r0 + kB, rows = end - c0, chunks = (rows * kB + 31) / 32;
+        for (int q = warp < 4 ? warp - 1 : warp - 2; q < 2 * chunks; q += kUpdaters) {
+            const bool ahead = q >= chunks;
+            const int e = (ahead ? q - chunks : q) * 32 + lane, i = c0 + e % max(rows, 1), j = (ahead ? c0 : r0) + e / max(rows, 1);
+            if (e >= rows * kB || i < j) continue;
+            const int k0 = ahead ? 0 : b0;
+            const double *x = s.A + i * kPitch, *y = s.A + j * kPitch;
+            double v = s.A[i * kPitch + j];
+#pragma unroll 8
+            for (int k = k0; k < r0; ++k) v = fma(-x[k], y[k], v);
+            s.A[i * kPitch + j] = v;
+        }
+    }
+}
+
+// CTAs 1 .. 3: the columns of G of their column blocks
+__device__ void inverse_cta(Smem &s, unsigned rank, double *G, int nb, int ld, int *info) {
+    const int tid = threadIdx.x;
+    const int blocks = (nb + kB - 1) / kB, end = blocks * kB;
+    int own[kOwn];
 #pragma unroll
-                for (int t = 0; t < kDiag; ++t) a = fma(-Pn[i * kPPitch + t], Pn[j * kPPitch + t], a);
-                As[i * kP + j] = a;
-            }
-            // the next block's rows below its diagonal block (the next panel's input), lanes along i
-            for (int e = ot; e < kDiag * m; e += kOthers) {
-                const int j = r0 + e / m, i = r0 + kDiag + e % m;
-                double a = As[i * kP + j];
+    for (int q = 0; q < kOwn; ++q) own[q] = c_own[rank][q];
+    // zero above the diagonal, and W
+    for (int e = tid; e < kOwn * kB * kLeafRows; e += kThreads) {
+        const int i = e % kLeafRows, c = e / kLeafRows, j = own[c / kB] * kB + c % kB;
+        s.G[i * kGPitch + c] = 0.0;
+        if (j >= 0 && j < nb && i < min(nb, own[c / kB] * kB)) G[(size_t)j * ld + i] = 0.0;
+    }
+    __syncthreads();
+    for (int b = 0; b < blocks; ++b) {
+        const int b0 = b * kB, r0 = b0 + kB;
+        if (tid == 0) s.ok = wait_flag(&s.flag_g[b]);
+        __syncthreads();
+        if (!s.ok) break;
+        // row block b of G: -Gd W for the column blocks before b, Gd for b itself
+        const int c = tid / kB, i = tid % kB, jb = c < kOwn * kB ? own[c / kB] : -1;
+        double v = 0.0;
+        if (jb >= 0 && jb < b) {
+            for (int t = 0; t <= i; ++t) v = fma(-s.Gd[b][i * kB + t], s.G[(b0 + t) * kGPitch + c], v);
+        } else if (jb == b) {
+            v = s.Gd[b][i * kB + c % kB];
+        }
+        __syncthreads();  // W has been read
+        if (jb >= 0 && jb <= b) {
+            s.G[(b0 + i) * kGPitch + c] = v;
+            const int j = jb * kB + c % kB;
+            if (b0 + i < nb && j < nb) G[(size_t)j * ld + b0 + i] = v;
+        }
+        if (b + 1 == blocks) break;
+        if (tid == 0) s.ok = wait_flag(&s.flag_p[b]);
+        __syncthreads();
+        if (!s.ok) break;
+        for (int e = tid; e < (end - r0) * kOwn * kB; e += kThreads) {  // W += L_b G_b, lanes along the rows
+            const int r = r0 + e % (end - r0), q = e / (end - r0);
+            if (own[q / kB] < 0 || own[q / kB] > b) continue;
+            double w = s.G[r * kGPitch + q];
 #pragma unroll
-                for (int t = 0; t < kDiag; ++t) a = fma(-Pn[i * kPPitch + t], Pn[j * kPPitch + t], a);
-                As[i * kP + j] = a;
-            }
-            if constexpr (L == 64) {
-                // the doubling inverse's products whose blocks are final, in the time warp 0's
-                // pivot chain leaves these warps idle (b: this block; the pair (2q, 2q + 1) of
-                // 8 rows, the quad of 16, the halves of 32)
-                const int b = b0 / kDiag;
-                double *W8 = Wm, *W16 = Wm + 4 * 64, *W32 = Wm + 4 * 64 + 2 * 256;
-                if ((b & 1) == 0)  // W of pair b / 2: L21 rows are the panel's (its copy into As is in flight)
-                    inv_w(Pn + (size_t)r0 * kPPitch, kPPitch, Gs, kP, W8 + (b / 2) * 64, 8, 16 * (b / 2), 0, 8, ot,
-                          kOthers);
-                else  // G21 of pair (b - 1) / 2: its second diagonal block was factored in the last block
-                    inv_g(Gs, kP, W8 + (b / 2) * 64, 8, 16 * (b / 2), ot, kOthers);
-                if (b == 2 || b == 6)  // W of quad b / 4: pairs inverted, panels final
-                    inv_w(As + (size_t)(32 * (b / 4) + 16) * kP + 32 * (b / 4), kP, Gs, kP, W16 + (b / 4) * 256, 16,
-                          32 * (b / 4), 0, 16, ot, kOthers);
-                if (b == 4)  // G21 of quad 0
-                    inv_g(Gs, kP, W16, 16, 0, ot, kOthers);
-                if (b >= 5)  // W of the halves, columns 0-15 then 16-31: the first half is inverted
-                    inv_w(As + (size_t)32 * kP, kP, Gs, kP, W32, 32, 0, 16 * (b - 5), 16 * (b - 4), ot, kOthers);
-            }
+            for (int t = 0; t < kB; ++t) w = fma(s.A[r * kPitch + b0 + t], s.G[(b0 + t) * kGPitch + q], w);
+            s.G[r * kGPitch + q] = w;
         }
         __syncthreads();
     }
-    if constexpr (L == 64) {  // the doubling inverse's last products (their other halves ran in the loop)
-        inv_g(Gs, kP, Wm + 3 * 64, 8, 48, tid, kThreads);  // pair 3
-        __syncthreads();
-        inv_g(Gs, kP, Wm + 4 * 64 + 256, 16, 32, tid, kThreads);  // quad 1
-        __syncthreads();
-        inv_g(Gs, kP, Wm + 4 * 64 + 2 * 256, 32, 0, tid, kThreads);  // the halves
-        __syncthreads();
-    } else
-    for (int s = kDiag; s < L; s *= 2) {  // inverse by doubling
-        const int per = s * s, count = (L / (2 * s)) * per;
-        // W = L21 G11 (G11 lower: t >= j), lanes along i: equal trips s - j
-        for (int e = tid; e < count; e += kThreads) {
-            const int blk = e / per, o = 2 * s * blk, j = (e % per) / s, i = e % s;
-            double a = 0.0;
-            for (int t = j; t < s; ++t) a = fma(As[(o + s + i) * kP + o + t], Gs[(o + t) * kP + o + j], a);
-            Wm[blk * per + i * s + j] = a;
-        }
-        __syncthreads();
-        // G21 = -G22 W (G22 lower: t <= i), lanes along j: equal trips i + 1
-        for (int e = tid; e < count; e += kThreads) {
-            const int blk = e / per, o = 2 * s * blk, i = (e % per) / s, j = e % s;
-            const double *W = Wm + blk * per;
-            double a = 0.0;
-            for (int t = 0; t <= i; ++t) a = fma(Gs[(o + s + i) * kP + o + s + t], W[t * s + j], a);
-            Gs[(o + s + i) * kP + o + j] = -a;
-        }
-        __syncthreads();
-    }
-    for (int e = tid; e < L * L; e += kThreads) {
-        const int i = e % L, j = e / L;
-        if (i < nb && j < nb) {
-            const bool low = i >= j;
-            G[(size_t)j * ld + i] = low ? Gs[i * kP + j] : 0.0;
-            A[(size_t)j * ld + i] = low ? As[i * kP + j] : 0.0;
+    if (tid == 0 && !s.ok) atomicExch(info + 1, ELHL_ERR_TIMEOUT);
+}
+
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads)
+    leaf_chol_inv64_kernel(double *A, double *G, int nb, int ld, int row0, int *info) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    Smem &s = *reinterpret_cast<Smem *>(raw);
+    const unsigned rank = cluster_rank();
+    const int tid = threadIdx.x;
+    if (tid < kBlocks) s.flag_g[tid] = s.flag_p[tid] = 0;
+    if (rank == 0) {
+        for (int e = tid; e < kLeafRows * kLeafRows; e += kThreads) {  // rows past nb: the identity
+            const int i = e % kLeafRows, j = e / kLeafRows;
+            double v = i == j ? 1.0 : 0.0;
+            if (i < nb && j < nb) v = i >= j ? A[(size_t)j * ld + i] : 0.0;
+            s.A[i * kPitch + j] = v;
         }
     }
+    cluster_barrier();  // flags and A in place
+    if (rank == 0) factor_cta(s, A, nb, ld, row0, info);
+    else inverse_cta(s, rank, G, nb, ld, info);
+    cluster_barrier();  // no CTA leaves while its shared memory may still be written
 }
 
 }  // namespace
@@ -274,13 +334,13 @@ int leaf_rows() { return kLeafRows; }
 cudaError_t leaf_chol_inv64(double *A, double *G, int nb, int ld, int row0, int *info, cudaStream_t st) {
     static bool attr = false;
     if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(leaf_chol_inv64_kernel<kLeafRows>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)leaf_smem<kLeafRows>());
+        cudaError_t e = cudaFuncSetAttribute(leaf_chol_inv64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(Smem));
         if (e != cudaSuccess) return e;
         attr = true;
     }
     if (nb <= 0 || nb > kLeafRows) return cudaErrorInvalidValue;
-    leaf_chol_inv64_kernel<kLeafRows><<<1, kThreads, leaf_smem<kLeafRows>(), st>>>(A, G, nb, ld, row0, info);
+    leaf_chol_inv64_kernel<<<kCluster, kThreads, sizeof(Smem), st>>>(A, G, nb, ld, row0, info);
     count_launch();
     return cudaGetLastError();
 }
