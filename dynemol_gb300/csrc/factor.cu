@@ -17,14 +17,16 @@
 //            columns after that up to date with every panel so far (left-looking, so
 //            that each step carries about the same work);
 //            warp 4 sends the finished panel and the diagonal block's inverse to the
-//            other CTAs (distributed shared memory) and writes L out.
+//            other CTAs (distributed shared memory).
 //   CTAs 1-3 G = L^-1 by column blocks, right-looking: W_ij += L_ib G_bj as panel b
 //            arrives, G_bj = -G_bb W_bj as the inverse of diagonal block b arrives, so
 //            that only one such product remains when the factor ends.
 // The pivots of F: reciprocal instead of reciprocal root in the chain (the roots of
 // all eight pivots together afterwards), the eliminated column of A replaced in place
 // by the inverse's, one FMA per lane and pivot for both.
-// 66 us per leaf before (one CTA, inverse included), see leaf_chol_inv64 for now.
+// 66 us per leaf of 64 rows in one CTA, 41 us on the cluster with the pivots' elements found
+// per lane in branches, 34.5 us with them in a table of offsets and L written after the loop:
+// F 5,000 cycles, P 1,100-1,900, the next diagonal block 1,000, eight times.
 #include "elhl_internal.cuh"
 #include "grid_sync.cuh"
 
@@ -104,66 +106,88 @@ struct Smem {
     double A[kLeafRows * kPitch];          // CTA 0: A, then L; others: the panels of L
     double Gd[kBlocks][kB * kB];           // inverses of the diagonal blocks (zero above the diagonal)
     double G[kLeafRows * kGPitch];         // others: W, then G, of the CTA's column blocks
-    double M[kB * (kB + 1)], Lr[kB * (kB + 1)], d[kB], rr[kB];  // F
+    // F: the block, its eliminated columns (unscaled), the pivots and their root's reciprocals
+    double M[kB * kB], Lr[kB * kB], d[kB], rr[kB];
+    double zero, one, dump;                // operands of F's lanes without an element, and where they write
     int flag_g[kBlocks], flag_p[kBlocks];  // others: Gd[b], panel b have arrived
     int ok;
 };
 
+// One lane's part of one pivot of F: out = m - (a u) / a_kk, with a also kept at `keep`
+// (offsets in doubles from the start of Smem).
+struct Step {
+    short a, u, m, out, keep;
+};
+__device__ __forceinline__ short at(const Smem &s, const double *p) { return (short)(p - s.A); }
+// The n-th element pivot k changes: a_ij (i >= j > k) and x_ij (j < k) take m = itself,
+// a = a_ik, u = a_jk or x_kj; the new column x_ik takes u = 1, m = 0 and keeps a_ik.
+__device__ __forceinline__ Step pivot_step(Smem &s, int k, int n) {
+    const int updates = (kB * (kB - 1) - k * (k + 1)) / 2;
+    if (n < updates) {
+        int i = k + 1, e = n;
+        while (e >= i) e -= i++;
+        const int j = e < k ? e : e + 1;
+        const short m = at(s, s.M + i * kB + j);
+        return Step{at(s, s.M + i * kB + k), at(s, j > k ? s.M + j * kB + k : s.M + k * kB + j), m, m, at(s, &s.dump)};
+    }
+    const int i = k + 1 + n - updates;
+    const short none = at(s, &s.dump), zero = at(s, &s.zero), c = at(s, s.M + i * kB + k);
+    if (i < kB) return Step{c, at(s, &s.one), zero, c, at(s, s.Lr + i * kB + k)};
+    return Step{zero, zero, zero, none, none};
+}
+constexpr int kTwice = 2;  // pivots with more than 32 elements (35, 33, then 30 and fewer)
+
 // F, warp 0: the 8 x 8 block at (b0, b0) of s.A, all of its updates done: its Cholesky
 // factor in place and the factor's inverse in s.Gd[b].  At pivot k, with m_i = a_ik / a_kk:
 // a_ij -= m_i a_jk for i >= j > k and, for the unit lower inverse x kept where the
-// columns <= k of A were, x_ij -= m_i x_kj for j < k and x_ik = -m_i.  act[k]: this
-// lane's element (i << 4 | j) of that update, or -1 (28 - k (k + 1) / 2 elements).  A
-// non-positive pivot of a real row (< nb) sets *info (first one found) and is carried
-// on with a zero scale, so the launch always ends.
-__device__ void factor_block(Smem &s, int b, int nb, int row0, const int (&act)[kB - 1], int *info) {
+// columns <= k of A were, x_ij -= m_i x_kj for j < k and x_ik = -m_i: at most 35
+// elements, one multiplication beside the reciprocal and one FMA after it.  A
+// non-positive pivot of a real row (< nb) sets *info (the first one); nothing after it
+// depends on the values.
+__device__ __forceinline__ void factor_block(Smem &s, int b, int nb, int row0, const Step (&step)[kB - 1], const Step (&more)[kTwice],
+                             int *info) {
     const int lane = threadIdx.x & 31, b0 = b * kB;
-    constexpr int p = kB + 1;
-    for (int e = lane; e < kB * (kB + 1) / 2; e += 32) {
-        int i, j;
-        tri_elem(e, i, j);
-        s.M[i * p + j] = s.A[(b0 + i) * kPitch + b0 + j];
+    double *w = s.A;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int e = lane + 32 * u;
+        s.M[e] = s.A[(b0 + e / kB) * kPitch + b0 + e % kB];  // above the diagonal: not read
     }
 #pragma unroll
     for (int k = 0; k < kB; ++k) {
         __syncwarp();
-        const double d = s.M[k * p + k];
-        const long long bits = __double_as_longlong(d);
-        const bool ok = bits > 0 && bits <= 0x7ff0000000000000ll;  // d > 0
-        const double inv = ok ? reciprocal(d) : 0.0;
-        if (lane == 0) {
-            s.d[k] = ok ? d : 0.0;
-            if (!ok && b0 + k < nb) atomicCAS(info, 0, row0 + b0 + k + 1);
-        }
-        if (k + 1 < kB) {
-            const int ij = act[k < kB - 1 ? k : 0], i = ij >> 4, j = ij & 15, ic = k + 1 + lane;
-            double v = 0.0, a = 0.0, x = 0.0;
-            if (ij >= 0) {
-                const double t = s.M[i * p + k] * (j > k ? s.M[j * p + k] : s.M[k * p + j]);
-                v = fma(-t, inv, s.M[i * p + j]);
-            }
-            if (ic < kB) {
-                a = s.M[ic * p + k];
-                x = -(a * inv);
-            }
+        const double d = s.M[k * kB + k];
+        if (lane == 0) s.d[k] = d;
+        if (k + 1 == kB) break;
+        const Step &q = step[k < kB - 1 ? k : 0];
+        const double a = w[q.a], m = w[q.m], t = a * w[q.u], inv = reciprocal(d), v = fma(-t, inv, m);
+        if (k < kTwice) {
+            const Step &r = more[k < kTwice ? k : 0];
+            const double a2 = w[r.a], v2 = fma(-(a2 * w[r.u]), inv, w[r.m]);
             __syncwarp();
-            if (ij >= 0) s.M[i * p + j] = v;
-            if (ic < kB) {
-                s.Lr[ic * p + k] = a;
-                s.M[ic * p + k] = x;
-            }
+            w[r.out] = v2;
+            w[r.keep] = a2;
+        } else {
+            __syncwarp();
         }
+        w[q.out] = v;
+        w[q.keep] = a;
     }
     __syncwarp();
-    if (lane < kB) s.rr[lane] = s.d[lane] > 0.0 ? rsqrt(s.d[lane]) : 0.0;
+    if (lane < kB) {
+        const double d = s.d[lane];
+        s.rr[lane] = rsqrt(d);
+        const unsigned bad = __ballot_sync(0xffu, !(d > 0.0) && b0 + lane < nb);
+        if (bad && lane == 0) atomicCAS(info, 0, row0 + b0 + __ffs(bad));
+    }
     __syncwarp();
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
         const int e = lane + 32 * u, i = e / kB, j = e % kB;
         double g = 0.0;
         if (i >= j) {
-            s.A[(b0 + i) * kPitch + b0 + j] = (i > j ? s.Lr[i * p + j] : s.d[j]) * s.rr[j];
-            g = i > j ? s.M[i * p + j] * s.rr[i] : s.rr[i];
+            s.A[(b0 + i) * kPitch + b0 + j] = (i > j ? s.Lr[e] : s.d[j]) * s.rr[j];
+            g = i > j ? s.M[e] * s.rr[i] : s.rr[i];
         }
         s.Gd[b][e] = g;
     }
@@ -174,14 +198,12 @@ __device__ void factor_block(Smem &s, int b, int nb, int row0, const int (&act)[
 __device__ void factor_cta(Smem &s, double *A, int nb, int ld, int row0, int *info) {
     const int tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
     const int blocks = (nb + kB - 1) / kB, end = blocks * kB;  // rows in use (padded to whole blocks)
-    int act[kB - 1];
+    Step step[kB - 1], more[kTwice];
 #pragma unroll
-    for (int k = 0; k < kB - 1; ++k) {
-        int i = k + 1, e = lane;
-        while (i < kB && e >= i) e -= i++;
-        act[k] = i < kB ? (i << 4) | (e < k ? e : e + 1) : -1;
-    }
-    if (warp == 0) factor_block(s, 0, nb, row0, act, info);
+    for (int k = 0; k < kB - 1; ++k) step[k] = pivot_step(s, k, lane);
+#pragma unroll
+    for (int k = 0; k < kTwice; ++k) more[k] = pivot_step(s, k, 32 + lane);
+    if (warp == 0) factor_block(s, 0, nb, row0, step, more, info);
     for (int b = 0; b < blocks; ++b) {
         const int b0 = b * kB, r0 = b0 + kB;
         const bool last = b + 1 == blocks;
@@ -215,14 +237,12 @@ __device__ void factor_cta(Smem &s, double *A, int nb, int ld, int row0, int *in
                 const double *v = s.A + (r0 + q / (kB / 2)) * kPitch + b0 + 2 * (q % (kB / 2));
                 for (int c = 1; c < kCluster; ++c) store_remote(remote(v, c), v[0], v[1]);
             }
-            raise_flag(&s.flag_p[b]);
-            for (int j = b0; j < min(r0, nb); ++j)  // column block b of L, zero above the diagonal
-                for (int i = lane; i < nb; i += 32) A[(size_t)j * ld + i] = i >= j ? s.A[i * kPitch + j] : 0.0;
+            if (!last) raise_flag(&s.flag_p[b]);
         }
         if (last) break;
         if (warp == 0) {
             asm volatile("bar.sync 1, 128;" ::: "memory");  // the next diagonal block is up to date
-            factor_block(s, b + 1, nb, row0, act, info);
+            factor_block(s, b + 1, nb, row0, step, more, info);
             continue;
         }
         if (warp == 4) continue;
@@ -253,6 +273,12 @@ __device__ void factor_cta(Smem &s, double *A, int nb, int ld, int row0, int *in
             for (int k = k0; k < r0; ++k) v = fma(-x[k], y[k], v);
             s.A[i * kPitch + j] = v;
         }
+    }
+    // L, zero above the diagonal
+#pragma unroll 4
+    for (int e = tid; e < kLeafRows * kLeafRows; e += kThreads) {
+        const int i = e % kLeafRows, j = e / kLeafRows;
+        if (i < nb && j < nb) A[(size_t)j * ld + i] = i >= j ? s.A[i * kPitch + j] : 0.0;
     }
 }
 
@@ -314,11 +340,22 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads)
     const int tid = threadIdx.x;
     if (tid < kBlocks) s.flag_g[tid] = s.flag_p[tid] = 0;
     if (rank == 0) {
-        for (int e = tid; e < kLeafRows * kLeafRows; e += kThreads) {  // rows past nb: the identity
-            const int i = e % kLeafRows, j = e / kLeafRows;
-            double v = i == j ? 1.0 : 0.0;
-            if (i < nb && j < nb) v = i >= j ? A[(size_t)j * ld + i] : 0.0;
-            s.A[i * kPitch + j] = v;
+        constexpr int kLoads = kLeafRows * kLeafRows / kThreads;
+        double v[kLoads];
+#pragma unroll
+        for (int q = 0; q < kLoads; ++q) {  // rows past nb: the identity
+            const int e = tid + q * kThreads, i = e % kLeafRows, j = e / kLeafRows;
+            v[q] = i == j ? 1.0 : 0.0;
+            if (i < nb && j < nb && i >= j) v[q] = A[(size_t)j * ld + i];
+        }
+#pragma unroll
+        for (int q = 0; q < kLoads; ++q) {
+            const int e = tid + q * kThreads, i = e % kLeafRows, j = e / kLeafRows;
+            s.A[i * kPitch + j] = v[q];
+        }
+        if (tid == 0) {
+            s.zero = 0.0;
+            s.one = 1.0;
         }
     }
     cluster_barrier();  // flags and A in place
