@@ -775,8 +775,8 @@ struct ChebState {
     // BF16X3 on the hand-written tcgen05 GEMM: Hs and the order's block split in three BF16 terms
     bool umma = false;
     int usplits = 1;           // K split of the tensor-core GEMM (partial tiles in Y)
-    __nv_bfloat16 *hsplit[3] = {nullptr, nullptr, nullptr};  // N rows of ld (Hs symmetric: row = column)
-    __nv_bfloat16 *vsplit[3] = {nullptr, nullptr, nullptr};  // 2m rows of ld (K-major block)
+    unsigned char *hpack = nullptr;  // Hs in three BF16 terms, packed for the tensor cores
+    unsigned char *vpack = nullptr;  // v_{k-1} likewise
     double *Ht = nullptr;    // FP64 H~
     void *Hs = nullptr;      // scaled, launch precision
     void *vbuf = nullptr;
@@ -839,11 +839,9 @@ struct ChebState {
         if (Y) cudaFree(Y);
         if (Vf) cudaFree(Vf);
         Y = Vf = nullptr;
-        for (int t = 0; t < 3; ++t) {
-            if (hsplit[t]) cudaFree(hsplit[t]);
-            if (vsplit[t]) cudaFree(vsplit[t]);
-            hsplit[t] = vsplit[t] = nullptr;
-        }
+        if (hpack) cudaFree(hpack);
+        if (vpack) cudaFree(vpack);
+        hpack = vpack = nullptr;
         umma = false;
         if (oz) {
             oz->release();
@@ -983,7 +981,7 @@ int cheb_prepare(ChebState &cs, double dt, double tol, const double *h = nullptr
     if (cs.oz && !cs.rows)  // the tensor-core propagation reads Hs as BF16 slices
         if (int rc = cs.oz->slice(static_cast<const double *>(cs.Hs), st)) return rc;
     if (cs.umma && !h) {  // the tensor-core GEMM reads Hs as three BF16 terms
-        if (int rc = split3_bf16(reinterpret_cast<const float *>(cs.Hs), cs.N, cs.N, cs.ld, cs.hsplit, cs.ld, false, st))
+        if (int rc = umma_pack_h(reinterpret_cast<const float *>(cs.Hs), cs.N, cs.ld, cs.hpack, st))
             return rc;
     }
     return ELHL_OK;
@@ -1317,10 +1315,8 @@ int cheb_gemm_enqueue(ChebState &cs, int parity) {
     for (int k = 1; k <= cs.K; ++k) {
         const float *vprev = reinterpret_cast<const float *>(vb + ((k + 2) % 3) * vs);
         if (cs.umma) {  // Y (N x 2m) = Hs V^T on the tensor cores (Hs symmetric), three BF16 terms each
-            if (int rc = split3_bf16(vprev, n, 2 * m, 2 * m, cs.vsplit, cs.ld, true, st)) return rc;
-            if (int rc = umma_bf16x3_gemm(cs.hsplit, cs.ld, cs.vsplit, cs.ld, n, n, 2 * m, cs.usplits, cs.Y,
-                                          g_ctx.err, st))
-                return rc;
+            if (int rc = umma_pack_v(vprev, n, 2 * m, cs.vpack, st)) return rc;
+            if (int rc = umma_bf16x3_gemm(cs.hpack, cs.vpack, n, n, 2 * m, cs.usplits, cs.Y, g_ctx.err, st)) return rc;
         } else if (int rc = gemm_vt(g_ctx.blas_tc, cs.precision, 2 * m, n, vprev,
                                     reinterpret_cast<const float *>(cs.Hs), cs.ld, cs.Y)) {
             return rc;
@@ -3094,10 +3090,9 @@ int elhl_traj_create(const elhl_basis_desc *basis, const double *coords, const e
             if (!rc) rc = dev_alloc(&cs.gpops, (size_t)cs.P * (cs.nfrag + 1));
             // BF16X3 with 16, 32 or 64 columns: the hand-written tcgen05 GEMM (else cuBLAS emulation)
             if (!rc && cs.precision == ELHL_PREC_BF16X3 && umma_supported_n2(2 * cs.m)) {
-                for (int t = 0; t < 3 && !rc; ++t)
-                    if (cudaMalloc(&cs.hsplit[t], (size_t)cs.ld * cs.N * sizeof(__nv_bfloat16)) != cudaSuccess ||
-                        cudaMalloc(&cs.vsplit[t], (size_t)cs.ld * 2 * cs.m * sizeof(__nv_bfloat16)) != cudaSuccess)
-                        rc = ELHL_ERR_OOM;
+                if (!rc && (cudaMalloc(&cs.hpack, umma_a_bytes(cs.N)) != cudaSuccess ||
+                            cudaMalloc(&cs.vpack, umma_b_bytes(cs.N, 2 * cs.m)) != cudaSuccess))
+                    rc = ELHL_ERR_OOM;
                 cs.usplits = umma_splits(cs.N, cs.N);
                 if (!rc && cs.usplits > 1) {  // Y holds one partial tile per split
                     cudaFree(cs.Y);
@@ -3107,8 +3102,7 @@ int elhl_traj_create(const elhl_basis_desc *basis, const double *coords, const e
                 }
                 if (!rc) {
                     cs.umma = true;
-                    rc = split3_bf16(reinterpret_cast<const float *>(cs.Hs), cs.N, cs.N, cs.ld, cs.hsplit, cs.ld,
-                                     false, g_ctx.stream);
+                    rc = umma_pack_h(reinterpret_cast<const float *>(cs.Hs), cs.N, cs.ld, cs.hpack, g_ctx.stream);
                 }
             }
         }

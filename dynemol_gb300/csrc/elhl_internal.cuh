@@ -190,15 +190,16 @@ cudaError_t launch_cheb_rows_df64(const RowsLaunch &L, int rows, cudaStream_t st
 
 // Split-precision tensor-core GEMM (umma_gemm.cu): sum over s < splits of Y_s
 // (rows x n2, row-major FP32, Y_s = Y + s rows n2) = sum over the BF16 terms
-// (i + j <= 2) of A_i (rows x K, K contiguous, ld lda) times B_j^T (B_j: n2 x K,
-// ld ldb).  n2 in {32, 64, 128}; umma_splits picks the K split.
-size_t umma_smem_bytes(int n2);
+// (i + j <= 2) of A_i (rows x K) times B_j^T (B_j: n2 x K), both packed by
+// umma_pack_h / umma_pack_v.  n2 in {32, 64, 128}; umma_splits picks the K split.
 int umma_supported_n2(int n2);
 int umma_splits(int rows, int K);
-int split3_bf16(const float *src, int rows, int cols, int lds, __nv_bfloat16 *const dst[3], int ldd, bool transpose,
-                cudaStream_t st);
-int umma_bf16x3_gemm(const __nv_bfloat16 *const A[3], int lda, const __nv_bfloat16 *const B[3], int ldb, int rows,
-                     int K, int n2, int splits, float *Y, int *d_error, cudaStream_t st);
+size_t umma_a_bytes(int N);
+size_t umma_b_bytes(int N, int n2);
+int umma_pack_h(const float *H, int N, int ld, void *dst, cudaStream_t st);
+int umma_pack_v(const float *v, int n, int n2, void *dst, cudaStream_t st);
+int umma_bf16x3_gemm(const void *A, const void *B, int rows, int K, int n2, int splits, float *Y, int *d_error,
+                     cudaStream_t st);
 
 // FP64 Chebyshev propagation by exact BF16 slices on the tensor cores
 // (ozaki.cu), one grid phase per order on an explicit Hs.  An order's work:

@@ -106,12 +106,6 @@ __device__ __forceinline__ int scale_exp(double x) {
 // byte offset of (row R, K index kk) in a 128B-swizzled K-major tile of 128-byte rows
 __device__ __forceinline__ int swz_off(int R, int kk) { return R * 128 + (((kk >> 3) ^ (R & 7)) << 4) + ((kk & 7) << 1); }
 
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
 // generic-proxy global writes made visible to (and ordered with) the async proxy
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
