@@ -190,7 +190,7 @@ __device__ void produce(const Ctx &c, const OzLaunch &L, const CUtensorMap *map,
             const int kb = walk_kb(sg, ki, rev);
             for (int a = 0; a < kS; ++a) {
                 const unsigned s = r.acnt % kAStages;
-                if (r.acnt >= kAStages && !mbar_wait(&c.empty[s], ((r.acnt / kAStages) - 1) & 1, now_ns(), kWaitNs)) {
+                if (r.acnt >= kAStages && !mbar_wait(&c.empty[s], ((r.acnt / kAStages) - 1) & 1, kWaitNs)) {
                     set_abort(c, L.error);
                     return;
                 }
@@ -205,19 +205,21 @@ __device__ void produce(const Ctx &c, const OzLaunch &L, const CUtensorMap *map,
 }
 
 // One block per accumulator buffer: over 64 K every weight's sum of slice
-// products stays below 2^23.2, exact in FP32.
+// products stays below 2^23.2, exact in FP32.  Warp 1 as one: descriptors that a
+// single lane computes cost 37 cycles per MMA, in a converged warp with one lane
+// elected around the MMAs they stay in uniform registers.
 __device__ void issue_mma(const Ctx &c, const OzLaunch &L, Roles &r, bool rev) {
     const int s0 = L.seg_begin[blockIdx.x], s1 = L.seg_begin[blockIdx.x + 1];
     for (int qi = 0; qi < s1 - s0; ++qi) {
         const OzSeg sg = L.segs[walk_seg(s0, s1, qi, rev)];
         for (int ki = 0; ki < sg.kb1 - sg.kb0; ++ki) {
             const unsigned tb = r.gcnt & 1;
-            if (r.gcnt >= 2 && !mbar_wait(&c.accempty[tb], ((r.gcnt >> 1) - 1) & 1, now_ns(), kWaitNs)) {
+            if (r.gcnt >= 2 && !mbar_wait_warp(&c.accempty[tb], ((r.gcnt >> 1) - 1) & 1, kWaitNs)) {
                 set_abort(c, L.error);
                 return;
             }
             const unsigned sb = r.bcnt % kBStages;
-            if (!mbar_wait(&c.bfull[sb], (r.bcnt / kBStages) & 1, now_ns(), kWaitNs)) {
+            if (!mbar_wait_warp(&c.bfull[sb], (r.bcnt / kBStages) & 1, kWaitNs)) {
                 set_abort(c, L.error);
                 return;
             }
@@ -226,7 +228,7 @@ __device__ void issue_mma(const Ctx &c, const OzLaunch &L, Roles &r, bool rev) {
 #pragma unroll
             for (int a = 0; a < kS; ++a) {
                 const unsigned s = r.acnt % kAStages;
-                if (!mbar_wait(&c.full[s], (r.acnt / kAStages) & 1, now_ns(), kWaitNs)) {
+                if (!mbar_wait_warp(&c.full[s], (r.acnt / kAStages) & 1, kWaitNs)) {
                     set_abort(c, L.error);
                     return;
                 }
@@ -235,15 +237,20 @@ __device__ void issue_mma(const Ctx &c, const OzLaunch &L, Roles &r, bool rev) {
                 const uint64_t db = smem_desc_sw128(btile + mma_brow(a) * 128);
                 const uint32_t acc = c.tmem + tb * kAccCols + (uint32_t)mma_col(a);
                 const uint32_t idesc = idesc_bf16(kTileM, mma_n(a));
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < kKB / 16; ++k)  // K = 16 per MMA: +32 bytes along the swizzled row
-                    umma_bf16(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, !(a == 0 && k == 0));
-                umma_commit(&c.empty[s]);  // the A stage is free once these MMAs have read it
+                    for (int k = 0; k < kKB / 16; ++k)  // K = 16 per MMA: +32 bytes along the swizzled row
+                        umma_bf16(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, !(a == 0 && k == 0));
+                    umma_commit(&c.empty[s]);  // the A stage is free once these MMAs have read it
+                    if (a == kS - 1) {
+                        umma_commit(&c.bempty[sb]);
+                        umma_commit(&c.accfull[tb]);
+                    }
+                }
+                __syncwarp();
                 ++r.acnt;
             }
-            umma_commit(&c.bempty[sb]);
             ++r.bcnt;
-            umma_commit(&c.accfull[tb]);
             ++r.gcnt;
         }
     }
@@ -635,7 +642,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(c.smem + SmemLayout::misc_off);
     c.abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
     c.last_flag = reinterpret_cast<unsigned *>(tmem_slot + 2);
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
     if (threadIdx.x == 0) {
         for (int s = 0; s < kAStages; ++s) {
             mbar_init(&c.full[s], 1);
@@ -683,7 +690,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             continue;
         }
         if (warp == 1) {
-            if ((threadIdx.x & 31) == 0) issue_mma(c, L, r, k & 1);
+            issue_mma(c, L, r, k & 1);
             ok = !aborted(c) && *(volatile int *)L.error == 0;
             continue;
         }
@@ -722,9 +729,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (unsigned q = r.bcnt - n; q < r.bcnt; ++q)
             mbar_wait(&c.bfull[q % kBStages], (q / kBStages) & 1, now_ns(), kWaitNs);
     }
-    if (threadIdx.x == 32) {
-        umma_commit(c.done);
-        mbar_wait(c.done, 0, now_ns(), kWaitNs);
+    if (warp == 1) {
+        __syncwarp();
+        if (elect_one()) umma_commit(c.done);
+        mbar_wait_warp(c.done, 0, kWaitNs);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();

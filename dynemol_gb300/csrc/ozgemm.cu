@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + Smem::misc_off);
     int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
     unsigned *flag = reinterpret_cast<unsigned *>(tmem_slot + 2);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kAStages; ++s) {
             mbar_init(&full[s], 1);
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         unsigned acnt = 0;
         for (int kb = kb0, bi = 0; kb < kb1; ++kb, ++bi) {
             const int sb = bi % kBStages;
-            if (bi >= kBStages && !mbar_wait(&bempty[sb], ((bi / kBStages) - 1) & 1, now_ns(), kWaitNs)) {
+            if (bi >= kBStages && !mbar_wait(&bempty[sb], ((bi / kBStages) - 1) & 1, kWaitNs)) {
                 atomicExch(abort_flag, 1);
                 break;
             }
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             bool stop = false;
             for (int a = 0; a < kS; ++a) {
                 const unsigned s = acnt % kAStages;
-                if (acnt >= kAStages && !mbar_wait(&empty[s], ((acnt / kAStages) - 1) & 1, now_ns(), kWaitNs)) {
+                if (acnt >= kAStages && !mbar_wait(&empty[s], ((acnt / kAStages) - 1) & 1, kWaitNs)) {
                     atomicExch(abort_flag, 1);
                     stop = true;
                     break;
@@ -276,25 +276,27 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (stop) break;
         }
         issued = acnt;
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issuer
+    } else if (warp == 1) {
+        // ---- MMA issuer (the warp as one, one lane elected around the MMAs: the
+        // descriptors stay in uniform registers)
         unsigned acnt = 0;
         for (int kb = kb0, bi = 0; kb < kb1; ++kb, ++bi) {
             const unsigned tb = bi & 1, sb = bi % kBStages;
-            if (bi >= 2 && !mbar_wait(&accempty[tb], ((bi >> 1) - 1) & 1, now_ns(), kWaitNs)) {
-                atomicExch(abort_flag, 1);
+            if (bi >= 2 && !mbar_wait_warp(&accempty[tb], ((bi >> 1) - 1) & 1, kWaitNs)) {
+                if (lane == 0) atomicExch(abort_flag, 1);
                 break;
             }
-            if (!mbar_wait(&bfull[sb], (bi / kBStages) & 1, now_ns(), kWaitNs)) {
-                atomicExch(abort_flag, 1);
+            if (!mbar_wait_warp(&bfull[sb], (bi / kBStages) & 1, kWaitNs)) {
+                if (lane == 0) atomicExch(abort_flag, 1);
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;");
             bool stop = false;
+#pragma unroll
             for (int a = 0; a < kS; ++a) {
                 const unsigned s = acnt % kAStages;
-                if (!mbar_wait(&full[s], (acnt / kAStages) & 1, now_ns(), kWaitNs)) {
-                    atomicExch(abort_flag, 1);
+                if (!mbar_wait_warp(&full[s], (acnt / kAStages) & 1, kWaitNs)) {
+                    if (lane == 0) atomicExch(abort_flag, 1);
                     stop = true;
                     break;
                 }
@@ -306,15 +308,20 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint64_t db = smem_desc_sw128(smem + Smem::b_off + (size_t)sb * kBStage);
                 const uint32_t acc = tmem + tb * kAccCols + (uint32_t)(a * kTN);
                 const uint32_t idesc = idesc_bf16(kTM, kTN * (kS - a));
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < kKB / 16; ++k)  // the first MMA (a = 0: all weights) starts the block
-                    umma_bf16(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, !(a == 0 && k == 0));
-                umma_commit(&empty[s]);
+                    for (int k = 0; k < kKB / 16; ++k)  // the first MMA (a = 0: all weights) starts the block
+                        umma_bf16(acc, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, !(a == 0 && k == 0));
+                    umma_commit(&empty[s]);
+                    if (a == kS - 1) {
+                        umma_commit(&bempty[sb]);
+                        umma_commit(&accfull[tb]);
+                    }
+                }
+                __syncwarp();
                 ++acnt;
             }
             if (stop) break;
-            umma_commit(&bempty[sb]);
-            umma_commit(&accfull[tb]);
         }
     } else if (warp >= 2) {
         // ---- fold the weights of each block into H and L, then write C
@@ -330,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         bool ok = true;
         for (int bi = 0; bi < kb1 - kb0; ++bi) {
             const unsigned tb = bi & 1;
-            if (t == 0) *flag = mbar_wait(&accfull[tb], (bi >> 1) & 1, now_ns(), kWaitNs) ? 1u : 0u;
+            if (t == 0) *flag = mbar_wait(&accfull[tb], (bi >> 1) & 1, kWaitNs) ? 1u : 0u;
             asm volatile("bar.sync 1, 128;" ::: "memory");
             ok = *(volatile unsigned *)flag != 0;
             asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -370,11 +377,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     // drain: loads and MMAs complete before the CTA frees its TMEM and leaves
     if (warp == 0 && lane == 0) {
         const unsigned n = min(issued, (unsigned)kAStages);
-        for (unsigned q = issued - n; q < issued; ++q) mbar_wait(&full[q % kAStages], (q / kAStages) & 1, now_ns(), kWaitNs);
+        for (unsigned q = issued - n; q < issued; ++q) mbar_wait(&full[q % kAStages], (q / kAStages) & 1, kWaitNs);
     }
-    if (warp == 1 && lane == 0) {
-        umma_commit(done);
-        mbar_wait(done, 0, now_ns(), kWaitNs);
+    if (warp == 1) {
+        __syncwarp();
+        if (elect_one()) umma_commit(done);
+        mbar_wait_warp(done, 0, kWaitNs);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();

@@ -60,6 +60,31 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, u
         : "memory");
 }
 
+// the same, limit_ns from the first look (the clock is read only if that fails)
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, unsigned long long limit_ns) {
+    const unsigned a = smem_u32(bar);
+    unsigned long long t0 = 0;
+    while (true) {
+        unsigned done = 0;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (done) return true;
+        const unsigned long long t = now_ns();
+        if (!t0) t0 = t;
+        if (t - t0 > limit_ns) return false;
+    }
+}
+
+// the same by a converged warp, which stays converged: one answer for all lanes
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned parity, unsigned long long limit_ns) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit_ns));
+}
+
 // `bytes` (a multiple of 16) from global to shared memory, counted on the mbarrier
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(

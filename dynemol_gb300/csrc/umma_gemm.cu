@@ -54,11 +54,6 @@ constexpr unsigned long long kWaitNs = 2000000000ull;
 
 using namespace tc;
 
-// bounded wait (kWaitNs) for the phase with the given parity
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, unsigned long long t0) {
-    return tc::mbar_wait(bar, parity, t0, kWaitNs);
-}
-
 struct UmmaParams {
     const unsigned char *A, *B;  // packed operands
     int rows, K;           // Y is rows x N2; the packed operands are zero past K
@@ -124,7 +119,6 @@ __global__ void __launch_bounds__(UmmaShape<N2>::kThreads, 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tmem_slot;
-    const unsigned long long t0 = now_ns();
 
     if (warp == 0 && lane == 0) {
         // ---- TMA producer
@@ -133,7 +127,7 @@ __global__ void __launch_bounds__(UmmaShape<N2>::kThreads, 1)
         int issued = 0;
         for (int kc = 0; kc < nk; ++kc) {
             const int s = kc % kStages;
-            if (kc >= kStages && !mbar_wait(&empty[s], ((kc / kStages) - 1) & 1, t0)) {
+            if (kc >= kStages && !mbar_wait(&empty[s], ((kc / kStages) - 1) & 1, kWaitNs)) {
                 atomicExch(abort_flag, 1);
                 break;
             }
@@ -149,7 +143,7 @@ __global__ void __launch_bounds__(UmmaShape<N2>::kThreads, 1)
         }
         // loads still in flight land before the CTA ends: wait for every issued stage
         for (int kc = (issued > kStages ? issued - kStages : 0); kc < issued; ++kc)
-            mbar_wait(&full[kc % kStages], (kc / kStages) & 1, now_ns());
+            mbar_wait(&full[kc % kStages], (kc / kStages) & 1, kWaitNs);
     } else if (warp == 1) {
         // ---- MMA issuer (the warp as one, so that descriptors stay in uniform registers)
         const uint32_t idesc = idesc_bf16(kBM, N2);
@@ -157,8 +151,8 @@ __global__ void __launch_bounds__(UmmaShape<N2>::kThreads, 1)
         const int pb[kNumPairs] = {0, 1, 0, 2, 1, 0};
         for (int kc = 0; kc < nk; ++kc) {
             const int s = kc % kStages, set = kc & 1;
-            if (!mbar_wait(&full[s], (kc / kStages) & 1, t0) ||
-                (kc >= 2 && !mbar_wait(&set_empty[set], ((kc >> 1) - 1) & 1, t0))) {
+            if (!mbar_wait_warp(&full[s], (kc / kStages) & 1, kWaitNs) ||
+                (kc >= 2 && !mbar_wait_warp(&set_empty[set], ((kc >> 1) - 1) & 1, kWaitNs))) {
                 if (lane == 0) atomicExch(abort_flag, 1);
                 break;
             }
@@ -195,7 +189,7 @@ __global__ void __launch_bounds__(UmmaShape<N2>::kThreads, 1)
         bool ok = true;
         for (int kc = 0; kc < nk; ++kc) {
             const int set = kc & 1;
-            if (lane == 0) ok = mbar_wait(&set_full[set], (kc >> 1) & 1, t0) && !*(volatile int *)abort_flag;
+            if (lane == 0) ok = mbar_wait(&set_full[set], (kc >> 1) & 1, kWaitNs) && !*(volatile int *)abort_flag;
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;");
@@ -229,7 +223,7 @@ __global__ void __launch_bounds__(UmmaShape<N2>::kThreads, 1)
         } else if (lane == 0) {
             atomicExch(abort_flag, 1);
         }
-        if (lane == 0) mbar_wait(done, 0, now_ns());  // no MMA in flight when the TMEM is freed
+        if (lane == 0) mbar_wait(done, 0, kWaitNs);  // no MMA in flight when the TMEM is freed
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
