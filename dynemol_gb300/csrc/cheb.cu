@@ -183,7 +183,7 @@ struct OrderEpi {
     const T2 *vprev2;
     T2 *vout;
     double2 *acc;
-    int k, m, g;
+    int k, m, col0;
     double cre, cim;
     const T2 *vprev1;  // implicit operator: y -= shift v_{k-1}; nullptr for an explicit Hs
     T shift;
@@ -210,7 +210,7 @@ struct OrderEpi {
                     v.y = two_sum_plus(__fmul_rn(2.f, yi), -w2.y, __fmul_rn(2.f, di));
                 }
                 vout[(size_t)i * MG + c] = v;
-                const size_t ao = (size_t)i * m + g * MG + c;
+                const size_t ao = (size_t)i * m + col0 + c;
                 double2 a = acc[ao];
                 const double vr = (double)v.x, vi = (double)v.y;
                 a.x += cre * vr - cim * vi;
@@ -234,7 +234,7 @@ struct OrderEpi {
             v.y = T(2) * yi - w2.y;
         }
         vout[(size_t)i * MG + c] = v;
-        const size_t ao = (size_t)i * m + g * MG + c;
+        const size_t ao = (size_t)i * m + col0 + c;
         double2 a = acc[ao];
         const double vr = (double)v.x, vi = (double)v.y;
         a.x += cre * vr - cim * vi;
@@ -255,22 +255,39 @@ struct AccEpi {
     }
 };
 
-// one order k >= 1 for the rows of segment sg, column group g (MG columns);
+// The column groups of m columns: as many of MG as fit, then two, then one.  A group's
+// vectors lie together, [ldv][width], after those of the columns before it.  One kernel
+// serves problems of any column counts side by side.
+// f(width as a type, first column)
+template <int MG, typename F>
+__device__ __forceinline__ void column_groups(int m, F f) {
+    int c = 0;
+    for (; c + MG <= m; c += MG) f(std::integral_constant<int, MG>{}, c);
+    if constexpr (MG > 2)
+        if (c + 2 <= m) {
+            f(std::integral_constant<int, 2>{}, c);
+            c += 2;
+        }
+    if constexpr (MG > 1)
+        if (c < m) f(std::integral_constant<int, 1>{}, c);
+}
+
+// one order k >= 1 for the rows of segment sg, the MG columns from col0 on;
 // jwin > 0: the previous vector is staged in windows of jwin rows
 template <typename T, int MG>
-__device__ void order_rows(const ChebProblem &pb, const ChebSegment &sg, int k, int g, int parity,
+__device__ void order_rows(const ChebProblem &pb, const ChebSegment &sg, int k, int col0, int parity,
                            typename Vec2<T>::type *s_v, T *s_part, double cre, double cim, int jwin,
                            typename Vec2<T>::type *s_y) {
     using T2 = typename Vec2<T>::type;
     const int tid = threadIdx.x;
     const int ld = pb.ld, m = pb.m;
     T2 *vbuf = reinterpret_cast<T2 *>(pb.vbuf);
-    const size_t gstride = (size_t)pb.ldv * MG;         // one column group
-    const size_t bstride = gstride * (m / MG);          // one of the three vector buffers
-    const T2 *vprev = vbuf + (size_t)((k + 2) % 3) * bstride + g * gstride;   // v_{k-1}
-    OrderEpi<T, MG> epi{vbuf + (size_t)((k + 1) % 3) * bstride + g * gstride,
-                        vbuf + (size_t)(k % 3) * bstride + g * gstride,
-                        pb.col[parity ^ 1], k, m, g, cre, cim, nullptr, T(0), pb.dcorr, vprev};
+    const size_t goff = (size_t)pb.ldv * col0;          // the column group
+    const size_t bstride = (size_t)pb.ldv * m;          // one of the three vector buffers
+    const T2 *vprev = vbuf + (size_t)((k + 2) % 3) * bstride + goff;   // v_{k-1}
+    OrderEpi<T, MG> epi{vbuf + (size_t)((k + 1) % 3) * bstride + goff,
+                        vbuf + (size_t)(k % 3) * bstride + goff,
+                        pb.col[parity ^ 1], k, m, col0, cre, cim, nullptr, T(0), pb.dcorr, vprev};
     if (jwin == 0 || ld <= jwin) {  // the whole previous vector in shared memory
         __syncthreads();
         for (int q = tid; q < ld * MG; q += kBlock) s_v[q] = ldcg2(vprev + q);  // padding rows are zero
@@ -310,21 +327,21 @@ struct StoreEpi {
     }
 };
 
-// Phase ph of order k >= 1 of an implicit problem, column group g, over the
-// CTA's segments [s0, s1): 0: w = G^T v_{k-1};  1: y = (h/b) w;
+// Phase ph of order k >= 1 of an implicit problem, the MG columns from col0 on, over
+// the CTA's segments [s0, s1): 0: w = G^T v_{k-1};  1: y = (h/b) w;
 // 2: v_k from G y - shift v_{k-1} (recurrence + accumulation).  The staged
 // vector is shared by all of the CTA's segments.
 template <typename T, int MG>
-__device__ void implicit_phase(const ChebLaunch &L, const ChebProblem &pb, int s0, int s1, int k, int ph, int g,
+__device__ void implicit_phase(const ChebLaunch &L, const ChebProblem &pb, int s0, int s1, int k, int ph, int col0,
                                typename Vec2<T>::type *s_v, T *s_part, double cre, double cim) {
     using T2 = typename Vec2<T>::type;
     const int ld = pb.ld, m = pb.m;
     T2 *vbuf = reinterpret_cast<T2 *>(pb.vbuf);
     T2 *wb = reinterpret_cast<T2 *>(pb.wb);
-    const size_t gstride = (size_t)pb.ldv * MG;
-    const size_t bstride = gstride * (m / MG);
-    const T2 *vprev = vbuf + (size_t)((k + 2) % 3) * bstride + g * gstride;  // v_{k-1}
-    const T2 *src = ph == 0 ? vprev : wb + (size_t)(ph - 1) * bstride + g * gstride;
+    const size_t goff = (size_t)pb.ldv * col0;
+    const size_t bstride = (size_t)pb.ldv * m;
+    const T2 *vprev = vbuf + (size_t)((k + 2) % 3) * bstride + goff;  // v_{k-1}
+    const T2 *src = ph == 0 ? vprev : wb + (size_t)(ph - 1) * bstride + goff;
     const ChebSegment *segs = L.segs;
     if (ph == 1 && L.segs_full) {  // the full phase has its own even row split
         segs = L.segs_full;
@@ -338,15 +355,15 @@ __device__ void implicit_phase(const ChebLaunch &L, const ChebProblem &pb, int s
     for (int s = s0; s < s1; ++s) {
         const ChebSegment sg = segs[s];
         if (ph == 0) {
-            StoreEpi<T, MG> epi{wb + g * gstride};
+            StoreEpi<T, MG> epi{wb + goff};
             rows_gemv<T, MG, 1>(reinterpret_cast<const T *>(pb.G), ld, s_v, sg.row0, sg.row1, s_part, epi);
         } else if (ph == 1) {
-            StoreEpi<T, MG> epi{wb + bstride + g * gstride};
+            StoreEpi<T, MG> epi{wb + bstride + goff};
             rows_gemv<T, MG, 0>(reinterpret_cast<const T *>(pb.H), ld, s_v, sg.row0, sg.row1, s_part, epi);
         } else {
-            OrderEpi<T, MG> epi{vbuf + (size_t)((k + 1) % 3) * bstride + g * gstride,
-                                vbuf + (size_t)(k % 3) * bstride + g * gstride,
-                                pb.col[L.parity ^ 1], k, m, g, cre, cim, vprev, (T)pb.shift, nullptr, nullptr};
+            OrderEpi<T, MG> epi{vbuf + (size_t)((k + 1) % 3) * bstride + goff,
+                                vbuf + (size_t)(k % 3) * bstride + goff,
+                                pb.col[L.parity ^ 1], k, m, col0, cre, cim, vprev, (T)pb.shift, nullptr, nullptr};
             rows_gemv<T, MG, 2>(reinterpret_cast<const T *>(pb.Gt), ld, s_v, sg.row0, sg.row1, s_part, epi);
         }
     }
@@ -358,13 +375,16 @@ __device__ void order_zero(const ChebProblem &pb, const ChebSegment &sg, int par
     using T2 = typename Vec2<T>::type;
     T2 *v0 = reinterpret_cast<T2 *>(pb.vbuf);
     const int m = pb.m;
-    const size_t gstride = (size_t)pb.ldv * MG;
     const double cre = pb.coef[0].x, cim = pb.coef[0].y;
     const double2 *phi = pb.col[parity];
     double2 *acc = pb.col[parity ^ 1];
     for (int q = threadIdx.x; q < (sg.row1 - sg.row0) * m; q += kBlock) {
         const int i = sg.row0 + q / m, col = q % m;
-        const int g = col / MG, c = col % MG;
+        int w = MG, c0 = col / MG * MG;  // the column's group
+        while (c0 + w > m) {
+            w >>= 1;
+            c0 = col / w * w;
+        }
         const size_t o = (size_t)i * m + col;
         double2 p = phi[o];
         if (pb.scale) {
@@ -375,7 +395,7 @@ __device__ void order_zero(const ChebProblem &pb, const ChebSegment &sg, int par
         T2 v;
         v.x = (T)p.x;
         v.y = (T)p.y;
-        v0[g * gstride + (size_t)i * MG + c] = v;
+        v0[(size_t)pb.ldv * c0 + (size_t)i * w + (col - c0)] = v;
         acc[o] = make_double2(cre * p.x - cim * p.y, cre * p.y + cim * p.x);
     }
 }
@@ -401,8 +421,9 @@ __global__ void __launch_bounds__(kBlock, 1) cheb_kernel(ChebLaunch L) {
                     for (int s = s0; s < s1; ++s) order_zero<T, MG>(pb, L.segs[s], L.parity);
                 } else if (k <= pb.K) {
                     const double cre = pb.coef[k].x, cim = pb.coef[k].y;
-                    for (int g = 0; g < pb.m / MG; ++g)
-                        implicit_phase<T, MG>(L, pb, s0, s1, k, ph, g, s_v, s_part, cre, cim);
+                    column_groups<MG>(pb.m, [&](auto w, int col0) {
+                        implicit_phase<T, decltype(w)::value>(L, pb, s0, s1, k, ph, col0, s_v, s_part, cre, cim);
+                    });
                 }
             } else {
                 for (int s = s0; s < s1; ++s) {
@@ -413,9 +434,10 @@ __global__ void __launch_bounds__(kBlock, 1) cheb_kernel(ChebLaunch L) {
                         order_zero<T, MG>(pb, sg, L.parity);
                     } else {
                         const double cre = pb.coef[k].x, cim = pb.coef[k].y;
-                        for (int g = 0; g < pb.m / MG; ++g)
-                            order_rows<T, MG>(pb, sg, k, g, L.parity, s_v, s_part, cre, cim, L.jwin,
-                                              s_v + (size_t)L.jwin * MG);
+                        column_groups<MG>(pb.m, [&](auto w, int col0) {
+                            order_rows<T, decltype(w)::value>(pb, sg, k, col0, L.parity, s_v, s_part, cre, cim, L.jwin,
+                                                              s_v + (size_t)L.jwin * MG);
+                        });
                     }
                 }
             }
@@ -453,23 +475,24 @@ __global__ void __launch_bounds__(kBlock, 1) readout_kernel(ChebLaunch L) {
             const T *M = reinterpret_cast<const T *>(pass == 0 ? pb.A : pb.B);
             const int src0 = (pass == 1 && m == 2 * P) ? P : 0;
             double2 *out = pass == 0 ? pb.psi : pb.bra;
-            for (int g = 0; g < P / MG; ++g) {
+            column_groups<MG>(P, [&](auto width, int col0) {
+                constexpr int W = decltype(width)::value;
                 __syncthreads();
-                for (int q = tid; q < ld * MG; q += kBlock) {
-                    const int j = q / MG, c = q % MG;
-                    const double2 v = j < pb.N ? __ldcg(cols + (size_t)j * m + src0 + g * MG + c) : make_double2(0, 0);
+                for (int q = tid; q < ld * W; q += kBlock) {
+                    const int j = q / W, c = q % W;
+                    const double2 v = j < pb.N ? __ldcg(cols + (size_t)j * m + src0 + col0 + c) : make_double2(0, 0);
                     T2 t;
                     t.x = (T)v.x;
                     t.y = (T)v.y;
                     s_v[q] = t;
                 }
                 __syncthreads();
-                ReadEpi<T, MG> epi{out, P, g * MG};
+                ReadEpi<T, W> epi{out, P, col0};
                 if (pass == 0)
-                    rows_gemv<T, MG, 1>(M, ld, s_v, sg.row0, sg.row1, s_part, epi);  // A = L^-1: j >= i
+                    rows_gemv<T, W, 1>(M, ld, s_v, sg.row0, sg.row1, s_part, epi);  // A = L^-1: j >= i
                 else
-                    rows_gemv<T, MG, 2>(M, ld, s_v, sg.row0, sg.row1, s_part, epi);  // B = L^T: j <= i
-            }
+                    rows_gemv<T, W, 2>(M, ld, s_v, sg.row0, sg.row1, s_part, epi);  // B = L^T: j <= i
+            });
         }
         __syncthreads();
         // population partials of this segment: Re conj(psi_ip) bra_ip per (column, fragment)
@@ -1049,11 +1072,11 @@ cudaError_t launch_readout_rows(const ChebProblem *probs, int N, int P, int pari
 int cheb_block() { return kBlock; }
 
 int cheb_group_size(int precision, int m, int max_ld, bool windowed) {
-    // the largest of 4, 2, 1 staged columns that divides m and fits in shared
-    // memory (windowed: the explicit propagation stages the vector in windows)
+    // the largest of 4, 2, 1 staged columns that is at most m (DF64: divides it) and fits
+    // in shared memory (windowed: the explicit propagation stages the vector in windows)
     const size_t c2 = (precision == ELHL_PREC_FP64 || precision == ELHL_PREC_DF64) ? sizeof(double2) : sizeof(float2);
     for (int mg : {4, 2, 1})
-        if (m % mg == 0 && (windowed || kCheb_part_bytes + (size_t)max_ld * mg * c2 <= kCheb_smem_limit)) return mg;
+        if ((precision == ELHL_PREC_DF64 ? m % mg == 0 : mg <= m) && (windowed || kCheb_part_bytes + (size_t)max_ld * mg * c2 <= kCheb_smem_limit)) return mg;
     return 0;
 }
 

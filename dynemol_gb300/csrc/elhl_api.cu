@@ -1396,7 +1396,7 @@ struct ChebPlan {
     int grid = 0, max_ld = 0, kmax = 0, mg = 0, mg_read = 0, precision = 0, parity = 0;
     int ro_precision = 0;      // element type of the read-out matrices (FP64 or the launch precision)
     int nphase = 1;            // 3: one implicit problem
-    int mgcd = 0;              // gcd of the problems' column counts
+    int mgcd = 0, mmax = 0;    // gcd and largest of the problems' column counts
     bool tuned = false;        // tile measured (on the plan's first run)
     OzRes *oz = nullptr;       // one ELHL_PREC_OZ64 trajectory: the tensor-core propagation
     ChebState *solo = nullptr; // the state of a plan of one problem
@@ -1407,10 +1407,19 @@ struct ChebPlan {
     }
 };
 
-int tune_plan(ChebPlan &pl, int mgcd);
+int tune_plan(ChebPlan &pl);
 
 // may the propagation stage its vector in windows? (explicit Hs, not in DF64)
 bool windowed_plan(int precision, bool implicit) { return !implicit && precision != ELHL_PREC_DF64; }
+
+// Time of one row of a problem relative to the other problems of a plan: its elements, in
+// FP64 and DF64 times its columns (the arithmetic), in FP32 times its column groups of up
+// to four (each reads the row again) and a quarter per column.
+double row_work(const ChebState &cs) {
+    const bool wide = cs.precision == ELHL_PREC_FP64 || cs.precision == ELHL_PREC_DF64;
+    const int rest = cs.m % 4, groups = cs.m / 4 + (rest & 1) + (rest >> 1);
+    return (double)cs.ld * (wide ? cs.m : groups + 0.25 * cs.m);
+}
 
 int cheb_plan(ChebPlan &pl, const std::vector<ChebState *> &states) {
     pl.release();
@@ -1424,28 +1433,27 @@ int cheb_plan(ChebPlan &pl, const std::vector<ChebState *> &states) {
     pl.kmax = 0;
     pl.precision = states[0]->precision;
     double work = 0.0;
-    int mgcd = 0;  // staged group size must divide every problem's column count
+    int mgcd = 0, mmax = 0, pmax = 1;
     for (auto *cs : states) {
+        mmax = std::max(mmax, cs->m);
+        pmax = std::max(pmax, cs->P);
         if (cs->precision != pl.precision || cs->m <= 0) return ELHL_ERR_BAD_ARG;
         pl.max_ld = std::max(pl.max_ld, cs->ld);
-        work += (double)cs->N * cs->ld;
+        work += (double)cs->N * row_work(*cs);
         int a = cs->m, b = mgcd;
         while (b) { const int t = a % b; a = b; b = t; }
         mgcd = a;
     }
     const bool implicit_plan = states[0]->implicit;
-    pl.mg = cheb_group_size(pl.precision, mgcd, pl.max_ld, windowed_plan(pl.precision, implicit_plan));
+    // DF64: the staged group divides every problem's column count; otherwise the kernels
+    // take the rest of a problem's columns in narrower groups
+    pl.mg = cheb_group_size(pl.precision, pl.precision == ELHL_PREC_DF64 ? mgcd : mmax, pl.max_ld,
+                            windowed_plan(pl.precision, implicit_plan));
     if (!pl.mg) return ELHL_ERR_UNSUPPORTED;
-    int pgcd = 0;  // read-out groups must divide every problem's ket columns
-    for (auto *cs : states) {
-        int a = std::max(cs->P, 1), b = pgcd;
-        while (b) { const int t = a % b; a = b; b = t; }
-        pgcd = a;
-    }
     pl.ro_precision = states[0]->ro64 ? ELHL_PREC_FP64 : pl.precision;
     for (auto *cs : states)
         if (cs->readout_ready && cs->ro64 != states[0]->ro64) return ELHL_ERR_UNSUPPORTED;  // one read-out type
-    pl.mg_read = cheb_group_size(pl.ro_precision, pgcd, pl.max_ld);
+    pl.mg_read = cheb_group_size(pl.ro_precision, pmax, pl.max_ld);
     pl.pops_per_step = 0;
     pl.parity = states[0]->parity;
     const bool implicit = states[0]->implicit;
@@ -1511,7 +1519,7 @@ int cheb_plan(ChebPlan &pl, const std::vector<ChebState *> &states) {
     double acc_w = 0.0;
     for (int q = 0; q < (int)states.size() && !implicit; ++q) {
         const ChebState *cs = states[q];
-        const double rw = cs->ld;  // work per row
+        const double rw = row_work(*cs);
         int r = 0;
         while (r < cs->N) {
             int take = cs->N - r;
@@ -1549,6 +1557,7 @@ int cheb_plan(ChebPlan &pl, const std::vector<ChebState *> &states) {
         CU_TRY(copy_h2d(pl.d_seg_full_begin, pl.seg_full_begin.data(), pl.seg_full_begin.size() * sizeof(int)));
     }
     pl.mgcd = mgcd;
+    pl.mmax = mmax;
     pl.tuned = false;  // measured on the first run (plans of batch members never run)
     pl.oz = states.size() == 1 ? states[0]->oz : nullptr;
     pl.solo = states.size() == 1 ? states[0] : nullptr;
@@ -1589,24 +1598,26 @@ ChebLaunch plan_launch(const ChebPlan &pl) {
 }
 
 // Autotuner of the propagation tile: the number of complex columns staged per
-// pass over the matrix (4, 2 or 1 where it divides every problem's column count
-// and fits in shared memory) sets the accumulator tile of every warp (row tile x
+// pass over the matrix (4, 2 or 1, at most the largest column count, where it fits in
+// shared memory; DF64: where it divides every problem's column count) sets the accumulator tile of every warp (row tile x
 // columns) and the passes per order.  Each candidate runs the plan itself for
 // up to 4 orders (twice; the second run is timed with CUDA events); the fastest
-// is kept per (precision, column gcd, phases, padded size, total elements).  A
+// is kept per (precision, column gcd and largest count, phases, padded size, total elements).  A
 // trial only writes the output columns and recurrence buffers, which the next
 // real launch overwrites.
-std::map<std::tuple<int, int, int, int, int>, int> g_tile_cache;
+std::map<std::tuple<int, int, int, int, int, int>, int> g_tile_cache;
 
-int tune_plan(ChebPlan &pl, int mgcd) {
+int tune_plan(ChebPlan &pl) {
     std::vector<int> cand;
     const bool windowed = windowed_plan(pl.precision, pl.nphase == 3);
     for (int mg : {4, 2, 1})
-        if (mgcd % mg == 0 && cheb_group_size(pl.precision, mg, pl.max_ld, windowed) == mg) cand.push_back(mg);
+        if ((pl.precision == ELHL_PREC_DF64 ? pl.mgcd % mg == 0 : mg <= pl.mmax) &&
+            cheb_group_size(pl.precision, mg, pl.max_ld, windowed) == mg)
+            cand.push_back(mg);
     if (cand.size() < 2 || pl.kmax < 1) return ELHL_OK;
     double elems = 0.0;
     for (const auto &p : pl.probs) elems += (double)p.N * p.ld;
-    const auto key = std::make_tuple(pl.precision, mgcd, pl.nphase, (pl.max_ld + 255) / 256, (int)std::log2(elems + 1));
+    const auto key = std::make_tuple(pl.precision, pl.mgcd, pl.mmax, pl.nphase, (pl.max_ld + 255) / 256, (int)std::log2(elems + 1));
     auto it = g_tile_cache.find(key);
     if (it != g_tile_cache.end()) {
         pl.mg = it->second;
@@ -1724,7 +1735,7 @@ int cheb_run(ChebPlan &pl) {
     if (pl.solo && pl.solo->rows && pl.nphase == 1) return rows_run(pl);
     if (pl.oz) return oz_run(pl);
     if (!pl.tuned) {
-        if (int rc = tune_plan(pl, pl.mgcd)) return rc;
+        if (int rc = tune_plan(pl)) return rc;
         pl.tuned = true;
     }
     CU_TRY(cudaMemsetAsync(g_ctx.err, 0, sizeof(int), st));

@@ -100,7 +100,7 @@ constexpr int kMaxCols = 64;  // ket columns per problem (read-out partial layou
 struct ChebProblem {
     int N, ld, ldv, m, K;   // size, matrix/vector leading dims (padded rows are 0), complex columns, last order
     const void *H;          // Hs = (H~ - a)/b in the launch precision, N columns of ld rows (symmetric)
-    void *vbuf;             // [3][m/MG][ldv][MG] complex vectors in the launch precision
+    void *vbuf;             // [3][column group][ldv][group width] complex vectors in the launch precision
     double2 *col[2];        // ping-pong columns [ldv][m] (FP64): col[parity] in, col[parity^1] out
     const double2 *coef;    // [K+1] expansion coefficients (phase folded in)
     const double *scale;    // [P] factor applied to the input columns (renormalisation) or nullptr
@@ -116,7 +116,7 @@ struct ChebProblem {
     // zeros above the diagonal), Gt = G^T (upper), and one order applies
     // Hs v = G (h/b) G^T v - shift v in three grid-synchronised phases.  G == nullptr: explicit Hs.
     const void *G, *Gt;
-    void *wb;               // [2][m/MG][ldv][MG] launch precision: w = G^T v, y = (h/b) w
+    void *wb;               // [2][column group][ldv][group width] launch precision: w = G^T v, y = (h/b) w
     double shift;           // a / b
     double *drift;          // largest relative change of a column's squared norm over a step (norm control)
     double *ntot;           // [P] total population of each particle after the step, in FP64 from the
