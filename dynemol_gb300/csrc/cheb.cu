@@ -93,13 +93,14 @@ __device__ void rows_gemv(const T *M, int ld, const typename Vec2<T>::type *s_v,
     constexpr int NW = NV < 32 ? NV : 32;
     constexpr int NB = NV / NW;        // warp-sum batches
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int rows = row1 - row0;
-    int WR = 1;
-    while (WR < kWarps && WR * kRT < rows) WR <<= 1;
-    const int WJ = kWarps / WR;
-    const int wr = warp / WJ, wj = warp % WJ;
-    for (int base = row0; base < row1; base += kRT * WR) {
-        const int tile_end = min(row1, base + kRT * WR);
+    for (int base = row0, tile_end; base < row1; base = tile_end) {
+        // WR warps along the rows that are left, WJ along j, so that the last super-tile of
+        // a segment keeps every warp busy (FP32, 157 rows in tiles of 128: the last 29 on
+        // four warps took as long as the first 128)
+        int WR = 1;
+        while (WR < kWarps && WR * kRT < row1 - base) WR <<= 1;
+        const int WJ = kWarps / WR, wr = warp / WJ, wj = warp % WJ;
+        tile_end = min(row1, base + kRT * WR);
         // j window [jw0, jw1) (multiples of 32; s_v holds x from row jw0 on)
         const int jlo = max(jw0, TRI == 1 ? (base & ~31) : 0);
         const int jhi = min(jw1, TRI == 2 ? min(ld, (tile_end + 31) & ~31) : ld);

@@ -1412,13 +1412,19 @@ int tune_plan(ChebPlan &pl);
 // may the propagation stage its vector in windows? (explicit Hs, not in DF64)
 bool windowed_plan(int precision, bool implicit) { return !implicit && precision != ELHL_PREC_DF64; }
 
-// Time of one row of a problem relative to the other problems of a plan: its elements, in
-// FP64 and DF64 times its columns (the arithmetic), in FP32 times its column groups of up
-// to four (each reads the row again) and a quarter per column.
+// Time of one row of a problem relative to the other problems of a plan, in elements: its
+// elements and what a row costs besides (warp sums, epilogue), in FP64 and DF64 times its
+// columns (the arithmetic), in FP32 times its column groups of up to four (each reads the
+// row again) and a quarter per column.  FP32: 5.4 elements per cycle in the sweep, 8,000
+// to 11,000 cycles per 128 rows besides.  Without the second term the CTAs of the small
+// members kept the others waiting a third of each order (24 members of N 270 to 2,930,
+// FP32: 3.45 ms per step, 2.64 so; their FP64 read-out 1.04 ms, 0.67 so).
+constexpr int kRowExtra = 400, kRowExtraWide = 100;
 double row_work(const ChebState &cs) {
     const bool wide = cs.precision == ELHL_PREC_FP64 || cs.precision == ELHL_PREC_DF64;
+    if (wide) return (double)(cs.ld + kRowExtraWide) * cs.m;
     const int rest = cs.m % 4, groups = cs.m / 4 + (rest & 1) + (rest >> 1);
-    return (double)cs.ld * (wide ? cs.m : groups + 0.25 * cs.m);
+    return (cs.ld + kRowExtra) * (groups + 0.25 * cs.m);
 }
 
 int cheb_plan(ChebPlan &pl, const std::vector<ChebState *> &states) {

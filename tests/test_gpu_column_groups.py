@@ -46,3 +46,17 @@ def test_mixed_column_counts_in_one_server(elhl, oracle_mod, prec, tol):
         pops = sv.result(i)[0]
         assert np.abs(pops[:, :-1] - _exact(oracle_mod, sysm, states, STEPS)[:, :-1]).max() < tol
     sv.close()
+
+
+def test_uneven_batch_with_more_rows_per_cta_than_a_tile(elhl):
+    """Forty FP32 members of N about 310 to 680: row ranges of more than 128 rows with every
+    kind of remainder, within 1e-6 of the same batch in FP64."""
+    systems_ = [systems.cubic_cluster(n_atoms=100 + 3 * q, seed=q, frag_atoms=16) for q in range(40)]
+    out = {}
+    for prec in (elhl.PREC_FP64, elhl.PREC_FP32):
+        b = elhl.Batch(systems_, dt=DT, precision=prec, ncols=2, cheb_tol=1e-12)
+        b.init_fmo()
+        b.compact()
+        out[prec] = b.step(nsteps=2)
+        b.close()
+    assert np.abs(out[elhl.PREC_FP32] - out[elhl.PREC_FP64])[..., :-1].max() < 1e-6
