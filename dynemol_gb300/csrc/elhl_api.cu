@@ -237,26 +237,33 @@ __global__ void lower_only_kernel(double *A, int n, int ld) {
 // Schur update and factors A22 (whose single-CTA leaves leave most SMs free).
 // It replaces the reference's LU inverse of S (MAGMA dgetrf + dgetri,
 // GPU_Interface.cpp:910-928; CPU dsytrf + dsytri, :936-947): S is symmetric
-// positive definite, so its Cholesky factor gives S^-1 = G^T G.  W holds the
-// n2 x n1 off-diagonal block of each split (leading dimension ld).  The upper
-// triangles of A and G are left undefined.
+// positive definite, so its Cholesky factor gives S^-1 = G^T G.  L21 is formed in W
+// (leading dimension ld), whose n1 columns are the split's until its side work is done
+// (the second block's splits take the columns after them); the second stream copies it
+// into place, so no copy waits between the products and the leaves (2 to 4 us per split).
+// The upper triangles of A and G are left undefined.
 bool chol_inv_fits(int n, int ld, size_t wcap) {
     const int leaf = leaf_rows();
     if (n <= leaf) return true;
     const int n1 = round_up(n / 2, leaf), n2 = n - n1;
-    return (size_t)ld * n1 <= wcap && chol_inv_fits(n1, ld, wcap) && chol_inv_fits(n2, ld, wcap);
+    return (size_t)ld * n1 <= wcap && chol_inv_fits(n1, ld, wcap) && chol_inv_fits(n2, ld, wcap - (size_t)ld * n1);
 }
 
 // An FP64 product of the factorisations: on the tensor cores from exact slices
 // (ozgemm) when tc is set and the product is large enough to fill the GPU, else
-// on the FP64 pipe (dgemm64).
+// on the FP64 pipe (dgemm64; dgemm_small for the smallest blocks).
 // Below 320 rows the FP64 pipe of all SMs (dgemm64's 16- and 32-row tiles) beats
 // the three launches of a sliced product: the factorisation at N = 3720 took
 // 15.7 ms with the cut at 64 rows, 12.4 at 192, 11.7 at 320, 11.8 at 448 and
 // 12.6 at 640.
 constexpr int kOzGemmMin = 320;
+// Up to 192 rows the small-block kernel: 3.2 against 10 us at 64 rows, 6 against 14 at
+// 128, 12 against 17 at 192; at 256 both take 22.
+constexpr int kSmallGemmMax = 192;
 cudaError_t fgemm(bool tc, int m, int n, int k, double alpha, const double *A, int lda, bool transA, const double *B,
                   int ldb, bool transB, double beta, double *C, int ldc, cudaStream_t st, int tri = 0, int lane = 0) {
+    if (m <= kSmallGemmMax && n <= kSmallGemmMax && k <= kSmallGemmMax)
+        return dgemm_small(m, n, k, alpha, A, lda, transA, B, ldb, transB, beta, C, ldc, st, tri);
     if (tc && m >= kOzGemmMin && n >= kOzGemmMin && k >= kOzGemmMin)
         return ozgemm(m, n, k, alpha, A, lda, transA, B, ldb, transB, beta, C, ldc, st, tri, lane);
     return dgemm64(m, n, k, alpha, A, lda, transA, B, ldb, transB, beta, C, ldc, st, tri, lane);
@@ -290,15 +297,15 @@ int chol_inv64(double *A, double *G, int n, int ld, int row0, double *W, int *in
     double *G12 = G + (size_t)n1 * ld;  // n1 x n2, above the diagonal: free until lower_only
     cudaStream_t side = g_ctx.aux_stream;
     if (int rc = chol_inv64(A, G, n1, ld, row0, W, info, tc)) return rc;
-    CU_TRY(cudaMemcpy2DAsync(W, ld * sizeof(double), A21, ld * sizeof(double), n2 * sizeof(double), n1,
-                             cudaMemcpyDeviceToDevice, st));
-    CU_TRY(fgemm(tc, n2, n1, n1, 1.0, W, ld, false, G, ld, true, 0.0, A21, ld, st, kTriBt));       // L21
+    CU_TRY(fgemm(tc, n2, n1, n1, 1.0, A21, ld, false, G, ld, true, 0.0, W, ld, st, kTriBt));       // L21
     CU_TRY(cudaEventRecord(g_ctx.ev_l21, st));
     CU_TRY(cudaStreamWaitEvent(side, g_ctx.ev_l21, 0));
-    CU_TRY(fgemm(tc, n1, n2, n1, 1.0, G, ld, true, A21, ld, true, 0.0, G12, ld, side, kTriAt, 1));  // (L21 G11)^T
+    CU_TRY(fgemm(tc, n1, n2, n1, 1.0, G, ld, true, W, ld, true, 0.0, G12, ld, side, kTriAt, 1));  // (L21 G11)^T
+    CU_TRY(cudaMemcpy2DAsync(A21, ld * sizeof(double), W, ld * sizeof(double), n2 * sizeof(double), n1,
+                             cudaMemcpyDeviceToDevice, side));
     CU_TRY(cudaEventRecord(g_ctx.ev_side, side));
-    CU_TRY(fgemm(tc, n2, n2, n1, -1.0, A21, ld, false, A21, ld, true, 1.0, A22, ld, st, kTriLowerC));  // Schur
-    if (int rc = chol_inv64(A22, G22, n2, ld, row0 + n1, W, info, tc)) return rc;
+    CU_TRY(fgemm(tc, n2, n2, n1, -1.0, W, ld, false, W, ld, true, 1.0, A22, ld, st, kTriLowerC));  // Schur
+    if (int rc = chol_inv64(A22, G22, n2, ld, row0 + n1, W + (size_t)n1 * ld, info, tc)) return rc;
     // the side stream is serial: its last recorded event covers this split's product
     CU_TRY(cudaStreamWaitEvent(st, g_ctx.ev_side, 0));
     CU_TRY(fgemm(tc, n2, n1, n2, -1.0, G22, ld, false, G12, ld, true, 0.0, G21, ld, st, kTriA));  // G21

@@ -253,6 +253,10 @@ constexpr int kTriA = 1, kTriB = 2, kTriBt = 4, kTriLowerC = 8, kTriAt = 16;
 // three quarters of the resident CTA slots.
 cudaError_t dgemm64(int m, int n, int k, double alpha, const double *A, int lda, bool transA, const double *B, int ldb,
                     bool transB, double beta, double *C, int ldc, cudaStream_t st, int tri = 0, int lane = 0);
+// The same for products of a latency, not of the FP64 pipe (dgemm_small.cu): any size, no
+// workspace, so any number of streams.
+cudaError_t dgemm_small(int m, int n, int k, double alpha, const double *A, int lda, bool transA, const double *B,
+                        int ldb, bool transB, double beta, double *C, int ldc, cudaStream_t st, int tri = 0);
 // The same product on the tensor cores from exact BF16 slices (ozgemm.cu):
 // FP64-accurate (each output exact until one rounding, products below 2^-64 of
 // the row and column scales dropped), for large products; lane as for dgemm64.
