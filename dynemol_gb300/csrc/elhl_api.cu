@@ -700,7 +700,7 @@ struct OzRes {
     double *v = nullptr, *part = nullptr;
     unsigned char *xs = nullptr;  // [3][2 tiles] sliced vectors (oz_vector_tile_bytes each)
     int *xe = nullptr;            // [3][2 tiles][8] their scale exponents, then [3][8] column maxima
-    unsigned *cnt = nullptr;
+    size_t parts = 0;  // partials (slots of one segment each)
     OzSeg *segs = nullptr;
     int *begin = nullptr, *base = nullptr, *count = nullptr;
     size_t xs_bytes() const { return (size_t)3 * 2 * ntiles * oz_vector_tile_bytes(); }
@@ -714,7 +714,6 @@ struct OzRes {
         CU_TRY(cudaMalloc(&xs, xs_bytes()));
         CU_TRY(cudaMemset(xs, 0, xs_bytes()));  // the zero slots of every tile stay zero
         if (int rc = dev_alloc(&xe, (size_t)3 * 2 * ntiles * 8 + 3 * 8)) return rc;
-        CU_TRY(cudaMalloc(&cnt, (size_t)ntiles * sizeof(unsigned)));
         std::vector<OzSeg> sg;
         std::vector<int> b, pb, pc;
         oz_schedule(N, grid, sg, b, pb, pc);
@@ -726,7 +725,8 @@ struct OzRes {
         CU_TRY(copy_h2d(begin, b.data(), b.size() * sizeof(int)));
         CU_TRY(copy_h2d(base, pb.data(), pb.size() * sizeof(int)));
         CU_TRY(copy_h2d(count, pc.data(), pc.size() * sizeof(int)));
-        return dev_alloc(&part, std::max<size_t>(sg.size(), 1) * oz_tile_rows() * 16);  // 128-bit partials
+        parts = std::max<size_t>(sg.size(), 1);
+        return dev_alloc(&part, parts * oz_tile_rows() * 16);  // 128-bit partials
     }
     // slices and row scales of Hs (FP64), allocated on first use
     int slice(const double *Hs, cudaStream_t st) {
@@ -743,11 +743,9 @@ struct OzRes {
         if (s) cudaFree(s);
         if (segs) cudaFree(segs);
         if (xs) cudaFree(xs);
-        if (cnt) cudaFree(cnt);
         s = nullptr;
         segs = nullptr;
         xs = nullptr;
-        cnt = nullptr;
         dev_free(r); dev_free(begin); dev_free(base); dev_free(count);
         dev_free(v); dev_free(xe); dev_free(part);
     }
@@ -1694,7 +1692,6 @@ int oz_run(ChebPlan &pl) {
     L.part_base = oz.base;
     L.part_count = oz.count;
     L.part = oz.part;
-    L.tile_cnt = oz.cnt;
     L.bar_count = g_ctx.bar;
     L.error = g_ctx.err;
     L.barrier_ns = g_dbg_barrier_ns;
@@ -1702,7 +1699,7 @@ int oz_run(ChebPlan &pl) {
     g_dbg_exit_cta1 = 0;  // one launch only
     CU_TRY(cudaMemsetAsync(g_ctx.err, 0, sizeof(int), st));
     CU_TRY(cudaMemsetAsync(g_ctx.bar, 0, 2 * sizeof(unsigned), st));
-    CU_TRY(cudaMemsetAsync(oz.cnt, 0, (size_t)oz.ntiles * sizeof(unsigned), st));
+    CU_TRY(cudaMemsetAsync(oz.part, 0, oz.parts * oz_tile_rows() * 16 * sizeof(double), st));  // tags
     CU_TRY(cudaMemsetAsync(oz.xe + (size_t)3 * 2 * oz.ntiles * 8, 0x80, 3 * 8 * sizeof(int), st));  // column maxima
     CU_TRY(cudaEventRecord(g_ctx.ev[0], st));
     CU_TRY(launch_oz_cheb(L, oz.s, oz.grid, st));
@@ -2209,11 +2206,11 @@ int rebuild(elhl_traj *tr, const double *d_coords) {
 }
 
 // ELHL_PREC_OZ64 up to this size propagates on the FP64 pipe (cheb_rows.cuh) instead of
-// the tensor cores: an order of oz_cheb_kernel costs at least 7 us of hand-overs
+// the tensor cores: an order of oz_cheb_kernel costs at least 5.5 us of hand-overs
 // (TMA, MMA, flush, partials, barrier) whatever its size.  Moving step, tensor cores /
-// FP64 pipe in ms of propagation: 0.98 / 0.23 at N = 62, 1.22 / 0.61 at 341, 1.89 /
-// 1.49 at 620, 1.92 / 2.04 at 775.
-constexpr int kOzRowsMax = 700;
+// FP64 pipe in ms of propagation: 0.81 / 0.21 at N = 62, 0.90 / 0.62 at 341, 1.10 / 0.98
+// at 496, 1.19 / 1.12 at 558, 1.24 / 1.43 at 620, 1.24 / 2.07 at 775.
+constexpr int kOzRowsMax = 580;
 
 // Moving nuclei: form H~ = G h G^T every step (1.5 N^3 flops), or apply its three
 // factors in every order (twice the elements, three grid phases per order instead

@@ -223,8 +223,7 @@ struct OzLaunch {
     const int *seg_begin;        // [grid + 1]
     const int *part_base;        // [tiles] first partial slot of a row tile
     const int *part_count;       // [tiles] segments of a row tile
-    double *part;                // partial tiles [slot][128][8] as 128-bit integers (16 bytes each)
-    unsigned *tile_cnt;          // [tiles] segments written, over all orders of the launch
+    double *part;                // partial tiles [slot][8][128] as 128-bit integers (16 bytes each)
     unsigned *bar_count;         // grid-barrier arrivals, over all orders of the launch (0 at the launch)
     int *error;
     unsigned long long barrier_ns;  // grid-barrier limit (0: default)

@@ -41,7 +41,7 @@
 //   warps 4-7  fold each block from TMEM (one thread per row); at the end of a
 //              segment they store its partial (exact 128-bit integers); a CTA
 //              designated per half of a 64-row chunk (4 of the 8 columns) sums
-//              the tile's partials once all are counted (exact, in any order),
+//              the tile's partials as they arrive (exact, in any order),
 //              applies the Chebyshev recurrence and the c_k v_k accumulation
 //              in FP64, and slices its rows of v_k for the next order.
 // Warps 2-7 meet the grid barrier of every order.  Every wait is bounded: on a
@@ -52,6 +52,7 @@
 #include <algorithm>
 
 #include "elhl_internal.cuh"
+#include "exchange.cuh"
 #include "grid_sync.cuh"
 #include "tc_ptx.cuh"
 
@@ -165,7 +166,6 @@ __device__ __forceinline__ bool grid_barrier_sub(unsigned *count, unsigned targe
                 atomicExch(err, ELHL_ERR_TIMEOUT);
                 break;
             }
-            __nanosleep(20);
         }
     }
     asm volatile("bar.sync 2, 192;" ::: "memory");
@@ -417,14 +417,29 @@ __device__ void slice_chunk_out(const Ctx &c, int h, int half, const EpiThread &
     fence_proxy_async_global();  // read by bulk copies after the next grid barrier
 }
 
-// bounded wait until *cnt reaches target (segments of a row tile written)
-__device__ __forceinline__ bool wait_count(const unsigned *cnt, unsigned target) {
-    const unsigned long long t0 = now_ns();
-    while (*(volatile const unsigned *)cnt < target) {
-        if (now_ns() - t0 > kWaitNs) return false;
-        __nanosleep(32);
-    }
-    return true;
+// A partial is one 16-byte word: the 128-bit integer (|s| < 2^116) with the order's tag in
+// the top ten bits of its high half, written and read whole (exchange.cuh), so that the
+// reader polls the words themselves: no fence, counter or second trip to L2 between a
+// tile's last segment and its epilogue.  A slot is written once per order, between two
+// grid barriers, and cleared before the launch: its tag is never the next order's.
+// Rows lie side by side ([slot][8 columns][128 rows]): with a row's eight words together
+// (16-byte stores 128 bytes apart) and a counter per tile an order took 13.2 us at N = 932
+// and 39.9 us at N = 3720, 8.2 and 36.8 us so (the operator's bytes alone: 1.5 and 28.7).
+constexpr int kTagShift = 54;
+__device__ __forceinline__ unsigned long long order_tag(int k) { return (unsigned long long)(k % 1023 + 1); }
+__device__ __forceinline__ I128 untag(const ulonglong2 &w) {
+    return I128{(long long)(w.y << (64 - kTagShift)) >> (64 - kTagShift), w.x};
+}
+// true in every thread if `ok` holds in all 128 threads of warps 4-7 (named barrier 1)
+__device__ __forceinline__ bool all_ok(bool ok) {
+    unsigned r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((unsigned)ok)
+        : "memory");
+    return r != 0;
 }
 
 // What a half-chunk epilogue reads besides the partials, loaded before it
@@ -444,30 +459,55 @@ __device__ __forceinline__ EpiPre epi_prefetch(const OzLaunch &L, const OrderIO 
     return q;
 }
 
-// Epilogue of half c of chunk h once its row tile's np segments are written:
-// the exact sum of their partials, the row's product in FP64, the recurrence
-// and accumulation of order k, and the slices of the half's rows of v_k for the
-// next order.  The rows and columns of a half are only ever touched by this
-// CTA (order 0 included), so v and acc use plain (L1) loads.
-__device__ void chunk_epilogue(const Ctx &c, const OzLaunch &L, const OrderIO &io, int h, int half, int np,
-                               const int (&E)[8], const EpiThread &et, const EpiPre &pre) {
-    const int rt = h >> 1, trow = (h & 1) * 64 + et.r;  // row tile, row in it
-    I128 S[2] = {I128{0, 0ull}, I128{0, 0ull}};
-    const longlong2 *p0 = reinterpret_cast<const longlong2 *>(L.part) +
-                          ((size_t)L.part_base[rt] * kTileM + trow) * 8 + et.col;
+// The exact sum of a row tile's np partials of the thread's row and two columns, polled
+// until this order's have all arrived; false when the wait (kWaitNs) runs out.  The warp
+// polls as one (votes), the words that are in are left alone.
+__device__ bool sum_partials(const OzLaunch &L, int k, int rt, int trow, int col, int np, I128 (&S)[2]) {
+    const ulonglong2 *p0 =
+        reinterpret_cast<const ulonglong2 *>(L.part) + ((size_t)L.part_base[rt] * 8 + col) * kTileM + trow;
+    const unsigned long long tag = order_tag(k);
+    S[0] = S[1] = I128{0, 0ull};
     for (int s0 = 0; s0 < np; s0 += 8) {  // up to 16 loads in flight
-        longlong2 v[8][2];
+        ulonglong2 v[8][2];
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            if (s0 + j < np)
 #pragma unroll
-                for (int u = 0; u < 2; ++u) v[j][u] = __ldcg(p0 + (size_t)(s0 + j) * kTileM * 8 + u);
+            for (int u = 0; u < 2; ++u)
+                v[j][u] = s0 + j < np ? fetch(p0 + ((s0 + j) * 8 + u) * kTileM)
+                                      : make_ulonglong2(0ull, tag << kTagShift);
+        unsigned long long t0 = 0;
+        for (unsigned polls = 1;; ++polls) {
+            bool miss = false;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) miss |= (v[j][u].y >> kTagShift) != tag;
+            if (!__any_sync(0xffffffffu, miss)) break;
+            if ((polls & 63u) == 0) {
+                const unsigned long long t = now_ns();
+                if (!t0) t0 = t;
+                if (__any_sync(0xffffffffu, t - t0 > kWaitNs)) return false;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    if ((v[j][u].y >> kTagShift) != tag) v[j][u] = fetch(p0 + ((s0 + j) * 8 + u) * kTileM);
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            if (s0 + j < np)
 #pragma unroll
-                for (int u = 0; u < 2; ++u) add128(S[u], I128{v[j][u].x, (unsigned long long)v[j][u].y});
+            for (int u = 0; u < 2; ++u) add128(S[u], untag(v[j][u]));
     }
+    return true;
+}
+
+// Epilogue of half c of chunk h from the exact sums S of its row tile's partials: the
+// row's product in FP64, the recurrence and accumulation of order k, and the slices of the
+// half's rows of v_k for the next order.  The rows and columns of a half are only ever
+// touched by this CTA (order 0 included), so v and acc use plain (L1) loads.
+__device__ void chunk_epilogue(const Ctx &c, const OzLaunch &L, const OrderIO &io, int h, int half, const I128 (&S)[2],
+                               const int (&E)[8], const EpiThread &et, const EpiPre &pre) {
     const double rs = L.rscale[et.row];
     double y[2];
 #pragma unroll
@@ -490,30 +530,22 @@ __device__ void chunk_epilogue(const Ctx &c, const OzLaunch &L, const OrderIO &i
     slice_chunk_out(c, h, half, et, y, io.xs_out, io.xe_out, io.emax_out);
 }
 
-// A row tile's partial (exact 128-bit integers, 8 columns per row) into its
-// slot.  It is counted at its row tile later (release_partials), once the next
-// segment's work has given the stores time to complete.
-__device__ __forceinline__ void store_partial(const OzLaunch &L, int slot, int t, const I128 (&A)[8]) {
-    longlong2 *part = reinterpret_cast<longlong2 *>(L.part) + ((size_t)slot * kTileM + t) * 8;
+// a row tile's partial (exact 128-bit integers, 8 columns per row) into its slot
+__device__ __forceinline__ void store_partial(const OzLaunch &L, int k, int slot, int t, const I128 (&A)[8]) {
+    ulonglong2 *part = reinterpret_cast<ulonglong2 *>(L.part) + (size_t)slot * 8 * kTileM + t;
+    constexpr unsigned long long kMask = (1ull << kTagShift) - 1;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) part[u] = make_longlong2(A[u].hi, (long long)A[u].lo);
-}
-// the stored partial of row tile `tile` (if >= 0) made visible, then counted
-__device__ __forceinline__ void release_partial(const OzLaunch &L, int &tile, int t) {
-    if (tile < 0) return;
-    __threadfence();
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (t == 0) atomicAdd(&L.tile_cnt[tile], 1u);
-    tile = -1;
+    for (int u = 0; u < 8; ++u)
+        publish(part + u * kTileM, A[u].lo, ((unsigned long long)A[u].hi & kMask) | (order_tag(k) << kTagShift));
 }
 
 // The CTA's segments: each 64-K block's weight sums folded, with that chunk's
 // vector scale, into one exact 128-bit integer per row and column, stored as
-// the segment's partial and counted at its row tile.  The chunk exponents of
+// the segment's partial.  The chunk exponents of
 // the order's vector are read once into shared memory.  Then the epilogues of
 // the half-chunks this CTA is designated for (half-chunk q = 2 h + c by CTA
 // floor(q grid / halves): spread over the grid, at most one per CTA while
-// halves <= grid), each once its row tile's segments are all counted.
+// halves <= grid), each once its row tile's partials are all in.
 __device__ void flush_and_epilogue(const Ctx &c, const OzLaunch &L, const OrderIO &io, Roles &r, bool rev) {
     const int t = threadIdx.x - 128;  // 0 .. 127: TMEM lane / row in the tile
     const int warp = threadIdx.x >> 5;
@@ -529,8 +561,8 @@ __device__ void flush_and_epilogue(const Ctx &c, const OzLaunch &L, const OrderI
         for (int i = t; i < nkb * 8; i += 128) c.xe[i] = __ldcg(io.xe_in + i);
         asm volatile("bar.sync 1, 128;" ::: "memory");
     }
-    int pend = -1;  // row tile of the stored, not yet counted partial
-    for (int qi = 0; qi < s1 - s0; ++qi) {
+    bool ok = true;  // of this warp; a warp that gave up still meets the others at their barriers
+    for (int qi = 0; ok && qi < s1 - s0; ++qi) {
         const OzSeg sg = L.segs[walk_seg(s0, s1, qi, rev)];
         I128 A[8];
 #pragma unroll
@@ -538,16 +570,7 @@ __device__ void flush_and_epilogue(const Ctx &c, const OzLaunch &L, const OrderI
         for (int ki = 0; ki < sg.kb1 - sg.kb0; ++ki) {
             const int kb = walk_kb(sg, ki, rev);
             const unsigned tb = r.gcnt & 1;
-            // one thread waits and all 128 follow its outcome, so that none is left
-            // alone at the named barriers
-            if (t == 0) *c.last_flag = mbar_wait(&c.accfull[tb], (r.gcnt >> 1) & 1, now_ns(), kWaitNs) ? 1u : 0u;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            const bool ready = *(volatile unsigned *)c.last_flag != 0;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (!ready) {
-                if (t == 0) set_abort(c, L.error);
-                return;
-            }
+            if (!(ok = mbar_wait_warp(&c.accfull[tb], (r.gcnt >> 1) & 1, kWaitNs))) break;
             asm volatile("tcgen05.fence::after_thread_sync;");
             long long H[8], Lo[8];
 #pragma unroll
@@ -566,11 +589,9 @@ __device__ void flush_and_epilogue(const Ctx &c, const OzLaunch &L, const OrderI
                 add128(A[u], group_term(H[u], Lo[u], max(0, E[u] - ec)));
             }
         }
-        release_partial(L, pend, t);
-        store_partial(L, L.part_base[sg.rt] + sg.slot, t, A);
-        pend = sg.rt;
+        if (ok) store_partial(L, io.k, L.part_base[sg.rt] + sg.slot, t, A);
     }
-    release_partial(L, pend, t);
+    if (!ok) set_abort(c, L.error);
     const int nhc = 4 * ntiles, G = gridDim.x;
     const int q1 = (int)(((long long)(blockIdx.x + 1) * nhc + G - 1) / G);
     for (int q = (int)(((long long)blockIdx.x * nhc + G - 1) / G); q < q1; ++q) {
@@ -578,17 +599,13 @@ __device__ void flush_and_epilogue(const Ctx &c, const OzLaunch &L, const OrderI
         const EpiThread et = epi_thread(h, half, t);
         const EpiPre pre = epi_prefetch(L, io, et);
         const int np = L.part_count[h >> 1];
-        // the count only grows (np per order, zero at the launch): order k waits for k np
-        if (t == 0) *c.last_flag = wait_count(&L.tile_cnt[h >> 1], (unsigned)(np * io.k)) ? 1u : 0u;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        const bool ready = *(volatile unsigned *)c.last_flag != 0;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (!ready) {
-            if (t == 0) set_abort(c, L.error);
+        I128 S[2];
+        ok = ok && sum_partials(L, io.k, h >> 1, (h & 1) * 64 + et.r, et.col, np, S);
+        if (!all_ok(ok)) {
+            set_abort(c, L.error);
             return;
         }
-        __threadfence();
-        chunk_epilogue(c, L, io, h, half, np, E, et, pre);
+        chunk_epilogue(c, L, io, h, half, S, E, et, pre);
     }
 }
 
