@@ -99,11 +99,6 @@ static_assert(kS == 7 && acc_layout_ok(), "accumulator layout");
 __device__ __forceinline__ double pow2(int e) {  // 2^e for |e| < 1000
     return __longlong_as_double((long long)(1023 + e) << 52);
 }
-// exponent e with |x| < 2^e for the non-zero finite x (0 for x = 0)
-__device__ __forceinline__ int scale_exp(double x) {
-    if (!(x > 0.0)) return 0;
-    return (int)((__double_as_longlong(x) >> 52) & 0x7ff) - 1022;
-}
 // byte offset of (row R, K index kk) in a 128B-swizzled K-major tile of 128-byte rows
 __device__ __forceinline__ int swz_off(int R, int kk) { return R * 128 + (((kk >> 3) ^ (R & 7)) << 4) + ((kk & 7) << 1); }
 
@@ -406,7 +401,7 @@ __device__ void slice_chunk_out(const Ctx &c, int h, int half, const EpiThread &
 #pragma unroll
         for (int b = 0; b < kS; ++b)
             *reinterpret_cast<__nv_bfloat16 *>(c.out + swz_off(8 * (b + 1) + et.col + u, et.r)) =
-                __float2bfloat16_rn((float)dig[b]);
+                __ushort_as_bfloat16((unsigned short)digit_bf16(dig[b]));
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");  // the rows are complete; c.red is free again
     constexpr int kPieces = kS * 4 * 8;  // slots 1-7 x the half's 4 rows x 8 pieces of 16 bytes
@@ -763,28 +758,28 @@ __global__ void __launch_bounds__(kThreads, 1)
 // on the scale 2^e_j of its largest element; out[s][j][i], rscale[j] = 2^e_j
 __global__ void oz_slice_kernel(const double *__restrict__ M, int n, int ld, __nv_bfloat16 *__restrict__ out,
                                 double *__restrict__ rscale) {
-    __shared__ double s_max[32];
+    __shared__ unsigned s_max[32];
     const int j = blockIdx.x;
-    const double *col = M + (size_t)j * ld;
-    double mx = 0.0;
-    for (int i = threadIdx.x; i < ld; i += blockDim.x) mx = fmax(mx, fabs(col[i]));
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const double2 *col = reinterpret_cast<const double2 *>(M + (size_t)j * ld);  // ld is a multiple of 32
+    unsigned mx = 0;
+    for (int i = threadIdx.x; i < ld / 2; i += blockDim.x) mx = max(mx, max(abs_key(col[i].x), abs_key(col[i].y)));
+    mx = __reduce_max_sync(0xffffffffu, mx);
     if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        mx = threadIdx.x < (blockDim.x >> 5) ? s_max[threadIdx.x] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (threadIdx.x == 0) s_max[0] = mx;
-    }
-    __syncthreads();
-    const int e = scale_exp(s_max[0]);
+    mx = 0;
+    for (int w = 0; w < (int)blockDim.x >> 5; ++w) mx = max(mx, s_max[w]);
+    const int e = key_exp(mx);
     if (threadIdx.x == 0) rscale[j] = pow2(e);
     const size_t sstride = (size_t)n * ld;
-    for (int i = threadIdx.x; i < ld; i += blockDim.x) {
-        int dig[kS];
-        slice7(col[i], e, dig);
+    for (int i = threadIdx.x; i < ld / 2; i += blockDim.x) {
+        const double2 x = col[i];
+        int d0[kS], d1[kS];
+        slice7(x.x, e, d0);
+        slice7(x.y, e, d1);
 #pragma unroll
-        for (int s = 0; s < kS; ++s) out[s * sstride + (size_t)j * ld + i] = __float2bfloat16_rn((float)dig[s]);
+        for (int s = 0; s < kS; ++s)
+            *reinterpret_cast<unsigned *>(out + s * sstride + (size_t)j * ld + 2 * i) =
+                digit_bf16(d0[s]) | (digit_bf16(d1[s]) << 16);
     }
 }
 

@@ -61,10 +61,6 @@ struct Smem {
 };
 
 __device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
-__device__ __forceinline__ int scale_exp(double x) {  // |x| < 2^e for the finite x > 0 (0 for x = 0)
-    if (!(x > 0.0)) return 0;
-    return (int)((__double_as_longlong(x) >> 52) & 0x7ff) - 1022;
-}
 
 // element (r, j) of an operand row: row r of op(A) (or column r of op(B)), j the K index
 struct OperandView {
@@ -108,8 +104,8 @@ __device__ __forceinline__ void load_tile(const OperandView &v, int r0, int j0, 
 
 // Slicing of both operands in two passes over pieces of 32 operand rows x
 // chunk K (blockIdx.z: 0 = op(A), 1 = op(B)^T), tiles of 32 x 32 loaded along
-// X's contiguous index: oz_partmax_kernel writes each row's largest |element|
-// of the piece to pm[r][piece]; oz_slice_kernel reduces a row's pieces to its
+// X's contiguous index: oz_partmax_kernel writes the key (abs_key) of each row's largest
+// |element| of the piece to pm[r][piece]; oz_slice_kernel reduces a row's pieces to its
 // scale 2^e_r (scale[r], written by the pieces at K = 0) and cuts every element
 // of its piece with slice7 into out[s][r][j] (row stride kp, zero for k <= j < kp).
 // The piece is 256 K, or 128 / 64 for K up to 1024 / 512: a piece's tiles run one
@@ -117,7 +113,7 @@ __device__ __forceinline__ void load_tile(const OperandView &v, int r0, int j0, 
 // with fewer dependent tile loads).
 __host__ __device__ constexpr int slice_chunk(int kp) { return kp <= 512 ? 64 : kp <= 1024 ? 128 : 256; }
 
-__global__ void __launch_bounds__(256) oz_partmax_kernel(OperandView va, OperandView vb, double *pmA, double *pmB,
+__global__ void __launch_bounds__(256) oz_partmax_kernel(OperandView va, OperandView vb, unsigned *pmA, unsigned *pmB,
                                                          int npiece, int chunk) {
     __shared__ double t[32][33];
     const bool isB = blockIdx.z == 1;
@@ -126,42 +122,42 @@ __global__ void __launch_bounds__(256) oz_partmax_kernel(OperandView va, Operand
     if (r0 >= v.rows) return;
     int lo, hi;  // the same for the 32 rows: they lie in one output tile
     read_range(v, r0, lo, hi);
-    double mx = 0.0;  // thread (x, y): row r0 + x over K columns y, y + 8, ... of each tile
+    unsigned mx = 0;  // thread (x, y): row r0 + x over K columns y, y + 8, ... of each tile
     for (int j0 = j00; j0 < min(v.k, j00 + chunk); j0 += 32) {
         if (j0 >= hi || j0 + 32 <= lo) continue;  // masked out: zero (uniform over the block)
         __syncthreads();
         load_tile(v, r0, j0, t);
         __syncthreads();
-        for (int q = threadIdx.y; q < 32; q += 8) mx = fmax(mx, fabs(t[threadIdx.x][q]));
+        for (int q = threadIdx.y; q < 32; q += 8) mx = max(mx, abs_key(t[threadIdx.x][q]));
     }
-    __shared__ double s_max[8][32];
+    __shared__ unsigned s_max[8][32];
     s_max[threadIdx.y][threadIdx.x] = mx;
     __syncthreads();
     if (threadIdx.y == 0 && r0 + threadIdx.x < v.rows) {
-        double m = s_max[0][threadIdx.x];
-        for (int q = 1; q < 8; ++q) m = fmax(m, s_max[q][threadIdx.x]);
+        unsigned m = s_max[0][threadIdx.x];
+        for (int q = 1; q < 8; ++q) m = max(m, s_max[q][threadIdx.x]);
         (isB ? pmB : pmA)[(size_t)(r0 + threadIdx.x) * npiece + blockIdx.x] = m;
     }
 }
 
-__global__ void __launch_bounds__(256) oz_slice_kernel(OperandView va, OperandView vb, const double *pmA,
-                                                       const double *pmB, int npiece, __nv_bfloat16 *outA,
+__global__ void __launch_bounds__(256) oz_slice_kernel(OperandView va, OperandView vb, const unsigned *pmA,
+                                                       const unsigned *pmB, int npiece, __nv_bfloat16 *outA,
                                                        __nv_bfloat16 *outB, int kp, double *scA, double *scB,
                                                        int chunk) {
     __shared__ double t[32][33];
     __shared__ int s_e[32];
     const bool isB = blockIdx.z == 1;
     const OperandView &v = isB ? vb : va;
-    const double *pm = isB ? pmB : pmA;
+    const unsigned *pm = isB ? pmB : pmA;
     __nv_bfloat16 *out = isB ? outB : outA;
     const int r0 = blockIdx.y * 32, j00 = blockIdx.x * chunk;
     if (r0 >= v.rows) return;
     if (threadIdx.y == 0) {
         const int r = r0 + threadIdx.x;
-        double m = 0.0;
+        unsigned m = 0;
         if (r < v.rows)
-            for (int q = 0; q < npiece; ++q) m = fmax(m, pm[(size_t)r * npiece + q]);
-        const int e = scale_exp(m);
+            for (int q = 0; q < npiece; ++q) m = max(m, pm[(size_t)r * npiece + q]);
+        const int e = key_exp(m);
         s_e[threadIdx.x] = e;
         if (blockIdx.x == 0 && r < v.rows) (isB ? scB : scA)[r] = pow2(e);
     }
@@ -173,13 +169,17 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(OperandView va, OperandVi
         __syncthreads();
         load_tile(v, r0, j0, t);
         __syncthreads();
-        for (int rr = threadIdx.y; rr < 32; rr += 8) {
-            const int r = r0 + rr, j = j0 + threadIdx.x;
+        // two consecutive K per thread (kp is a multiple of 8), two rows per warp
+        for (int rr = 2 * threadIdx.y + threadIdx.x / 16; rr < 32; rr += 16) {
+            const int jj = 2 * (threadIdx.x % 16), r = r0 + rr, j = j0 + jj;
             if (r >= v.rows || j >= kp) continue;
-            int dig[kS];
-            slice7(t[rr][threadIdx.x], s_e[rr], dig);
+            int d0[kS], d1[kS];
+            slice7(t[rr][jj], s_e[rr], d0);
+            slice7(t[rr][jj + 1], s_e[rr], d1);
 #pragma unroll
-            for (int sl = 0; sl < kS; ++sl) out[sl * sstride + (size_t)r * kp + j] = __float2bfloat16_rn((float)dig[sl]);
+            for (int sl = 0; sl < kS; ++sl)
+                *reinterpret_cast<unsigned *>(out + sl * sstride + (size_t)r * kp + j) =
+                    digit_bf16(d0[sl]) | (digit_bf16(d1[sl]) << 16);
         }
     }
 }
@@ -429,7 +429,7 @@ struct Lane {
     size_t sl_elems = 0;
     double *sc = nullptr;
     size_t rows_cap = 0;
-    double *pm = nullptr;    // row maxima per K piece of both operands
+    unsigned *pm = nullptr;  // keys of the row maxima per K piece of both operands
     size_t pm_cap = 0;
     int *err = nullptr;
 };
@@ -465,7 +465,7 @@ cudaError_t ensure_pm(Lane &ln, size_t n) {
     if (ln.pm) cudaFree(ln.pm);
     ln.pm = nullptr;
     ln.pm_cap = 0;
-    cudaError_t e = cudaMalloc(&ln.pm, n * sizeof(double));
+    cudaError_t e = cudaMalloc(&ln.pm, n * sizeof(unsigned));
     if (e == cudaSuccess) ln.pm_cap = n;
     return e;
 }
