@@ -82,23 +82,29 @@ __device__ __forceinline__ void read_range(const OperandView &v, int r, int &lo,
     hi = v.mask == 1 ? (min(v.k, t0 + v.tile) + kKB - 1) / kKB * kKB : 1 << 30;
 }
 
-// 32 x 32 tile of the operand rows [r0, r0+32) x K [j0, j0+32) in shared memory
-// (t[rr][jj]), loaded along X's contiguous index; masked and out-of-range entries 0
-__device__ __forceinline__ void load_tile(const OperandView &v, int r0, int j0, double (&t)[32][33]) {
-    for (int q = threadIdx.y; q < 32; q += blockDim.y) {
-        int r, j;
-        if (v.kcontig) {
-            r = r0 + q;
-            j = j0 + threadIdx.x;
-        } else {
-            r = r0 + threadIdx.x;
-            j = j0 + q;
-        }
-        double x = 0.0;
+// 32 x 32 tile of the operand rows [r0, r0+32) x K [j0, j0+32): the thread's four
+// elements, loaded along X's contiguous index (masked and out-of-range ones 0), and their
+// places in shared memory (t[rr][jj])
+struct Tile4 {
+    double x[4];
+};
+__device__ __forceinline__ Tile4 load_tile(const OperandView &v, int r0, int j0) {
+    Tile4 o;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int q = threadIdx.y + 8 * i, r = r0 + (v.kcontig ? q : (int)threadIdx.x),
+                  j = j0 + (v.kcontig ? (int)threadIdx.x : q);
         const bool keep = r < v.rows && j < v.k && !(v.mask == 1 && j > r) && !(v.mask == 2 && j < r);
-        if (keep) x = v.kcontig ? v.X[(size_t)r * v.ld + j] : v.X[(size_t)j * v.ld + r];
-        if (v.kcontig) t[q][threadIdx.x] = x;
-        else t[threadIdx.x][q] = x;
+        o.x[i] = keep ? (v.kcontig ? v.X[(size_t)r * v.ld + j] : v.X[(size_t)j * v.ld + r]) : 0.0;
+    }
+    return o;
+}
+__device__ __forceinline__ void put_tile(const OperandView &v, const Tile4 &o, double (&t)[32][33]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int q = threadIdx.y + 8 * i;
+        if (v.kcontig) t[q][threadIdx.x] = o.x[i];
+        else t[threadIdx.x][q] = o.x[i];
     }
 }
 
@@ -109,8 +115,8 @@ __device__ __forceinline__ void load_tile(const OperandView &v, int r0, int j0, 
 // scale 2^e_r (scale[r], written by the pieces at K = 0) and cuts every element
 // of its piece with slice7 into out[s][r][j] (row stride kp, zero for k <= j < kp).
 // The piece is 256 K, or 128 / 64 for K up to 1024 / 512: a piece's tiles run one
-// after another, so short operands take more, shorter pieces (more CTAs, each
-// with fewer dependent tile loads).
+// after another (the next one's loads under way), so short operands take more, shorter
+// pieces (more CTAs, each with fewer tiles).
 __host__ __device__ constexpr int slice_chunk(int kp) { return kp <= 512 ? 64 : kp <= 1024 ? 128 : 256; }
 
 __global__ void __launch_bounds__(256) oz_partmax_kernel(OperandView va, OperandView vb, unsigned *pmA, unsigned *pmB,
@@ -123,10 +129,14 @@ __global__ void __launch_bounds__(256) oz_partmax_kernel(OperandView va, Operand
     int lo, hi;  // the same for the 32 rows: they lie in one output tile
     read_range(v, r0, lo, hi);
     unsigned mx = 0;  // thread (x, y): row r0 + x over K columns y, y + 8, ... of each tile
-    for (int j0 = j00; j0 < min(v.k, j00 + chunk); j0 += 32) {
-        if (j0 >= hi || j0 + 32 <= lo) continue;  // masked out: zero (uniform over the block)
+    // tiles outside the range are masked out: zero (uniform over the block)
+    const int ja = max(j00, lo), je = min(min(v.k, j00 + chunk), hi);
+    Tile4 x{};
+    if (ja < je) x = load_tile(v, r0, ja);
+    for (int j0 = ja; j0 < je; j0 += 32) {
         __syncthreads();
-        load_tile(v, r0, j0, t);
+        put_tile(v, x, t);
+        if (j0 + 32 < je) x = load_tile(v, r0, j0 + 32);
         __syncthreads();
         for (int q = threadIdx.y; q < 32; q += 8) mx = max(mx, abs_key(t[threadIdx.x][q]));
     }
@@ -164,10 +174,14 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(OperandView va, OperandVi
     const size_t sstride = (size_t)v.rows * kp;
     int lo, hi;  // the same for the 32 rows: they lie in one output tile
     read_range(v, r0, lo, hi);
-    for (int j0 = j00; j0 < min(kp, j00 + chunk); j0 += 32) {
-        if (j0 >= hi || j0 + 32 <= lo) continue;  // never read by the product (uniform over the block)
+    // tiles outside the range are never read by the product (uniform over the block)
+    const int ja = max(j00, lo), je = min(min(kp, j00 + chunk), hi);
+    Tile4 x{};
+    if (ja < je) x = load_tile(v, r0, ja);
+    for (int j0 = ja; j0 < je; j0 += 32) {
         __syncthreads();
-        load_tile(v, r0, j0, t);
+        put_tile(v, x, t);
+        if (j0 + 32 < je) x = load_tile(v, r0, j0 + 32);
         __syncthreads();
         // two consecutive K per thread (kp is a multiple of 8), two rows per warp
         for (int rr = 2 * threadIdx.y + threadIdx.x / 16; rr < 32; rr += 16) {
