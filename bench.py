@@ -256,8 +256,8 @@ def run_ours(args, rank, world):
         m = 4 if moving else 2
         # bytes per matrix element: FP64 / DF64 pairs 8, FP32 4, OZ64 seven BF16 slices 14
         bH = {"fp64": 8.0, "df64": 8.0, "oz64": 14.0}.get(args.precision, 4.0)
-        # the implicit operator (three grid phases) reads 2 N^2 elements per order, an
-        # explicit H~ (one phase: fixed nuclei, and OZ64 moving nuclei) N^2
+        # the implicit operator (three grid phases: large bases with moving nuclei) reads
+        # 2 N^2 elements per order, an explicit H~ (one phase) N^2
         implicit = st.phases == 3 if method == api.METHOD_CHEBYSHEV else False
         elems, vec = (2.0 * N * N, 144.0) if implicit else (1.0 * N * N, 80.0)
         per_launch_orders = orders / max(1, K) / m

@@ -56,7 +56,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned nblocks, 
 // one thread waits for `target` = nblocks x (barriers so far).  Against
 // grid_barrier an arrival needs no answer, the poll does not sleep, and *err is
 // read by the waiting thread alone, every 64th poll, instead of by every thread
-// after each barrier: 3,500 cycles per Taylor round before, 2,000 after (117
+// after each barrier: 3,500 cycles per Taylor round before, 2,750 after (117
 // CTAs).  grid_poll returns false on a timeout (which it reports) or when
 // another CTA has reported one; the caller broadcasts the answer.
 __device__ __forceinline__ void grid_arrive(unsigned *count) {

@@ -114,7 +114,7 @@ enum {
                              Cholesky factor with inverse and spectral bounds; with >= 16 ket columns
                              (one per particle) and N >= 2048, H~.Psi runs as FP32 GEMMs on the FP32
                              pipes (cuBLAS, FP32 sums along N) */
-    ELHL_PREC_DF64 = 3,   /* Chebyshev, implicit operator: operator and series vectors as FP32 pairs
+    ELHL_PREC_DF64 = 3,   /* Chebyshev: operator and series vectors as FP32 pairs
                              hi + lo (48-bit significands) with exact-product / TwoSum arithmetic on the
                              FP32 pipes, FP64 recurrence and sums: FP64-level accuracy (1e-10 populations)
                              without the FP64 pipe; FP64 factor, bounds and read-out */
@@ -125,7 +125,8 @@ enum {
     ELHL_PREC_OZ64 = 4    /* Chebyshev, trajectories with ncols <= 4: FP64 operator, vectors and
                              recurrence, with every operator product computed exactly on the tensor
                              cores from 7 bf16 slices of 8 bits per operand (Ozaki scheme I, products
-                             below 2^-64 of a row's scale dropped) and rounded once to FP64; moving
+                             below 2^-64 of a row's scale dropped) and rounded once to FP64 (small
+                             bases propagate on the FP64 pipe, which is faster there); moving
                              nuclei form H~ = G h G^T every step the same way, and the factorisation's
                              products of 320 or more rows too; bounds and read-out in FP64 */
 };
@@ -297,11 +298,12 @@ typedef struct {
     int prop_launches;    /* propagation kernel launches */
     int rebuild_count;    /* rebuilds */
     int tile_cols;        /* Chebyshev: complex columns per matrix pass chosen by the autotuner (0: GEMM regime) */
-    int phases;           /* Chebyshev: grid phases per order (1 explicit H~, 3 implicit G h G^T) */
+    int phases;           /* Chebyshev: grid phases per order (1 explicit H~, 3 implicit G h G^T; moving
+                             nuclei form H~ where that is faster) */
     double sh_ms;         /* moving nuclei: device time of the S, h build */
     double factor_ms;     /* ... of the Cholesky factorisation of S with G = L^-1 */
-    double inverse_ms;    /* ... of the operator formed from them: H~ = G h G^T (ELHL_PREC_OZ64),
-                             the zeroed upper triangles of L and G (implicit operator) */
+    double inverse_ms;    /* ... of the operator formed from them: H~ = G h G^T (explicit), the zeroed
+                             upper triangles of L and G (implicit operator) */
     int cheb_retries;     /* Chebyshev steps redone on a widened spectral interval */
     double norm_drift;    /* Chebyshev: largest relative change of a column's squared norm in one step
                              (before renormalisation), over the call's accepted steps */
