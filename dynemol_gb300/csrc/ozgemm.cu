@@ -24,7 +24,7 @@
 //              of A slice a against the B slices b <= 6 - a at once (N = 32 (7 - a),
 //              D from column 32 a, so that B slice b lands on the weight
 //              accumulator a + b) in one of two 224-column buffers;
-//   warps 2-5  fold each block's accumulators into H and L (one thread per row)
+//   warps 2-9  fold each block's accumulators into H and L (a thread per row and 16 columns)
 //              and write C.
 // Operands are sliced by oz_partmax_kernel and oz_slice_kernel beforehand
 // (K-major, zero outside the triangle a flag names).  Every wait is bounded (ELHL_ERR_TIMEOUT).
@@ -44,7 +44,8 @@ constexpr int kS = 7;
 constexpr int kTM = 128, kTN = 32, kKB = 64;
 constexpr int kAStages = 8;
 constexpr int kBStages = 2;
-constexpr int kThreads = 192;
+constexpr int kFoldCols = 16, kFoldWarps = 4 * (kTN / kFoldCols);  // a fold warp: 32 rows x kFoldCols columns
+constexpr int kThreads = 64 + 32 * kFoldWarps;
 constexpr int kATile = kTM * kKB * 2;       // 16 KB
 constexpr int kBSlice = kTN * kKB * 2;      // 4 KB
 constexpr int kBStage = kS * kBSlice;       // 28 KB
@@ -231,7 +232,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint64_t *accfull = bempty + kBStages, *accempty = accfull + 2, *done = accempty + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + Smem::misc_off);
     int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
-    unsigned *flag = reinterpret_cast<unsigned *>(tmem_slot + 2);
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kAStages; ++s) {
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&accfull[s], 1);
-            mbar_init(&accempty[s], 128);
+            mbar_init(&accempty[s], kFoldWarps);  // one arrival per fold warp
         }
         mbar_init(done, 1);
         *abort_flag = 0;
@@ -338,49 +338,56 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (stop) break;
         }
     } else if (warp >= 2) {
-        // ---- fold the weights of each block into H and L, then write C
-        const int t = threadIdx.x - 64;          // 0 .. 127
+        // ---- fold the weights of each block into H and L, then write C: eight warps, the
+        // buffer released as soon as it is read (2,100 of a block's 3,560 cycles, beside the
+        // 28 MMAs of the next, 3,100; four warps that released it after the fold: 122.7 us
+        // per product of a rebuild at N = 3720, 118.1 so)
         const int quad = warp & 3;               // TMEM lanes [32 quad, 32 quad + 32)
-        const int row = i0 + quad * 32 + lane;
-        long long H[kTN], L[kTN];
+        const int row = i0 + quad * 32 + lane, c0 = (warp - 2) / 4 * kFoldCols;
+        long long H[kFoldCols], L[kFoldCols];
 #pragma unroll
-        for (int c = 0; c < kTN; ++c) {
+        for (int c = 0; c < kFoldCols; ++c) {
             H[c] = 0;
             L[c] = 0;
         }
         bool ok = true;
         for (int bi = 0; bi < kb1 - kb0; ++bi) {
             const unsigned tb = bi & 1;
-            if (t == 0) *flag = mbar_wait(&accfull[tb], (bi >> 1) & 1, kWaitNs) ? 1u : 0u;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            ok = *(volatile unsigned *)flag != 0;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (!ok) {
-                if (t == 0) atomicExch(abort_flag, 1);
+            if (!(ok = mbar_wait_warp(&accfull[tb], (bi >> 1) & 1, kWaitNs))) {
+                if (lane == 0) atomicExch(abort_flag, 1);
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;");
-            const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + tb * kAccCols;
+            const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + tb * kAccCols + (uint32_t)c0;
+            auto fold = [&](int d, const uint32_t (&v)[kFoldCols]) {
 #pragma unroll
-            for (int d = 0; d < kS; ++d) {
-                uint32_t v[32];
-                tmem_ld32(taddr + (uint32_t)(d * kTN), v);
-                tmem_wait_ld();
-#pragma unroll
-                for (int c = 0; c < kTN; ++c) {
+                for (int c = 0; c < kFoldCols; ++c) {
                     const long long x = (long long)__float2int_rn(__uint_as_float(v[c]));
                     if (d <= 2) H[c] += x * (1ll << (8 * (2 - d)));
                     else L[c] += x * (1ll << (8 * (kS - 1 - d)));
                 }
-            }
+            };
+            constexpr int kFirst = 3;  // weights read before the first fold
+            uint32_t v[kS - kFirst][kFoldCols];
+#pragma unroll
+            for (int d = 0; d < kFirst; ++d) tmem_ld16(taddr + (uint32_t)(d * kTN), v[d]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int d = 0; d < kFirst; ++d) fold(d, v[d]);
+#pragma unroll
+            for (int d = kFirst; d < kS; ++d) tmem_ld16(taddr + (uint32_t)(d * kTN), v[d - kFirst]);
+            tmem_wait_ld();
             asm volatile("tcgen05.fence::before_thread_sync;");
-            mbar_arrive(&accempty[tb]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&accempty[tb]);  // the warp has read the buffer
+#pragma unroll
+            for (int d = kFirst; d < kS; ++d) fold(d, v[d - kFirst]);
         }
         if (ok && row < g.m) {
             const double rs = g.rs[row] * pow2(-64);
 #pragma unroll
-            for (int c = 0; c < kTN; ++c) {
-                const int col = j0 + c;
+            for (int c = 0; c < kFoldCols; ++c) {
+                const int col = j0 + c0 + c;
                 if (col >= g.n) continue;
                 const double val = ((double)H[c] * 0x1p32 + (double)L[c]) * rs * g.cs[col];
                 double *cp = g.C + (size_t)col * g.ldc + row;
