@@ -394,6 +394,7 @@ struct TaylorBuffers {
     double2 *slots = nullptr;
     TaylorParticle *part = nullptr;
     double *tfinal = nullptr;
+    ulonglong2 *words = nullptr;  // vectors and records on their way between the CTAs
     int reserve(int N_, int P_) {
         const int ldv_ = round_up(N_, 32);
         if (slots && N_ <= N && P_ <= P && ldv_ <= ldv) return ELHL_OK;
@@ -404,11 +405,12 @@ struct TaylorBuffers {
         if (int rc = dev_alloc(&slots, (size_t)P * kSlots * 2 * ldv)) return rc;
         if (int rc = dev_alloc(&part, (size_t)P)) return rc;
         if (int rc = dev_alloc(&tfinal, 1)) return rc;
+        if (int rc = dev_alloc(&words, taylor_words(N, g_ctx.grid))) return rc;
         CU_TRY(cudaMemset(slots, 0, (size_t)P * kSlots * 2 * ldv * sizeof(double2)));
         return ELHL_OK;
     }
     void release() {
-        dev_free(slots); dev_free(part); dev_free(tfinal);
+        dev_free(slots); dev_free(part); dev_free(tfinal); dev_free(words);
         N = 0;
         P = 0;
     }
@@ -452,6 +454,7 @@ int run_taylor(const double *Hp, int N, int ld, TaylorBuffers &tb, int P, const 
     L.partials = g_ctx.partials;
     L.bar_count = g_ctx.bar;
     L.error = g_ctx.err;
+    L.words = tb.words;
     CU_TRY(cudaEventRecord(g_ctx.ev[0], st));
     CU_TRY(launch_taylor(L, g_ctx.grid, kTaylorBlock, st));
     CU_TRY(cudaEventRecord(g_ctx.ev[1], st));

@@ -85,8 +85,10 @@ struct TaylorLaunch {
     double *pop_partials; // [grid][nparticles][kMaxFrag+1]
     unsigned *bar_count;  // grid barrier: two words, one 64-bit count (8-byte aligned, zero at the launch)
     int *error;           // global error flag
+    ulonglong2 *words;    // taylor_words(N, grid) words exchanged in place of the barrier, or nullptr
 };
 constexpr int kSlots = 6;
+size_t taylor_words(int N, int grid);
 
 cudaError_t launch_taylor(const TaylorLaunch &L, int grid, int block, cudaStream_t st);
 int taylor_grid_size(int block, int *grid_out);

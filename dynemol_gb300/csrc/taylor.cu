@@ -14,7 +14,11 @@
 //   epilogue   one warp per eight rows forms the scaled term, the partial sum
 //              and, where the round decides something, the CTA's record
 //              (max |delta|^2 of bra and ket, <bra|ket>);
-//   barrier    bounded grid barrier (gives up after kBarrierNs and reports
+//   exchange   the vector that follows (as a rule) and the records go from CTA to
+//              CTA as words tagged with the round, polled by their readers
+//              (exchange.cuh); a bounded grid barrier instead where the kernel is not
+//              resident, without L.words, at a step's first round and where another
+//              vector follows (both give up after kBarrierNs and report
 //              ELHL_ERR_TIMEOUT instead of hanging);
 //   advance    one warp per particle sums the records in a fixed order and
 //              advances an identical copy of the particle's state machine in
@@ -43,14 +47,16 @@
 //     cost more than the products saved;
 //   - grid_arrive / grid_poll (grid_sync.cuh) instead of grid_barrier.
 // Measured, one particle at N = 465 (the 150-atom drop-in call, 3254 rounds): 23 us
-// per round before (one thread per column, 32 accumulators each), 6.4 us now:
-// products 5,900 cycles (5,400 is the FP64 unit's time for the 72 warp instructions
-// of each sub-partition), barrier 2,750, epilogue 1,950, vectors 850.  N = 62: 4 us.
+// per round before (one thread per column, 32 accumulators each), 6.4 us with a barrier
+// per round (products 5,900 cycles, 5,400 of them the FP64 unit's time for the 72 warp
+// instructions of each sub-partition, barrier 2,750, epilogue 1,950, vectors 850), 4.8 us
+// with the words.
 #include <cooperative_groups.h>
 
 #include <algorithm>
 
 #include "elhl_internal.cuh"
+#include "exchange.cuh"
 #include "grid_sync.cuh"
 
 namespace elhl {
@@ -235,7 +241,7 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
     __shared__ Ctrl ctrl[P];
     __shared__ double red[kWarps][16 * P];       // non-resident: a chunk's warp sums
     __shared__ double unit_rec[kWarps][4];       // records of the epilogue's units
-    __shared__ int s_step, s_it, s_ok;
+    __shared__ int s_step, s_it, s_ok, s_abort;
     __shared__ double s_tinit, s_tmax;
 
     const int G = gridDim.x;
@@ -255,6 +261,7 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
     };
 
     if (tid == 0) {
+        s_abort = 0;
         s_step = 0;
         s_it = L.it0;
         s_tinit = L.t_init;
@@ -408,6 +415,37 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
         }
     };
 
+    // Exchange without the barrier (resident, L.words): the round's next source and its
+    // records go out as words tagged with the round, which the readers poll.  Two buffers
+    // suffice: a CTA publishes round r + 2 once it has every CTA's words of round r + 1,
+    // and those follow their CTA's use of round r.
+    const bool words = kResident && L.words != nullptr;
+    unsigned long long round = 0;
+    auto word = [&](int p) { return L.words + ((size_t)(round & 1) * PMAX + p) * 4 * N; };
+    auto rec_word = [&](int p) {
+        return L.words + (size_t)2 * PMAX * 4 * N + ((size_t)(round & 1) * PMAX + p) * 4 * G;
+    };
+    // particle p's published vectors into shared memory as they arrive
+    auto stage_words = [&](int p) {
+        constexpr int U = 8;
+        const ulonglong2 *src = word(p);
+        double *dst = sv + (size_t)p * np * 4;
+        for (int base = 0; base < 4 * N; base += U * kTaylorBlock) {
+            ulonglong2 w[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int e = base + u * kTaylorBlock + tid;
+                w[u] = e < 4 * N ? fetch(src + e) : make_ulonglong2(0ull, round);
+            }
+            if (!await_words(w, round, src + base + tid, kTaylorBlock, L.error, kBarrierNs)) s_abort = 1;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int e = base + u * kTaylorBlock + tid;
+                if (e < 4 * N) dst[e] = __longlong_as_double((long long)w[u].x);
+            }
+        }
+    };
+
     int parity = 0;
     unsigned long long arrivals = 0;  // of the whole grid, at the next barrier's end
     double keep[P];                   // this lane's element of the last partial sum (first unit) ...
@@ -421,6 +459,11 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
     auto record = [&](int p, int q) -> double * {
         return L.partials + (((size_t)parity * PMAX + p) * G + blockIdx.x) * PW + q;
     };
+    // this CTA's record field q of particle p in a decision of an expansion
+    auto put_record = [&](int p, int q, double x) {
+        if (words) publish(rec_word(p) + 4 * blockIdx.x + q, (unsigned long long)__double_as_longlong(x), round);
+        else *record(p, q) = x;
+    };
     // wait for the round's arrivals; false: the launch ends with an error
     auto wait_round = [&]() -> bool {
         arrivals += G;
@@ -430,9 +473,10 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
     };
     bool ready = false;  // the next round's products are formed
     for (;;) {
+        ++round;
         int src[P];
         bool act[P];
-        bool norm = false;
+        bool norm = false;  // of every particle that is not done, or of none
 #pragma unroll
         for (int p = 0; p < P; ++p) {
             src[p] = ctrl[p].src;
@@ -477,6 +521,7 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
             const Ctrl &c = ctrl[p];
             const bool rec = decides(c);
             const double gk = c.g[c.k - 1];
+            const bool give_sum = c.phase == PH_MAIN && c.k >= c.kmax;  // the next source, as guessed below
             double best = 0.0, dot = 0.0;  // lanes of component 0 / 1: Re / Im of <bra|ket>
             // units dealt so that both particles' first units go to different warps
             for (int u = (warp + kWarps - p) % kWarps; u < groups; u += kWarps) {
@@ -506,6 +551,9 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
                 if (in) {
                     reinterpret_cast<double *>(vec(p, c.out_term, comp < 2))[e] = t;
                     reinterpret_cast<double *>(vec(p, c.out_acc, comp < 2))[e] = n;
+                    if (words)
+                        publish(word(p) + (size_t)i * 4 + comp,
+                                (unsigned long long)__double_as_longlong(give_sum ? n : t), round);
                 }
                 if (u == 0) keep[p] = n;
                 if (rec) {
@@ -530,12 +578,12 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
                 if (groups <= 1) {
                     if (warp == p) {
                         if (lane == 0) {
-                            *record(p, 1) = best;
-                            *record(p, 2) = dot;
+                            put_record(p, 1, best);
+                            put_record(p, 2, dot);
                         } else if (lane == 1) {
-                            *record(p, 3) = dot;
+                            put_record(p, 3, dot);
                         } else if (lane == 2) {
-                            *record(p, 0) = best;
+                            put_record(p, 0, best);
                         }
                     }
                 } else {
@@ -552,20 +600,23 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
                         double s = unit_rec[0][tid];
                         for (int w = 1; w < kWarps; ++w)
                             s = tid < 2 ? max_bits(s, unit_rec[w][tid]) : s + unit_rec[w][tid];
-                        *record(p, tid) = s;
+                        put_record(p, tid, s);
                     }
                     __syncthreads();
                 }
             }
             keep_slot[p] = c.out_acc;
         }
-        if (P == 1 && groups <= 1) {  // warp 0 alone wrote global memory in this round
-            __syncwarp();
-        } else {
-            __syncthreads();
+        const bool barrier = !words || norm;
+        if (barrier) {
+            if (P == 1 && groups <= 1) {  // warp 0 alone wrote global memory in this round
+                __syncwarp();
+            } else {
+                __syncthreads();
+            }
+            if (tid == 0) grid_arrive(L.bar_count);
+            if (!wait_round()) break;
         }
-        if (tid == 0) grid_arrive(L.bar_count);
-        if (!wait_round()) break;
 
         // ------------------------------------------------ advance
         // The next round's source unless the advance decides otherwise: this round's
@@ -579,9 +630,13 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
         if constexpr (kResident) {
 #pragma unroll
             for (int p = 0; p < P; ++p)
-                if (act[p]) stage(p, guess[p]);
+                if (act[p]) {
+                    if (words) stage_words(p);
+                    else stage(p, guess[p]);
+                }
         }
         __syncthreads();  // ctrl has been read by every thread; the staged vectors are complete
+        if (s_abort) break;
         if (warp < P) {
             // warp p: particle p's records summed in a fixed order (identical in every CTA)
             Ctrl &c = ctrl[warp];
@@ -590,10 +645,36 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
                 // lanes 0-15 sum fields 0 and 2 (bra maximum, Re <bra|ket>), lanes 16-31 fields 1 and 3
                 const double *rec = L.partials + ((size_t)parity * PMAX + warp) * G * PW + (lane >> 4);
                 double m = 0.0, d = 0.0;
+                if (barrier) {
 #pragma unroll 5
-                for (int g = lane & 15; g < G; g += 16) {
-                    m = max_bits(m, __ldcg(rec + (size_t)g * PW));
-                    d += __ldcg(rec + (size_t)g * PW + 2);
+                    for (int g = lane & 15; g < G; g += 16) {
+                        m = max_bits(m, __ldcg(rec + (size_t)g * PW));
+                        d += __ldcg(rec + (size_t)g * PW + 2);
+                    }
+                } else {
+                    constexpr int U = 5;
+                    const ulonglong2 *rw = rec_word(warp) + (lane >> 4);
+                    for (int g0 = 0; g0 < G; g0 += 16 * U) {
+                        ulonglong2 a[U], b[U];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const int g = g0 + 16 * u + (lane & 15);
+                            a[u] = b[u] = make_ulonglong2(0ull, round);
+                            if (g < G) {
+                                a[u] = fetch(rw + 4 * g);
+                                b[u] = fetch(rw + 4 * g + 2);
+                            }
+                        }
+                        const ulonglong2 *at = rw + 4 * (g0 + (lane & 15));
+                        if (!await_words(a, round, at, 64, L.error, kBarrierNs) ||
+                            !await_words(b, round, at + 2, 64, L.error, kBarrierNs))
+                            s_abort = 1;
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            m = max_bits(m, __longlong_as_double((long long)a[u].x));
+                            d += __longlong_as_double((long long)b[u].x);
+                        }
+                    }
                 }
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) {
@@ -612,6 +693,7 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
         }
         products(guess, act);
         __syncthreads();
+        if (s_abort) break;
         parity ^= 1;
 
         bool all_done = true;
@@ -622,7 +704,13 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
             all_done &= c.phase == PH_DONE;
             if (c.phase == PH_CONV || c.phase == PH_MAIN) ready &= c.src == guess[p];
         }
-        if (!all_done) continue;
+        if (!all_done) {
+            if (!ready && !barrier) {  // another source than guessed: its slots, written before this barrier
+                if (tid == 0) grid_arrive(L.bar_count);
+                if (!wait_round()) break;
+            }
+            continue;
+        }
         ready = false;
 
         // ---- step finished for every particle: population round + step driver
@@ -718,6 +806,10 @@ cudaError_t launch_taylor_t(const TaylorLaunch &L, int grid, int block, size_t s
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     TaylorLaunch copy = L;
+    if (kResident && L.words) {  // no word carries a round's tag before the launch
+        e = cudaMemsetAsync(L.words, 0, taylor_words(L.N, grid) * sizeof(ulonglong2), st);
+        if (e != cudaSuccess) return e;
+    }
     void *args[] = {&copy};
     e = cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(block), args, smem, st);
     count_launch();
@@ -725,6 +817,8 @@ cudaError_t launch_taylor_t(const TaylorLaunch &L, int grid, int block, size_t s
 }
 
 }  // namespace
+
+size_t taylor_words(int N, int grid) { return (size_t)2 * PMAX * 4 * ((size_t)N + grid); }
 
 int taylor_grid_size(int block, int *grid_out) {
     int dev = 0, sms = 0, per_sm = 0;
