@@ -1236,32 +1236,20 @@ __global__ void gemm_order0_kernel(const double2 *__restrict__ phi, const double
     acc[q] = make_double2(c0.x * p.x - c0.y * p.y, c0.x * p.y + c0.y * p.x);
 }
 
-// y = sum of the nsplit partial products (fixed order, as an FP32 pair: TwoSum, so
-// exact to 2^-48), v_k = 2 y - v_{k-2} (v_1 = y) rounded once to FP32, acc += c_k v_k
-// in FP64.  The sums in FP64 bound this kernel by the FP64 unit (32 of its 40 FP64
-// instructions per element at 16 splits): 30 us per order at N = 4092, 64 columns,
-// 8 us on the FP32 pipes.
-__global__ void __launch_bounds__(256) gemm_epilogue_kernel(const float2 *__restrict__ Y, int nsplit,
-                                                            size_t split_stride, const float2 *__restrict__ vprev2,
+// v_k = 2 y - v_{k-2} (v_1 = y), acc += c_k v_k in FP64 (y: one product, summed in FP32)
+__global__ void __launch_bounds__(256) gemm_epilogue_kernel(const float2 *__restrict__ Y,
+                                                            const float2 *__restrict__ vprev2,
                                                             float2 *__restrict__ vout, double2 *__restrict__ acc,
                                                             const double2 *coef, int k, int nm) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nm) return;
     double2 a = acc[q];
-    const float2 w = k == 1 ? make_float2(0.f, 0.f) : vprev2[q];
-    float2 h = Y[q], l = make_float2(0.f, 0.f);
-#pragma unroll 8
-    for (int s = 1; s < nsplit; ++s) {
-        const float2 t = Y[s * split_stride + q];
-        df_add(h.x, l.x, t.x, 0.f);
-        df_add(h.y, l.y, t.y, 0.f);
-    }
-    float2 v;
-    if (k == 1) {
-        v = make_float2(__fadd_rn(h.x, l.x), __fadd_rn(h.y, l.y));
-    } else {
-        v.x = two_sum_plus(__fmul_rn(2.f, h.x), -w.x, __fmul_rn(2.f, l.x));
-        v.y = two_sum_plus(__fmul_rn(2.f, h.y), -w.y, __fmul_rn(2.f, l.y));
+    const float2 y = Y[q];
+    float2 v = y;
+    if (k > 1) {
+        const float2 w = vprev2[q];
+        v.x = __fsub_rn(__fmul_rn(2.f, y.x), w.x);
+        v.y = __fsub_rn(__fmul_rn(2.f, y.y), w.y);
     }
     vout[q] = v;
     const double2 c = coef[k];
@@ -1320,18 +1308,20 @@ int cheb_gemm_enqueue(ChebState &cs, int parity) {
     const bool renorm = true;
     gemm_order0_kernel<<<nb, tb, 0, st>>>(in, renorm ? cs.scale : nullptr, cs.P, n, m, cs.c0, vb, out);
     count_launch();
+    if (cs.umma)
+        if (int rc = umma_pack_v(reinterpret_cast<const float *>(vb), n, 2 * m, cs.vpack, st)) return rc;
     for (int k = 1; k <= cs.K; ++k) {
-        const float *vprev = reinterpret_cast<const float *>(vb + ((k + 2) % 3) * vs);
+        const float2 *vprev = vb + ((k + 2) % 3) * vs, *vprev2 = vb + ((k + 1) % 3) * vs;
+        float2 *vk = vb + (k % 3) * vs;
         if (cs.umma) {  // Y (N x 2m) = Hs V^T on the tensor cores (Hs symmetric), three BF16 terms each
-            if (int rc = umma_pack_v(vprev, n, 2 * m, cs.vpack, st)) return rc;
             if (int rc = umma_bf16x3_gemm(cs.hpack, cs.vpack, n, n, 2 * m, cs.usplits, cs.Y, g_ctx.err, st)) return rc;
-        } else if (int rc = gemm_vt(g_ctx.blas_tc, cs.precision, 2 * m, n, vprev,
-                                    reinterpret_cast<const float *>(cs.Hs), cs.ld, cs.Y)) {
-            return rc;
+            if (int rc = umma_epilogue(cs.Y, cs.usplits, vprev2, vk, out, cs.coef, k, n, m, cs.vpack, st)) return rc;
+            continue;
         }
-        gemm_epilogue_kernel<<<nb, tb, 0, st>>>(reinterpret_cast<const float2 *>(cs.Y), cs.umma ? cs.usplits : 1,
-                                                (size_t)n * m, vb + ((k + 1) % 3) * vs,
-                                                vb + (k % 3) * vs, out, cs.coef, k, nm);
+        if (int rc = gemm_vt(g_ctx.blas_tc, cs.precision, 2 * m, n, reinterpret_cast<const float *>(vprev),
+                             reinterpret_cast<const float *>(cs.Hs), cs.ld, cs.Y))
+            return rc;
+        gemm_epilogue_kernel<<<nb, tb, 0, st>>>(reinterpret_cast<const float2 *>(cs.Y), vprev2, vk, out, cs.coef, k, nm);
         count_launch();
     }
     norm_drift_cols_kernel<<<m, kDriftBlock, 0, st>>>(in, out, n, m, cs.P, renorm ? cs.scale : nullptr, cs.drift);

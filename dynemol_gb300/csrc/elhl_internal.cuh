@@ -200,6 +200,9 @@ size_t umma_a_bytes(int N);
 size_t umma_b_bytes(int N, int n2);
 int umma_pack_h(const float *H, int N, int ld, void *dst, cudaStream_t st);
 int umma_pack_v(const float *v, int n, int n2, void *dst, cudaStream_t st);
+// the order's epilogue: recurrence and accumulation from the partials Y, v_k packed for the next product
+int umma_epilogue(const float *Y, int nsplit, const float2 *vprev2, float2 *vout, double2 *acc, const double2 *coef, int k,
+                  int n, int m, void *dst, cudaStream_t st);
 int umma_bf16x3_gemm(const void *A, const void *B, int rows, int K, int n2, int splits, float *Y, int *d_error,
                      cudaStream_t st);
 

@@ -40,6 +40,7 @@
 // nearly empty) were the earlier form.
 #include <algorithm>
 
+#include "df64.cuh"
 #include "elhl_internal.cuh"
 #include "tc_ptx.cuh"
 
@@ -249,50 +250,117 @@ int launch_umma(const UmmaParams &p, cudaStream_t st) {
 
 // Packed operand: for each tile of `tile` rows and each chunk of 64 K, the three terms'
 // tiles as they lie in shared memory (rows of 128 B, 16-byte piece c of row r at piece
-// c ^ (r & 7): the 128B swizzle), so that a chunk is one contiguous run of memory.  A
-// thread splits eight consecutive K of one row: x = x0 + x1 + x2 in BF16 terms, each the
-// rounding of the remainder.  Zero outside rows x K.
-// get(row, k): the operand's element
-template <typename Get>
-__device__ __forceinline__ void pack8(unsigned char *dst, int tile, int nk, int row, int k0, Get get) {
-    uint4 t[3];
-    unsigned *w = reinterpret_cast<unsigned *>(t);
+// c ^ (r & 7): the 128B swizzle), so that a chunk is one contiguous run of memory.
+// KN (4 or 8) consecutive K from k0 on of one row: x = x0 + x1 + x2 in BF16 terms, each the
+// rounding of the remainder.
+template <int KN>
+__device__ __forceinline__ void pack_row(unsigned char *dst, int tile, int nk, int row, int k0, const float (&x)[KN]) {
+    unsigned w[3][KN / 2];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < KN / 2; ++q) {
         unsigned short v[2][3];
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-            const float x = get(row, k0 + 2 * q + u);
-            const __nv_bfloat16 a = __float2bfloat16_rn(x);
-            const float ra = x - __bfloat162float(a);
+            const __nv_bfloat16 a = __float2bfloat16_rn(x[2 * q + u]);
+            const float ra = x[2 * q + u] - __bfloat162float(a);
             const __nv_bfloat16 b = __float2bfloat16_rn(ra);
             v[u][0] = __bfloat16_as_ushort(a);
             v[u][1] = __bfloat16_as_ushort(b);
             v[u][2] = __bfloat16_as_ushort(__float2bfloat16_rn(ra - __bfloat162float(b)));
         }
 #pragma unroll
-        for (int s = 0; s < 3; ++s) w[4 * s + q] = (unsigned)v[0][s] | ((unsigned)v[1][s] << 16);
+        for (int s = 0; s < 3; ++s) w[s][q] = (unsigned)v[0][s] | ((unsigned)v[1][s] << 16);
     }
     const int r = row % tile, c = (k0 % kBK) / 8;
     unsigned char *d = dst + ((size_t)(row / tile) * nk + k0 / kBK) * (3 * (size_t)tile * kBK * 2) + (size_t)r * kBK * 2 +
-                       (size_t)((c ^ (r & 7)) * 16);
+                       (size_t)((c ^ (r & 7)) * 16 + (k0 & 4) * 2);
 #pragma unroll
-    for (int s = 0; s < 3; ++s) *reinterpret_cast<uint4 *>(d + s * (size_t)tile * kBK * 2) = t[s];
+    for (int s = 0; s < 3; ++s) {
+        unsigned char *t = d + s * (size_t)tile * kBK * 2;
+        if constexpr (KN == 8) *reinterpret_cast<uint4 *>(t) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+        else *reinterpret_cast<uint2 *>(t) = make_uint2(w[s][0], w[s][1]);
+    }
 }
 
 // A of a symmetric H in FP32 (N columns of ld rows): a row's K are a column
 __global__ void pack_h_kernel(const float *__restrict__ H, int N, int ld, unsigned char *dst, int nk) {
     const int k0 = 8 * (blockIdx.x * blockDim.x + threadIdx.x), row = blockIdx.y;
     if (k0 >= nk * kBK) return;
-    pack8(dst, kBM, nk, row, k0,
-          [&](int r, int k) { return r < N && k < N ? H[(size_t)r * ld + k] : 0.f; });
+    float x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = row < N && k0 + u < N ? H[(size_t)row * ld + k0 + u] : 0.f;
+    pack_row(dst, kBM, nk, row, k0, x);
 }
 
 // B of the Chebyshev block v (n rows of n2 reals): one row of B per column of v
 __global__ void pack_v_kernel(const float *__restrict__ v, int n, int n2, unsigned char *dst, int nk) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x, c = t % n2, k0 = 8 * (t / n2);
     if (k0 >= nk * kBK) return;
-    pack8(dst, n2, nk, c, k0, [&](int r, int k) { return k < n ? v[(size_t)k * n2 + r] : 0.f; });
+    float x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = k0 + u < n ? v[(size_t)(k0 + u) * n2 + c] : 0.f;
+    pack_row(dst, n2, nk, c, k0, x);
+}
+
+// y = sum of the nsplit partial products (fixed order, as an FP32 pair: TwoSum, so
+// exact to 2^-48), v_k = 2 y - v_{k-2} (v_1 = y) rounded once to FP32, acc += c_k v_k
+// in FP64, and v_k packed as the next product's B (rows past n keep the zeros that
+// packing v_0 left).  A thread takes kEpiRows rows of one complex column, everything it
+// reads asked for before the first result: bound by the FP64 unit (eight of its
+// instructions per element, 4 us at N = 4092, 64 columns).  There 9.4 us, against 7.0 + 2.8
+// and a launch with the packing apart; eight rows one after another took 17.6.
+constexpr int kEpiRows = 4;
+__global__ void __launch_bounds__(128) umma_epilogue_kernel(const float2 *__restrict__ Y, int nsplit,
+                                                            size_t split_stride, const float2 *__restrict__ vprev2,
+                                                            float2 *__restrict__ vout, double2 *__restrict__ acc,
+                                                            const double2 *coef, int k, int n, int m,
+                                                            unsigned char *dst, int nk) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, c = t % m, r0 = kEpiRows * (t / m);
+    if (r0 >= n) return;
+    const int rows = min(kEpiRows, n - r0);
+    double2 a[kEpiRows];
+    float2 w[kEpiRows], h[kEpiRows], l[kEpiRows];
+#pragma unroll
+    for (int i = 0; i < kEpiRows; ++i) {
+        const size_t q = (size_t)(r0 + min(i, rows - 1)) * m + c;
+        a[i] = acc[q];
+        w[i] = k == 1 ? make_float2(0.f, 0.f) : vprev2[q];
+        h[i] = Y[q];
+        l[i] = make_float2(0.f, 0.f);
+    }
+    const double2 ck = coef[k];
+#pragma unroll 4
+    for (int s = 1; s < nsplit; ++s) {
+#pragma unroll
+        for (int i = 0; i < kEpiRows; ++i) {
+            const float2 y = Y[s * split_stride + (size_t)(r0 + min(i, rows - 1)) * m + c];
+            df_add(h[i].x, l[i].x, y.x, 0.f);
+            df_add(h[i].y, l[i].y, y.y, 0.f);
+        }
+    }
+    float re[kEpiRows], im[kEpiRows];
+#pragma unroll
+    for (int i = 0; i < kEpiRows; ++i) {
+        float2 v;
+        if (k == 1) {
+            v = make_float2(__fadd_rn(h[i].x, l[i].x), __fadd_rn(h[i].y, l[i].y));
+        } else {
+            v.x = two_sum_plus(__fmul_rn(2.f, h[i].x), -w[i].x, __fmul_rn(2.f, l[i].x));
+            v.y = two_sum_plus(__fmul_rn(2.f, h[i].y), -w[i].y, __fmul_rn(2.f, l[i].y));
+        }
+        re[i] = im[i] = 0.f;
+        if (i >= rows) continue;
+        re[i] = v.x;
+        im[i] = v.y;
+        const size_t q = (size_t)(r0 + i) * m + c;
+        vout[q] = v;
+        double2 s = a[i];
+        s.x += ck.x * (double)v.x - ck.y * (double)v.y;
+        s.y += ck.x * (double)v.y + ck.y * (double)v.x;
+        acc[q] = s;
+    }
+    pack_row(dst, 2 * m, nk, 2 * c, r0, re);
+    pack_row(dst, 2 * m, nk, 2 * c + 1, r0, im);
 }
 
 }  // namespace
@@ -314,6 +382,17 @@ int umma_pack_h(const float *H, int N, int ld, void *dst, cudaStream_t st) {
 int umma_pack_v(const float *v, int n, int n2, void *dst, cudaStream_t st) {
     const int nk = (n + kBK - 1) / kBK;
     pack_v_kernel<<<(nk * (kBK / 8) * n2 + 127) / 128, 128, 0, st>>>(v, n, n2, static_cast<unsigned char *>(dst), nk);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? ELHL_OK : ELHL_ERR_CUDA;
+}
+
+int umma_epilogue(const float *Y, int nsplit, const float2 *vprev2, float2 *vout, double2 *acc, const double2 *coef, int k,
+                  int n, int m, void *dst, cudaStream_t st) {
+    const int threads = (n + kEpiRows - 1) / kEpiRows * m;
+    umma_epilogue_kernel<<<(threads + 127) / 128, 128, 0, st>>>(reinterpret_cast<const float2 *>(Y), nsplit,
+                                                                (size_t)n * m, vprev2, vout, acc, coef, k, n, m,
+                                                                static_cast<unsigned char *>(dst),
+                                                                (n + kBK - 1) / kBK);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? ELHL_OK : ELHL_ERR_CUDA;
 }
