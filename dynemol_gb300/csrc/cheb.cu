@@ -410,6 +410,7 @@ __global__ void __launch_bounds__(kBlock, 1) cheb_kernel(ChebLaunch L) {
     const int G = gridDim.x;
     const int s0 = L.seg_begin[blockIdx.x], s1 = L.seg_begin[blockIdx.x + 1];
     const unsigned long long bar_ns = L.barrier_ns ? L.barrier_ns : kBarrierNs;
+    if (__syncthreads_or(*(volatile const int *)L.error)) return;  // an earlier launch of this call gave up
     if ((int)blockIdx.x + 1 == L.exit_cta1) return;  // test hook: the other CTAs' barrier waits run out
     __shared__ int s_ok;
     unsigned long long arrivals = 0;
@@ -966,6 +967,7 @@ __global__ void __launch_bounds__(kBlock, 1) cheb_df_kernel(ChebLaunch L) {
     const int s0 = L.seg_begin[blockIdx.x], s1 = L.seg_begin[blockIdx.x + 1];
     const ChebProblem &pb = L.probs[0];
     const unsigned long long bar_ns = L.barrier_ns ? L.barrier_ns : kBarrierNs;
+    if (__syncthreads_or(*(volatile const int *)L.error)) return;  // an earlier launch of this call gave up
     if ((int)blockIdx.x + 1 == L.exit_cta1) return;  // test hook: the other CTAs' barrier waits run out
     __shared__ int s_ok;
     unsigned long long arrivals = 0;

@@ -180,6 +180,7 @@ __global__ void __launch_bounds__(kThreads, 1) cheb_rows_kernel(const RowsLaunch
     const int r0 = blockIdx.x * R;
     H *sh = reinterpret_cast<H *>(dyn);
     Sum *part = reinterpret_cast<Sum *>(sh + (size_t)R * np);
+    if (__syncthreads_or(*(volatile const int *)L.error)) return;  // an earlier launch of this call gave up
     if ((int)blockIdx.x + 1 == L.exit_cta1) return;  // test hook: the other CTAs' waits run out
     const unsigned long long limit = L.barrier_ns ? L.barrier_ns : kBarrierNs;
     if (tid == 0) s_abort = 0;

@@ -109,6 +109,10 @@ cudaError_t copy_d2h(void *dst, const void *src, size_t bytes) {
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, g_ctx.stream);
     return e != cudaSuccess ? e : cudaStreamSynchronize(g_ctx.stream);
 }
+// The error word of the propagation kernels, cleared once at the start of what is checked
+// as a whole (a call's steps, or an attempt at them) and read at its end: no launch in
+// between clears it, so a step that timed out is seen whatever the steps after it do.
+cudaError_t clear_error() { return cudaMemsetAsync(g_ctx.err, 0, sizeof(int), g_ctx.stream); }
 
 int ensure_context_locked(int device) {
     if (g_ctx.ready && (device < 0 || device == g_ctx.device)) return ELHL_OK;
@@ -1635,7 +1639,6 @@ int tune_plan(ChebPlan &pl) {
     for (int mg : cand) {
         float ms = 0.0f;
         for (int rep = 0; rep < 2; ++rep) {
-            CU_TRY(cudaMemsetAsync(g_ctx.err, 0, sizeof(int), st));
             CU_TRY(cudaMemsetAsync(g_ctx.bar, 0, 2 * sizeof(unsigned), st));
             CU_TRY(cudaEventRecord(g_ctx.ev[0], st));
             CU_TRY(launch_cheb(L, pl.precision, mg, st));
@@ -1690,7 +1693,6 @@ int oz_run(ChebPlan &pl) {
     L.barrier_ns = g_dbg_barrier_ns;
     L.exit_cta1 = g_dbg_exit_cta1;
     g_dbg_exit_cta1 = 0;  // one launch only
-    CU_TRY(cudaMemsetAsync(g_ctx.err, 0, sizeof(int), st));
     CU_TRY(cudaMemsetAsync(g_ctx.bar, 0, 2 * sizeof(unsigned), st));
     CU_TRY(cudaMemsetAsync(oz.part, 0, oz.parts * oz_tile_rows() * 16 * sizeof(double), st));  // tags
     CU_TRY(cudaMemsetAsync(oz.xe + (size_t)3 * 2 * oz.ntiles * 8, 0x80, 3 * 8 * sizeof(int), st));  // column maxima
@@ -1725,7 +1727,6 @@ int rows_run(ChebPlan &pl) {
     L.barrier_ns = g_dbg_barrier_ns;
     L.exit_cta1 = g_dbg_exit_cta1;
     g_dbg_exit_cta1 = 0;  // one launch only
-    CU_TRY(cudaMemsetAsync(g_ctx.err, 0, sizeof(int), st));
     CU_TRY(cudaEventRecord(g_ctx.ev[0], st));
     CU_TRY(launch_cheb_rows(L, pl.precision, cs.rows, st));
     CU_TRY(cudaEventRecord(g_ctx.ev[1], st));
@@ -1741,7 +1742,6 @@ int cheb_run(ChebPlan &pl) {
         if (int rc = tune_plan(pl)) return rc;
         pl.tuned = true;
     }
-    CU_TRY(cudaMemsetAsync(g_ctx.err, 0, sizeof(int), st));
     CU_TRY(cudaMemsetAsync(g_ctx.bar, 0, 2 * sizeof(unsigned), st));
     ChebLaunch L{};
     L.probs = pl.d_probs;
@@ -2383,6 +2383,7 @@ int cheb_run_checked(elhl_traj *tr, double *drift) {
     cudaStream_t st = g_ctx.stream;
     const double ntol = cheb_norm_tolerance(tr->cfg);
     for (int attempt = 0;; ++attempt) {
+        CU_TRY(clear_error());
         CU_TRY(cudaMemsetAsync(tr->plan.d_drift, 0, sizeof(double), st));
         if (int rc = cheb_run(tr->plan)) return rc;
         if (int rc = launch_norm_drift(tr->plan)) return rc;
@@ -2429,6 +2430,7 @@ int cheb_step_impl(elhl_traj *tr, const double *coords, bool coords_on_device, i
         double *d_drift = cs.gemm ? cs.drift : tr->plan.d_drift;
         double drift = 0.0;
         for (int attempt = 0;; ++attempt) {
+            CU_TRY(clear_error());
             CU_TRY(cudaMemsetAsync(d_drift, 0, sizeof(double), st));
             CU_TRY(cudaEventRecord(g_ctx.ev[2], st));
             for (int s = 0; s < nsteps; ++s) {
@@ -3652,6 +3654,7 @@ int elhl_batch_step(elhl_batch *b, int nsteps, double *pops) {
         if (!tr->cs.cols_current)
             if (int rc = cheb_load_columns(tr)) return rc;
     (void)per_traj;
+    CU_TRY(clear_error());
     CU_TRY(cudaMemsetAsync(b->plan.d_drift, 0, nt * sizeof(double), st));
     for (int s = 0; s < nsteps; ++s) {
         if (int rc = cheb_dev_step(b->plan, b->states, b->pops + s * per_step)) return rc;
@@ -3900,6 +3903,7 @@ int elhl_server_step(elhl_server *sv, int *n_active, int *n_pending) {
     if (!sv->active.empty()) {
         std::lock_guard<std::mutex> lk(g_ctx.mu);
         cudaStream_t st = g_ctx.stream;
+        CU_TRY(clear_error());
         // one cooperative launch per non-empty group, one step graph per GEMM-regime request
         for (auto &g : sv->groups) {
             if (g.reqs.empty()) continue;

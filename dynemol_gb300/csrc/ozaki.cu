@@ -636,6 +636,7 @@ __device__ void order_zero(const Ctx &c, const OzLaunch &L) {
 __global__ void __launch_bounds__(kThreads, 1)
     oz_cheb_kernel(const __grid_constant__ CUtensorMap mH, OzLaunch L) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
+    if (__syncthreads_or(*(volatile const int *)L.error)) return;  // an earlier launch of this call gave up
     if ((int)blockIdx.x + 1 == L.exit_cta1) return;  // test hook: the other CTAs' barrier waits run out
     Ctx c;
     c.smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
