@@ -252,9 +252,9 @@ cudaError_t dgemm64(int m, int n, int k, double alpha, const double *A, int lda,
     if (!ln.part) {
         cudaError_t e = cudaMalloc(&ln.part, (size_t)kMaxPartials * kMaxTile * kMaxTile * sizeof(double));
         if (e == cudaSuccess) e = cudaMalloc(&ln.count, (size_t)kMaxPartials * 16 * sizeof(int));
-        if (e == cudaSuccess) e = cudaMemset(ln.count, 0, (size_t)kMaxPartials * 16 * sizeof(int));
+        if (e == cudaSuccess) e = cudaMemsetAsync(ln.count, 0, (size_t)kMaxPartials * 16 * sizeof(int), st);
         if (e == cudaSuccess) e = cudaMalloc(&ln.sched, 4 * sizeof(int));
-        if (e == cudaSuccess) e = cudaMemset(ln.sched, 0, 4 * sizeof(int));
+        if (e == cudaSuccess) e = cudaMemsetAsync(ln.sched, 0, 4 * sizeof(int), st);
         if (e != cudaSuccess) return e;
     }
     const int kt = std::max(1, (k + kBK - 1) / kBK);

@@ -100,13 +100,18 @@ struct Context {
 Context g_ctx;
 
 // Copies ordered with the library stream.  The library's streams are created
-// non-blocking, so a plain cudaMemcpy (legacy default stream) is not ordered
-// with their work; device-to-host copies also wait for the data.
+// non-blocking, so a plain cudaMemcpy or cudaMemset (legacy default stream, which may be
+// busy with another library's work) is not ordered with theirs: copies and clears go to
+// g_ctx.stream; device-to-host copies also wait for the data.
 cudaError_t copy_h2d(void *dst, const void *src, size_t bytes) {
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, g_ctx.stream);
 }
 cudaError_t copy_d2h(void *dst, const void *src, size_t bytes) {
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, g_ctx.stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(g_ctx.stream);
+}
+cudaError_t copy2d_d2h(void *dst, size_t dpitch, const void *src, size_t spitch, size_t width, size_t rows) {
+    cudaError_t e = cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, rows, cudaMemcpyDeviceToHost, g_ctx.stream);
     return e != cudaSuccess ? e : cudaStreamSynchronize(g_ctx.stream);
 }
 // The error word of the propagation kernels, cleared once at the start of what is checked
@@ -144,8 +149,8 @@ int ensure_context_locked(int device) {
     if (int rc = dev_alloc(&g_ctx.bar, 2)) return rc;
     if (int rc = dev_alloc(&g_ctx.err, 1)) return rc;
     if (int rc = dev_alloc(&g_ctx.partials, (size_t)2 * 2 * g_ctx.grid * 16)) return rc;
-    CU_TRY(cudaMemset(g_ctx.bar, 0, 2 * sizeof(unsigned)));
-    CU_TRY(cudaMemset(g_ctx.err, 0, sizeof(int)));
+    CU_TRY(cudaMemsetAsync(g_ctx.bar, 0, 2 * sizeof(unsigned), g_ctx.stream));
+    CU_TRY(cudaMemsetAsync(g_ctx.err, 0, sizeof(int), g_ctx.stream));
     for (auto &e : g_ctx.ev) CU_TRY(cudaEventCreate(&e));
     // make the allocation-free entry point's fixed array resident now, before
     // a caller's pool allocator or stream capture can start
@@ -279,9 +284,9 @@ int ozgemm_status() {
         int *e = ozgemm_error(lane);
         if (!e) continue;
         int h = 0;
-        CU_TRY(cudaMemcpy(&h, e, sizeof(int), cudaMemcpyDeviceToHost));
+        CU_TRY(copy_d2h(&h, e, sizeof(int)));
         if (h) {
-            CU_TRY(cudaMemset(e, 0, sizeof(int)));
+            CU_TRY(cudaMemsetAsync(e, 0, sizeof(int), g_ctx.stream));
             return h;
         }
     }
@@ -335,7 +340,7 @@ struct Factor {
         if (int rc = dev_alloc(&G, (size_t)ld * N)) return rc;
         if (int rc = dev_alloc(&W, (size_t)ld * N)) return rc;
         if (int rc = dev_alloc(&info, 2)) return rc;
-        CU_TRY(cudaMemset(info, 0, 2 * sizeof(int)));
+        CU_TRY(cudaMemsetAsync(info, 0, 2 * sizeof(int), g_ctx.stream));
         if (int rc = dev_alloc(&cols, (size_t)4 * ld)) return rc;
         return ELHL_OK;
     }
@@ -410,7 +415,7 @@ struct TaylorBuffers {
         if (int rc = dev_alloc(&part, (size_t)P)) return rc;
         if (int rc = dev_alloc(&tfinal, 1)) return rc;
         if (int rc = dev_alloc(&words, taylor_words(N, g_ctx.grid))) return rc;
-        CU_TRY(cudaMemset(slots, 0, (size_t)P * kSlots * 2 * ldv * sizeof(double2)));
+        CU_TRY(cudaMemsetAsync(slots, 0, (size_t)P * kSlots * 2 * ldv * sizeof(double2), g_ctx.stream));
         return ELHL_OK;
     }
     void release() {
@@ -717,9 +722,9 @@ struct OzRes {
         grid = grid_;
         ntiles = (N + oz_tile_rows() - 1) / oz_tile_rows();
         if (int rc = dev_alloc(&v, (size_t)3 * ld * 8)) return rc;
-        CU_TRY(cudaMemset(v, 0, (size_t)3 * ld * 8 * sizeof(double)));
+        CU_TRY(cudaMemsetAsync(v, 0, (size_t)3 * ld * 8 * sizeof(double), g_ctx.stream));
         CU_TRY(cudaMalloc(&xs, xs_bytes()));
-        CU_TRY(cudaMemset(xs, 0, xs_bytes()));  // the zero slots of every tile stay zero
+        CU_TRY(cudaMemsetAsync(xs, 0, xs_bytes(), g_ctx.stream));  // the zero slots of every tile stay zero
         if (int rc = dev_alloc(&xe, (size_t)3 * 2 * ntiles * 8 + 3 * 8)) return rc;
         std::vector<OzSeg> sg;
         std::vector<int> b, pb, pc;
@@ -741,7 +746,7 @@ struct OzRes {
             CU_TRY(cudaMalloc(&s, (size_t)oz_slices() * N * ld * sizeof(__nv_bfloat16)));
             const size_t nr = (size_t)ntiles * oz_tile_rows();
             if (int rc = dev_alloc(&r, nr)) return rc;
-            CU_TRY(cudaMemset(r, 0, nr * sizeof(double)));  // rows past N: scale 0
+            CU_TRY(cudaMemsetAsync(r, 0, nr * sizeof(double), g_ctx.stream));  // rows past N: scale 0
         }
         CU_TRY(oz_slice_matrix(Hs, N, ld, s, r, st));
         return ELHL_OK;
@@ -826,19 +831,19 @@ struct ChebState {
         if (int rc = dev_alloc(&Ht, (size_t)ld * N)) return rc;
         CU_TRY(cudaMalloc(&Hs, (size_t)ld * N * tsz));
         CU_TRY(cudaMalloc(&vbuf, (size_t)3 * ld * m * 2 * tsz));
-        CU_TRY(cudaMemset(vbuf, 0, (size_t)3 * ld * m * 2 * tsz));
+        CU_TRY(cudaMemsetAsync(vbuf, 0, (size_t)3 * ld * m * 2 * tsz, g_ctx.stream));
         if (int rc = dev_alloc(&phi, (size_t)ld * m)) return rc;
         if (int rc = dev_alloc(&acc, (size_t)ld * m)) return rc;
-        CU_TRY(cudaMemset(phi, 0, (size_t)ld * m * sizeof(double2)));
-        CU_TRY(cudaMemset(acc, 0, (size_t)ld * m * sizeof(double2)));
+        CU_TRY(cudaMemsetAsync(phi, 0, (size_t)ld * m * sizeof(double2), g_ctx.stream));
+        CU_TRY(cudaMemsetAsync(acc, 0, (size_t)ld * m * sizeof(double2), g_ctx.stream));
         // 6 Lanczos vectors, per-CTA partial sums, the tridiagonal record
         if (int rc = dev_alloc(&lz, (size_t)6 * ld + kLzPart + 128)) return rc;
-        CU_TRY(cudaMemset(lz, 0, (size_t)4 * ld * sizeof(double)));  // exchanged words: no tag
+        CU_TRY(cudaMemsetAsync(lz, 0, (size_t)4 * ld * sizeof(double), g_ctx.stream));  // exchanged words: no tag
         if (int rc = dev_alloc(&cscratch, (size_t)2 * m * ld)) return rc;
         if (int rc = dev_alloc(&scale, (size_t)kMaxCols)) return rc;
         if (int rc = dev_alloc(&drift, 1)) return rc;
         if (int rc = dev_alloc(&ntot, (size_t)kMaxCols)) return rc;
-        CU_TRY(cudaMemset(drift, 0, sizeof(double)));
+        CU_TRY(cudaMemsetAsync(drift, 0, sizeof(double), g_ctx.stream));
         std::vector<double> ones(kMaxCols, 1.0);
         CU_TRY(copy_h2d(scale, ones.data(), kMaxCols * sizeof(double)));
         return ELHL_OK;
@@ -1082,7 +1087,7 @@ int cheb_prepare_implicit(ChebState &cs, const double *Lfac, const double *h, do
     if (!cs.Gt) CU_TRY(cudaMalloc(&cs.Gt, (size_t)ld * n * tsz));
     if (!cs.wb) {
         CU_TRY(cudaMalloc(&cs.wb, (size_t)2 * ld * cs.m * 2 * tsz));
-        CU_TRY(cudaMemset(cs.wb, 0, (size_t)2 * ld * cs.m * 2 * tsz));
+        CU_TRY(cudaMemsetAsync(cs.wb, 0, (size_t)2 * ld * cs.m * 2 * tsz, g_ctx.stream));
     }
     // L with a zero upper triangle (the recursion leaves S's there): the dense column transforms read all of it
     lower_only_kernel<<<dim3((ld + 127) / 128, n), 128, 0, st>>>(const_cast<double *>(Lfac), n, ld);
@@ -2778,11 +2783,12 @@ int cheb_set_psi(elhl_traj *tr, const elhl_zcomplex *bra, const elhl_zcomplex *k
     if (!bra && !tr->S) return ELHL_ERR_BAD_ARG;  // S was released by elhl_batch_compact
     const size_t e = sizeof(double2);
     const int P = tr->P, n = tr->N;
+    cudaStream_t st = g_ctx.stream;
     for (int p = 0; p < P; ++p)
-        CU_TRY(cudaMemcpy2D(tr->psi_ao + p, P * e, ket + (size_t)p * n, e, e, n, cudaMemcpyHostToDevice));
+        CU_TRY(cudaMemcpy2DAsync(tr->psi_ao + p, P * e, ket + (size_t)p * n, e, e, n, cudaMemcpyHostToDevice, st));
     if (bra) {
         for (int p = 0; p < P; ++p)
-            CU_TRY(cudaMemcpy2D(tr->bra_ao + p, P * e, bra + (size_t)p * n, e, e, n, cudaMemcpyHostToDevice));
+            CU_TRY(cudaMemcpy2DAsync(tr->bra_ao + p, P * e, bra + (size_t)p * n, e, e, n, cudaMemcpyHostToDevice, st));
     } else {
         // bra = S ket: the complex columns as a 2P x N real matrix times S (symmetric)
         CU_TRY(dgemm64(2 * P, n, n, 1.0, (const double *)tr->psi_ao, 2 * P, false, tr->S, tr->ld, false, 0.0,
@@ -3089,8 +3095,9 @@ int elhl_traj_create(const elhl_basis_desc *basis, const double *coords, const e
         if (!rc) rc = dev_alloc(&tr->psi_ao, (size_t)tr->ld * tr->P);
         if (!rc) rc = dev_alloc(&tr->bra_ao, (size_t)tr->ld * tr->P);
         if (!rc) rc = dev_alloc(&tr->target, (size_t)tr->P);
-        if (!rc && cudaMemset(tr->psi_ao, 0, (size_t)tr->ld * tr->P * sizeof(double2)) != cudaSuccess) rc = ELHL_ERR_CUDA;
-        if (!rc && cudaMemset(tr->bra_ao, 0, (size_t)tr->ld * tr->P * sizeof(double2)) != cudaSuccess) rc = ELHL_ERR_CUDA;
+        const size_t ao = (size_t)tr->ld * tr->P * sizeof(double2);
+        if (!rc && cudaMemsetAsync(tr->psi_ao, 0, ao, g_ctx.stream) != cudaSuccess) rc = ELHL_ERR_CUDA;
+        if (!rc && cudaMemsetAsync(tr->bra_ao, 0, ao, g_ctx.stream) != cudaSuccess) rc = ELHL_ERR_CUDA;
         const bool df = tr->cfg.precision == ELHL_PREC_DF64;  // DF64: implicit operator from the start
         if (!rc) rc = cheb_rebuild_operator(tr, df, df);
         ChebState &cs = tr->cs;
@@ -3270,9 +3277,9 @@ int elhl_traj_get_matrices(elhl_traj *tr, double *S, double *h, double *Hp) {
     std::lock_guard<std::mutex> lk(g_ctx.mu);
     CU_TRY(cudaStreamSynchronize(g_ctx.stream));
     const size_t col = tr->N * sizeof(double), ldb = tr->ld * sizeof(double);
-    if (S) CU_TRY(cudaMemcpy2D(S, col, tr->S, ldb, col, tr->N, cudaMemcpyDeviceToHost));
-    if (h) CU_TRY(cudaMemcpy2D(h, col, tr->h, ldb, col, tr->N, cudaMemcpyDeviceToHost));
-    if (Hp && tr->Hp) CU_TRY(cudaMemcpy2D(Hp, col, tr->Hp, ldb, col, tr->N, cudaMemcpyDeviceToHost));
+    if (S) CU_TRY(copy2d_d2h(S, col, tr->S, ldb, col, tr->N));
+    if (h) CU_TRY(copy2d_d2h(h, col, tr->h, ldb, col, tr->N));
+    if (Hp && tr->Hp) CU_TRY(copy2d_d2h(Hp, col, tr->Hp, ldb, col, tr->N));
     return ELHL_OK;
 }
 
@@ -3283,12 +3290,12 @@ int elhl_traj_get_factor(elhl_traj *tr, double *L, double *G) {
     CU_TRY(cudaStreamSynchronize(g_ctx.stream));
     const size_t col = tr->N * sizeof(double), ldb = tr->ld * sizeof(double);
     if (L) {
-        CU_TRY(cudaMemcpy2D(L, col, tr->fac.L, ldb, col, tr->N, cudaMemcpyDeviceToHost));
+        CU_TRY(copy2d_d2h(L, col, tr->fac.L, ldb, col, tr->N));
         for (int j = 1; j < tr->N; ++j)  // the explicit operator's factor keeps S above the diagonal
             std::memset(L + (size_t)j * tr->N, 0, j * sizeof(double));
     }
     if (G) {
-        CU_TRY(cudaMemcpy2D(G, col, traj_inverse(tr), ldb, col, tr->N, cudaMemcpyDeviceToHost));
+        CU_TRY(copy2d_d2h(G, col, traj_inverse(tr), ldb, col, tr->N));
         for (int j = 1; j < tr->N; ++j)  // zero above the diagonal, whatever the recursion left there
             std::memset(G + (size_t)j * tr->N, 0, j * sizeof(double));
     }
@@ -3359,8 +3366,8 @@ int traj_psi_host(elhl_traj *tr, std::vector<double2> &bra, std::vector<double2>
                                 reinterpret_cast<elhl_zcomplex *>(ket.data()));
     CU_TRY(cudaStreamSynchronize(g_ctx.stream));
     for (int p = 0; p < P; ++p) {
-        CU_TRY(cudaMemcpy(bra.data() + (size_t)p * N, tr->tb.bra(p), N * e, cudaMemcpyDeviceToHost));
-        CU_TRY(cudaMemcpy(ket.data() + (size_t)p * N, tr->tb.ket(p), N * e, cudaMemcpyDeviceToHost));
+        CU_TRY(copy_d2h(bra.data() + (size_t)p * N, tr->tb.bra(p), N * e));
+        CU_TRY(copy_d2h(ket.data() + (size_t)p * N, tr->tb.ket(p), N * e));
     }
     return ELHL_OK;
 }
@@ -3413,11 +3420,11 @@ int traj_snapshot_impl(elhl_traj *tr, const char *path) {
         ChebState &cs = tr->cs;
         rh.emin = cs.emin;
         rh.emax = cs.emax;
-        CU_TRY(cudaMemcpy(target.data(), tr->target, P * sizeof(double), cudaMemcpyDeviceToHost));
+        CU_TRY(copy_d2h(target.data(), tr->target, P * sizeof(double)));
         if (cs.cols_current) {  // fixed-nuclei steps continue from them (moving ones reload them from Psi)
             rh.has_cols = 1;
             cols.resize((size_t)N * cs.m);
-            CU_TRY(cudaMemcpy(cols.data(), cs.cin(), cols.size() * sizeof(double2), cudaMemcpyDeviceToHost));
+            CU_TRY(copy_d2h(cols.data(), cs.cin(), cols.size() * sizeof(double2)));
         }
     }
     // Net_Charge(atom) = sum_n sign_n |sum_{i in atom} DUAL_bra_i DUAL_ket_i|, sign -1 el / +1 hl
@@ -3512,13 +3519,15 @@ int traj_restore_impl(elhl_traj *tr, const char *path) {
     if (tr->cheb()) {
         ChebState &cs = tr->cs;
         for (int p = 0; p < P; ++p) {
-            CU_TRY(cudaMemcpy2D(tr->psi_ao + p, P * e, ket.data() + (size_t)p * N, e, e, N, cudaMemcpyHostToDevice));
-            CU_TRY(cudaMemcpy2D(tr->bra_ao + p, P * e, bra.data() + (size_t)p * N, e, e, N, cudaMemcpyHostToDevice));
+            CU_TRY(cudaMemcpy2DAsync(tr->psi_ao + p, P * e, ket.data() + (size_t)p * N, e, e, N, cudaMemcpyHostToDevice,
+                                     g_ctx.stream));
+            CU_TRY(cudaMemcpy2DAsync(tr->bra_ao + p, P * e, bra.data() + (size_t)p * N, e, e, N, cudaMemcpyHostToDevice,
+                                     g_ctx.stream));
         }
         if (res.empty()) {
             if (int rc = cheb_set_target(tr)) return rc;
         } else {
-            CU_TRY(cudaMemcpy(tr->target, target.data(), P * sizeof(double), cudaMemcpyHostToDevice));
+            CU_TRY(copy_h2d(tr->target, target.data(), P * sizeof(double)));
             cs.cols_current = false;
             if (!cs.implicit && (rh.emin != cs.emin || rh.emax != cs.emax)) {  // an interval widened by norm control
                 cs.emin = rh.emin;
@@ -3530,17 +3539,17 @@ int traj_restore_impl(elhl_traj *tr, const char *path) {
                 }
             }
             if (rh.has_cols) {
-                CU_TRY(cudaMemcpy(cs.cin(), res.data() + sizeof(rh) + P * sizeof(double), (size_t)N * cs.m * e,
-                                  cudaMemcpyHostToDevice));
+                CU_TRY(copy_h2d(cs.cin(), res.data() + sizeof(rh) + P * sizeof(double), (size_t)N * cs.m * e));
                 cs.cols_current = true;
             }
         }
     } else {
         for (int p = 0; p < P; ++p) {
-            CU_TRY(cudaMemcpy(tr->tb.bra(p), bra.data() + (size_t)p * N, N * e, cudaMemcpyHostToDevice));
-            CU_TRY(cudaMemcpy(tr->tb.ket(p), ket.data() + (size_t)p * N, N * e, cudaMemcpyHostToDevice));
+            CU_TRY(copy_h2d(tr->tb.bra(p), bra.data() + (size_t)p * N, N * e));
+            CU_TRY(copy_h2d(tr->tb.ket(p), ket.data() + (size_t)p * N, N * e));
         }
     }
+    CU_TRY(cudaStreamSynchronize(g_ctx.stream));  // the host columns have been read
     tr->t = t;
     tr->it = it;
     if (!res.empty()) {

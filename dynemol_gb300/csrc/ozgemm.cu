@@ -456,10 +456,10 @@ struct Lane {
 };
 Lane g_lane[2];
 
-cudaError_t ensure(Lane &ln, size_t sl_elems, size_t rows) {
+cudaError_t ensure(Lane &ln, size_t sl_elems, size_t rows, cudaStream_t st) {
     if (!ln.err) {
         cudaError_t e = cudaMalloc(&ln.err, sizeof(int));
-        if (e == cudaSuccess) e = cudaMemset(ln.err, 0, sizeof(int));
+        if (e == cudaSuccess) e = cudaMemsetAsync(ln.err, 0, sizeof(int), st);
         if (e != cudaSuccess) return e;
     }
     if (sl_elems > ln.sl_elems) {
@@ -509,7 +509,7 @@ cudaError_t ozgemm(int m, int n, int k, double alpha, const double *A, int lda, 
     // one set of slices and scales serves both operands
     const bool same = A == B && lda == ldb && va.kcontig == vb.kcontig && m == n && va.mask == vb.mask;
     const size_t sa = (size_t)kS * m * kp, sb = same ? 0 : (size_t)kS * n * kp;
-    if (cudaError_t e = ensure(ln, sa + sb, (size_t)m + n)) return e;
+    if (cudaError_t e = ensure(ln, sa + sb, (size_t)m + n, st)) return e;
     __nv_bfloat16 *slA = ln.sl, *slB = same ? ln.sl : ln.sl + sa;  // sa is a multiple of 8 elements: 16-byte aligned
     double *scB = same ? ln.sc : ln.sc + m;
     const int chunk = slice_chunk(kp), npiece = (kp + chunk - 1) / chunk;
