@@ -2107,7 +2107,6 @@ struct elhl_traj {
     ChebState cs;
     ChebPlan plan;
     double2 *psi_ao = nullptr, *bra_ao = nullptr;
-    double2 *psi_cols = nullptr;  // [2][P][N] their columns, for reading back (allocated on first use)
     double *target = nullptr;  // per-particle total population to hold (reduced precision)
     bool cheb() const { return cfg.method == ELHL_METHOD_CHEBYSHEV; }
 };
@@ -2753,24 +2752,24 @@ __global__ void __launch_bounds__(256) columns_kernel(const double2 *__restrict_
 }
 
 // Psi as host columns.  The AO arrays hold the particles side by side ([ld][P]); they
-// are transposed on the device and copied whole: a strided copy of 16-byte elements
-// per particle and state took 18 us each (64 columns: 2.3 ms).
+// are transposed on the device, into the column transforms' scratch (2 m ld doubles, m >= P:
+// no allocation, so that reading a state cannot fail for memory), and copied whole: a
+// strided copy of 16-byte elements per particle and state took 18 us each (64 columns:
+// 2.3 ms).
 int cheb_psi_columns(elhl_traj *tr, elhl_zcomplex *bra, elhl_zcomplex *ket) {
     cudaStream_t st = g_ctx.stream;
     const int P = tr->P, n = tr->N;
-    const size_t len = (size_t)n * P;
-    if (!tr->psi_cols)
-        if (int rc = dev_alloc(&tr->psi_cols, 2 * len)) return rc;
+    double2 *cols = reinterpret_cast<double2 *>(tr->cs.cscratch);
     const dim3 grid((n + 31) / 32, (P + 31) / 32);
-    if (ket) {
-        columns_kernel<<<grid, 256, 0, st>>>(tr->psi_ao, tr->psi_cols, n, P);
+    const struct {
+        const double2 *src;
+        elhl_zcomplex *dst;
+    } parts[] = {{tr->psi_ao, ket}, {tr->bra_ao, bra}};
+    for (const auto &p : parts) {
+        if (!p.dst) continue;
+        columns_kernel<<<grid, 256, 0, st>>>(p.src, cols, n, P);
         count_launch();
-        CU_TRY(cudaMemcpyAsync(ket, tr->psi_cols, len * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    }
-    if (bra) {
-        columns_kernel<<<grid, 256, 0, st>>>(tr->bra_ao, tr->psi_cols + len, n, P);
-        count_launch();
-        CU_TRY(cudaMemcpyAsync(bra, tr->psi_cols + len, len * sizeof(double2), cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(p.dst, cols, (size_t)n * P * sizeof(double2), cudaMemcpyDeviceToHost, st));
     }
     CU_TRY(cudaGetLastError());
     CU_TRY(cudaStreamSynchronize(st));
@@ -3154,7 +3153,7 @@ int elhl_traj_destroy(elhl_traj *tr) {
     tr->tb.release();
     tr->cs.release();
     tr->plan.release();
-    dev_free(tr->psi_ao); dev_free(tr->bra_ao); dev_free(tr->psi_cols); dev_free(tr->target);
+    dev_free(tr->psi_ao); dev_free(tr->bra_ao); dev_free(tr->target);
     delete tr;
     return ELHL_OK;
 }
