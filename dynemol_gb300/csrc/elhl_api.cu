@@ -3973,12 +3973,14 @@ int elhl_server_step(elhl_server *sv, int *n_active, int *n_pending) {
             const size_t np = (size_t)r->P * (r->nfrag + 1);
             if (!(drift[q] <= cheb_norm_tolerance(r->tr->cfg))) r->status = ELHL_ERR_NO_CONVERGENCE;
             if (r->done_steps >= r->nsteps || r->status) {
+                // a request whose results cannot be read still leaves, with that status: a
+                // return from here would leave those already in `finished` in `active` too
                 r->pops.resize(np);
-                const double *src = r->group < 0 ? r->tr->cs.gpops : sv->groups[r->group].pops + r->pops_off;
-                CU_TRY(copy_d2h(r->pops.data(), src, np * sizeof(double)));
                 r->psi.resize((size_t)r->nao * r->P);
-                if (int rc = cheb_psi_columns(r->tr, nullptr, reinterpret_cast<elhl_zcomplex *>(r->psi.data())))
-                    return rc;
+                const double *src = r->group < 0 ? r->tr->cs.gpops : sv->groups[r->group].pops + r->pops_off;
+                int rc = copy_d2h(r->pops.data(), src, np * sizeof(double)) == cudaSuccess ? ELHL_OK : ELHL_ERR_CUDA;
+                if (!rc) rc = cheb_psi_columns(r->tr, nullptr, reinterpret_cast<elhl_zcomplex *>(r->psi.data()));
+                if (rc) r->status = rc;
                 r->t_done = now_s();
                 sv->used -= r->bytes;
                 if (r->group >= 0) {
