@@ -3781,6 +3781,18 @@ static double request_bytes(const elhl_traj_config &cfg, int nao, int P) {
     return ld * nao * (5 * 8.0 + tsz + 2 * 8.0) + ld * cfg.ncols / cfg.nparticles * P * (3 * 2 * tsz + 2 * 16.0) +
            slices + 1e6;
 }
+// What its propagation holds besides: the exchange words of the shared-memory row kernel (a
+// request that runs alone), or the packed operands and partial products of the tensor-core
+// block product.  A request waits for these too, but one that exceeds the budget by them
+// alone is not refused: it is admitted when no other is active.
+static double request_exchange_bytes(const elhl_traj_config &cfg, int nao, int P) {
+    double b = 0.0;
+    if (cheb_rows_fit(cfg.precision, nao, P, g_ctx.sms)) b += 32.0 * (double)cheb_rows_words(cfg.precision, nao, P);
+    if (cfg.precision == ELHL_PREC_BF16X3 && P >= kGemmMinCols && nao >= kGemmMinN && umma_supported_n2(2 * P))
+        b += (double)umma_a_bytes(nao) + (double)umma_b_bytes(nao, 2 * P) +
+             8.0 * nao * P * umma_splits(nao, nao);
+    return b;
+}
 
 static int server_admit(elhl_server *sv, ServerRequest *r) {
     elhl_basis_desc d{};
@@ -3877,6 +3889,7 @@ static int server_submit(elhl_server *sv, const elhl_request *q, const char *res
         delete r;
         return ELHL_ERR_OOM;  // can never be admitted
     }
+    r->bytes += request_exchange_bytes(sv->cfg, b->nao, r->P);
     r->id = sv->next_id++;
     r->t_submit = now_s();
     sv->pending.push_back(r);
@@ -3887,7 +3900,8 @@ static int server_submit(elhl_server *sv, const elhl_request *q, const char *res
 int elhl_server_step(elhl_server *sv, int *n_active, int *n_pending) {
     if (!sv) return ELHL_ERR_BAD_ARG;
     // admission, FIFO, within the budget
-    while (!sv->pending.empty() && sv->used + sv->pending.front()->bytes <= sv->budget) {
+    while (!sv->pending.empty() &&
+           (sv->active.empty() || sv->used + sv->pending.front()->bytes <= sv->budget)) {
         ServerRequest *r = sv->pending.front();
         sv->pending.pop_front();
         r->t_admit = now_s();
