@@ -2227,10 +2227,15 @@ bool moving_explicit(const elhl_traj *tr) {
     }
 }
 
-// Cholesky factor, then the operator for the current S, h: explicit H~ (formed
-// once for fixed nuclei; for moving nuclei as moving_explicit says, unless the
-// caller asks for the factors) or implicit G h G^T; bounds and coefficients.
-int cheb_rebuild_operator(elhl_traj *tr, bool implicit = false, bool factors = false) {
+// What cheb_rebuild_operator forms: H~ once for fixed nuclei, or for moving nuclei (fewer
+// Lanczos steps) H~, its factors, or whichever of the two moving_explicit says.
+enum class Rebuild { kFixed, kMoving, kMovingExplicit, kMovingImplicit };
+
+// Cholesky factor, then the operator for the current S, h: explicit H~ or implicit
+// G h G^T; bounds and coefficients.
+int cheb_rebuild_operator(elhl_traj *tr, Rebuild what) {
+    const bool moving = what != Rebuild::kFixed;
+    const bool implicit = what == Rebuild::kMovingImplicit || (what == Rebuild::kMoving && !moving_explicit(tr));
     cudaStream_t st = g_ctx.stream;
     ChebState &cs = tr->cs;
     // S = L L^T and G = L^-1 in one recursion, in FP64 for every precision: on the
@@ -2238,7 +2243,7 @@ int cheb_rebuild_operator(elhl_traj *tr, bool implicit = false, bool factors = f
     // 320 or more rows exact on the tensor cores for the others (Factor::tc).
     // The implicit operator keeps G in cs.Ht, the explicit one in the factor's G.
     cs.moving = false;
-    if (implicit && !factors && moving_explicit(tr)) {
+    if (moving && !implicit) {
         if (int rc = tr->fac.factor(tr->S, tr->N)) return rc;
         CU_TRY(cudaEventRecord(g_ctx.ev[5], st));
         if (int rc = tr->fac.check_info(false)) return rc;
@@ -2415,7 +2420,7 @@ int cheb_step_impl(elhl_traj *tr, const double *coords, bool coords_on_device, i
     int rc = ELHL_OK;
     if (!coords && cs.implicit && cs.gemm) {
         // GEMM regime after moving steps: form H~ for the current geometry
-        if ((rc = cheb_rebuild_operator(tr, false))) return rc;
+        if ((rc = cheb_rebuild_operator(tr, Rebuild::kFixed))) return rc;
         if ((rc = cheb_prepare_readout(cs, tr->fac.L, traj_inverse(tr)))) return rc;
         if ((rc = cheb_plan(tr->plan, one))) return rc;
     }
@@ -2499,7 +2504,7 @@ int cheb_step_impl(elhl_traj *tr, const double *coords, bool coords_on_device, i
                 break;
             }
             if (cudaEventRecord(g_ctx.ev[4], st) != cudaSuccess) { rc = ELHL_ERR_CUDA; break; }
-            if ((rc = cheb_rebuild_operator(tr, true))) break;  // implicit: A, B follow the new L
+            if ((rc = cheb_rebuild_operator(tr, Rebuild::kMoving))) break;
             if ((rc = cheb_load_columns(tr))) break;
             if (cudaEventRecord(g_ctx.ev[3], st) != cudaSuccess) { rc = ELHL_ERR_CUDA; break; }
             if ((rc = cheb_plan_refresh(tr->plan, one))) break;
@@ -3098,7 +3103,7 @@ int elhl_traj_create(const elhl_basis_desc *basis, const double *coords, const e
         if (!rc && cudaMemsetAsync(tr->psi_ao, 0, ao, g_ctx.stream) != cudaSuccess) rc = ELHL_ERR_CUDA;
         if (!rc && cudaMemsetAsync(tr->bra_ao, 0, ao, g_ctx.stream) != cudaSuccess) rc = ELHL_ERR_CUDA;
         const bool df = tr->cfg.precision == ELHL_PREC_DF64;  // DF64: implicit operator from the start
-        if (!rc) rc = cheb_rebuild_operator(tr, df, df);
+        if (!rc) rc = cheb_rebuild_operator(tr, df ? Rebuild::kMovingImplicit : Rebuild::kFixed);
         ChebState &cs = tr->cs;
         cs.P = tr->P; cs.nfrag = tr->nfrag; cs.psi_out = tr->psi_ao; cs.bra_out = tr->bra_ao;
         cs.ao_frag = tr->basis.ao_frag; cs.target = tr->target;
@@ -3331,9 +3336,11 @@ constexpr char kResumeMagic[8] = {'E', 'L', 'H', 'L', 'R', 'S', 'M', '1'};
 
 struct ResumeHead {
     char magic[8];
-    int method, precision, N, P, ncols, first_call, has_cols, pad;
+    int method, precision, N, P, ncols, first_call, has_cols;
+    int form;  // Chebyshev operator: kFormExplicit, kFormImplicit; 0 in files that do not say
     double save_tau[2], emin, emax;
 };
+constexpr int kFormExplicit = 1, kFormImplicit = 2;
 
 bool put_record(FILE *f, const void *p, size_t n) {
     const uint32_t m = (uint32_t)n;
@@ -3419,6 +3426,7 @@ int traj_snapshot_impl(elhl_traj *tr, const char *path) {
         ChebState &cs = tr->cs;
         rh.emin = cs.emin;
         rh.emax = cs.emax;
+        rh.form = cs.implicit ? kFormImplicit : kFormExplicit;
         CU_TRY(copy_d2h(target.data(), tr->target, P * sizeof(double)));
         if (cs.cols_current) {  // fixed-nuclei steps continue from them (moving ones reload them from Psi)
             rh.has_cols = 1;
@@ -3528,14 +3536,24 @@ int traj_restore_impl(elhl_traj *tr, const char *path) {
         } else {
             CU_TRY(copy_h2d(tr->target, target.data(), P * sizeof(double)));
             cs.cols_current = false;
-            if (!cs.implicit && (rh.emin != cs.emin || rh.emax != cs.emax)) {  // an interval widened by norm control
+            // Fixed-nuclei steps go on with the operator in the form the steps before the
+            // snapshot left it in (moving steps and creation differ in that), on their
+            // interval.  In the GEMM regime fixed steps form H~ anew after implicit ones.
+            const bool implicit = rh.form ? rh.form == kFormImplicit : cs.implicit;
+            std::vector<ChebState *> one{&cs};
+            if (implicit != cs.implicit && !cs.gemm && tr->S) {
+                if (int rc = cheb_rebuild_operator(tr, implicit ? Rebuild::kMovingImplicit : Rebuild::kMovingExplicit)) return rc;
+                if (int rc = cheb_plan_refresh(tr->plan, one)) return rc;
+                cs.cols_current = false;
+            }
+            if (implicit == cs.implicit && (rh.emin != cs.emin || rh.emax != cs.emax)) {  // a widened interval, or a moving rebuild's
                 cs.emin = rh.emin;
                 cs.emax = rh.emax;
-                if (int rc = cheb_prepare(cs, tr->cfg.dt * tr->cfg.frame_step, tr->cfg.cheb_tol)) return rc;
-                if (!tr->plan.probs.empty()) {
-                    std::vector<ChebState *> one{&cs};
+                if (int rc = cheb_prepare(cs, tr->cfg.dt * tr->cfg.frame_step, tr->cfg.cheb_tol,
+                                          cs.implicit ? tr->h : nullptr))
+                    return rc;
+                if (!tr->plan.probs.empty())
                     if (int rc = cheb_plan_refresh(tr->plan, one)) return rc;
-                }
             }
             if (rh.has_cols) {
                 CU_TRY(copy_h2d(cs.cin(), res.data() + sizeof(rh) + P * sizeof(double), (size_t)N * cs.m * e));
