@@ -960,6 +960,7 @@ int cheb_prepare(ChebState &cs, double dt, double tol, const double *h = nullptr
     const double binv = 1.0 / cs.b;
     dim3 grid((cs.ld + 127) / 128, cs.N);
     const double *src = h ? h : cs.Ht;
+    if (!src) return ELHL_ERR_BAD_ARG;  // released by elhl_batch_compact: the interval cannot change any more
     const double a = h ? 0.0 : cs.a;
     if (cs.precision == ELHL_PREC_DF64) {
         split_df_kernel<<<grid, 128, 0, st>>>(src, (float2 *)cs.Hs, cs.N, cs.ld, a, binv, false);
