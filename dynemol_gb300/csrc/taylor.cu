@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
     const int r0 = min(N, blockIdx.x * rows), r1 = min(N, r0 + rows), nrow = r1 - r0;
     const int np = pad8(N);
     const int nf = L.nfrag < kMaxFrag ? L.nfrag : kMaxFrag;
-    const double tol2 = L.tol * L.tol;
+    const double tol2 = L.tol < 0.0 ? -1.0 : L.tol * L.tol;  // |delta| > tol < 0 always holds
     double *sv = dyn;                                    // resident: [P][np][4] ket re, im, bra re, im
     double *sh = dyn + (size_t)P * np * 4;               // resident: [rows][np][2] H'(i, j), H'(j, i)
     double *sy = kResident ? sh + (size_t)rows * np * 2 : dyn;  // [kWarps][P][rows][4] or [P][rows][4]
