@@ -132,7 +132,8 @@ struct Ctx {
     unsigned char *out;
     uint32_t tmem;
     int *abort_flag;
-    unsigned *last_flag;
+    int *go;  // the grid barrier's answer
+    __device__ bool grid_barrier_sub(unsigned *count, unsigned target, int *err, unsigned long long limit_ns) const;
 };
 
 __device__ __forceinline__ bool aborted(const Ctx &c) { return *(volatile int *)c.abort_flag != 0; }
@@ -146,25 +147,35 @@ __device__ __forceinline__ void set_abort(const Ctx &c, int *err) {
 // the launch) and waits, with acquire loads, until all nblocks CTAs have
 // arrived at this barrier (the count reaches `target` = nblocks x barriers so
 // far).  No reset and no generation word: the last arrival itself releases
-// the others.  Bounded: false (with ELHL_ERR_TIMEOUT) after limit_ns.
-__device__ __forceinline__ bool grid_barrier_sub(unsigned *count, unsigned target, int *err,
-                                                 unsigned long long limit_ns) {
+// the others.  Bounded: false (with ELHL_ERR_TIMEOUT) after limit_ns, and where this CTA
+// or another has given up.  Thread 64 looks once for all 192: threads that each read the
+// error word, which another CTA may set between their reads, could part here, and those
+// that went on would wait at the next barrier for those that left.
+__device__ __forceinline__ bool Ctx::grid_barrier_sub(unsigned *count, unsigned target, int *err,
+                                                      unsigned long long limit_ns) const {
     asm volatile("bar.sync 2, 192;" ::: "memory");
     if (threadIdx.x == 64) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
         const unsigned long long t0 = globaltimer_ns();
-        while (true) {
+        bool all = true;
+        while (all) {
             unsigned v;
+            int e;  // beside the count: no second trip to L2 after the wait
+            asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(e) : "l"(err) : "memory");
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            all = e == 0;
             if (v >= target) break;
-            if (globaltimer_ns() - t0 > limit_ns) {
+            if (all && globaltimer_ns() - t0 > limit_ns) {
                 atomicExch(err, ELHL_ERR_TIMEOUT);
-                break;
+                all = false;
             }
         }
+        all = all && !aborted(*this);
+        if (!all) atomicExch(abort_flag, 1);  // stops this CTA's producer and MMA issuer
+        *(volatile int *)go = all;
     }
     asm volatile("bar.sync 2, 192;" ::: "memory");
-    return *(volatile int *)err == 0;
+    return *(volatile int *)go != 0;
 }
 
 // ---- phase roles ----------------------------------------------------------------
@@ -654,7 +665,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     c.xe = reinterpret_cast<int *>(c.smem + SmemLayout::xe_off);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(c.smem + SmemLayout::misc_off);
     c.abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
-    c.last_flag = reinterpret_cast<unsigned *>(tmem_slot + 2);
+    c.go = reinterpret_cast<int *>(tmem_slot + 2);
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
     if (threadIdx.x == 0) {
         for (int s = 0; s < kAStages; ++s) {
@@ -693,7 +704,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // barrier.  So the next order's loads and MMAs overlap the barrier.  Warps
     // 2-7 meet every grid barrier on named barrier 2.
     bool ok = true;
-    if (warp >= 2) ok = grid_barrier_sub(L.bar_count, (unsigned)G, L.error, bar_ns);
+    if (warp >= 2) ok = c.grid_barrier_sub(L.bar_count, (unsigned)G, L.error, bar_ns);
     // the sliced vector v_k is in buffer k % 3
     for (int k = 1; ok && k <= L.K; ++k) {
         const int bin = (k + 2) % 3, bout = k % 3;
@@ -704,7 +715,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (warp == 1) {
             issue_mma(c, L, r, k & 1);
-            ok = !aborted(c) && *(volatile int *)L.error == 0;
+            // one answer for the warp: the next order's waits and its elected lane are the whole warp's
+            ok = __all_sync(0xffffffffu, !aborted(c) && *(volatile int *)L.error == 0);
             continue;
         }
         if (warp < 4) {
@@ -727,8 +739,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             io.emax_out = L.emax[bout];
             flush_and_epilogue(c, L, io, r, k & 1);
         }
-        ok = grid_barrier_sub(L.bar_count, (unsigned)G * (unsigned)(k + 1), L.error, bar_ns) && !aborted(c);
-        if (!ok && threadIdx.x == 64) atomicExch(c.abort_flag, 1);  // stops this CTA's producer and MMA issuer
+        ok = c.grid_barrier_sub(L.bar_count, (unsigned)G * (unsigned)(k + 1), L.error, bar_ns);
     }
     // drain: copies issued into the A ring and every MMA complete before the CTA
     // leaves and frees its TMEM (all consumed already unless a wait gave up)
