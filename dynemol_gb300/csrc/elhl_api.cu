@@ -2856,6 +2856,21 @@ int elhl_debug_barrier(double limit_s, int exit_cta) {
     return ELHL_OK;
 }
 
+int elhl_debug_reciprocal(const double *x, double *y, double *q, int n) {
+    if (!x || !y || !q || n <= 0) return ELHL_ERR_BAD_ARG;
+    std::lock_guard<std::mutex> lk(g_ctx.mu);
+    if (int rc = ensure_context_locked(-1)) return rc;
+    double *d = nullptr;
+    if (int rc = dev_alloc(&d, (size_t)3 * n)) return rc;
+    cudaError_t e = copy_h2d(d, x, n * sizeof(double));
+    if (e == cudaSuccess) e = launch_reciprocal(d, d + n, d + 2 * (size_t)n, n, g_ctx.stream);
+    if (e == cudaSuccess) e = copy_d2h(y, d + n, n * sizeof(double));
+    if (e == cudaSuccess) e = copy_d2h(q, d + 2 * (size_t)n, n * sizeof(double));
+    dev_free(d);
+    CU_TRY(e);
+    return ELHL_OK;
+}
+
 int elhl_set_stream(void *stream) {
     std::lock_guard<std::mutex> lk(g_ctx.mu);
     if (int rc = ensure_context_locked(-1)) return rc;

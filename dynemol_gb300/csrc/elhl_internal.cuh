@@ -275,6 +275,8 @@ size_t ozgemm_smem_bytes();
 // info[0] (if still 0) to row0 + column + 1, a wait that gave up info[1].
 int leaf_rows();
 cudaError_t leaf_chol_inv64(double *A, double *G, int nb, int ld, int row0, int *info, cudaStream_t st);
+// the pivots' reciprocal y of x, and CUDA's division q = 1 / x (for its test)
+cudaError_t launch_reciprocal(const double *x, double *y, double *q, int n, cudaStream_t st);
 
 // Lanczos recursion of k steps for the spectral bounds, FP64, one cooperative
 // launch (lanczos.cu): explicit H (G == nullptr; both triangles stored) or

@@ -50,8 +50,14 @@ __device__ __forceinline__ void tri_elem(int e, int &i, int &j) {
     j = e - i * (i + 1) / 2;
 }
 
-// 1 / d for a normal d > 0: third-order Householder iteration y (1 + e + e^2), e = 1 - d y,
-// on the hardware's approximation (20 bits: error e^3 below 2^-57 before rounding)
+// 1 / d by one step of Householder's third-order iteration for the root of 1 / y - d (A. S.
+// Householder, The Numerical Treatment of a Single Nonlinear Equation, 1970; the geometric
+// series of 1 / (1 - e)): y (1 + e + e^2), e = 1 - d y.  The start is rcp.approx.ftz.f64,
+// whose result has 20 fraction bits: e is below 2^-19, so 1 - d y is exact in an FMA, the
+// terms left out are below 2^-57, and the result is within 0.63 ulp of 1 / d (tested against
+// exact quotients and against CUDA's division).  d and the start have to be normal; outside
+// 2^-999 .. 2^998, well inside the normal range on either side, and for zero, infinities
+// and NaN, the division.
 __device__ __forceinline__ double reciprocal(double d) {
     const int ex = (__double2hiint(d) >> 20) & 0x7ff;
     if (ex < 24 || ex > 2020) return 1.0 / d;
@@ -364,9 +370,23 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads)
     cluster_barrier();  // no CTA leaves while its shared memory may still be written
 }
 
+__global__ void reciprocal_kernel(const double *x, double *y, double *q, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    y[i] = reciprocal(x[i]);
+    q[i] = 1.0 / x[i];
+}
+
 }  // namespace
 
 int leaf_rows() { return kLeafRows; }
+
+cudaError_t launch_reciprocal(const double *x, double *y, double *q, int n, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    reciprocal_kernel<<<(n + 255) / 256, 256, 0, st>>>(x, y, q, n);
+    count_launch();
+    return cudaGetLastError();
+}
 
 cudaError_t leaf_chol_inv64(double *A, double *G, int nb, int ld, int row0, int *info, cudaStream_t st) {
     static bool attr = false;

@@ -382,6 +382,10 @@ int elhl_set_stream(void *stream);
  * is bounded. */
 int elhl_debug_barrier(double limit_s, int exit_cta);
 
+/* Test hook of the factorisation's arithmetic: y[i] = the reciprocal its pivots take of
+ * x[i], q[i] = 1 / x[i] by CUDA's division (host arrays of n). */
+int elhl_debug_reciprocal(const double *x, double *y, double *q, int n);
+
 /* Kernels of this library launched so far in this process (each kernel node
  * of a replayed step graph counted; library calls such as cuBLAS not
  * counted): benchmarks read it before and after a timed region. */
