@@ -33,7 +33,7 @@ EXPORTED_SYMBOLS = (
     "propagationelhl_gpucaller_", "elhl_last_status", "elhl_status_string", "elhl_traj_config_default",
     "elhl_traj_create", "elhl_traj_destroy", "elhl_traj_init_fmo", "elhl_traj_init_fmo_states", "elhl_traj_set_psi", "elhl_traj_get_psi", "elhl_traj_step",
     "elhl_traj_step_device", "elhl_traj_energies", "elhl_traj_get_matrices", "elhl_traj_get_factor", "elhl_traj_get_stats", "elhl_traj_snapshot", "elhl_traj_restore", "elhl_device_count",
-    "elhl_sm_count", "elhl_set_stream", "elhl_debug_barrier", "elhl_debug_reciprocal", "elhl_kernel_launches", "elhl_propagate_fixed_scratch", "elhl_bessel_j",
+    "elhl_sm_count", "elhl_set_stream", "elhl_debug_barrier", "elhl_debug_stall", "elhl_debug_reciprocal", "elhl_kernel_launches", "elhl_propagate_fixed_scratch", "elhl_bessel_j",
     "elhl_chebyshev_coefficients", "elhl_batch_create", "elhl_batch_size", "elhl_batch_member",
     "elhl_batch_compact", "elhl_batch_step", "elhl_batch_get_stats", "elhl_batch_destroy",
     "elhl_server_create", "elhl_server_submit", "elhl_server_step", "elhl_server_poll", "elhl_server_result",
@@ -132,6 +132,7 @@ def load(path: str = LIB_PATH):
     L.elhl_sm_count.restype = ci
     L.elhl_set_stream.argtypes = [vp]
     L.elhl_debug_barrier.argtypes = [ctypes.c_double, ci]
+    L.elhl_debug_stall.argtypes = [ci]
     L.elhl_debug_reciprocal.argtypes = [vp, vp, vp, ci]
     L.elhl_kernel_launches.argtypes = []
     L.elhl_kernel_launches.restype = ctypes.c_longlong
@@ -446,9 +447,15 @@ def set_stream(stream_handle: int | None):
 
 
 def debug_barrier(limit_s: float = 0.0, exit_cta: int = -1):
-    """Failure-detection test hook: grid-barrier limit (s, <= 0: default) and a
+    """Failure-detection test hook: limit of the kernels' waits (s, <= 0: default) and a
     CTA of the next propagation launch that leaves before its first barrier."""
     _check(load().elhl_debug_barrier(float(limit_s), int(exit_cta)), "elhl_debug_barrier")
+
+
+def debug_stall(where: int):
+    """Failure-detection test hook: 1 a CTA of the next Lanczos launch leaves, 2 the factor's CTA
+    of the next leaf raises no flag, 3 a CTA of the next OZ64 propagation withholds partial sums."""
+    _check(load().elhl_debug_stall(int(where)), "elhl_debug_stall")
 
 
 def debug_reciprocal(x: np.ndarray):

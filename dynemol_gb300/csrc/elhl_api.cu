@@ -258,6 +258,19 @@ bool chol_inv_fits(int n, int ld, size_t wcap) {
     return (size_t)ld * n1 <= wcap && chol_inv_fits(n1, ld, wcap) && chol_inv_fits(n2, ld, wcap - (size_t)ld * n1);
 }
 
+// Failure-detection test hooks (elhl_debug_barrier, elhl_debug_stall): the limit of the
+// kernels' waits, a one-shot early exit of one CTA of a propagation launch, and a one-shot
+// stall elsewhere.
+unsigned long long g_dbg_barrier_ns = 0;
+int g_dbg_exit_cta1 = 0;
+enum Stall { kStallNone = 0, kStallBounds = 1, kStallLeaf = 2, kStallPartials = 3 };
+int g_dbg_stall = kStallNone;
+bool take_stall(Stall s) {
+    if (g_dbg_stall != s) return false;
+    g_dbg_stall = kStallNone;
+    return true;
+}
+
 // An FP64 product of the factorisations: on the tensor cores from exact slices
 // (ozgemm) when tc is set and the product is large enough to fill the GPU, else
 // on the FP64 pipe (dgemm64; dgemm_small for the smallest blocks).
@@ -280,24 +293,21 @@ cudaError_t fgemm(bool tc, int m, int n, int k, double alpha, const double *A, i
 
 // ELHL_ERR_TIMEOUT if a tensor-core product gave up a wait since the last check (then cleared)
 int ozgemm_status() {
-    for (int lane = 0; lane < 2; ++lane) {
-        int *e = ozgemm_error(lane);
-        if (!e) continue;
-        int h = 0;
-        CU_TRY(copy_d2h(&h, e, sizeof(int)));
-        if (h) {
-            CU_TRY(cudaMemsetAsync(e, 0, sizeof(int), g_ctx.stream));
-            return h;
-        }
-    }
-    return ELHL_OK;
+    int h[2] = {0, 0};
+    for (int lane = 0; lane < 2; ++lane)
+        if (const int *e = ozgemm_error(lane))
+            CU_TRY(cudaMemcpyAsync(&h[lane], e, sizeof(int), cudaMemcpyDeviceToHost, g_ctx.stream));
+    CU_TRY(cudaStreamSynchronize(g_ctx.stream));
+    for (int lane = 0; lane < 2; ++lane)
+        if (h[lane]) CU_TRY(cudaMemsetAsync(ozgemm_error(lane), 0, sizeof(int), g_ctx.stream));
+    return h[0] ? h[0] : h[1];
 }
 
 int chol_inv64(double *A, double *G, int n, int ld, int row0, double *W, int *info, bool tc = false) {
     cudaStream_t st = g_ctx.stream;
     const int leaf = leaf_rows();
     if (n <= leaf) {
-        CU_TRY(leaf_chol_inv64(A, G, n, ld, row0, info, st));
+        CU_TRY(leaf_chol_inv64(A, G, n, ld, row0, info, st, g_dbg_barrier_ns, take_stall(kStallLeaf)));
         return ELHL_OK;
     }
     const int n1 = round_up(n / 2, leaf), n2 = n - n1;
@@ -464,6 +474,9 @@ int run_taylor(const double *Hp, int N, int ld, TaylorBuffers &tb, int P, const 
     L.bar_count = g_ctx.bar;
     L.error = g_ctx.err;
     L.words = tb.words;
+    L.barrier_ns = g_dbg_barrier_ns;
+    L.exit_cta1 = g_dbg_exit_cta1;
+    g_dbg_exit_cta1 = 0;  // one launch only
     CU_TRY(cudaEventRecord(g_ctx.ev[0], st));
     CU_TRY(launch_taylor(L, g_ctx.grid, kTaylorBlock, st));
     CU_TRY(cudaEventRecord(g_ctx.ev[1], st));
@@ -930,7 +943,7 @@ int lanczos_bounds(ChebState &cs, int ksteps, const double *h = nullptr, const d
     CU_TRY(cudaMemsetAsync(rec, 0, (2 * k + 1) * sizeof(double), st));
     CU_TRY(cudaMemsetAsync(g_ctx.err, 0, sizeof(int), st));
     CU_TRY(launch_lanczos64(n, ld, k, h ? h : cs.Ht, h ? cs.Ht : nullptr, Gt, cs.lz, cs.lz + 4 * ld, part, kLzPart,
-                            rec, g_ctx.bar, g_ctx.err, st));
+                            rec, g_ctx.bar, g_ctx.err, st, g_dbg_barrier_ns, take_stall(kStallBounds) ? 1 : 0));
     int err = 0;
     CU_TRY(copy_d2h(&err, g_ctx.err, sizeof(int)));
     if (err) return err;
@@ -1665,11 +1678,6 @@ int tune_plan(ChebPlan &pl) {
     return ELHL_OK;
 }
 
-// Failure-detection test hook (elhl_debug_barrier): the grid-barrier limit of
-// the propagation launches and a one-shot early exit of one CTA.
-unsigned long long g_dbg_barrier_ns = 0;
-int g_dbg_exit_cta1 = 0;
-
 // The propagation launch of an ELHL_PREC_OZ64 plan (one problem, m <= 4, explicit Hs).
 int oz_run(ChebPlan &pl) {
     cudaStream_t st = g_ctx.stream;
@@ -1699,6 +1707,7 @@ int oz_run(ChebPlan &pl) {
     L.barrier_ns = g_dbg_barrier_ns;
     L.exit_cta1 = g_dbg_exit_cta1;
     g_dbg_exit_cta1 = 0;  // one launch only
+    L.mute_cta1 = take_stall(kStallPartials) ? oz.grid : 0;  // the last CTA always has a segment
     CU_TRY(cudaMemsetAsync(g_ctx.bar, 0, 2 * sizeof(unsigned), st));
     CU_TRY(cudaMemsetAsync(oz.part, 0, oz.parts * oz_tile_rows() * 16 * sizeof(double), st));  // tags
     CU_TRY(cudaMemsetAsync(oz.xe + (size_t)3 * 2 * oz.ntiles * 8, 0x80, 3 * 8 * sizeof(int), st));  // column maxima
@@ -2853,6 +2862,13 @@ int elhl_debug_barrier(double limit_s, int exit_cta) {
     if (limit_s > 10.0 || exit_cta < -1 || exit_cta >= 1 << 20) return ELHL_ERR_BAD_ARG;
     g_dbg_barrier_ns = limit_s > 0.0 ? (unsigned long long)(limit_s * 1e9) : 0ULL;
     g_dbg_exit_cta1 = exit_cta + 1;
+    return ELHL_OK;
+}
+
+int elhl_debug_stall(int where) {
+    std::lock_guard<std::mutex> lk(g_ctx.mu);
+    if (where < kStallNone || where > kStallPartials) return ELHL_ERR_BAD_ARG;
+    g_dbg_stall = where;
     return ELHL_OK;
 }
 

@@ -70,6 +70,7 @@ struct TaylorLaunch {
     TaylorParticle *part; // [nparticles]
     double t_init, t_max;
     double tol, norm_tol;
+    double tol2;          // what |delta|^2 is compared with (set by launch_taylor)
     int max_conv_calls;
     // multi-step mode (fixed nuclei): nsteps > 1 runs the step driver on the device
     int nsteps;
@@ -86,6 +87,8 @@ struct TaylorLaunch {
     unsigned *bar_count;  // grid barrier: two words, one 64-bit count (8-byte aligned, zero at the launch)
     int *error;           // global error flag
     ulonglong2 *words;    // taylor_words(N, grid) words exchanged in place of the barrier, or nullptr
+    unsigned long long barrier_ns;  // limit of the grid barrier (0: default)
+    int exit_cta1;        // test hook: 1 + the CTA that leaves after the first round (0: none)
 };
 constexpr int kSlots = 6;
 size_t taylor_words(int N, int grid);
@@ -231,8 +234,9 @@ struct OzLaunch {
     double *part;                // partial tiles [slot][8][128] as 128-bit integers (16 bytes each)
     unsigned *bar_count;         // grid-barrier arrivals, over all orders of the launch (0 at the launch)
     int *error;
-    unsigned long long barrier_ns;  // grid-barrier limit (0: default)
+    unsigned long long barrier_ns;  // limit of the grid barrier and of the partials (0: defaults)
     int exit_cta1;                  // test hook: 1 + the CTA that leaves before its first barrier
+    int mute_cta1;                  // test hook: 1 + the CTA that withholds its partials of order 2
 };
 int oz_slices();
 int oz_tile_rows();
@@ -272,9 +276,11 @@ size_t ozgemm_smem_bytes();
 // Diagonal-block leaves of the recursive factorisation (factor.cu), in shared
 // memory, blocks of leaf_rows() = 64 rows: leaf_chol_inv64: A (nb x nb,
 // nb <= 64) <- chol(A), G <- its inverse, in FP64; a non-positive pivot sets
-// info[0] (if still 0) to row0 + column + 1, a wait that gave up info[1].
+// info[0] (if still 0) to row0 + column + 1, a wait that gave up info[1].  wait_ns: limit of
+// the waits (0: default); mute: test hook, the factor's CTA raises no flag.
 int leaf_rows();
-cudaError_t leaf_chol_inv64(double *A, double *G, int nb, int ld, int row0, int *info, cudaStream_t st);
+cudaError_t leaf_chol_inv64(double *A, double *G, int nb, int ld, int row0, int *info, cudaStream_t st,
+                            unsigned long long wait_ns = 0, bool mute = false);
 // the pivots' reciprocal y of x, and CUDA's division q = 1 / x (for its test)
 cudaError_t launch_reciprocal(const double *x, double *y, double *q, int n, cudaStream_t st);
 
@@ -286,7 +292,8 @@ cudaError_t launch_reciprocal(const double *x, double *y, double *q, int n, cuda
 // barrier that gave up.
 cudaError_t launch_lanczos64(int n, int ld, int k, const double *H, const double *G, const double *Gt, double *r,
                              double *t, double *part, int part_cap, double *rec, unsigned *bar, int *err,
-                             cudaStream_t st);
+                             cudaStream_t st,
+                             unsigned long long wait_ns = 0, int exit_cta1 = 0);
 
 int bessel_j_sequence(double beta, int kmax, double *J);
 int chebyshev_coefficients(double dt, double emin, double emax, double tol, int kcap, std::vector<double> &cre,

@@ -93,7 +93,7 @@ __device__ __forceinline__ void raise_flag(int *flag) {
         asm volatile("st.release.cluster.shared::cluster.u32 [%0], %1;" ::"r"(remote(flag, lane)), "r"(1) : "memory");
 }
 // one thread: bounded wait for a flag of this CTA
-__device__ __forceinline__ bool wait_flag(const int *flag) {
+__device__ __forceinline__ bool wait_flag(const int *flag, unsigned long long limit_ns) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(flag);
     unsigned long long t0 = 0;
     for (unsigned n = 1;; ++n) {
@@ -103,7 +103,7 @@ __device__ __forceinline__ bool wait_flag(const int *flag) {
         if ((n & 63u) == 0) {
             const unsigned long long t = globaltimer_ns();
             if (!t0) t0 = t;
-            if (t - t0 > kWaitNs) return false;
+            if (t - t0 > limit_ns) return false;
         }
     }
 }
@@ -201,7 +201,7 @@ __device__ __forceinline__ void factor_block(Smem &s, int b, int nb, int row0, c
 }
 
 // CTA 0: the factor
-__device__ void factor_cta(Smem &s, double *A, int nb, int ld, int row0, int *info) {
+__device__ void factor_cta(Smem &s, double *A, int nb, int ld, int row0, int *info, bool mute) {
     const int tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
     const int blocks = (nb + kB - 1) / kB, end = blocks * kB;  // rows in use (padded to whole blocks)
     Step step[kB - 1], more[kTwice];
@@ -238,12 +238,12 @@ __device__ void factor_cta(Smem &s, double *A, int nb, int ld, int row0, int *in
             // the inverse of the diagonal block, then the panel, to the CTAs 1 .. 3
             for (int c = 1; c < kCluster; ++c)
                 store_remote(remote(&s.Gd[b][2 * lane], c), s.Gd[b][2 * lane], s.Gd[b][2 * lane + 1]);
-            raise_flag(&s.flag_g[b]);
+            if (!mute) raise_flag(&s.flag_g[b]);
             for (int q = lane; q < (end - r0) * (kB / 2); q += 32) {
                 const double *v = s.A + (r0 + q / (kB / 2)) * kPitch + b0 + 2 * (q % (kB / 2));
                 for (int c = 1; c < kCluster; ++c) store_remote(remote(v, c), v[0], v[1]);
             }
-            if (!last) raise_flag(&s.flag_p[b]);
+            if (!last && !mute) raise_flag(&s.flag_p[b]);
         }
         if (last) break;
         if (warp == 0) {
@@ -289,7 +289,8 @@ __device__ void factor_cta(Smem &s, double *A, int nb, int ld, int row0, int *in
 }
 
 // CTAs 1 .. 3: the columns of G of their column blocks
-__device__ void inverse_cta(Smem &s, unsigned rank, double *G, int nb, int ld, int *info) {
+__device__ void inverse_cta(Smem &s, unsigned rank, double *G, int nb, int ld, int *info,
+                            unsigned long long limit_ns) {
     const int tid = threadIdx.x;
     const int blocks = (nb + kB - 1) / kB, end = blocks * kB;
     int own[kOwn];
@@ -304,7 +305,7 @@ __device__ void inverse_cta(Smem &s, unsigned rank, double *G, int nb, int ld, i
     __syncthreads();
     for (int b = 0; b < blocks; ++b) {
         const int b0 = b * kB, r0 = b0 + kB;
-        if (tid == 0) s.ok = wait_flag(&s.flag_g[b]);
+        if (tid == 0) s.ok = wait_flag(&s.flag_g[b], limit_ns);
         __syncthreads();
         if (!s.ok) break;
         // row block b of G: -Gd W for the column blocks before b, Gd for b itself
@@ -322,7 +323,7 @@ __device__ void inverse_cta(Smem &s, unsigned rank, double *G, int nb, int ld, i
             if (b0 + i < nb && j < nb) G[(size_t)j * ld + b0 + i] = v;
         }
         if (b + 1 == blocks) break;
-        if (tid == 0) s.ok = wait_flag(&s.flag_p[b]);
+        if (tid == 0) s.ok = wait_flag(&s.flag_p[b], limit_ns);
         __syncthreads();
         if (!s.ok) break;
         for (int e = tid; e < (end - r0) * kOwn * kB; e += kThreads) {  // W += L_b G_b, lanes along the rows
@@ -339,7 +340,8 @@ __device__ void inverse_cta(Smem &s, unsigned rank, double *G, int nb, int ld, i
 }
 
 __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads)
-    leaf_chol_inv64_kernel(double *A, double *G, int nb, int ld, int row0, int *info) {
+    leaf_chol_inv64_kernel(double *A, double *G, int nb, int ld, int row0, int *info, unsigned long long wait_ns,
+                           bool mute) {
     extern __shared__ __align__(16) unsigned char raw[];
     Smem &s = *reinterpret_cast<Smem *>(raw);
     const unsigned rank = cluster_rank();
@@ -365,8 +367,8 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads)
         }
     }
     cluster_barrier();  // flags and A in place
-    if (rank == 0) factor_cta(s, A, nb, ld, row0, info);
-    else inverse_cta(s, rank, G, nb, ld, info);
+    if (rank == 0) factor_cta(s, A, nb, ld, row0, info, mute);
+    else inverse_cta(s, rank, G, nb, ld, info, wait_ns ? wait_ns : kWaitNs);
     cluster_barrier();  // no CTA leaves while its shared memory may still be written
 }
 
@@ -388,7 +390,8 @@ cudaError_t launch_reciprocal(const double *x, double *y, double *q, int n, cuda
     return cudaGetLastError();
 }
 
-cudaError_t leaf_chol_inv64(double *A, double *G, int nb, int ld, int row0, int *info, cudaStream_t st) {
+cudaError_t leaf_chol_inv64(double *A, double *G, int nb, int ld, int row0, int *info, cudaStream_t st,
+                            unsigned long long wait_ns, bool mute) {
     static bool attr = false;
     if (!attr) {
         cudaError_t e = cudaFuncSetAttribute(leaf_chol_inv64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -397,7 +400,7 @@ cudaError_t leaf_chol_inv64(double *A, double *G, int nb, int ld, int row0, int 
         attr = true;
     }
     if (nb <= 0 || nb > kLeafRows) return cudaErrorInvalidValue;
-    leaf_chol_inv64_kernel<<<kCluster, kThreads, sizeof(Smem), st>>>(A, G, nb, ld, row0, info);
+    leaf_chol_inv64_kernel<<<kCluster, kThreads, sizeof(Smem), st>>>(A, G, nb, ld, row0, info, wait_ns, mute);
     count_launch();
     return cudaGetLastError();
 }

@@ -221,12 +221,15 @@ struct LrArgs {
     unsigned long long tag0;  // a value no earlier launch used, its low 32 bits zero
     double *rec;              // alpha [k], beta [k], steps used [1]
     int *err;
+    unsigned long long limit;  // of the waits
+    int exit_cta1;             // test hook: 1 + the CTA that leaves at once (0: none)
 };
 
 __global__ void __launch_bounds__(kLrThreads, 1) lanczos_rows_kernel(const LrArgs a) {
     extern __shared__ double dyn[];
     __shared__ double s_red[2][kLrWarps], s_sc[4];
     __shared__ int s_abort;
+    if ((int)blockIdx.x + 1 == a.exit_cta1) return;  // test hook: the other CTAs' waits run out
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int n = a.n, rows = (n + gridDim.x - 1) / gridDim.x;
     const int r0 = min(n, (int)blockIdx.x * rows), nrow = min(n, r0 + rows) - r0;
@@ -272,7 +275,7 @@ __global__ void __launch_bounds__(kLrThreads, 1) lanczos_rows_kernel(const LrArg
                 w[u] = make_ulonglong2(0ull, tag);
                 if (i < n) w[u] = fetch(x + i);
             }
-            if (!await_words(w, tag, x + i0 + lane, kLrThreads, a.err, kBarrierNs)) s_abort = 1;
+            if (!await_words(w, tag, x + i0 + lane, kLrThreads, a.err, a.limit)) s_abort = 1;
 #pragma unroll
             for (int u = 0; u < kLrBatch; ++u) {
                 const int i = i0 + u * kLrThreads + lane;
@@ -355,13 +358,14 @@ __global__ void __launch_bounds__(kLrThreads, 1) lanczos_rows_kernel(const LrArg
 size_t rows_smem(int n, int sms) { return (size_t)(2 + (n + sms - 1) / sms) * n * sizeof(double); }
 
 cudaError_t launch_rows(int n, int ld, int k, const double *H, double *x, double *rec, int *err, int sms,
-                        cudaStream_t st) {
+                        cudaStream_t st, unsigned long long wait_ns, int exit_cta1) {
     static unsigned long long launches = 0;  // under the library's lock
     const int rows = (n + sms - 1) / sms, grid = (n + rows - 1) / rows;
     const size_t smem = rows_smem(n, sms);
     cudaError_t e = cudaFuncSetAttribute(lanczos_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    LrArgs a{n, ld, k, H, reinterpret_cast<ulonglong2 *>(x), ++launches << 32, rec, err};
+    LrArgs a{n, ld, k, H, reinterpret_cast<ulonglong2 *>(x), ++launches << 32, rec, err, wait_ns ? wait_ns : kBarrierNs,
+             std::min(exit_cta1, grid)};
     void *args[] = {&a};
     e = cudaLaunchCooperativeKernel((const void *)lanczos_rows_kernel, dim3(grid), dim3(kLrThreads), args, smem, st);
     count_launch();
@@ -372,7 +376,8 @@ cudaError_t launch_rows(int n, int ld, int k, const double *H, double *x, double
 
 cudaError_t launch_lanczos64(int n, int ld, int k, const double *H, const double *G, const double *Gt, double *r,
                              double *t, double *part, int part_cap, double *rec, unsigned *bar, int *err,
-                             cudaStream_t st) {
+                             cudaStream_t st,
+                             unsigned long long wait_ns, int exit_cta1) {
     static int grid = 0;
     if (!grid) {  // one CTA per SM, co-resident at the largest shared-memory size
         const int smem_max = (int)((kXsCap + kRedSlots) * sizeof(double));
@@ -390,7 +395,7 @@ cudaError_t launch_lanczos64(int n, int ld, int k, const double *H, const double
     // a step at N = 3720 takes 57 us against lanczos64_kernel's 43): the words' [2][n] x 16
     // bytes lie in r's 4 x ld doubles
     if (!G && n >= 1 && k >= 1 && rows_smem(n, grid) <= kLrSmem)
-        return launch_rows(n, ld, k, H, r, rec, err, grid, st);
+        return launch_rows(n, ld, k, H, r, rec, err, grid, st, wait_ns, exit_cta1);
     const size_t smem = (size_t)(std::min(n, kXsCap) + kRedSlots) * sizeof(double);
     if (grid > part_cap || k < 1 || n < 1 || (G && !Gt)) return cudaErrorInvalidValue;
     LzArgs a{n, ld, k, H, G, Gt, r, t, part, rec, bar, err};

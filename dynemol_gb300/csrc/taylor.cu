@@ -251,7 +251,6 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
     const int r0 = min(N, blockIdx.x * rows), r1 = min(N, r0 + rows), nrow = r1 - r0;
     const int np = pad8(N);
     const int nf = L.nfrag < kMaxFrag ? L.nfrag : kMaxFrag;
-    const double tol2 = L.tol < 0.0 ? -1.0 : L.tol * L.tol;  // |delta| > tol < 0 always holds
     double *sv = dyn;                                    // resident: [P][np][4] ket re, im, bra re, im
     double *sh = dyn + (size_t)P * np * 4;               // resident: [rows][np][2] H'(i, j), H'(j, i)
     double *sy = kResident ? sh + (size_t)rows * np * 2 : dyn;  // [kWarps][P][rows][4] or [P][rows][4]
@@ -261,7 +260,7 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
     };
 
     if (tid == 0) {
-        s_abort = 0;
+        s_abort = (int)blockIdx.x + 1 == L.exit_cta1;  // test hook: it leaves after the first round, the others' waits run out
         s_step = 0;
         s_it = L.it0;
         s_tinit = L.t_init;
@@ -415,6 +414,8 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
         }
     };
 
+    // (The words' waits take kBarrierNs, the barrier's L.barrier_ns: a limit that is no
+    // constant costs the words' rounds 0.5 %.)
     // Exchange without the barrier (resident, L.words): the round's next source and its
     // records go out as words tagged with the round, which the readers poll.  Two buffers
     // suffice: a CTA publishes round r + 2 once it has every CTA's words of round r + 1,
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
     // wait for the round's arrivals; false: the launch ends with an error
     auto wait_round = [&]() -> bool {
         arrivals += G;
-        if (tid == 0) s_ok = grid_poll(L.bar_count, arrivals, L.error);
+        if (tid == 0) s_ok = grid_poll(L.bar_count, arrivals, L.error, L.barrier_ns);
         __syncthreads();
         return s_ok;
     };
@@ -687,7 +688,7 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
                 v[3] = __shfl_sync(0xffffffffu, d, 16);
             }
             int need = 0;
-            if (lane == 0) need = advance(c, v, tol2, L.norm_tol, L.max_conv_calls, s_tinit, s_tmax);
+            if (lane == 0) need = advance(c, v, L.tol2, L.norm_tol, L.max_conv_calls, s_tinit, s_tmax);
             need = __shfl_sync(0xffffffffu, need, 0);
             if (need) set_coefficients(c, need, lane);
         }
@@ -806,6 +807,9 @@ cudaError_t launch_taylor_t(const TaylorLaunch &L, int grid, int block, size_t s
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     TaylorLaunch copy = L;
+    if (copy.exit_cta1 > grid) copy.exit_cta1 = grid;
+    if (!copy.barrier_ns) copy.barrier_ns = kBarrierNs;
+    copy.tol2 = L.tol < 0.0 ? -1.0 : L.tol * L.tol;  // |delta| > tol < 0 always holds
     if (kResident && L.words) {  // no word carries a round's tag before the launch
         e = cudaMemsetAsync(L.words, 0, taylor_words(L.N, grid) * sizeof(ulonglong2), st);
         if (e != cudaSuccess) return e;

@@ -374,13 +374,20 @@ int elhl_server_destroy(elhl_server *sv);
 int elhl_set_stream(void *stream);
 
 /* Test hook for failure detection (no counterpart in the reference): the
- * grid-barrier wait limit of the Chebyshev propagation launches (limit_s <= 0
- * restores the default 5 s; at most 10 s) and, when exit_cta >= 0, one CTA of
- * the next propagation launch that leaves before its first grid barrier, so
- * that the other CTAs' waits run out and the call returns ELHL_ERR_TIMEOUT
+ * limit of the waits of the propagation, bounds and leaf kernels (limit_s <= 0
+ * restores the defaults, 5 s and 2 s; at most 10 s; the tagged words of the Taylor kernel
+ * keep theirs of 5 s) and, when exit_cta >= 0, one CTA of
+ * the next propagation launch that leaves before its first grid barrier (Taylor: after its
+ * first round), so that the other CTAs' waits run out and the call returns ELHL_ERR_TIMEOUT
  * with the device context intact.  No fault or hang is involved: every wait
  * is bounded. */
 int elhl_debug_barrier(double limit_s, int exit_cta);
+
+/* The same for waits that no early exit reaches; where = 1: a CTA of the next Lanczos launch
+ * (explicit operator in shared memory) leaves at once, 2: the factor's CTA of the next
+ * leaf raises no flag, 3: a CTA of the next ELHL_PREC_OZ64 tensor-core propagation withholds
+ * its partial sums of order 2; 0: none. */
+int elhl_debug_stall(int where);
 
 /* Test hook of the factorisation's arithmetic: y[i] = the reciprocal its pivots take of
  * x[i], q[i] = 1 / x[i] by CUDA's division (host arrays of n). */
