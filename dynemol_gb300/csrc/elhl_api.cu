@@ -2219,22 +2219,35 @@ int rebuild(elhl_traj *tr, const double *d_coords) {
 // at 496, 1.19 / 1.12 at 558, 1.24 / 1.43 at 620, 1.24 / 2.07 at 775.
 constexpr int kOzRowsMax = 580;
 
-// Moving nuclei: form H~ = G h G^T every step (1.5 N^3 flops), or apply its three
-// factors in every order (twice the elements, three grid phases per order instead
-// of one, and the same in the Lanczos recursion)?  H~ wins until its N^3 overtakes
-// the N^2 saved per order (143 orders of a 0.5 fs step): measured whole steps,
-// factors / H~ in ms, FP32 5.8 / 3.4 at N = 744, 24.1 / 20.0 at 3720, 45.5 / 41.8 at
-// 5580; DF64 16.0 / 9.7 at 1860, 85.2 / 63.0 at 5580; FP64, whose H~ is formed on
-// the FP64 pipe, 15.5 / 9.2 at 1032, 31.6 / 28.4 at 1860.  Beyond the measured sizes
-// the lines lie where the two costs extrapolated as N^2 and N^3 meet.  The OZ64
-// kernel propagates an explicit operator only.
+// Moving nuclei: form H~ = G h G^T every step (N^3 flops), or apply its three factors in
+// every order (twice the elements, three grid phases per order instead of one, and the
+// same in the Lanczos recursion)?  H~ pays once, the factors in each of the K orders of
+// the step, so the rule weighs what H~ costs beyond what it saves in the bounds against K
+// times what it saves per order, both fitted (in 1e-9 ms) to whole steps of N = 341 to 5,580
+// at 20 to 150 orders with two and four columns.  FP64, whose H~ is formed on the FP64 pipe:
+// N^3 against 33e6 + 4.2 m N^2 per order; the other precisions (sliced products) 0.037 N^3 -
+// 450e6 - 67 N^2 against 10e6 + (0.7 + 0.3 m) N^2 in FP32 and 15e6 + 1.45 m N^2 in DF64.
+// Steps in ms, factors / H~, four columns: FP64 N = 1032 4.5 / 4.4 at 19 orders and
+// 13.5 / 6.8 at 133; N = 1860 14.7 / 18.5 at 46 and 29.1 / 24.3 at 145; N = 2480 25.3 / 36.7
+// and 47.5 / 46.7; FP32 N = 3720 11.8 / 11.6 at 20 and 19.4 / 14.1 at 147, N = 5580 25.2 /
+// 25.8 at 48 and 36.9 / 30.7 at 152; DF64 N = 5580 27.8 / 27.2 at 21 and 79.6 / 53.0 at 152.
+// Of the 128 pairs measured the rule takes the slower form in two, by 3.4 % at most (by size
+// alone, at 2,000 AOs in FP64, N = 1860 took 1.67 times as long at 20 orders).  K is the last step's; a form is left when the other is ahead by 5 % (a change of form makes a new
+// plan).  The OZ64 kernel propagates an explicit operator only.
 bool moving_explicit(const elhl_traj *tr) {
+    const ChebState &cs = tr->cs;
+    const double n = tr->N, n2 = n * n, n3 = n2 * n, m = cs.m;
+    double form = 0.037 * n3 - 450e6 - 67.0 * n2, order = 10e6 + (0.7 + 0.3 * m) * n2;
     switch (tr->cfg.precision) {
         case ELHL_PREC_OZ64: return true;
-        case ELHL_PREC_FP64: return tr->N <= 2000;
-        case ELHL_PREC_DF64: return tr->N <= 12000;
-        default: return tr->N <= 6000;
+        case ELHL_PREC_FP64:
+            form = n3;
+            order = 33e6 + 4.2 * m * n2;
+            break;
+        case ELHL_PREC_DF64: order = 15e6 + 1.45 * m * n2; break;
+        default: break;
     }
+    return form <= cs.K * order * (cs.implicit ? 0.95 : 1.05);
 }
 
 // What cheb_rebuild_operator forms: H~ once for fixed nuclei, or for moving nuclei (fewer
