@@ -277,7 +277,7 @@ size_t ozgemm_smem_bytes();
 // memory, blocks of leaf_rows() = 64 rows: leaf_chol_inv64: A (nb x nb,
 // nb <= 64) <- chol(A), G <- its inverse, in FP64; a non-positive pivot sets
 // info[0] (if still 0) to row0 + column + 1, a wait that gave up info[1].  wait_ns: limit of
-// the waits (0: default); mute: test hook, the factor's CTA raises no flag.
+// the waits (0: default); mute: test hook, the factor's CTA does nothing.
 int leaf_rows();
 cudaError_t leaf_chol_inv64(double *A, double *G, int nb, int ld, int row0, int *info, cudaStream_t st,
                             unsigned long long wait_ns = 0, bool mute = false);
