@@ -2214,10 +2214,13 @@ int rebuild(elhl_traj *tr, const double *d_coords) {
 
 // ELHL_PREC_OZ64 up to this size propagates on the FP64 pipe (cheb_rows.cuh) instead of
 // the tensor cores: an order of oz_cheb_kernel costs at least 5.5 us of hand-overs
-// (TMA, MMA, flush, partials, barrier) whatever its size.  Moving step, tensor cores /
-// FP64 pipe in ms of propagation: 0.81 / 0.21 at N = 62, 0.90 / 0.62 at 341, 1.10 / 0.98
-// at 496, 1.19 / 1.12 at 558, 1.24 / 1.43 at 620, 1.24 / 2.07 at 775.
-constexpr int kOzRowsMax = 580;
+// (TMA, MMA, flush, partials, barrier) whatever its size and columns, one of the row kernel
+// its rows per CTA times its columns.  So the lines lie where a CTA of 152 takes a fifth
+// row (four columns) or a seventh (two).  Propagation of a moving step, tensor cores / FP64 pipe
+// in ms: four columns 0.81 / 0.21 at N = 62, 1.11 / 0.97 at 496, 1.21 / 1.17 at 589, 1.24 /
+// 1.44 at 620; two columns 1.23 / 0.64 at 558, 1.27 / 0.95 at 744, 1.23 / 1.17 at 868, 1.06 /
+// 1.33 at 930.  Fixed nuclei cross at the same sizes.
+int oz_rows_max(int m) { return m <= 2 ? 912 : 608; }
 
 // Moving nuclei: form H~ = G h G^T every step (N^3 flops), or apply its three factors in
 // every order (twice the elements, three grid phases per order instead of one, and the
@@ -3138,7 +3141,7 @@ int elhl_traj_create(const elhl_basis_desc *basis, const double *coords, const e
         if (!rc) {
             int sms = 0;
             rc = cheb_grid_size(&sms) ? ELHL_ERR_CUDA : ELHL_OK;
-            if (!oz || tr->N <= kOzRowsMax) tr->cs.rows = cheb_rows_fit(tr->cs.precision, tr->N, tr->cs.m, sms);
+            if (!oz || tr->N <= oz_rows_max(tr->cs.m)) tr->cs.rows = cheb_rows_fit(tr->cs.precision, tr->N, tr->cs.m, sms);
         }
         tr->cs.guard = tr->cfg.lanczos_guard;
         if (!rc) rc = dev_alloc(&tr->psi_ao, (size_t)tr->ld * tr->P);

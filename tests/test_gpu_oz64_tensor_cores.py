@@ -1,5 +1,5 @@
 """ELHL_PREC_OZ64 where its propagation runs on the tensor cores (oz_cheb_kernel, beyond the
-sizes that the FP64 row kernel takes over: kOzRowsMax AOs, more with two columns): fixed and
+sizes that the FP64 row kernel takes over, 608 AOs with four columns, 912 with two): fixed and
 moving nuclei against exact propagation in the generalized eigenbasis at the FP64 bars, and
 many steps.  One order is one hand-over of tagged partial sums whose tags come round after
 1,023 orders, and the step count covers that within a launch of many orders too."""
@@ -28,8 +28,8 @@ def _system(n_atoms):
     return sysm, homo
 
 
-# row tiles of 128: eight with 3 rows in the last, five with 108, ten with 88
-@pytest.mark.parametrize("n_atoms,ncols", [(290, 2), (200, 4), (400, 4)])
+# row tiles of 128: nine with 3 rows in the last, five with 108, ten with 88
+@pytest.mark.parametrize("n_atoms,ncols", [(331, 2), (200, 4), (400, 4)])
 def test_fixed_nuclei_vs_exact(elhl, oracle_mod, n_atoms, ncols):
     sysm, homo = _system(n_atoms)
     S = oracle_mod.overlap(sysm)
@@ -49,7 +49,7 @@ def test_fixed_nuclei_vs_exact(elhl, oracle_mod, n_atoms, ncols):
 
 def test_many_steps_and_many_orders(elhl, oracle_mod):
     """300 steps of about 40 orders, then one step of 6 fs: more than 1,023 orders in a launch."""
-    sysm, homo = _system(290)
+    sysm, homo = _system(300)
     S = oracle_mod.overlap(sysm)
     bra, ket = oracle_mod.initial_states(sysm, S, homo + 1, homo)
     for dt, nsteps, orders in ((1e-4, 300, 0), (6e-3, 1, 1024)):
@@ -64,7 +64,7 @@ def test_many_steps_and_many_orders(elhl, oracle_mod):
         assert st.orders // (2 * nsteps) > orders
 
 
-@pytest.mark.parametrize("n_atoms,ncols", [(190, 4), (290, 2)])
+@pytest.mark.parametrize("n_atoms,ncols", [(200, 4), (331, 2)])
 def test_moving_then_fixed_vs_exact(elhl, oracle_mod, n_atoms, ncols):
     sysm, homo = _system(n_atoms)
     coords = np.stack([systems.perturbed_coords(sysm.coords, i, seed=3) for i in range(3)])
@@ -83,3 +83,27 @@ def test_moving_then_fixed_vs_exact(elhl, oracle_mod, n_atoms, ncols):
             bra = oracle_mod.overlap(sysm, g) @ ket
         bra, ket = _exact(oracle_mod, sysm, bra, ket, g, 5e-4)
         assert np.abs(p - _pops(oracle_mod, sysm, bra, ket)).max() < 1e-10
+
+
+@pytest.mark.parametrize("n_atoms,ncols,on_tensor_cores", [(294, 2, False), (295, 2, True), (196, 4, False), (197, 4, True)])
+def test_line_between_the_kernels(elhl, n_atoms, ncols, on_tensor_cores):
+    """The last size of the FP64 row kernel and the first of the tensor cores, by the column
+    counts: both agree with the FP64 path; which kernel ran shows in the launches of a step."""
+    sysm, homo = _system(n_atoms)
+    assert (sysm.nao > (912 if ncols == 2 else 608)) == on_tensor_cores
+    out = {}
+    for prec in ("PREC_FP64", "PREC_OZ64"):
+        tr = elhl.Trajectory(sysm, dt=1e-4, method=elhl.METHOD_CHEBYSHEV, precision=getattr(elhl, prec), ncols=ncols,
+                             cheb_tol=1e-14)
+        tr.init_fmo(homo + 1, homo)
+        tr.step(None, nsteps=1)
+        before = elhl.kernel_launches()
+        pops = tr.step(None, nsteps=4)
+        launches = elhl.kernel_launches() - before
+        out[prec] = (pops, tr.get_psi()[1], launches)
+        tr.close()
+    assert np.abs(out["PREC_OZ64"][0] - out["PREC_FP64"][0]).max() < 1e-12
+    assert np.abs(out["PREC_OZ64"][1] - out["PREC_FP64"][1]).max() < 1e-11
+    # the row kernel's step is two launches, the tensor cores' one and the separate read-out's
+    assert out["PREC_FP64"][2] == 8
+    assert (out["PREC_OZ64"][2] == 8) != on_tensor_cores
