@@ -1448,6 +1448,17 @@ double row_work(const ChebState &cs) {
     return (cs.ld + kRowExtra) * (groups + 0.25 * cs.m);
 }
 
+// read-out matrices of a problem (or none), and what only a device read-out does
+void plan_readout(ChebProblem &p, const ChebState &cs, bool dev) {
+    p.A = dev ? cs.A : nullptr;
+    p.B = dev ? cs.B : nullptr;
+    const bool renorm = dev && reduced_precision(cs.precision);
+    p.scale = renorm ? cs.scale : nullptr;
+    p.scale_out = renorm ? cs.scale : nullptr;
+    p.target = renorm ? cs.target : nullptr;
+    p.ntot = renorm ? cs.ntot : nullptr;
+}
+
 int cheb_plan(ChebPlan &pl, const std::vector<ChebState *> &states) {
     pl.release();
     pl.probs.clear();
@@ -1491,16 +1502,9 @@ int cheb_plan(ChebPlan &pl, const std::vector<ChebState *> &states) {
         p.N = cs->N; p.ld = cs->ld; p.ldv = cs->ld; p.m = cs->m; p.K = cs->K;
         p.H = cs->Hs; p.vbuf = cs->vbuf; p.col[0] = cs->phi; p.col[1] = cs->acc; p.coef = cs->coef;
         p.P = cs->P;
-        const bool dev = cs->readout_ready && pl.mg_read;
-        p.A = dev ? cs->A : nullptr;
-        p.B = dev ? cs->B : nullptr;
+        plan_readout(p, *cs, cs->readout_ready && pl.mg_read);
         p.psi = cs->psi_out; p.bra = cs->bra_out; p.ao_frag = cs->ao_frag; p.nfrag = cs->nfrag;
         p.pops_off = (int)pl.pops_per_step;
-        const bool renorm = dev && reduced_precision(cs->precision);
-        p.scale = renorm ? cs->scale : nullptr;
-        p.scale_out = renorm ? cs->scale : nullptr;
-        p.target = renorm ? cs->target : nullptr;
-        p.ntot = renorm ? cs->ntot : nullptr;
         if (cs->implicit) {
             p.G = cs->A;
             p.Gt = cs->Gt;
@@ -1603,6 +1607,17 @@ int cheb_plan_refresh(ChebPlan &pl, const std::vector<ChebState *> &states) {
     }
     CU_TRY(copy_h2d(pl.d_probs, pl.probs.data(), pl.probs.size() * sizeof(ChebProblem)));
     return ELHL_OK;
+}
+
+// The plan after cheb_prepare_readout: as it is, with the matrices' addresses, where their type
+// is the one it was made for (no allocation, so that runs that alternate moving and fixed
+// steps pay for the matrices only).
+int cheb_plan_readout(ChebPlan &pl, const std::vector<ChebState *> &states) {
+    bool same = pl.probs.size() == states.size() && pl.mg_read > 0;
+    for (auto *cs : states) same &= pl.ro_precision == (cs->ro64 ? ELHL_PREC_FP64 : cs->precision);
+    if (!same) return cheb_plan(pl, states);
+    for (size_t q = 0; q < states.size(); ++q) plan_readout(pl.probs[q], *states[q], true);
+    return cheb_plan_refresh(pl, states);
 }
 
 ChebLaunch plan_launch(const ChebPlan &pl) {
@@ -2453,7 +2468,7 @@ int cheb_step_impl(elhl_traj *tr, const double *coords, bool coords_on_device, i
     if (!coords && !cs.readout_ready && tr->fac.L && cs.precision != ELHL_PREC_DF64) {
         // fixed nuclei after moving steps: factor-based read-out matrices for the current L
         if ((rc = cheb_prepare_readout(cs, tr->fac.L, traj_inverse(tr)))) return rc;
-        if ((rc = cheb_plan(tr->plan, one))) return rc;
+        if ((rc = cheb_plan_readout(tr->plan, one))) return rc;
     }
     if (!coords && cs.readout_ready && (tr->plan.mg_read || cs.gemm)) {
         // ---- fixed nuclei, device read-out: two launches (or one graph) per step, no host sync;
