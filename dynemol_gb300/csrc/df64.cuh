@@ -37,6 +37,33 @@ __device__ __forceinline__ void df_add(float &ah, float &al, float bh, float bl)
     ah = t;
 }
 
+// s + e = a + b exactly (Knuth's TwoSum), s in a, e in b
+__device__ __forceinline__ void two_sum(float &a, float &b) {
+    const float s = __fadd_rn(a, b);
+    const float z = __fsub_rn(s, a);
+    b = __fadd_rn(__fsub_rn(a, __fsub_rn(s, z)), __fsub_rn(b, z));
+    a = s;
+}
+
+// FP32 triples s[0] + s[1] + s[2]: sums of FP32 numbers with less error (2^-70 of the largest
+// partial sum) than FP64 makes, without the FP64 pipe.
+__device__ __forceinline__ void ts_add(float (&s)[3], float y) {
+    two_sum(s[0], y);
+    two_sum(s[1], y);
+    s[2] = __fadd_rn(s[2], y);
+}
+// A triple rounded to FP32, to nearest of the triple's value: b + c is rounded to odd (its last
+// bit set where something lies below it, so that no tie is seen where there is none), then a
+// added (S. Boldo, G. Melquiond, Emulation of FMA and correctly rounded sums: proved
+// algorithms using rounding to odd, 2008).
+__device__ __forceinline__ float ts_round(float a, float b, float c) {
+    two_sum(a, b);
+    two_sum(b, c);
+    int i = __float_as_int(b);
+    if (c != 0.f && !(i & 1)) i += (i ^ __float_as_int(c)) < 0 ? -1 : 1;
+    return __fadd_rn(a, __int_as_float(i));
+}
+
 // (a + b) + c rounded once for |c| far below ulp(a + b): TwoSum gives a + b = t + e
 // exactly, then t + (e + c)
 __device__ __forceinline__ float two_sum_plus(float a, float b, float c) {

@@ -302,8 +302,8 @@ __global__ void pack_v_kernel(const float *__restrict__ v, int n, int n2, unsign
     pack_row(dst, n2, nk, c, k0, x);
 }
 
-// y = sum of the nsplit partial products (fixed order, as an FP32 pair: TwoSum, so
-// exact to 2^-48), v_k = 2 y - v_{k-2} (v_1 = y) rounded once to FP32, acc += c_k v_k
+// y = sum of the nsplit partial products (fixed order, as an FP32 triple: closer than an FP64
+// sum), v_k = 2 y - v_{k-2} (v_1 = y) rounded once to FP32, acc += c_k v_k
 // in FP64, and v_k packed as the next product's B (rows past n keep the zeros that
 // packing v_0 left).  A thread takes kEpiRows rows of one complex column, everything it
 // reads asked for before the first result: bound by the FP64 unit (eight of its
@@ -319,14 +319,17 @@ __global__ void __launch_bounds__(128) umma_epilogue_kernel(const float2 *__rest
     if (r0 >= n) return;
     const int rows = min(kEpiRows, n - r0);
     double2 a[kEpiRows];
-    float2 w[kEpiRows], h[kEpiRows], l[kEpiRows];
+    float2 w[kEpiRows];
+    float yr[kEpiRows][3], yi[kEpiRows][3];
 #pragma unroll
     for (int i = 0; i < kEpiRows; ++i) {
         const size_t q = (size_t)(r0 + min(i, rows - 1)) * m + c;
         a[i] = acc[q];
         w[i] = k == 1 ? make_float2(0.f, 0.f) : vprev2[q];
-        h[i] = Y[q];
-        l[i] = make_float2(0.f, 0.f);
+        const float2 y = Y[q];
+        yr[i][0] = y.x;
+        yi[i][0] = y.y;
+        yr[i][1] = yr[i][2] = yi[i][1] = yi[i][2] = 0.f;
     }
     const double2 ck = coef[k];
 #pragma unroll 4
@@ -334,20 +337,23 @@ __global__ void __launch_bounds__(128) umma_epilogue_kernel(const float2 *__rest
 #pragma unroll
         for (int i = 0; i < kEpiRows; ++i) {
             const float2 y = Y[s * split_stride + (size_t)(r0 + min(i, rows - 1)) * m + c];
-            df_add(h[i].x, l[i].x, y.x, 0.f);
-            df_add(h[i].y, l[i].y, y.y, 0.f);
+            ts_add(yr[i], y.x);
+            ts_add(yi[i], y.y);
         }
     }
     float re[kEpiRows], im[kEpiRows];
 #pragma unroll
     for (int i = 0; i < kEpiRows; ++i) {
-        float2 v;
-        if (k == 1) {
-            v = make_float2(__fadd_rn(h[i].x, l[i].x), __fadd_rn(h[i].y, l[i].y));
-        } else {
-            v.x = two_sum_plus(__fmul_rn(2.f, h[i].x), -w[i].x, __fmul_rn(2.f, l[i].x));
-            v.y = two_sum_plus(__fmul_rn(2.f, h[i].y), -w[i].y, __fmul_rn(2.f, l[i].y));
+        if (k > 1) {
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                yr[i][s] = __fmul_rn(2.f, yr[i][s]);
+                yi[i][s] = __fmul_rn(2.f, yi[i][s]);
+            }
+            ts_add(yr[i], -w[i].x);
+            ts_add(yi[i], -w[i].y);
         }
+        const float2 v = make_float2(ts_round(yr[i][0], yr[i][1], yr[i][2]), ts_round(yi[i][0], yi[i][1], yi[i][2]));
         re[i] = im[i] = 0.f;
         if (i >= rows) continue;
         re[i] = v.x;
