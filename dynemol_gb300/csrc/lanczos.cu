@@ -207,12 +207,14 @@ __global__ void __launch_bounds__(kLzThreads) lanczos64_kernel(const LzArgs a) {
 // its rows and publishes them (exchange.cuh); every CTA then reads all of w and
 // carries q_j and q_{j-1} and the scalars itself, by the same operations in the same
 // order, so that all agree to the bit.  p = w - beta_{j-1} q_{j-1}, alpha = p . q and
-// beta^2 = |p|^2 - alpha^2 from one pass over p (a second pass sums |p - alpha q|^2
-// where that difference would cancel).  Bound: the FP64 unit for the products above
+// beta^2 = |p|^2 - alpha^2 from one pass over p; a second pass sums |p - alpha q|^2 where
+// that difference would cancel by more than a factor of eight (beta loses two bits at most;
+// on the C/H/O systems beta^2 stays above a quarter of |p|^2, so the second pass is rare).  Bound: the FP64 unit for the products above
 // about N = 700, latency below.  Twenty steps: N = 62 217 -> 75 us, N = 744 272 -> 174,
 // N = 932 275 -> 193, N = 1860 379 -> 300.
 constexpr int kLrThreads = 256, kLrWarps = kLrThreads / 32, kLrBatch = 4;
 constexpr size_t kLrSmem = 220 * 1024;
+constexpr double kLrCancel = 0.125;
 
 struct LrArgs {
     int n, ld, k;
@@ -308,7 +310,7 @@ __global__ void __launch_bounds__(kLrThreads, 1) lanczos_rows_kernel(const LrArg
             if (lane == 0) {
                 const double b2 = p2 - alpha * alpha, ib = rsqrt(b2);
                 s_sc[0] = alpha;
-                s_sc[1] = b2 > 1.0e-6 * p2 ? 1.0 : 0.0;  // else |p - alpha q|^2 is summed
+                s_sc[1] = b2 > kLrCancel * p2 ? 1.0 : 0.0;  // else |p - alpha q|^2 is summed
                 s_sc[2] = b2 * ib;
                 s_sc[3] = ib;
             }
