@@ -1,5 +1,6 @@
 // Chebyshev propagation of one trajectory on an explicit Hs whose rows stay in
-// shared memory for the whole launch (bases up to about 1,900 AOs in FP64).
+// shared memory for the whole launch (FP64 and DF64: up to 1,250 AOs with four columns and
+// about 1,900 with two; FP32: 2,432).
 //
 // At these sizes an order of cheb_kernel (cheb.cu) is latency, not work: a grid
 // barrier (2,750 cycles with the fastest form of it), the previous vector staged

@@ -1,4 +1,4 @@
-// FP64 products of the factorisations' smallest blocks (64 to 128 rows):
+// FP64 products of the factorisations' smallest blocks (up to 192 rows):
 //   C = alpha op(A) op(B) + beta C, flags and masking as in dgemm.cu.
 // At these sizes the product is a matter of latency, not of the FP64 pipe (64^3: 0.5 us
 // if every SM took part): dgemm.cu's 16 x 16 tiles of one 64^3 product are 16 CTAs whose

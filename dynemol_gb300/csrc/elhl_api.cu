@@ -243,7 +243,7 @@ __global__ void lower_only_kernel(double *A, int n, int ld) {
 // 64-row diagonal blocks as leaves (leaf_chol_inv64), splits on multiples of 64.
 // G11^T L21^T, the first factor of G21 = -G22 (L21 G11) stored transposed in the
 // unused upper block G12, runs on a second stream while the main stream does the
-// Schur update and factors A22 (whose single-CTA leaves leave most SMs free).
+// Schur update and factors A22 (whose leaves, clusters of four CTAs, leave most SMs free).
 // It replaces the reference's LU inverse of S (MAGMA dgetrf + dgetri,
 // GPU_Interface.cpp:910-928; CPU dsytrf + dsytri, :936-947): S is symmetric
 // positive definite, so its Cholesky factor gives S^-1 = G^T G.  L21 is formed in W
@@ -313,7 +313,7 @@ int chol_inv64(double *A, double *G, int n, int ld, int row0, double *W, int *in
     const int n1 = round_up(n / 2, leaf), n2 = n - n1;
     double *A21 = A + n1, *A22 = A + (size_t)n1 * ld + n1;
     double *G21 = G + n1, *G22 = G + (size_t)n1 * ld + n1;
-    double *G12 = G + (size_t)n1 * ld;  // n1 x n2, above the diagonal: free until lower_only
+    double *G12 = G + (size_t)n1 * ld;  // n1 x n2, above the diagonal: not read as part of G
     cudaStream_t side = g_ctx.aux_stream;
     if (int rc = chol_inv64(A, G, n1, ld, row0, W, info, tc)) return rc;
     CU_TRY(fgemm(tc, n2, n1, n1, 1.0, A21, ld, false, G, ld, true, 0.0, W, ld, st, kTriBt));       // L21
@@ -1047,8 +1047,7 @@ bool readout_fp64(const ChebState &cs) {
 }
 
 // A = L^-1 and B = L^T for the device read-out of fixed nuclei, in FP64
-// (readout_fp64) or the launch precision.  L and G = L^-1 both FP64 with zero
-// upper triangles.
+// (readout_fp64) or the launch precision.  L and G = L^-1 both FP64 (lower triangles).
 int cheb_prepare_readout(ChebState &cs, const double *Lfac, const double *G) {
     cudaStream_t st = g_ctx.stream;
     const int n = cs.N, ld = cs.ld;
@@ -1103,7 +1102,7 @@ int cheb_prepare_implicit(ChebState &cs, const double *Lfac, const double *h, do
         CU_TRY(cudaMalloc(&cs.wb, (size_t)2 * ld * cs.m * 2 * tsz));
         CU_TRY(cudaMemsetAsync(cs.wb, 0, (size_t)2 * ld * cs.m * 2 * tsz, g_ctx.stream));
     }
-    // L with a zero upper triangle (the recursion leaves S's there): the dense column transforms read all of it
+    // zero upper triangles, whatever the recursion left there: split_df_kernel reads whole columns
     lower_only_kernel<<<dim3((ld + 127) / 128, n), 128, 0, st>>>(const_cast<double *>(Lfac), n, ld);
     count_launch();
     CU_TRY(cudaGetLastError());
@@ -1944,7 +1943,8 @@ __global__ void cols_mt_kernel(const double *__restrict__ M, int ld, int n, cons
     if ((lane & 3) == 0 && r < R) Y[(size_t)j * R + r] = acc[0];
 }
 
-// The same four transforms with dense FP64 factors (zeros above the diagonal):
+// The same four transforms with dense FP64 factors (lower triangles; what is above the
+// diagonal is not read):
 // M = G = L^-1 for the inverse ones, M = L otherwise, X op(M) into scratch
 // (2 ncols x n) and a strided copy back.  op(M) = M, and op(M) = M^T when the
 // FP64 transpose Mt (Lt for L, Gt for G) is resident, run as cols_mt_kernel;
@@ -2333,7 +2333,7 @@ int cheb_load_columns(elhl_traj *tr) {
     CU_TRY(cudaMemcpy2DAsync(in, cs.m * e, tr->psi_ao, P * e, P * e, n, cudaMemcpyDeviceToDevice, st));
     if (cs.m == 2 * P)
         CU_TRY(cudaMemcpy2DAsync(in + P, cs.m * e, tr->bra_ao, P * e, P * e, n, cudaMemcpyDeviceToDevice, st));
-    if (cs.implicit) {  // dense L (zeroed upper triangle) and G = L^-1
+    if (cs.implicit) {  // G = L^-1 lies in cs.Ht
         const double *Lt = cs.lt64(), *Gt = cs.gt64();
         if (int rc = cols_apply_dense(tr->fac.L, cs.Ht, tr->ld, n, in, cs.m, 0, P, false, false, cs.cscratch, Lt, Gt))
             return rc;
