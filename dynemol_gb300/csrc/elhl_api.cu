@@ -2117,6 +2117,8 @@ struct elhl_traj {
     std::vector<int> h_ao0, h_nao, h_n, h_l, h_m, h_nz;
     std::vector<double> h_zeta, h_coef, h_ip, h_kwh, h_vs;
     const double *last_coords = nullptr;  // device coordinates of the current S, h
+    double *coords2 = nullptr;            // Chebyshev, moving nuclei: the other buffer for them
+    int lost = ELHL_OK;                   // why there is no operator (a refused geometry, and no way back)
     int N = 0, ld = 0, natoms = 0, nfrag = 0, P = 2;
     elhl_traj_config cfg;
     double *S = nullptr, *h = nullptr, *Hp = nullptr, *coords = nullptr, *pops = nullptr;
@@ -2451,6 +2453,34 @@ int cheb_run_checked(elhl_traj *tr, double *drift) {
     }
 }
 
+// What the operator was before a rebuild, to go back to if its geometry is refused.
+struct OperatorState {
+    bool moving, implicit;
+    double emin, emax;
+};
+OperatorState operator_state(const ChebState &cs) { return {cs.moving, cs.implicit, cs.emin, cs.emax}; }
+
+// After a rebuild that failed: S, h, the factor and the operator of the last geometry
+// (tr->last_coords) again, in their form and on their interval, so that the trajectory is
+// where it was before the step.
+int cheb_return_to_geometry(elhl_traj *tr, const OperatorState &was) {
+    ChebState &cs = tr->cs;
+    std::vector<ChebState *> one{&cs};
+    CU_TRY(launch_build_sh(tr->basis, tr->last_coords, tr->cfg.cutoff, tr->S, tr->h, tr->ld, g_ctx.stream));
+    const Rebuild what = !was.moving ? Rebuild::kFixed
+                         : was.implicit ? Rebuild::kMovingImplicit : Rebuild::kMovingExplicit;
+    if (int rc = cheb_rebuild_operator(tr, what)) return rc;
+    if (!cs.implicit) cs.readout_ready = false;
+    if (cs.emin != was.emin || cs.emax != was.emax) {  // an interval widened by norm control
+        cs.emin = was.emin;
+        cs.emax = was.emax;
+        if (int rc = cheb_prepare(cs, tr->cfg.dt * tr->cfg.frame_step, tr->cfg.cheb_tol,
+                                  cs.implicit ? tr->h : nullptr))
+            return rc;
+    }
+    return cheb_plan_refresh(tr->plan, one);
+}
+
 int cheb_step_impl(elhl_traj *tr, const double *coords, bool coords_on_device, int nsteps, double *d_pops) {
     cudaStream_t st = g_ctx.stream;
     ChebState &cs = tr->cs;
@@ -2459,6 +2489,7 @@ int cheb_step_impl(elhl_traj *tr, const double *coords, bool coords_on_device, i
     const size_t nc = (size_t)tr->natoms * 3;
     std::vector<ChebState *> one{&cs};
     int rc = ELHL_OK;
+    if (!coords && tr->lost) return tr->lost;
     if (!coords && cs.implicit && cs.gemm) {
         // GEMM regime after moving steps: form H~ for the current geometry
         if ((rc = cheb_rebuild_operator(tr, Rebuild::kFixed))) return rc;
@@ -2530,22 +2561,40 @@ int cheb_step_impl(elhl_traj *tr, const double *coords, bool coords_on_device, i
     if (!coords && !cs.cols_current) rc = cheb_load_columns(tr);
     for (int s = 0; s < nsteps && !rc; ++s) {
         if (coords) {
-            const double *dc;
-            if (coords_on_device) {
-                dc = coords + s * nc;
-            } else {
-                if (cudaMemcpyAsync(tr->coords, coords + s * nc, nc * sizeof(double), cudaMemcpyHostToDevice, st) !=
-                    cudaSuccess) { rc = ELHL_ERR_CUDA; break; }
-                dc = tr->coords;
+            // the buffer that does not hold the last geometry, which stays for a refused one
+            double *own = tr->last_coords == tr->coords ? tr->coords2 : tr->coords;
+            if (!own) {
+                if ((rc = dev_alloc(&tr->coords2, nc))) break;
+                own = tr->coords2;
             }
-            tr->last_coords = dc;
+            const double *dc = coords_on_device ? coords + s * nc : own;
+            if (!coords_on_device && cudaMemcpyAsync(own, coords + s * nc, nc * sizeof(double), cudaMemcpyHostToDevice,
+                                                     st) != cudaSuccess) { rc = ELHL_ERR_CUDA; break; }
+            const OperatorState was = operator_state(cs);
             if (cudaEventRecord(g_ctx.ev[2], st) != cudaSuccess) { rc = ELHL_ERR_CUDA; break; }
             if (launch_build_sh(tr->basis, dc, tr->cfg.cutoff, tr->S, tr->h, tr->ld, st) != cudaSuccess) {
                 rc = ELHL_ERR_CUDA;
                 break;
             }
             if (cudaEventRecord(g_ctx.ev[4], st) != cudaSuccess) { rc = ELHL_ERR_CUDA; break; }
-            if ((rc = cheb_rebuild_operator(tr, Rebuild::kMoving))) break;
+            if ((rc = cheb_rebuild_operator(tr, Rebuild::kMoving))) {
+                tr->lost = cheb_return_to_geometry(tr, was);
+                if (tr->last_coords != tr->coords && tr->last_coords != tr->coords2) {  // the caller's buffer is valid during the call only
+                    (void)cudaMemcpyAsync(own, tr->last_coords, nc * sizeof(double), cudaMemcpyDeviceToDevice, st);
+                    (void)cudaStreamSynchronize(st);
+                    tr->last_coords = own;
+                }
+                break;
+            }
+            tr->lost = ELHL_OK;
+            tr->last_coords = dc;
+            if (coords_on_device && s + 1 == nsteps) {  // as the call returns
+                if (cudaMemcpyAsync(own, dc, nc * sizeof(double), cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
+                    rc = ELHL_ERR_CUDA;
+                    break;
+                }
+                tr->last_coords = own;
+            }
             if ((rc = cheb_load_columns(tr))) break;
             if (cudaEventRecord(g_ctx.ev[3], st) != cudaSuccess) { rc = ELHL_ERR_CUDA; break; }
             if ((rc = cheb_plan_refresh(tr->plan, one))) break;
@@ -3221,7 +3270,7 @@ int elhl_traj_destroy(elhl_traj *tr) {
     tr->tb.release();
     tr->cs.release();
     tr->plan.release();
-    dev_free(tr->psi_ao); dev_free(tr->bra_ao); dev_free(tr->target);
+    dev_free(tr->psi_ao); dev_free(tr->bra_ao); dev_free(tr->target); dev_free(tr->coords2);
     delete tr;
     return ELHL_OK;
 }
