@@ -332,14 +332,22 @@ __global__ void __launch_bounds__(128) umma_epilogue_kernel(const float2 *__rest
         yr[i][1] = yr[i][2] = yi[i][1] = yi[i][2] = 0.f;
     }
     const double2 ck = coef[k];
-#pragma unroll 4
-    for (int s = 1; s < nsplit; ++s) {
+    constexpr int kAhead = 3;  // partials under way together
+    for (int s0 = 1; s0 < nsplit; s0 += kAhead) {
+        float2 y[kAhead][kEpiRows];
 #pragma unroll
-        for (int i = 0; i < kEpiRows; ++i) {
-            const float2 y = Y[s * split_stride + (size_t)(r0 + min(i, rows - 1)) * m + c];
-            ts_add(yr[i], y.x);
-            ts_add(yi[i], y.y);
-        }
+        for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+            for (int i = 0; i < kEpiRows; ++i)
+                y[u][i] = s0 + u < nsplit ? Y[(s0 + u) * split_stride + (size_t)(r0 + min(i, rows - 1)) * m + c]
+                                          : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+            for (int i = 0; i < kEpiRows; ++i) {
+                ts_add(yr[i], y[u][i].x);
+                ts_add(yi[i], y[u][i].y);
+            }
     }
     float re[kEpiRows], im[kEpiRows];
 #pragma unroll
