@@ -474,7 +474,6 @@ int run_taylor(const double *Hp, int N, int ld, TaylorBuffers &tb, int P, const 
     L.bar_count = g_ctx.bar;
     L.error = g_ctx.err;
     L.words = tb.words;
-    L.barrier_ns = g_dbg_barrier_ns;
     L.exit_cta1 = g_dbg_exit_cta1;
     g_dbg_exit_cta1 = 0;  // one launch only
     CU_TRY(cudaEventRecord(g_ctx.ev[0], st));

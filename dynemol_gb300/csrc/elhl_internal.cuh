@@ -87,7 +87,6 @@ struct TaylorLaunch {
     unsigned *bar_count;  // grid barrier: two words, one 64-bit count (8-byte aligned, zero at the launch)
     int *error;           // global error flag
     ulonglong2 *words;    // taylor_words(N, grid) words exchanged in place of the barrier, or nullptr
-    unsigned long long barrier_ns;  // limit of the grid barrier (0: default)
     int exit_cta1;        // test hook: 1 + the CTA that leaves after the first round (0: none)
 };
 constexpr int kSlots = 6;

@@ -414,8 +414,7 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
         }
     };
 
-    // (The words' waits take kBarrierNs, the barrier's L.barrier_ns: a limit that is no
-    // constant costs the words' rounds 0.5 %.)
+    // (All waits take kBarrierNs: a limit that is no constant costs a round 0.3 to 0.5 %.)
     // Exchange without the barrier (resident, L.words): the round's next source and its
     // records go out as words tagged with the round, which the readers poll.  Two buffers
     // suffice: a CTA publishes round r + 2 once it has every CTA's words of round r + 1,
@@ -468,7 +467,7 @@ __global__ void __launch_bounds__(kTaylorBlock, 1) taylor_kernel(TaylorLaunch L)
     // wait for the round's arrivals; false: the launch ends with an error
     auto wait_round = [&]() -> bool {
         arrivals += G;
-        if (tid == 0) s_ok = grid_poll(L.bar_count, arrivals, L.error, L.barrier_ns);
+        if (tid == 0) s_ok = grid_poll(L.bar_count, arrivals, L.error);
         __syncthreads();
         return s_ok;
     };
@@ -808,7 +807,6 @@ cudaError_t launch_taylor_t(const TaylorLaunch &L, int grid, int block, size_t s
     if (e != cudaSuccess) return e;
     TaylorLaunch copy = L;
     if (copy.exit_cta1 > grid) copy.exit_cta1 = grid;
-    if (!copy.barrier_ns) copy.barrier_ns = kBarrierNs;
     copy.tol2 = L.tol < 0.0 ? -1.0 : L.tol * L.tol;  // |delta| > tol < 0 always holds
     if (kResident && L.words) {  // no word carries a round's tag before the launch
         e = cudaMemsetAsync(L.words, 0, taylor_words(L.N, grid) * sizeof(ulonglong2), st);

@@ -374,9 +374,8 @@ int elhl_server_destroy(elhl_server *sv);
 int elhl_set_stream(void *stream);
 
 /* Test hook for failure detection (no counterpart in the reference): the
- * limit of the waits of the propagation, bounds and leaf kernels (limit_s <= 0
- * restores the defaults, 5 s and 2 s; at most 10 s; the tagged words of the Taylor kernel
- * keep theirs of 5 s) and, when exit_cta >= 0, one CTA of
+ * limit of the waits of the Chebyshev, bounds and leaf kernels (limit_s <= 0
+ * restores the defaults, 5 s and 2 s; at most 10 s; the Taylor kernel keeps its 5 s) and, when exit_cta >= 0, one CTA of
  * the next propagation launch that leaves before its first grid barrier (Taylor: after its
  * first round), so that the other CTAs' waits run out and the call returns ELHL_ERR_TIMEOUT
  * with the device context intact.  No fault or hang is involved: every wait

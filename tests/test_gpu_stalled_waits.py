@@ -1,7 +1,7 @@
 """Every bounded wait of the cooperative kernels that can run out is made to, once, by the
 test hooks: a CTA that leaves or withholds what the others wait for.  The call returns
-ELHL_ERR_TIMEOUT after the hook's limit (0.2 s; the Taylor kernel's tagged words after
-theirs, 5 s), and the next call on the same context succeeds.  (The Chebyshev row kernels
+ELHL_ERR_TIMEOUT after the hook's limit (0.2 s; the Taylor kernel after its
+own, 5 s), and the next call on the same context succeeds.  (The Chebyshev row kernels
 and the tensor-core kernel's grid barrier: test_gpu_stalled_step.py.)"""
 import numpy as np
 import pytest
