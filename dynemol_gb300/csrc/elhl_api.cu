@@ -780,6 +780,7 @@ struct ChebState {
     int parity = 0;            // phi/acc role of col[0], col[1] for the device read-out path
     void *A = nullptr, *B = nullptr;   // L^-1, L^T in the launch precision (fixed nuclei read-out)
     bool readout_ready = false, cols_current = false;
+    unsigned long long version = 0;  // counts the operators and read-out matrices made: plans of several states follow it
     double *scale = nullptr;   // [P] pending renormalisation factor (reduced precision), 1 otherwise
     double *drift = nullptr;   // norm drift word of the GEMM-regime step (plans keep their own)
     double *ntot = nullptr;    // [kMaxCols] FP64 totals of the last step's columns (renormalisation)
@@ -1008,6 +1009,7 @@ int cheb_prepare(ChebState &cs, double dt, double tol, const double *h = nullptr
     CU_TRY(cudaMemcpyAsync(cs.coef, c.data(), (K + 1) * sizeof(double2), cudaMemcpyHostToDevice, st));
     CU_TRY(cudaStreamSynchronize(st));  // c is a host temporary
     cs.K = K;
+    ++cs.version;
     if (cs.oz && !cs.rows)  // the tensor-core propagation reads Hs as BF16 slices
         if (int rc = cs.oz->slice(static_cast<const double *>(cs.Hs), st)) return rc;
     if (cs.umma && !h) {  // the tensor-core GEMM reads Hs as three BF16 terms
@@ -1076,6 +1078,7 @@ int cheb_prepare_readout(ChebState &cs, const double *Lfac, const double *G) {
     CU_TRY(cudaGetLastError());
     CU_TRY(cudaStreamSynchronize(st));
     cs.readout_ready = true;
+    ++cs.version;
     return ELHL_OK;
 }
 
@@ -2117,6 +2120,7 @@ struct elhl_traj {
     std::vector<double> h_zeta, h_coef, h_ip, h_kwh, h_vs;
     const double *last_coords = nullptr;  // device coordinates of the current S, h
     double *coords2 = nullptr;            // Chebyshev, moving nuclei: the other buffer for them
+    bool shared = false;                  // member of a batch or request of a server: its operator stays explicit
     int lost = ELHL_OK;                   // why there is no operator (a refused geometry, and no way back)
     int N = 0, ld = 0, natoms = 0, nfrag = 0, P = 2;
     elhl_traj_config cfg;
@@ -2489,6 +2493,8 @@ int cheb_step_impl(elhl_traj *tr, const double *coords, bool coords_on_device, i
     std::vector<ChebState *> one{&cs};
     int rc = ELHL_OK;
     if (!coords && tr->lost) return tr->lost;
+    if (coords && !tr->S) return ELHL_ERR_BAD_ARG;  // released by elhl_batch_compact
+    tr->plan.parity = cs.parity;  // a batch or server step may have moved the columns
     if (!coords && cs.implicit && cs.gemm) {
         // GEMM regime after moving steps: form H~ for the current geometry
         if ((rc = cheb_rebuild_operator(tr, Rebuild::kFixed))) return rc;
@@ -3652,7 +3658,7 @@ int traj_restore_impl(elhl_traj *tr, const char *path) {
             // interval.  In the GEMM regime fixed steps form H~ anew after implicit ones.
             const bool implicit = rh.form ? rh.form == kFormImplicit : cs.implicit;
             std::vector<ChebState *> one{&cs};
-            if (implicit != cs.implicit && !cs.gemm && tr->S) {
+            if (implicit != cs.implicit && !cs.gemm && !tr->shared && tr->S) {
                 if (int rc = cheb_rebuild_operator(tr, implicit ? Rebuild::kMovingImplicit : Rebuild::kMovingExplicit)) return rc;
                 if (int rc = cheb_plan_refresh(tr->plan, one)) return rc;
                 cs.cols_current = false;
@@ -3717,11 +3723,42 @@ struct elhl_batch {
     std::vector<elhl_traj *> members;
     ChebPlan plan;
     std::vector<ChebState *> states;
+    std::vector<unsigned long long> versions;  // of the states the plan was made for
     double *pops = nullptr;
     size_t pops_cap = 0;
     bool compact = false;
     elhl_traj_stats stats{};
 };
+
+// What members have done by themselves since the batch's last step (a step of their own, a
+// checkpoint on another interval): columns in the plan's input buffers, explicit operators
+// with read-out matrices, and a plan with their present orders and addresses.
+static int batch_follow(elhl_batch *b) {
+    bool changed = false;
+    for (size_t i = 0; i < b->members.size(); ++i) {
+        elhl_traj *tr = b->members[i];
+        ChebState &cs = tr->cs;
+        if (tr->lost) return tr->lost;
+        if (cs.parity != b->plan.parity) {
+            const double2 *src = cs.cin();
+            cs.parity = b->plan.parity;
+            CU_TRY(cudaMemcpyAsync(cs.cin(), src, (size_t)cs.ld * cs.m * sizeof(double2), cudaMemcpyDeviceToDevice,
+                                   g_ctx.stream));
+        }
+        if (cs.implicit && b->members.size() > 1) {
+            if (!tr->S) return ELHL_ERR_UNSUPPORTED;  // compacted
+            if (int rc = cheb_rebuild_operator(tr, Rebuild::kFixed)) return rc;
+            cs.readout_ready = false;
+        }
+        if (!cs.readout_ready && cs.precision != ELHL_PREC_DF64)
+            if (int rc = cheb_prepare_readout(cs, tr->fac.L, traj_inverse(tr))) return rc;
+        changed |= cs.version != b->versions[i];
+    }
+    if (!changed) return ELHL_OK;
+    if (int rc = cheb_plan(b->plan, b->states)) return rc;
+    for (size_t i = 0; i < b->members.size(); ++i) b->versions[i] = b->states[i]->version;
+    return ELHL_OK;
+}
 
 extern "C" {
 
@@ -3736,8 +3773,10 @@ int elhl_batch_create(int ntraj, const elhl_basis_desc *bases, const double *con
         elhl_traj *tr = nullptr;
         rc = elhl_traj_create(&bases[i], coords[i], cfg, &tr);
         if (!rc) {
+            tr->shared = true;
             b->members.push_back(tr);
             b->states.push_back(&tr->cs);
+            b->versions.push_back(tr->cs.version);
             if (tr->nfrag != b->members[0]->nfrag || tr->P != b->members[0]->P) rc = ELHL_ERR_BAD_ARG;
         }
     }
@@ -3786,6 +3825,7 @@ int elhl_batch_step(elhl_batch *b, int nsteps, double *pops) {
         b->pops_cap = per_step * nsteps;
     }
     memset(&b->stats, 0, sizeof(b->stats));
+    if (int rc = batch_follow(b)) return rc;
     if (!b->plan.mg_read) return ELHL_ERR_UNSUPPORTED;
     for (auto *tr : b->members)
         if (!tr->cs.cols_current)
@@ -3939,6 +3979,7 @@ static int server_admit(elhl_server *sv, ServerRequest *r) {
         return rc;
     std::lock_guard<std::mutex> lk(g_ctx.mu);
     elhl_traj *tr = r->tr;
+    tr->shared = true;
     if (tr->cs.gemm) {
         r->group = -1;  // many columns on a large basis: one GEMM per order, its own step graph
     } else {
