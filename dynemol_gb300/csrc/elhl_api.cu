@@ -3144,6 +3144,19 @@ int elhl_huckel_with_fields(const elhl_basis_desc *basis, const double *coords, 
     return rc;
 }
 
+// everything a trajectory holds (also one whose creation failed half way); the lock is held
+static void release_traj(elhl_traj *tr) {
+    cudaStreamSynchronize(g_ctx.stream);
+    free_basis(tr->basis);
+    dev_free(tr->S); dev_free(tr->h); dev_free(tr->Hp); dev_free(tr->coords); dev_free(tr->pops);
+    tr->fac.release();
+    tr->tb.release();
+    tr->cs.release();
+    tr->plan.release();
+    dev_free(tr->psi_ao); dev_free(tr->bra_ao); dev_free(tr->target); dev_free(tr->coords2);
+    delete tr;
+}
+
 int elhl_traj_create(const elhl_basis_desc *basis, const double *coords, const elhl_traj_config *cfg,
                      elhl_traj **out) {
     if (!out || !coords) return ELHL_ERR_BAD_ARG;
@@ -3254,11 +3267,7 @@ int elhl_traj_create(const elhl_basis_desc *basis, const double *coords, const e
         if (!rc) rc = cheb_plan(tr->plan, one);
     }
     if (rc) {
-        free_basis(tr->basis);
-        dev_free(tr->S); dev_free(tr->h); dev_free(tr->Hp); dev_free(tr->coords);
-        tr->fac.release();
-        tr->tb.release();
-        delete tr;
+        release_traj(tr);
         return rc;
     }
     *out = tr;
@@ -3268,15 +3277,7 @@ int elhl_traj_create(const elhl_basis_desc *basis, const double *coords, const e
 int elhl_traj_destroy(elhl_traj *tr) {
     if (!tr) return ELHL_ERR_BAD_ARG;
     std::lock_guard<std::mutex> lk(g_ctx.mu);
-    cudaStreamSynchronize(g_ctx.stream);
-    free_basis(tr->basis);
-    dev_free(tr->S); dev_free(tr->h); dev_free(tr->Hp); dev_free(tr->coords); dev_free(tr->pops);
-    tr->fac.release();
-    tr->tb.release();
-    tr->cs.release();
-    tr->plan.release();
-    dev_free(tr->psi_ao); dev_free(tr->bra_ao); dev_free(tr->target); dev_free(tr->coords2);
-    delete tr;
+    release_traj(tr);
     return ELHL_OK;
 }
 
